@@ -424,6 +424,15 @@ bool run_launch(km_handle* h, int cls, F&& f) {
 #define KL(h, cls, expr) run_launch(h, cls, [&]() -> bool { return (expr); })
 #define KLV(h, cls, expr) run_launch(h, cls, [&]() -> bool { expr; return true; })
 
+// FP64 leaf Cholesky, d_K into d_Lf; false if a leaf is too large
+bool leaf_chol_f64(km_handle* h) {
+  int n = 0;
+  const bool ok = KL(h, KM_PROF_LEAF_CHOL,
+                     (n = launch_leaf_chol_f64(h->d_K, h->d_Lf, h->tree, h->d_info, h->stream)) > 0);
+  h->stats.kernel_launches += n - 1;
+  return ok;
+}
+
 int sync(km_handle* h, const char* where) {
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return cuda_fail(h, e, where);
@@ -1437,7 +1446,7 @@ static int general_factorize(km_handle* h) {
   int rc;
   timer_start(h);
   KM_CUDA(h, cudaMemsetAsync(h->d_info, 0, sizeof(int) * (t.nleaf + nb + 1), st));  // + grid-barrier word
-  if (!KL(h, KM_PROF_LEAF_CHOL, launch_leaf_chol<double>(h->d_K, h->d_Lf, t, h->d_info, st)))
+  if (!leaf_chol_f64(h))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the leaf Cholesky kernel");
   if (nb > 0) {
     // leaf triangular solves of every panel (invapply!, src/HODLR/src/utils.jl:54-65)
@@ -1751,7 +1760,7 @@ static int factorize_launches(km_handle* h) {
     }
     if (fwd) aux_fwd_leaf<ff>(h);
   } else if (!(h->mixed ? KL(h, KM_PROF_LEAF_CHOL, launch_leaf_chol<ff>(h->d_K, P<ff>(h->d_Lf), t, h->d_info, st))
-                        : KL(h, KM_PROF_LEAF_CHOL, launch_leaf_chol<double>(h->d_K, h->d_Lf, t, h->d_info, st)))) {
+                        : leaf_chol_f64(h))) {
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the leaf Cholesky kernel");
   }
   // A = L^{-1} Phi on every leaf, then Householder QR of each leaf panel

@@ -60,7 +60,8 @@ __global__ void k_chol_small(double* __restrict__ A, int n, int* __restrict__ in
 }
 
 // ---------------------------------------------------------------------------------------------
-// Batched leaf Cholesky: Lf_j = chol(K_j) (lower), blocked right-looking, one CTA per leaf.
+// Batched leaf Cholesky in float pairs: Lf_j = chol(K_j) (lower), blocked right-looking, one CTA
+// per leaf (the FP64 form is in km_chol.cu).
 // The current column panel (rows below the diagonal block) lives in shared memory.
 // info[j] = first failing column (1-based) of leaf j, 0 if positive definite.
 // ---------------------------------------------------------------------------------------------
@@ -1018,10 +1019,8 @@ template <typename T>
 bool launch_leaf_chol(const double* K, T* Lf, const Tree& t, int* info, cudaStream_t st) {
   const int64_t m = t.max_leaf;
   auto fits = [&](int nb) { return (size_t)(m + nb) * (nb + 1) * sizeof(T) <= 200 * 1024; };
-  // float pairs need twice the registers per value: use the 16-wide panel for them
-  if (sizeof(T) == sizeof(double) && std::is_same<T, double>::value && fits(32)) {
-    leaf_chol_launch<T, 32>(K, Lf, t, info, st);
-  } else if (fits(16)) {
+  // (float pairs need twice the registers per value: the widest panel is 16 columns)
+  if (fits(16)) {
     leaf_chol_launch<T, 16>(K, Lf, t, info, st);
   } else if (fits(8)) {
     leaf_chol_launch<T, 8>(K, Lf, t, info, st);
@@ -1332,7 +1331,6 @@ template void launch_node_finalize<double>(const double*, const double*, const d
 template void launch_node_finalize<ff>(const ff*, const ff*, const ff*, const ff*, int, int, const Tree&, ff*, ff*,
                                        ff*, ff*, ff*, ff*, cudaStream_t);
 
-template bool launch_leaf_chol<double>(const double*, double*, const Tree&, int*, cudaStream_t);
 template bool launch_leaf_chol<ff>(const double*, ff*, const Tree&, int*, cudaStream_t);
 template void launch_leaf_qr<double>(double*, int, const Tree&, double*, double*, cudaStream_t);
 template void launch_leaf_qr<ff>(ff*, int, const Tree&, ff*, ff*, cudaStream_t);

@@ -94,6 +94,9 @@ void launch_gather_points(const double* pts, const int64_t* idx, int r, double* 
 bool launch_chol_small(double* A, int n, int* info, cudaStream_t st);
 template <typename T>
 bool launch_leaf_chol(const double* K, T* Lf, const Tree& t, int* info, cudaStream_t st);
+// FP64 leaf Cholesky over all SMs (km_chol.cu): lower triangles of Lf only; info zero on entry.
+// Returns the number of kernels launched, 0 if a leaf is too large.
+int launch_leaf_chol_f64(const double* K, double* Lf, const Tree& t, int* info, cudaStream_t st);
 template <typename T>
 bool launch_leaf_tri(const T* Lf, const Tree& t, int op, T* Bptr, int64_t bmul, int64_t bld, int bld_is_m, T* Xptr,
                      int64_t xmul, int64_t xld, int xld_is_m, int ncols, cudaStream_t st);
