@@ -1,6 +1,6 @@
 // ACA assembly and the general (per-block basis) HODLR factorisation used for ACA blocks.
 //
-// ACA: one CTA per off-diagonal block runs the partially pivoted adaptive cross approximation of
+// ACA: one cluster of CTAs per off-diagonal block runs the partially pivoted adaptive cross approximation of
 // the reference (src/factorizations.jl:9-84) step for step: the start-row search, the pivot
 // rule of restrictedmaxabs (src/utils.jl:2-15: first strict maximum of |x| outside the used set,
 // the first unused index when nothing is non-zero), residual updates as a multiply followed by a
@@ -13,12 +13,16 @@
 // node's V (rows c1) and U (rows c2) panels with explicit Q, C = R1 R2', L22 = chol(I - C'C),
 // and the application of W_N^{-1} to the coarser panels.  In the QR bases W_N^{-1} only changes
 // the c2 rows:  y_c2 -= Q2 (z2 - L22^{-1}(z2 - C' z1)),  z1 = Q1' y_c1, z2 = Q2' y_c2.
-#include <climits>
+#include <cooperative_groups.h>
 
+#include <atomic>
+#include <climits>
 
 #include "km_kernels.h"
 
 namespace km {
+
+namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------------------------
 // CTA-wide reductions (deterministic order)
@@ -39,237 +43,444 @@ __device__ double cta_sum(double v, double* sred) {
   return t;
 }
 
-// restrictedmaxabs over x[0..n) with excluded flags: returns (value, index).
-__device__ void cta_restricted_argmax(const double* x, const uint8_t* excl, int64_t n, double* sval,
-                                     long long* sidx, double* out_val, int64_t* out_idx) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double best = 0.0;
-  long long bi = LLONG_MAX, first = LLONG_MAX;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    if (excl[i]) continue;
-    if (first == LLONG_MAX) first = i;
-    const double a = fabs(x[i]);
-    if (a > best) {
-      best = a;
-      bi = i;
-    }
-  }
-  // reduce: larger |x| wins, ties go to the smaller index; first = min over threads
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    const long long of = __shfl_xor_sync(0xffffffffu, first, o);
-    if (ob > best || (ob == best && oi < bi)) {
-      best = ob;
-      bi = oi;
-    }
-    first = min(first, of);
-  }
-  if (lane == 0) {
-    sval[w] = best;
-    sidx[w] = bi;
-    sidx[32 + w] = first;
-  }
+// ---------------------------------------------------------------------------------------------
+// Grid barrier of a cooperative launch.  It spins a bounded number of times; one that runs out sets
+// an error word that every CTA sees at its next barrier, so the launch ends early as a whole.
+// ---------------------------------------------------------------------------------------------
+constexpr long long kGridSpinLimit = 1ll << 20;  // L2 polls per barrier wait (~0.3 s)
+
+struct GridBar {
+  unsigned* count;
+  volatile unsigned* gen;
+  volatile int* err;
+  long long limit;  // polls before a wait gives up (< 0: kGridSpinLimit; 0: at the first poll, as
+                    // if the other CTAs never arrived: the test of the timeout path)
+};
+
+// Returns true when every CTA has arrived and no barrier of this launch has run out; the answer
+// is the same for all threads of the CTA (thread 0's view, passed through shared memory), so the
+// CTA leaves its loop as a whole.
+__device__ bool grid_barrier(GridBar gb) {
+  __shared__ int s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double b = 0.0;
-    long long ib = LLONG_MAX, f = LLONG_MAX;
-    for (int q = 0; q < nw; ++q) {
-      if (sval[q] > b || (sval[q] == b && sidx[q] < ib)) {
-        b = sval[q];
-        ib = sidx[q];
-      }
-      f = min(f, sidx[32 + q]);
-    }
-    if (b > 0.0) {
-      sval[32] = x[ib];
-      sidx[64] = ib;
+    const long long lim = gb.limit < 0 ? kGridSpinLimit : gb.limit;
+    const unsigned g = *gb.gen;
+    __threadfence();
+    if (atomicAdd(gb.count, 1u) == gridDim.x - 1) {
+      *gb.count = 0;
+      __threadfence();
+      atomicExch((unsigned*)gb.gen, g + 1);
     } else {
-      sval[32] = 0.0;
-      sidx[64] = (f == LLONG_MAX) ? n - 1 : f;
+      long long spins = 0;
+      while ((gb.limit == 0 || *gb.gen == g) && *gb.err == 0) {
+        if (++spins > lim) {
+          atomicExch((int*)gb.err, 1);
+          break;
+        }
+      }
     }
+    __threadfence();
+    s_ok = *gb.err == 0;
   }
   __syncthreads();
-  *out_val = sval[32];
-  *out_idx = sidx[64];
-  __syncthreads();
+  return s_ok != 0;
 }
 
 // ---------------------------------------------------------------------------------------------
-// ACA, one CTA (1024 threads) per block.  status: 0 ok, 1 "Incompatible maxrank or matrix
-// dimensions." (factorizations.jl:30), 2 rank capacity of the panel reached before convergence.
+// ACA of one block by a team of CTAs: a thread-block cluster (k_aca) or, for blocks of 8192 points
+// and more, every SM (k_aca_grid, a cooperative launch).  status: 0 ok, 1 "Incompatible maxrank or
+// matrix dimensions." (factorizations.jl:30), 2 rank capacity of the panel reached before
+// convergence, 3 a grid barrier ran out.
+//
+// Each CTA owns a slice of the rows and a slice of the columns.  A step takes three team barriers
+// (0.2 us in a cluster, about 1.5 us over the grid): the CTAs' candidates for the column pivot; those
+// for the next row pivot with the squared norms and the dots with the earlier columns; the shares
+// of the norm update.  Candidates are compared by |x| (as integers) with ties to the smaller
+// index, so every CTA takes the pivots of a scan over the whole row.
+//
+// A residual entry is a chain of one multiply and one subtract per earlier column, in the
+// reference's order, and a warp's FP64 instruction takes 65 cycles of its quarter of the SM however
+// few lanes are active: the chains bound the kernel.  One CTA per block ran a 512 x 512 block of
+// rank 496 (the README example: unsorted points, tolerance 1e-12) in 147 ms.  Split over 16 SMs a
+// slice holds 32 entries, and where a slice has at most 64 the multiplies, which do not wait for
+// one another, go to the quarters that the subtractions leave idle: 25.9 ms.  The 4096-point blocks
+// of a 2^14 matrix went from 191 to 25.8 ms, its 8192-point block (every SM in both forms; before
+// with seven barriers a step, searches by one thread and unbatched loads) from 74 to 29 ms.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) k_aca(const double* __restrict__ pts, KParams kp,
-                                              const AcaBlock* __restrict__ blocks, double* __restrict__ P,
-                                              uint8_t* __restrict__ F, int* __restrict__ piv, double rtol,
-                                              int* __restrict__ rank_out, int* __restrict__ status, int only) {
-  extern __shared__ double dsm[];  // 2 * cap: dots with previous columns
-  __shared__ double sred[40];
-  __shared__ double sval[40];
-  __shared__ long long sidx[72];
-  const int bid = only >= 0 ? only : (int)blockIdx.x;
-  const AcaBlock B = blocks[bid];
-  if (only < 0 && B.grid) return;  // compressed by k_aca_grid
+namespace {
+
+constexpr int kAcaThreads = 256;
+constexpr int kAcaChunk = 32;   // earlier columns per stage of the split residual
+constexpr int kAcaSplit = 64;   // widest slice whose multiplies and subtractions go to different warps
+
+struct AcaRec {                 // one CTA's part of a search and of the sums
+  unsigned long long key;       // bits of the largest |x| outside the used set (0: none is non-zero)
+  long long idx, first;         // its index; the first unused index
+  double val;                   // x[idx]
+  double z;                     // share of the norm update
+};
+
+struct AcaShared {
+  AcaRec rec[3];                // column search, row search, norm update: the barriers of a step apart
+  AcaRec win;                   // combined search of this step (same in every CTA)
+  AcaRec part[kAcaThreads / 32];
+  double sums[2];               // squared norms of the new row and column
+  double zpart[kAcaThreads / 32];
+  int stop;
+};
+
+__device__ __forceinline__ bool aca_better(unsigned long long k, long long i, const AcaRec& r) {
+  return k > r.key || (k == r.key && i < r.idx);
+}
+
+__device__ __forceinline__ void aca_warp_best(AcaRec& r) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long k = __shfl_xor_sync(0xffffffffu, r.key, o);
+    const long long i = __shfl_xor_sync(0xffffffffu, r.idx, o), f = __shfl_xor_sync(0xffffffffu, r.first, o);
+    const double v = __shfl_xor_sync(0xffffffffu, r.val, o);
+    if (aca_better(k, i, r)) {
+      r.key = k;
+      r.idx = i;
+      r.val = v;
+    }
+    r.first = min(r.first, f);
+  }
+}
+
+// Entry x of index i offered to a thread's candidate; a NaN is never the largest.
+__device__ __forceinline__ void aca_offer(AcaRec& r, double x, long long i, bool used) {
+  if (used) return;
+  if (r.first == LLONG_MAX) r.first = i;
+  const unsigned long long k = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+  if (k <= 0x7ff0000000000000ull && k > r.key) {
+    r.key = k;
+    r.idx = i;
+    r.val = x;
+  }
+}
+
+// The CTAs of a cluster exchange records and partial dots through distributed shared memory.
+struct ClusterTeam {
+  static constexpr int kLanes = 4;  // lanes that sum one column's partial dots over the CTAs
+  AcaShared* S;
+  double* d;                        // 2 x (cap + 1): partial dots of U_j . col, then of V_j . row
+  int cap1;
+  __device__ int size() const { return (int)cg::this_cluster().num_blocks(); }
+  __device__ int rank() const { return (int)cg::this_cluster().block_rank(); }
+  __device__ bool barrier() const {
+    cg::this_cluster().sync();
+    return true;
+  }
+  __device__ AcaRec* mine(int s) const { return S->rec + s; }
+  __device__ double* dots(int side) const { return d + side * cap1; }
+  __device__ AcaRec get(int s, int q) const { return cg::this_cluster().map_shared_rank(S, q)->rec[s]; }
+  __device__ double get_z(int q) const { return cg::this_cluster().map_shared_rank(S, q)->rec[2].z; }
+  __device__ double dot(int side, int q, int j) const {
+    return *cg::this_cluster().map_shared_rank(d + side * cap1 + j, q);
+  }
+};
+
+// The CTAs of a cooperative launch exchange them through L2.
+struct GridTeam {
+  static constexpr int kLanes = 32;
+  GridBar gb;
+  AcaRec* recs;   // 3 x CTAs
+  double* d;      // CTAs x 2 x (cap + 1)
+  int cap1;
+  __device__ int size() const { return (int)gridDim.x; }
+  __device__ int rank() const { return (int)blockIdx.x; }
+  __device__ bool barrier() const { return grid_barrier(gb); }
+  __device__ AcaRec* mine(int s) const { return recs + s * gridDim.x + blockIdx.x; }
+  __device__ double* dots(int side) const { return d + (2 * (int64_t)blockIdx.x + side) * cap1; }
+  __device__ AcaRec get(int s, int q) const {
+    const AcaRec* r = recs + s * gridDim.x + q;
+    return AcaRec{__ldcg(&r->key), __ldcg(&r->idx), __ldcg(&r->first), __ldcg(&r->val), 0.0};
+  }
+  __device__ double get_z(int q) const { return __ldcg(&recs[2 * gridDim.x + q].z); }
+  __device__ double dot(int side, int q, int j) const { return __ldcg(d + (2 * (int64_t)q + side) * cap1 + j); }
+};
+
+// The team's winner of record slot s, the same in every CTA; ends with a CTA barrier.
+template <typename Team>
+__device__ void aca_combine(const Team& team, AcaShared& S, int s, int64_t n) {
+  if (threadIdx.x < 32) {
+    AcaRec r{0, LLONG_MAX, LLONG_MAX, 0.0, 0.0};
+    for (int q = threadIdx.x; q < team.size(); q += 32) {
+      const AcaRec o = team.get(s, q);
+      if (aca_better(o.key, o.idx, r)) {
+        r.key = o.key;
+        r.idx = o.idx;
+        r.val = o.val;
+      }
+      r.first = min(r.first, o.first);
+    }
+    aca_warp_best(r);
+    if (threadIdx.x == 0) {
+      if (r.key == 0) {  // nothing non-zero is left: the first unused index
+        r.val = 0.0;
+        r.idx = r.first == LLONG_MAX ? n - 1 : r.first;
+      }
+      S.win = r;
+    }
+  }
+  __syncthreads();
+}
+
+// This CTA's candidate into its record of slot s (a team barrier follows).
+__device__ void aca_publish(AcaShared& S, AcaRec* out, AcaRec r) {
+  aca_warp_best(r);
+  if ((threadIdx.x & 31) == 0) S.part[threadIdx.x >> 5] = r;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    r = S.part[0];
+    for (int q = 1; q < kAcaThreads / 32; ++q) {
+      if (aca_better(S.part[q].key, S.part[q].idx, r)) {
+        r.key = S.part[q].key;
+        r.idx = S.part[q].idx;
+        r.val = S.part[q].val;
+      }
+      r.first = min(r.first, S.part[q].first);
+    }
+    out->key = r.key;
+    out->idx = r.idx;
+    out->first = r.first;
+    out->val = r.val;
+  }
+}
+
+// Residual entries e in [lo, hi) of a row or column: out[e] = k(e) - sum_j coef[j] M[e, j], one
+// multiply and one subtract per j in order; returns the thread's candidate among those not in
+// `used`.  role: this warp's number, rotated between the clusters so that the subtraction warps
+// of co-resident CTAs fall on different quarters of the SM.
+template <typename Eval>
+__device__ AcaRec aca_residual(Eval&& eval, const double* M, int64_t ld, int64_t lo, int64_t hi, double* out,
+                               const uint8_t* used, const double* coef, int nj, double* prod, int role) {
+  AcaRec r{0, LLONG_MAX, LLONG_MAX, 0.0, 0.0};
+  const int lane = threadIdx.x & 31;
+  if (hi - lo > kAcaSplit) {
+    for (int64_t e = lo + role * 32 + lane; e < hi; e += kAcaThreads) {
+      double v = eval(e);
+      int j = 0;
+      for (; j + 8 <= nj; j += 8) {
+        double m[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) m[q] = M[e + (int64_t)(j + q) * ld];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v = __dsub_rn(v, __dmul_rn(coef[j + q], m[q]));
+      }
+      for (; j < nj; ++j) v = __dsub_rn(v, __dmul_rn(coef[j], M[e + (int64_t)j * ld]));
+      out[e] = v;
+      aca_offer(r, v, e, used[e]);
+    }
+    return r;
+  }
+  const int nc = hi - lo > 32 ? 2 : 1;             // subtraction warps: roles 0 .. nc-1
+  const int np = (kAcaThreads / 128) * (4 - nc);   // multiply warps: roles with role % 4 >= nc
+  const int64_t e = lo + role * 32 + lane;
+  const bool mine = role < nc && e < hi;
+  double v = mine ? eval(e) : 0.0;
+  const int nchunk = (nj + kAcaChunk - 1) / kAcaChunk;
+  for (int t = 0; t <= nchunk; ++t) {
+    if ((role & 3) >= nc) {
+      if (t < nchunk) {
+        double* buf = prod + (t & 1) * kAcaChunk * kAcaSplit;
+        const int jn = min(kAcaChunk, nj - t * kAcaChunk);
+        const int pw = (role >> 2) * (4 - nc) + (role & 3) - nc;
+#pragma unroll 4
+        for (int it = pw; it < jn * nc; it += np) {
+          const int jj = it / nc, h = it - jj * nc;
+          const int64_t ee = lo + h * 32 + lane;
+          const int j = t * kAcaChunk + jj;
+          if (ee < hi) buf[jj * kAcaSplit + h * 32 + lane] = __dmul_rn(coef[j], M[ee + (int64_t)j * ld]);
+        }
+      }
+    } else if (mine && t > 0) {
+      const double* buf = prod + ((t - 1) & 1) * kAcaChunk * kAcaSplit + role * 32 + lane;
+      const int jn = min(kAcaChunk, nj - (t - 1) * kAcaChunk);
+#pragma unroll 8
+      for (int jj = 0; jj < jn; ++jj) v = __dsub_rn(v, buf[jj * kAcaSplit]);
+    }
+    __syncthreads();
+  }
+  if (mine) {
+    out[e] = v;
+    aca_offer(r, v, e, used[e]);
+  }
+  return r;
+}
+
+// The whole approximation; false if a barrier ran out (every CTA of the team then leaves).
+template <typename Team>
+__device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, const double* __restrict__ pts,
+                        const KParams& kp, const AcaBlock& B, double* P, uint8_t* F, int* __restrict__ piv,
+                        double rtol, int* __restrict__ rank_out, int* __restrict__ status) {
+  const int G = team.size(), g = team.rank();
   const int64_t nro = B.nro, ncl = B.ncl;
+  const int cap = B.cap;
+  double* coef = dsm;              // cap: U[ri, j] or V[cj, j] of the earlier columns
+  double* prod = coef + cap;       // 2 x kAcaChunk x kAcaSplit
+  double* da = team.dots(0);       // cap + 1: this CTA's part of U_j . col; entry frnk: |col|^2
+  double* db = team.dots(1);       // cap + 1: V_j . row; |row|^2
   double* U = P + B.offU;
   double* V = P + B.offV;
-  uint8_t* urow = F + B.offFlag;
+  uint8_t* urow = F + B.offFlag;   // a CTA reads and sets the flags of its own slices only
   uint8_t* ucol = urow + nro;
   int* prow = piv + 2 * B.offPiv;
-  int* pcol = prow + B.cap;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
+  int* pcol = prow + cap;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  constexpr int nw = kAcaThreads / 32;
+  const int role = (w + turn) & (nw - 1);
+  const int64_t rs = (nro + G - 1) / G, cs = (ncl + G - 1) / G;
+  const int64_t r_lo = min(nro, g * rs), r_hi = min(nro, r_lo + rs);
+  const int64_t c_lo = min(ncl, g * cs), c_hi = min(ncl, c_lo + cs);
   const double* xr = pts + 2 * B.row0;
   const double* xc = pts + 2 * B.col0;
-  for (int64_t i = tid; i < nro; i += blockDim.x) urow[i] = 0;
-  for (int64_t i = tid; i < ncl; i += blockDim.x) ucol[i] = 0;
-  const int maxsz = B.maxsz;
-  auto eval_row = [&](int64_t i, double* out) {
-    const double px = xr[2 * i], py = xr[2 * i + 1];
-    for (int64_t c = tid; c < ncl; c += blockDim.x) out[c] = kernel_value(kp, px, py, xc[2 * c], xc[2 * c + 1]);
-  };
-  auto eval_col = [&](int64_t j, double* out) {
-    const double px = xc[2 * j], py = xc[2 * j + 1];
-    for (int64_t i = tid; i < nro; i += blockDim.x) out[i] = kernel_value(kp, xr[2 * i], xr[2 * i + 1], px, py);
-  };
-  auto sumsq = [&](const double* x, int64_t n) {
-    double a = 0.0;
-    for (int64_t i = tid; i < n; i += blockDim.x) a += x[i] * x[i];
-    return cta_sum(a, sred);
-  };
-  // first row (factorizations.jl:24-30)
-  int64_t strt = 0;
-  eval_row(strt, V);
+  for (int64_t i = r_lo + tid; i < r_hi; i += kAcaThreads) urow[i] = 0;
+  for (int64_t c = c_lo + tid; c < c_hi; c += kAcaThreads) ucol[c] = 0;
   __syncthreads();
-  {
-    double mx = 0.0;
-    for (int64_t c = tid; c < ncl; c += blockDim.x) mx = fmax(mx, fabs(V[c]));
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) sred[w] = mx;
-    __syncthreads();
-    if (tid == 0) {
-      double m = 0.0;
-      for (int q = 0; q < nw; ++q) m = fmax(m, sred[q]);
-      sred[34] = m;
-    }
-    __syncthreads();
-    mx = sred[34];
-    __syncthreads();
-    while (mx == 0.0 && strt + 1 < maxsz) {
-      ++strt;
-      eval_row(strt, V);
+  const int maxsz = B.maxsz;
+  auto row_of = [&](int64_t i) {
+    const double px = xr[2 * i], py = xr[2 * i + 1];
+    return [=](int64_t c) { return kernel_value(kp, px, py, xc[2 * c], xc[2 * c + 1]); };
+  };
+  auto col_of = [&](int64_t j) {
+    const double px = xc[2 * j], py = xc[2 * j + 1];
+    return [=](int64_t i) { return kernel_value(kp, xr[2 * i], xr[2 * i + 1], px, py); };
+  };
+  int st = 0, frnk = 0;
+  double znorm2 = 0.0;
+  // first row not all zero (factorizations.jl:24-30)
+  int64_t ri = 0;
+  for (;;) {
+    aca_publish(S, team.mine(0), aca_residual(row_of(ri), V, ncl, c_lo, c_hi, V, ucol, coef, 0, prod, role));
+    if (!team.barrier()) return false;
+    aca_combine(team, S, 0, ncl);
+    if (S.win.key != 0 || ri + 1 >= maxsz) break;
+    ++ri;
+    if (!team.barrier()) return false;  // the records have been read
+  }
+  if (ri + 1 == maxsz) {
+    st = 1;
+  } else {
+    for (;;) {
+      // S.win: the column pivot; row `frnk` of V holds the unscaled residual row of row pivot ri
+      const double cv = S.win.val;
+      const int64_t cj = S.win.idx;
+      if (frnk > 0 && cv == 0.0) break;
+      double* row = V + (int64_t)frnk * ncl;
+      double* col = U + (int64_t)frnk * nro;
+      if (tid == 0) {
+        if (ri >= r_lo && ri < r_hi) urow[ri] = 1;
+        if (cj >= c_lo && cj < c_hi) ucol[cj] = 1;
+        if (g == 0) {
+          prow[frnk] = (int)ri;
+          pcol[frnk] = (int)cj;
+        }
+      }
+      for (int j = tid; j < frnk; j += kAcaThreads) coef[j] = __ldcg(V + cj + (int64_t)j * ncl);
+      for (int64_t c = c_lo + tid; c < c_hi; c += kAcaThreads) row[c] = __ddiv_rn(row[c], cv);
       __syncthreads();
-      double m2 = 0.0;
-      for (int64_t c = tid; c < ncl; c += blockDim.x) m2 = fmax(m2, fabs(V[c]));
-      for (int o = 16; o > 0; o >>= 1) m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-      if (lane == 0) sred[w] = m2;
+      const AcaRec rr = aca_residual(col_of(cj), U, nro, r_lo, r_hi, col, urow, coef, frnk, prod, role);
+      __syncthreads();
+      // this CTA's parts of the dots with the earlier columns and (entry frnk) of the squared
+      // norms: 4 lanes per column, so that a warp reduces 8 columns by two shuffle steps
+      for (int j0 = 0; j0 <= frnk; j0 += kAcaThreads / 4) {
+        const int j = j0 + (tid >> 2), p = tid & 3;
+        double a = 0.0, b = 0.0;
+        if (j <= frnk) {
+          const double* uj = U + (int64_t)j * nro;
+          const double* vj = V + (int64_t)j * ncl;
+#pragma unroll 4
+          for (int64_t i = r_lo + p; i < r_hi; i += 4) a += uj[i] * col[i];
+#pragma unroll 4
+          for (int64_t c = c_lo + p; c < c_hi; c += 4) b += vj[c] * row[c];
+        }
+        if (j0 + (w << 3) <= frnk) {
+          a += __shfl_xor_sync(0xffffffffu, a, 1);
+          b += __shfl_xor_sync(0xffffffffu, b, 1);
+          a += __shfl_xor_sync(0xffffffffu, a, 2);
+          b += __shfl_xor_sync(0xffffffffu, b, 2);
+          if (p == 0 && j <= frnk) {
+            da[j] = a;
+            db[j] = b;
+          }
+        }
+      }
+      aca_publish(S, team.mine(1), rr);
+      if (!team.barrier()) return false;
+      aca_combine(team, S, 1, nro);
+      ri = S.win.idx;
+      // sums over the CTAs: CTA g takes the columns j = g, g + G, ...; every CTA the norms
+      {
+        constexpr int kL = Team::kLanes, kPer = 32 / kL;  // columns per warp
+        const int p = lane % kL, nmine = g < frnk ? (frnk - g + G - 1) / G : 0;
+        double z = 0.0;
+        for (int t0 = w * kPer; t0 <= nmine; t0 += nw * kPer) {
+          const int t = t0 + lane / kL, j = t < nmine ? g + t * G : frnk;
+          double a = 0.0, b = 0.0;
+          if (t <= nmine)
+            for (int q = p; q < G; q += kL) {
+              a += team.dot(0, q, j);
+              b += team.dot(1, q, j);
+            }
+#pragma unroll
+          for (int o = 1; o < kL; o <<= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+          }
+          if (t < nmine && p == 0) z += __dmul_rn(__dmul_rn(2.0, fabs(a)), fabs(b));
+          if (t == nmine && p == 0) {
+            S.sums[0] = b;
+            S.sums[1] = a;
+          }
+        }
+        if (w * kPer <= nmine) {  // (warps without a column hold zero)
+#pragma unroll
+          for (int o = kL; o < 32; o <<= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+        }
+        if (lane == 0) S.zpart[w] = z;
+      }
       __syncthreads();
       if (tid == 0) {
-        double m = 0.0;
-        for (int q = 0; q < nw; ++q) m = fmax(m, sred[q]);
-        sred[34] = m;
+        double z = S.zpart[0];
+        const int used_w = min(nw, (g < frnk ? (frnk - g + G - 1) / G : 0) * Team::kLanes / 32 + 1);
+        for (int q = 1; q < used_w; ++q) z += S.zpart[q];
+        team.mine(2)->z = z;
+      }
+      if (!team.barrier()) return false;
+      if (w == 0) {
+        double z = 0.0;
+        for (int q = lane; q < G; q += 32) z += team.get_z(q);
+        z = warp_sum(z);
+        const double sr = S.sums[0], sc = S.sums[1];
+        znorm2 = __dadd_rn(__dadd_rn(znorm2, z), __dmul_rn(sr, sc));
+        const bool go = __dmul_rn(sqrt(sr), sqrt(sc)) > __dmul_rn(rtol, sqrt(znorm2)) && frnk + 1 < maxsz;
+        if (lane == 0) S.stop = !go;
       }
       __syncthreads();
-      mx = sred[34];
+      ++frnk;
+      if (S.stop) break;
+      if (frnk >= cap) {
+        st = 2;
+        break;
+      }
+      // residual row of the next row pivot, and its largest entry outside the used columns
+      for (int j = tid; j < frnk; j += kAcaThreads) coef[j] = __ldcg(U + ri + (int64_t)j * nro);
       __syncthreads();
+      if (tid == 0 && ri >= r_lo && ri < r_hi) urow[ri] = 1;
+      aca_publish(S, team.mine(0), aca_residual(row_of(ri), V, ncl, c_lo, c_hi, V + (int64_t)frnk * ncl, ucol, coef, frnk, prod,
+                                     role));
+      if (!team.barrier()) return false;
+      aca_combine(team, S, 0, ncl);
     }
   }
-  if (strt + 1 == maxsz) {
-    if (tid == 0) {
-      status[bid] = 1;
-      rank_out[bid] = 0;
-    }
-    return;
+  if (g == 0 && tid == 0) {
+    *rank_out = frnk;
+    *status = st;
   }
-  if (tid == 0) {
-    urow[strt] = 1;
-    prow[0] = (int)strt;
-  }
-  __syncthreads();
-  double mv;
-  int64_t mi;
-  cta_restricted_argmax(V, ucol, ncl, sval, sidx, &mv, &mi);
-  for (int64_t c = tid; c < ncl; c += blockDim.x) V[c] = __ddiv_rn(V[c], mv);
-  eval_col(mi, U);
-  __syncthreads();
-  double sr = sumsq(V, ncl), sc = sumsq(U, nro);
-  double znorm2 = __dmul_rn(sr, sc);
-  if (tid == 0) {
-    ucol[mi] = 1;
-    pcol[0] = (int)mi;
-  }
-  __syncthreads();
-  int frnk = 1;
-  int st = 0;
-  while (__dmul_rn(sqrt(sr), sqrt(sc)) > __dmul_rn(rtol, sqrt(znorm2)) && frnk < maxsz) {
-    const double* lastcol = U + (int64_t)(frnk - 1) * nro;
-    int64_t ri;
-    double rv;
-    cta_restricted_argmax(lastcol, urow, nro, sval, sidx, &rv, &ri);
-    if (tid == 0) urow[ri] = 1;
-    if (frnk >= B.cap) {
-      st = 2;
-      break;
-    }
-    double* row = V + (int64_t)frnk * ncl;
-    {
-      const double px = xr[2 * ri], py = xr[2 * ri + 1];
-      for (int64_t c = tid; c < ncl; c += blockDim.x) {
-        double v = kernel_value(kp, px, py, xc[2 * c], xc[2 * c + 1]);
-        for (int j = 0; j < frnk; ++j) v = __dsub_rn(v, __dmul_rn(U[ri + (int64_t)j * nro], V[c + (int64_t)j * ncl]));
-        row[c] = v;
-      }
-    }
-    __syncthreads();
-    double cv;
-    int64_t cj;
-    cta_restricted_argmax(row, ucol, ncl, sval, sidx, &cv, &cj);
-    if (cv == 0.0) break;
-    if (tid == 0) ucol[cj] = 1;
-    for (int64_t c = tid; c < ncl; c += blockDim.x) row[c] = __ddiv_rn(row[c], cv);
-    double* col = U + (int64_t)frnk * nro;
-    {
-      const double px = xc[2 * cj], py = xc[2 * cj + 1];
-      for (int64_t i = tid; i < nro; i += blockDim.x) {
-        double v = kernel_value(kp, xr[2 * i], xr[2 * i + 1], px, py);
-        for (int j = 0; j < frnk; ++j) v = __dsub_rn(v, __dmul_rn(V[cj + (int64_t)j * ncl], U[i + (int64_t)j * nro]));
-        col[i] = v;
-      }
-    }
-    __syncthreads();
-    // dots with the previous columns, one warp per j
-    for (int j = w; j < frnk; j += nw) {
-      const double* uj = U + (int64_t)j * nro;
-      const double* vj = V + (int64_t)j * ncl;
-      double a = 0.0, b = 0.0;
-      for (int64_t i = lane; i < nro; i += 32) a += uj[i] * col[i];
-      for (int64_t c = lane; c < ncl; c += 32) b += vj[c] * row[c];
-      a = warp_sum(a);
-      b = warp_sum(b);
-      if (lane == 0) {
-        dsm[j] = a;
-        dsm[B.cap + j] = b;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double z = znorm2;
-      for (int j = 0; j < frnk; ++j) z = __dadd_rn(z, __dmul_rn(__dmul_rn(2.0, fabs(dsm[j])), fabs(dsm[B.cap + j])));
-      sred[36] = z;
-      prow[frnk] = (int)ri;
-      pcol[frnk] = (int)cj;
-    }
-    __syncthreads();
-    znorm2 = sred[36];
-    __syncthreads();
-    sr = sumsq(row, ncl);
-    sc = sumsq(col, nro);
-    znorm2 = __dadd_rn(znorm2, __dmul_rn(sr, sc));
-    ++frnk;
-  }
-  if (tid == 0) {
-    rank_out[bid] = frnk;
-    status[bid] = st;
-  }
+  return team.barrier();  // no CTA leaves while another may still read its shared memory
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -808,370 +1019,43 @@ __global__ void k_glogdet(const GNodeDesc* __restrict__ nodes, int nn, double* _
   partial[q] = s;
 }
 
-// ---------------------------------------------------------------------------------------------
-// ACA of one large block by every SM (cooperative launch, one CTA per SM).  The steps are those
-// of k_aca (factorizations.jl:9-84): each CTA owns a slice of the rows and a slice of the
-// columns, evaluates its part of the residual row / column, and the argmax searches and the
-// norms are reduced over the CTAs' partial results in a fixed order, so every CTA takes the
-// same pivots.  Values written by other CTAs (records, pivots' entries, the published norms) are
-// read with ld.global.cg (L2, the coherence point); a CTA sets the used-row/column flags of its
-// own slices only.  Grid barriers spin a bounded number of times; a barrier that runs out sets the
-// block's status to 3 (timeout) and the CTAs leave the loop together at the next check.
-// ---------------------------------------------------------------------------------------------
-constexpr long long kGridSpinLimit = 1ll << 20;  // L2 polls per barrier wait (~0.3 s)
+}  // namespace
 
-struct GridBar {
-  unsigned* count;
-  volatile unsigned* gen;
-  volatile int* err;
-  long long limit;  // polls before a wait gives up (< 0: kGridSpinLimit; 0: at the first poll, as
-                    // if the other CTAs never arrived: the test of the timeout path)
-};
-
-// Returns true when every CTA has arrived and no barrier of this launch has run out; the answer
-// is the same for all threads of the CTA (thread 0's view, passed through shared memory), so the
-// CTA leaves its loop as a whole.
-__device__ bool grid_barrier(GridBar gb) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const long long lim = gb.limit < 0 ? kGridSpinLimit : gb.limit;
-    const unsigned g = *gb.gen;
-    __threadfence();
-    if (atomicAdd(gb.count, 1u) == gridDim.x - 1) {
-      *gb.count = 0;
-      __threadfence();
-      atomicExch((unsigned*)gb.gen, g + 1);
-    } else {
-      long long spins = 0;
-      while ((gb.limit == 0 || *gb.gen == g) && *gb.err == 0) {
-        if (++spins > lim) {
-          atomicExch((int*)gb.err, 1);
-          break;
-        }
-      }
-    }
-    __threadfence();
-    s_ok = *gb.err == 0;
-  }
-  __syncthreads();
-  return s_ok != 0;
+__global__ void __launch_bounds__(kAcaThreads) k_aca(const double* __restrict__ pts, KParams kp,
+                                                     const AcaBlock* __restrict__ blocks, int nblocks, int last_first,
+                                                     double* P, uint8_t* F, int* __restrict__ piv, double rtol,
+                                                     int* __restrict__ rank_out, int* __restrict__ status, int only) {
+  extern __shared__ double dsm[];
+  __shared__ AcaShared S;
+  const int cid = (int)(blockIdx.x / cg::this_cluster().num_blocks());
+  const int bid = only >= 0 ? only : (last_first ? nblocks - 1 - cid : cid);
+  const AcaBlock B = blocks[bid];
+  if (only < 0 && B.grid) return;  // compressed by k_aca_grid (the whole cluster leaves)
+  const ClusterTeam team{&S, dsm + B.cap + 2 * kAcaChunk * kAcaSplit, B.cap + 1};
+  aca_run(team, S, dsm, cid, pts, kp, B, P, F, piv, rtol, rank_out + bid, status + bid);
 }
 
-// partial argmax record of one CTA: (|x| best, its index, first unflagged index)
-__device__ void slice_argmax(const double* x, const uint8_t* excl, int64_t lo, int64_t hi, double* sval,
-                             long long* sidx, double* pval, long long* pidx) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double best = 0.0;
-  long long bi = LLONG_MAX, first = LLONG_MAX;
-  for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-    if (excl[i]) continue;
-    if (first == LLONG_MAX) first = i;
-    const double a = fabs(x[i]);
-    if (a > best) {
-      best = a;
-      bi = i;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    const long long of = __shfl_xor_sync(0xffffffffu, first, o);
-    if (ob > best || (ob == best && oi < bi)) {
-      best = ob;
-      bi = oi;
-    }
-    first = min(first, of);
-  }
-  if (lane == 0) {
-    sval[w] = best;
-    sidx[w] = bi;
-    sidx[32 + w] = first;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = 0.0;
-    long long ib = LLONG_MAX, f = LLONG_MAX;
-    for (int q = 0; q < nw; ++q) {
-      if (sval[q] > b || (sval[q] == b && sidx[q] < ib)) {
-        b = sval[q];
-        ib = sidx[q];
-      }
-      f = min(f, sidx[32 + q]);
-    }
-    *pval = b;
-    pidx[0] = ib;
-    pidx[1] = f;
-  }
-  __syncthreads();
-}
-
-// combine the CTAs' argmax records (same order in every CTA): restrictedmaxabs semantics.
-// CTA g's record: value at pval[g * stride], indices at pidx[2 g] (best) and pidx[2 g + 1] (first).
-__device__ void grid_argmax(const double* x, int64_t n, const double* pval, const long long* pidx, int stride,
-                            double* sh, long long* shi, double* out_val, int64_t* out_idx) {
-  if (threadIdx.x == 0) {
-    double b = 0.0;
-    long long ib = LLONG_MAX, f = LLONG_MAX;
-    for (int g = 0; g < (int)gridDim.x; ++g) {
-      const double v = __ldcg(pval + (int64_t)g * stride);
-      const long long i = __ldcg(pidx + 2 * g), fi = __ldcg(pidx + 2 * g + 1);
-      if (v > b || (v == b && i < ib)) {
-        b = v;
-        ib = i;
-      }
-      f = min(f, fi);
-    }
-    if (b > 0.0) {
-      sh[0] = __ldcg(x + ib);
-      shi[0] = ib;
-    } else {
-      sh[0] = 0.0;
-      shi[0] = (f == LLONG_MAX) ? n - 1 : f;
-    }
-  }
-  __syncthreads();
-  *out_val = sh[0];
-  *out_idx = shi[0];
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(512) k_aca_grid(const double* __restrict__ pts, KParams kp,
-                                                  const AcaBlock* __restrict__ blocks, int bidx,
-                                                  double* __restrict__ P, uint8_t* __restrict__ F,
-                                                  int* __restrict__ piv, double rtol, int* __restrict__ rank_out,
-                                                  int* __restrict__ status, double* __restrict__ scr,
-                                                  GridBar gb) {
-  extern __shared__ double coef[];  // cap: U[ri, j] or V[cj, j] of the previous columns
-  __shared__ double sred[40];
-  __shared__ double sval[40];
-  __shared__ long long sidx[72];
-  __shared__ double sh[4];
-  __shared__ long long shi[2];
+__global__ void __launch_bounds__(kAcaThreads) k_aca_grid(const double* __restrict__ pts, KParams kp,
+                                                          const AcaBlock* __restrict__ blocks, int bidx, double* P,
+                                                          uint8_t* F, int* __restrict__ piv, double rtol,
+                                                          int* __restrict__ rank_out, int* __restrict__ status,
+                                                          double* scr, GridBar gb) {
+  extern __shared__ double dsm[];
+  __shared__ AcaShared S;
   const AcaBlock B = blocks[bidx];
-  const int64_t nro = B.nro, ncl = B.ncl;
-  const int cap = B.cap;
-  double* U = P + B.offU;
-  double* V = P + B.offV;
-  uint8_t* urow = F + B.offFlag;
-  uint8_t* ucol = urow + nro;
-  int* prow = piv + 2 * B.offPiv;
-  int* pcol = prow + cap;
-  const int G = gridDim.x, g = blockIdx.x;
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-  const int64_t rs = (nro + G - 1) / G, cs = (ncl + G - 1) / G;
-  auto mn = [](int64_t a, int64_t b) { return a < b ? a : b; };
-  const int64_t r_lo = mn(nro, (int64_t)g * rs), r_hi = mn(nro, r_lo + rs);
-  const int64_t c_lo = mn(ncl, (int64_t)g * cs), c_hi = mn(ncl, c_lo + cs);
-  const double* xr = pts + 2 * B.row0;
-  const double* xc = pts + 2 * B.col0;
-  // scratch: per CTA a record of stride S doubles: [0] argmax value, [1] sum 1, [2] sum 2,
-  // [3 .. 3+cap) dots a_j, [3+cap .. 3+2cap) dots b_j; then 2 long longs per CTA; then scalars
-  const int S = 3 + 2 * cap;
-  double* rec = scr + (int64_t)g * S;
-  long long* irec = reinterpret_cast<long long*>(scr + (int64_t)G * S);
-  double* scal = scr + (int64_t)G * S + 2 * G;  // [0] znorm2, [1] sr, [2] sc
-  for (int64_t i = r_lo + tid; i < r_hi; i += blockDim.x) urow[i] = 0;
-  for (int64_t c = c_lo + tid; c < c_hi; c += blockDim.x) ucol[c] = 0;
-  if (!grid_barrier(gb)) goto done;
-  {
-    const int maxsz = B.maxsz;
-    auto slice_max = [&](const double* x) {
-      double mx = 0.0;
-      for (int64_t c = c_lo + tid; c < c_hi; c += blockDim.x) mx = fmax(mx, fabs(x[c]));
-      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if (lane == 0) sred[w] = mx;
-      __syncthreads();
-      if (tid == 0) {
-        double m = 0.0;
-        for (int q = 0; q < nw; ++q) m = fmax(m, sred[q]);
-        rec[0] = m;
-      }
-      __syncthreads();
-    };
-    auto all_max = [&]() {
-      if (tid == 0) {
-        double m = 0.0;
-        for (int q = 0; q < G; ++q) m = fmax(m, __ldcg(scr + (int64_t)q * S));
-        sh[2] = m;
-      }
-      __syncthreads();
-      const double m = sh[2];
-      __syncthreads();
-      return m;
-    };
-    auto slice_sum = [&](const double* x, int64_t lo, int64_t hi) {
-      double a = 0.0;
-      for (int64_t i = lo + tid; i < hi; i += blockDim.x) a += x[i] * x[i];
-      return cta_sum(a, sred);
-    };
-    // first row not all zero (factorizations.jl:24-30)
-    int64_t strt = 0;
-    for (;;) {
-      const double px = xr[2 * strt], py = xr[2 * strt + 1];
-      for (int64_t c = c_lo + tid; c < c_hi; c += blockDim.x) V[c] = kernel_value(kp, px, py, xc[2 * c], xc[2 * c + 1]);
-      __syncthreads();
-      slice_max(V);
-      if (!grid_barrier(gb)) goto done;
-      const double m = all_max();
-      if (m != 0.0 || strt + 1 >= maxsz) break;
-      ++strt;
-      if (!grid_barrier(gb)) goto done;  // records are rewritten by the next row
-    }
-    if (strt + 1 == maxsz) {
-      if (g == 0 && tid == 0) {
-        status[bidx] = 1;
-        rank_out[bidx] = 0;
-      }
-      goto done;
-    }
-    if (tid == 0 && strt >= r_lo && strt < r_hi) urow[strt] = 1;  // flags are set by their slice's owner
-    if (g == 0 && tid == 0) prow[0] = (int)strt;
-    double mv;
-    int64_t mi;
-    slice_argmax(V, ucol, c_lo, c_hi, sval, sidx, rec, irec + 2 * g);
-    if (!grid_barrier(gb)) goto done;
-    grid_argmax(V, ncl, scr, irec, S, sh, shi, &mv, &mi);
-    if (!grid_barrier(gb)) goto done;  // V[mi] is read before the division below
-    for (int64_t c = c_lo + tid; c < c_hi; c += blockDim.x) V[c] = __ddiv_rn(V[c], mv);
-    {
-      const double px = xc[2 * mi], py = xc[2 * mi + 1];
-      for (int64_t i = r_lo + tid; i < r_hi; i += blockDim.x) U[i] = kernel_value(kp, xr[2 * i], xr[2 * i + 1], px, py);
-    }
-    __syncthreads();
-    {
-      const double a = slice_sum(V, c_lo, c_hi), b = slice_sum(U, r_lo, r_hi);
-      if (tid == 0) {
-        rec[1] = a;
-        rec[2] = b;
-      }
-    }
-    if (tid == 0 && mi >= c_lo && mi < c_hi) ucol[mi] = 1;
-    if (g == 0 && tid == 0) pcol[0] = (int)mi;
-    if (!grid_barrier(gb)) goto done;
-    double sr = 0.0, sc = 0.0;
-    for (int q = 0; q < G; ++q) {
-      sr += __ldcg(scr + (int64_t)q * S + 1);
-      sc += __ldcg(scr + (int64_t)q * S + 2);
-    }
-    double znorm2 = __dmul_rn(sr, sc);
-    int frnk = 1, st = 0;
-    while (__dmul_rn(sqrt(sr), sqrt(sc)) > __dmul_rn(rtol, sqrt(znorm2)) && frnk < maxsz) {
-      // next row pivot: argmax of the last column over unused rows
-      const double* lastcol = U + (int64_t)(frnk - 1) * nro;
-      double rv;
-      int64_t ri;
-      if (!grid_barrier(gb)) goto done;  // the records of the previous step have been read
-      slice_argmax(lastcol, urow, r_lo, r_hi, sval, sidx, rec, irec + 2 * g);
-      if (!grid_barrier(gb)) goto done;
-      grid_argmax(lastcol, nro, scr, irec, S, sh, shi, &rv, &ri);
-      if (frnk >= cap) {
-        st = 2;
-        break;
-      }
-      for (int j = tid; j < frnk; j += blockDim.x) coef[j] = __ldcg(U + ri + (int64_t)j * nro);
-      __syncthreads();
-      double* row = V + (int64_t)frnk * ncl;
-      {
-        const double px = xr[2 * ri], py = xr[2 * ri + 1];
-        for (int64_t c = c_lo + tid; c < c_hi; c += blockDim.x) {
-          double v = kernel_value(kp, px, py, xc[2 * c], xc[2 * c + 1]);
-          for (int j = 0; j < frnk; ++j) v = __dsub_rn(v, __dmul_rn(coef[j], V[c + (int64_t)j * ncl]));
-          row[c] = v;
-        }
-      }
-      if (!grid_barrier(gb)) goto done;  // urow[ri] is set after every CTA searched
-      if (tid == 0 && ri >= r_lo && ri < r_hi) urow[ri] = 1;
-      double cv;
-      int64_t cj;
-      slice_argmax(row, ucol, c_lo, c_hi, sval, sidx, rec, irec + 2 * g);
-      if (!grid_barrier(gb)) goto done;
-      grid_argmax(row, ncl, scr, irec, S, sh, shi, &cv, &cj);
-      if (cv == 0.0) break;
-      if (!grid_barrier(gb)) goto done;  // row[cj] is read before the division below
-      if (tid == 0 && cj >= c_lo && cj < c_hi) ucol[cj] = 1;
-      for (int64_t c = c_lo + tid; c < c_hi; c += blockDim.x) row[c] = __ddiv_rn(row[c], cv);
-      for (int j = tid; j < frnk; j += blockDim.x) coef[j] = __ldcg(V + cj + (int64_t)j * ncl);
-      __syncthreads();
-      double* col = U + (int64_t)frnk * nro;
-      {
-        const double px = xc[2 * cj], py = xc[2 * cj + 1];
-        for (int64_t i = r_lo + tid; i < r_hi; i += blockDim.x) {
-          double v = kernel_value(kp, xr[2 * i], xr[2 * i + 1], px, py);
-          for (int j = 0; j < frnk; ++j) v = __dsub_rn(v, __dmul_rn(coef[j], U[i + (int64_t)j * nro]));
-          col[i] = v;
-        }
-      }
-      __syncthreads();
-      // partial dots with the previous columns and the new squared norms
-      for (int j = w; j < frnk; j += nw) {
-        const double* uj = U + (int64_t)j * nro;
-        const double* vj = V + (int64_t)j * ncl;
-        double a = 0.0, b = 0.0;
-        for (int64_t i = r_lo + lane; i < r_hi; i += 32) a += uj[i] * col[i];
-        for (int64_t c = c_lo + lane; c < c_hi; c += 32) b += vj[c] * row[c];
-        a = warp_sum(a);
-        b = warp_sum(b);
-        if (lane == 0) {
-          rec[3 + j] = a;
-          rec[3 + cap + j] = b;
-        }
-      }
-      {
-        const double a = slice_sum(row, c_lo, c_hi), b = slice_sum(col, r_lo, r_hi);
-        if (tid == 0) {
-          rec[1] = a;
-          rec[2] = b;
-        }
-      }
-      if (!grid_barrier(gb)) goto done;
-      if (g == 0) {
-        // dots summed over the CTAs in a fixed order, one warp per j
-        for (int j = w; j < frnk; j += nw) {
-          double a = 0.0, b = 0.0;
-          for (int q = lane; q < G; q += 32) {
-            a += __ldcg(scr + (int64_t)q * S + 3 + j);
-            b += __ldcg(scr + (int64_t)q * S + 3 + cap + j);
-          }
-          a = warp_sum(a);
-          b = warp_sum(b);
-          if (lane == 0) coef[j] = __dmul_rn(__dmul_rn(2.0, fabs(a)), fabs(b));
-        }
-        __syncthreads();
-        if (tid == 0) {
-          double z = znorm2;
-          for (int j = 0; j < frnk; ++j) z = __dadd_rn(z, coef[j]);
-          double s1 = 0.0, s2 = 0.0;
-          for (int q = 0; q < G; ++q) {
-            s1 += __ldcg(scr + (int64_t)q * S + 1);
-            s2 += __ldcg(scr + (int64_t)q * S + 2);
-          }
-          scal[0] = __dadd_rn(z, __dmul_rn(s1, s2));
-          scal[1] = s1;
-          scal[2] = s2;
-          prow[frnk] = (int)ri;
-          pcol[frnk] = (int)cj;
-        }
-      }
-      if (!grid_barrier(gb)) goto done;
-      znorm2 = __ldcg(scal);
-      sr = __ldcg(scal + 1);
-      sc = __ldcg(scal + 2);
-      ++frnk;
-    }
-    if (g == 0 && tid == 0) {
-      rank_out[bidx] = frnk;
-      status[bidx] = st;
-    }
-  }
-done:
-  if (g == 0 && tid == 0 && *gb.err) status[bidx] = 3;
+  const GridTeam team{gb, reinterpret_cast<AcaRec*>(scr), scr + 3 * gridDim.x * (sizeof(AcaRec) / sizeof(double)),
+                      B.cap + 1};
+  aca_run(team, S, dsm, 0, pts, kp, B, P, F, piv, rtol, rank_out + bidx, status + bidx);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && *gb.err) status[bidx] = 3;
 }
 
-int64_t aca_grid_scratch(int cap) {
-  const int G = 152 * 2;  // upper bound of the grid
-  return (int64_t)G * (3 + 2 * cap) + 2 * G + 8 + 4;
+constexpr int kAcaGridMaxCtas = 152 * 2;
+
+// records, partial dots and (last) the barrier words of up to kAcaGridMaxCtas CTAs, in doubles
+static int64_t aca_grid_words_at(int G, int cap) {
+  return (int64_t)G * (3 * (int64_t)(sizeof(AcaRec) / sizeof(double)) + 2 * (cap + 1));
 }
+int64_t aca_grid_scratch(int cap) { return aca_grid_words_at(kAcaGridMaxCtas, cap) + 2; }
 
 bool launch_aca_grid(const double* pts, KParams kp, const AcaBlock* blocks, int b, int cap, double* P, uint8_t* F,
                      int* piv, double rtol, int* rank, int* status, double* scratch, cudaStream_t st,
@@ -1181,41 +1065,81 @@ bool launch_aca_grid(const double* pts, KParams kp, const AcaBlock* blocks, int 
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (!coop) return false;
-  const size_t sm = (size_t)std::max(cap, 1) * sizeof(double);
+  const size_t sm = ((size_t)std::max(cap, 1) + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
   smem_limit((const void*)k_aca_grid, sm);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aca_grid, 512, sm) != cudaSuccess || per < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aca_grid, kAcaThreads, sm) != cudaSuccess || per < 1) {
     cudaGetLastError();
     return false;
   }
-  const int G = std::min(nsm, 152 * 2);
-  // barrier words live after the records in the scratch
-  unsigned* words = reinterpret_cast<unsigned*>(scratch + (int64_t)G * (3 + 2 * cap) + 2 * G + 8);
+  const int G = std::min(nsm, kAcaGridMaxCtas);
+  unsigned* words = reinterpret_cast<unsigned*>(scratch + aca_grid_words_at(G, cap));
   if (cudaMemsetAsync(words, 0, 4 * sizeof(unsigned), st) != cudaSuccess) return false;
   GridBar gb{words, words + 1, reinterpret_cast<volatile int*>(words + 2), wait_limit};
   void* args[] = {(void*)&pts, (void*)&kp, (void*)&blocks, (void*)&b, (void*)&P, (void*)&F, (void*)&piv,
                   (void*)&rtol, (void*)&rank, (void*)&status, (void*)&scratch, (void*)&gb};
-  if (cudaLaunchCooperativeKernel((const void*)k_aca_grid, dim3(G), dim3(512), args, sm, st) != cudaSuccess) {
+  if (cudaLaunchCooperativeKernel((const void*)k_aca_grid, dim3(G), dim3(kAcaThreads), args, sm, st) !=
+      cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   return true;
 }
 
+// CTAs per cluster of k_aca: 16 where clusters of that size can be scheduled, else 8
+static int aca_cluster(size_t sm) {
+  static std::atomic<int> known{0};
+  int v = known.load();
+  if (v == 0) {
+    v = 8;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(kAcaThreads);
+    cfg.dynamicSmemBytes = sm;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {16, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute((const void*)k_aca, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, (const void*)k_aca, &cfg) == cudaSuccess && n > 0)
+      v = 16;
+    cudaGetLastError();  // a refused query leaves clusters of 8
+    known.store(v);
+  }
+  return v;
+}
+
+static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int last_first, int only,
+                       int maxcap, double* P, uint8_t* F, int* piv, double rtol, int* rank, int* status,
+                       cudaStream_t st) {
+  const size_t sm = ((size_t)3 * std::max(maxcap, 1) + 2 + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
+  smem_limit((const void*)k_aca, sm);
+  const int cs = aca_cluster(sm);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((only >= 0 ? 1 : nblocks) * cs));
+  cfg.blockDim = dim3(kAcaThreads);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {(unsigned)cs, 1, 1};
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_aca, pts, kp, blocks, nblocks, last_first, P, F, piv, rtol, rank, status, only);
+}
+
 void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b, int maxcap, double* P,
                     uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st) {
-  const size_t sm = (size_t)2 * std::max(maxcap, 1) * sizeof(double);
-  smem_limit((const void*)k_aca, sm);
-  k_aca<<<1, 1024, sm, st>>>(pts, kp, blocks, P, F, piv, rtol, rank, status, b);
+  aca_launch(pts, kp, blocks, 1, 0, b, maxcap, P, F, piv, rtol, rank, status, st);
 }
 
 // ---------------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------------
 void launch_aca(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int maxcap, double* P,
-                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st) {
-  const size_t sm = (size_t)2 * std::max(maxcap, 1) * sizeof(double);
-  smem_limit((const void*)k_aca, sm);
-  k_aca<<<nblocks, 1024, sm, st>>>(pts, kp, blocks, P, F, piv, rtol, rank, status, -1);
+                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first) {
+  aca_launch(pts, kp, blocks, nblocks, last_first, -1, maxcap, P, F, piv, rtol, rank, status, st);
 }
 
 void launch_panel_qr(const PanelDesc* descs, int n, int kmax, double* taus, double* Ts, cudaStream_t st) {

@@ -1364,7 +1364,7 @@ static int aca_assemble(km_handle* h, const double* pts, bool dev, const Tree& t
   KLV(h, KM_PROF_EVAL, launch_eval_leaves(h->d_pts, t, h->kp, -1, h->d_K, st));
   if (nb > 0)
     KLV(h, KM_PROF_ACA, launch_aca(h->d_pts, h->kp, h->d_blk, nb, maxcap, h->d_panels, h->d_flags, h->d_piv, tol,
-                                   h->d_brank, h->d_bstatus, st));
+                                   h->d_brank, h->d_bstatus, st, 1));
   // large blocks: one cooperative launch each, all SMs on one block
   {
     int gmax = 0;

@@ -215,19 +215,20 @@ void launch_col_dots(const double* A, int64_t lda, const double* B, int64_t ldb,
                      double* out, cudaStream_t st);
 
 // ACA and the general factorisation
-constexpr int kAcaMaxCap = 4096;       // ACA panel columns per block (2 x 4096 doubles of shared memory)
+constexpr int kAcaMaxCap = 4096;       // ACA panel columns per block (3 x 4096 doubles of shared memory)
 constexpr int64_t kAcaGridMin = 8192;  // blocks at least this wide run the grid-wide ACA kernel
+// last_first: start with the last blocks (they are the large ones of a HODLR level order)
 void launch_aca(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int maxcap, double* P,
-                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st);
+                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first = 0);
 // ACA of one large block (blocks[b].grid == 1) by all SMs in one cooperative launch, with
 // bounded grid barriers; scratch of aca_grid_scratch(cap) doubles.  Returns false when the
-// cooperative launch is unavailable (the caller then runs the block in the one-CTA kernel).
+// cooperative launch is unavailable (the caller then runs the block in one cluster).
 // wait_limit: polls before a grid barrier gives up (< 0: default; 0: at the first poll)
 bool launch_aca_grid(const double* pts, KParams kp, const AcaBlock* blocks, int b, int cap, double* P, uint8_t* F,
                      int* piv, double rtol, int* rank, int* status, double* scratch, cudaStream_t st,
                      long long wait_limit = -1);
 int64_t aca_grid_scratch(int cap);
-// one-CTA ACA of a single block regardless of its grid flag (fallback)
+// ACA of a single block by one cluster regardless of its grid flag (fallback)
 void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b, int maxcap, double* P,
                     uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st);
 // Householder QR with explicit Q of n panels (largest column count kmax); scratch of
