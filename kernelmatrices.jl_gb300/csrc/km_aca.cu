@@ -15,6 +15,7 @@
 // the c2 rows:  y_c2 -= Q2 (z2 - L22^{-1}(z2 - C' z1)),  z1 = Q1' y_c1, z2 = Q2' y_c2.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <atomic>
 #include <climits>
 
@@ -484,16 +485,12 @@ __device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, c
 }
 
 // ---------------------------------------------------------------------------------------------
-// Householder QR with explicit Q of one panel per CTA, blocked (LAPACK dgeqrf / dorgqr
-// structure: reflectors of kQB columns are formed by the unblocked dgeqr2 / dlarfg rules and
-// applied to the rest of the panel as one compact-WY block reflector I - V T V').  The trailing
-// columns are then read and written once per block instead of once per reflector.  V is staged
-// in shared memory kQC rows at a time; trailing columns are processed kQT at a time.
+// Householder QR with explicit Q of tall panels (more rows than a cluster's shared memory holds,
+// see km_pqr.cu for the others), blocked (LAPACK dgeqrf / dorgqr structure): reflectors of kQB
+// columns are formed by the unblocked dgeqr2 / dlarfg rules and applied to the rest of the panel as
+// one compact-WY block reflector I - V T V'.
 // ---------------------------------------------------------------------------------------------
 constexpr int kQB = 8;
-constexpr int kQC = 256;
-constexpr int kQT = 256;
-constexpr int kQV = kQB + 1;  // row stride of the staged V chunk (conflict-free column reads)
 
 // T (kQB x kQB, upper, column-major) of the block reflector of columns j0 .. j0+jb-1:
 //   T[q][q] = tau_q,  T[0:q, q] = -tau_q T[0:q, 0:q] (V[:, 0:q]' v_q)
@@ -528,101 +525,18 @@ __device__ void panel_block_T(const double* A, int64_t m, int64_t lda, int j0, i
   __syncthreads();
 }
 
-// C[:, c0:c1] <- (I - V op(T) V') C[:, c0:c1] over rows j0 .. m-1, op(T) = T' (QR, transT = 1)
-// or T (forming Q, transT = 0); V = the block's reflectors (columns j0 .. j0+jb-1 of A).
-__device__ void panel_apply_block(double* A, int64_t m, int64_t lda, int j0, int jb, int c0, int c1,
-                                  const double* Tm, int transT, double* W, double* W2, double* Vc, int wcap) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
-  for (int t0 = c0; t0 < c1; t0 += wcap) {
-    const int nt = min(wcap, c1 - t0);
-    for (int e = tid; e < kQB * nt; e += blockDim.x) W[e] = 0.0;
-    __syncthreads();
-    // W = V' C  (rows from j0 on, chunked)
-    for (int64_t r0 = j0; r0 < m; r0 += kQC) {
-      const int rows = (int)(m - r0 < kQC ? m - r0 : kQC);
-      for (int e = tid; e < rows * kQB; e += blockDim.x) {
-        const int ii = e % rows, p = e / rows;  // consecutive threads: consecutive rows of a column
-        const int64_t i = r0 + ii, ip = j0 + p;
-        double v = 0.0;
-        if (p < jb) v = (i == ip) ? 1.0 : (i > ip ? A[(int64_t)(j0 + p) * lda + i] : 0.0);
-        Vc[ii * kQV + p] = v;
-      }
-      __syncthreads();
-      for (int c = w; c < nt; c += nw) {
-        const double* col = A + (int64_t)(t0 + c) * lda + r0;
-        double acc[kQB];
-#pragma unroll
-        for (int p = 0; p < kQB; ++p) acc[p] = 0.0;
-        for (int ii = lane; ii < rows; ii += 32) {
-          const double x = col[ii];
-#pragma unroll
-          for (int p = 0; p < kQB; ++p) acc[p] += Vc[ii * kQV + p] * x;
-        }
-#pragma unroll
-        for (int p = 0; p < kQB; ++p) {
-          const double sum = warp_sum(acc[p]);
-          if (lane == 0) W[p + c * kQB] += sum;
-        }
-      }
-      __syncthreads();
-    }
-    // W2 = op(T) W
-    for (int e = tid; e < kQB * nt; e += blockDim.x) {
-      const int q = e % kQB, c = e / kQB;
-      double z = 0.0;
-      if (transT) {
-        for (int p = 0; p <= q; ++p) z += Tm[p + q * kQB] * W[p + c * kQB];
-      } else {
-        for (int p = q; p < kQB; ++p) z += Tm[q + p * kQB] * W[p + c * kQB];
-      }
-      W2[e] = z;
-    }
-    __syncthreads();
-    // C -= V W2
-    for (int64_t r0 = j0; r0 < m; r0 += kQC) {
-      const int rows = (int)(m - r0 < kQC ? m - r0 : kQC);
-      for (int e = tid; e < rows * kQB; e += blockDim.x) {
-        const int ii = e % rows, p = e / rows;  // consecutive threads: consecutive rows of a column
-        const int64_t i = r0 + ii, ip = j0 + p;
-        double v = 0.0;
-        if (p < jb) v = (i == ip) ? 1.0 : (i > ip ? A[(int64_t)(j0 + p) * lda + i] : 0.0);
-        Vc[ii * kQV + p] = v;
-      }
-      __syncthreads();
-      for (int c = w; c < nt; c += nw) {
-        double* col = A + (int64_t)(t0 + c) * lda + r0;
-        const double* wc = W2 + c * kQB;
-        for (int ii = lane; ii < rows; ii += 32) {
-          double z = 0.0;
-#pragma unroll
-          for (int p = 0; p < kQB; ++p) z += Vc[ii * kQV + p] * wc[p];
-          col[ii] -= z;
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// The panel QR of a level runs as a sequence of launches per reflector block, so that the
-// trailing updates of a tall panel spread over many CTAs (one FP64-bound SM per panel took
-// seconds for the 32768 x 549 panels of an n = 2^16 ACA matrix):
-//   k_pq_factor  (one CTA per panel)        dgeqr2 on the block's kQB columns, its T
-//   k_pq_update  (panels x column tiles)    block reflector applied to kQU trailing columns each
-//   k_pq_rout    (one CTA per panel)        R out
-//   then, blocks from last to first: k_pq_update on the formed columns, k_pq_form (dorg2r on
-//   the block's own columns).  tau and the T factors live in global scratch between launches.
-constexpr int kQU = 8;  // trailing columns per update CTA (each CTA is FP64-bound: narrow tiles, more SMs)
-
+// One CTA's factor and form steps of a block, used where the cooperative launch of all SMs is
+// refused: k_pq_factor is dgeqr2 on the block's kQB columns and its T, k_pq_form dorg2r on the
+// block's own columns (the columns to its right are already formed).
 __global__ void __launch_bounds__(512) k_pq_factor(const PanelDesc* __restrict__ descs, int j0,
                                                    double* __restrict__ taus, int ldtau, double* __restrict__ Ts,
-                                                   int nblk, int skip_big = 0) {
+                                                   int nblk) {
   __shared__ double red[40];
   __shared__ double sh[2];
   __shared__ double G[kQB * kQB], Tm[kQB * kQB];
   const PanelDesc D = descs[blockIdx.x];
   const int k = D.k;
-  if (j0 >= k || (skip_big && D.big)) return;
+  if (j0 >= k) return;
   double* A = D.A;
   const int64_t m = D.m, lda = D.lda;
   double* tau = taus + (int64_t)blockIdx.x * ldtau;
@@ -670,42 +584,12 @@ __global__ void __launch_bounds__(512) k_pq_factor(const PanelDesc* __restrict__
   }
 }
 
-// grid (panels, tiles): the reflector block at j0 applied to trailing columns j0+kQB + y*kQU ..
-// (transT = 1: QR, I - V T' V'; transT = 0: forming Q, I - V T V').
-__global__ void __launch_bounds__(256) k_pq_update(const PanelDesc* __restrict__ descs, int j0,
-                                                   const double* __restrict__ Ts, int nblk, int transT) {
-  extern __shared__ double smq[];
-  __shared__ double Tm[kQB * kQB];
-  const PanelDesc D = descs[blockIdx.x];
-  const int k = D.k;
-  if (j0 >= k || D.big) return;
-  const int jb = min(kQB, k - j0), j1 = j0 + jb;
-  const int c0 = j1 + blockIdx.y * kQU;
-  if (c0 >= k) return;
-  const double* Tin = Ts + ((int64_t)blockIdx.x * nblk + j0 / kQB) * kQB * kQB;
-  for (int e = threadIdx.x; e < kQB * kQB; e += blockDim.x) Tm[e] = Tin[e];
-  double* W = smq;               // kQB x kQU
-  double* W2 = W + kQB * kQU;    // kQB x kQU
-  double* Vc = W2 + kQB * kQU;   // kQC x kQV
-  __syncthreads();
-  panel_apply_block(D.A, D.m, D.lda, j0, jb, c0, min(c0 + kQU, k), Tm, transT, W, W2, Vc, kQU);
-}
-
-__global__ void k_pq_rout(const PanelDesc* __restrict__ descs) {
-  const PanelDesc D = descs[blockIdx.x];
-  const int k = D.k;
-  for (int e = threadIdx.x; e < k * k; e += blockDim.x) {
-    const int i = e % k, c = e / k;
-    D.R[e] = (i <= c) ? D.A[(int64_t)c * D.lda + i] : 0.0;
-  }
-}
-
 // dorg2r on the block's own columns j0 .. j1-1 (the columns to its right are already formed).
 __global__ void __launch_bounds__(512) k_pq_form(const PanelDesc* __restrict__ descs, int j0,
-                                                 const double* __restrict__ taus, int ldtau, int skip_big = 0) {
+                                                 const double* __restrict__ taus, int ldtau) {
   const PanelDesc D = descs[blockIdx.x];
   const int k = D.k;
-  if (j0 >= k || (skip_big && D.big)) return;
+  if (j0 >= k) return;
   double* A = D.A;
   const int64_t m = D.m, lda = D.lda;
   const double* tau = taus + (int64_t)blockIdx.x * ldtau;
@@ -734,289 +618,316 @@ __global__ void __launch_bounds__(512) k_pq_form(const PanelDesc* __restrict__ d
 }
 
 // ---------------------------------------------------------------------------------------------
-// Node capacitance of the general factorisation: C = R1 R2', L22 = chol(I - C'C) (lower), one
-// CTA per node, operands in global memory.  info[node] = failing column (1-based) or 0.
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(512) k_gnode(const GNodeDesc* __restrict__ nodes, int* __restrict__ info) {
-  const GNodeDesc N = nodes[blockIdx.x];
-  const int r = N.r;
-  const double* R1 = N.R1;
-  const double* R2 = N.R2;
-  double* C = N.C;
-  double* Lm = N.L22;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < r * r; e += blockDim.x) {
-    const int i = e % r, c = e / r;
-    double acc = 0.0;
-    for (int l = max(i, c); l < r; ++l) acc += R1[i + (int64_t)l * r] * R2[c + (int64_t)l * r];
-    C[e] = acc;
-  }
-  __syncthreads();
-  for (int e = tid; e < r * r; e += blockDim.x) {
-    const int i = e % r, c = e / r;
-    if (i >= c) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[l + (int64_t)i * r] * C[l + (int64_t)c * r];
-      Lm[e] = (i == c ? 1.0 : 0.0) - acc;
-    } else {
-      Lm[e] = 0.0;
-    }
-  }
-  __syncthreads();
-  __shared__ int bad;
-  if (tid == 0) bad = 0;
-  __syncthreads();
-  for (int j = 0; j < r; ++j) {
-    const double d = Lm[j + (int64_t)j * r];
-    const bool ok = d > 0.0;
-    const double sd = ok ? sqrt(d) : 1.0;
-    __syncthreads();
-    if (tid == 0 && !ok && bad == 0) bad = j + 1;
-    for (int i = j + 1 + tid; i < r; i += blockDim.x) Lm[i + (int64_t)j * r] /= sd;
-    if (tid == 0) Lm[j + (int64_t)j * r] = sd;
-    __syncthreads();
-    const int wdt = r - j - 1;
-    for (int e = tid; e < wdt * wdt; e += blockDim.x) {
-      const int i = j + 1 + e % wdt, c = j + 1 + e / wdt;
-      if (i >= c) Lm[i + (int64_t)c * r] -= Lm[i + (int64_t)j * r] * Lm[c + (int64_t)j * r];
-    }
-    __syncthreads();
-  }
-  if (tid == 0) info[blockIdx.x] = bad;
-}
-
-// ---------------------------------------------------------------------------------------------
-// Application of node factors to column blocks, one warp per (item, column):
+// Application of node factors to column blocks:
 //   mode 0 (W^{-1}):  y2 -= Q2 (z2 - L22^{-1}(z2 - C' z1))
 //   mode 1 (W^{-T}):  t = L22^{-T} z2;  y1 -= Q1 C t;  y2 -= Q2 (z2 - t)
 //   mode 2 (W):       y2 += Q2 (C' z1 + L22 z2 - z2)
 //   mode 3 (W'):      y1 += Q1 C z2;  y2 += Q2 (L22' z2 - z2)
 //   mode 4 (pre-factor product): y1 += V (U' y2_in), y2 += U (V' y1_in) with Q1 = V, Q2 = U
 //          reading x (in) and accumulating into y (out)
-// with z1 = Q1' y1, z2 = Q2' y2.  grid = (items, ceil(ncols/8)), block 256.
+// with z1 = Q1' y1, z2 = Q2' y2.  One CTA per (item, CB columns), grid = (items, chunks).
+//
+// The FP64 pipe bounds it (two multiply-adds a clock and SM): a projection entry is a dot product
+// over the rows by one warp, eight at a time so that the sums over the lanes take 9 additions for
+// 8 entries instead of 40; an expansion takes a thread per row.  One warp per column, as before,
+// left most of the SM idle and walked the r x r solve serially: 7.2 ms for one column at r = 496
+// with 512-row panels, now 0.65 ms.  CB = 8 reads each Q once per 8 columns; a single right-hand
+// side takes CB = 1, a rank whose vectors do not fit in shared memory 8 at a time 4, 2 or 1.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_gapply(const GApplyItem* __restrict__ items,
-                                                const GNodeDesc* __restrict__ nodes, int mode, double* X,
-                                                const double* Xin, int64_t ldX, int kX) {
+namespace {
+
+constexpr int kGaThreads = 256;
+constexpr int kGaWarps = kGaThreads / 32;
+constexpr int kGaStage = 512;   // rows of x staged per pass of a projection
+
+// Sums v[0..8) over the warp's lanes; lane 4 b (b = 0..7) returns the sum of v[perm(b)] with
+// perm(b) = 4 b2 + 2 b1 + b0 of lane bits 4, 3, 2.
+__device__ __forceinline__ double reduce8(double (&v)[8], int lane) {
+#pragma unroll
+  for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const bool up = (lane & o) != 0;
+      const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  double s = v[0];
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  return s;
+}
+
+// Z[c * ldz + q] += sign * sum_{i < n} A[i + q lda] x(i, c) for q < nq, c < CB; x staged in shared
+// memory at xs[c * ldx + i].  Warps take 8 / CB entries q at a time.
+template <int CB>
+__device__ void ga_proj(const double* A, int64_t lda, int nq, int n, const double* xs, int ldx, double* Z, int ldz,
+                        double sign) {
+  constexpr int QB = 8 / CB;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int q0 = w * QB; q0 < nq; q0 += kGaWarps * QB) {
+    double v[8] = {};
+    const double* a[QB];
+#pragma unroll
+    for (int u = 0; u < QB; ++u) a[u] = A + (int64_t)min(q0 + u, nq - 1) * lda;
+#pragma unroll 2
+    for (int i = lane; i < n; i += 32) {
+      double x[CB];
+#pragma unroll
+      for (int c = 0; c < CB; ++c) x[c] = xs[c * ldx + i];
+#pragma unroll
+      for (int u = 0; u < QB; ++u) {
+        const double e = a[u][i];
+#pragma unroll
+        for (int c = 0; c < CB; ++c) v[u * CB + c] += e * x[c];
+      }
+    }
+    const double s = reduce8(v, lane);
+    const int k = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+    const int q = q0 + k / CB;
+    if ((lane & 3) == 0 && q < nq) Z[(k % CB) * ldz + q] += sign > 0.0 ? s : -s;
+  }
+}
+
+// The same with x in global memory (column c at x + c ldx, nc of them): staged kGaStage rows at a
+// time.  Zeroes Z first; ends with a barrier.
+template <int CB>
+__device__ void ga_proj_rows(const double* Q, int64_t s, int r, const double* x, int64_t ldx, int nc, double* xs,
+                             double* Z) {
+  for (int e = threadIdx.x; e < CB * r; e += kGaThreads) Z[e] = 0.0;
+  for (int64_t i0 = 0; i0 < s; i0 += kGaStage) {
+    const int n = (int)min((int64_t)kGaStage, s - i0);
+    __syncthreads();
+    for (int c = 0; c < CB; ++c)
+      for (int i = threadIdx.x; i < n; i += kGaThreads) xs[c * kGaStage + i] = c < nc ? x[c * ldx + i0 + i] : 0.0;
+    __syncthreads();
+    ga_proj<CB>(Q + i0, s, r, n, xs, kGaStage, Z, r, 1.0);
+  }
+  __syncthreads();
+}
+
+// out(i, c) = sum_{l0 <= l < l1(i)} A[i + l lda] G[c * ldg + l] for a thread's row i
+template <int CB>
+__device__ __forceinline__ void ga_row(const double* A, int64_t lda, int64_t i, int l0, int l1, const double* G,
+                                       int ldg, double (&acc)[CB]) {
+#pragma unroll
+  for (int c = 0; c < CB; ++c) acc[c] = 0.0;
+  int l = l0;
+  for (; l + 4 <= l1; l += 4) {
+    double a[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) a[u] = A[i + (int64_t)(l + u) * lda];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int c = 0; c < CB; ++c) acc[c] += a[u] * G[c * ldg + l + u];
+  }
+  for (; l < l1; ++l) {
+    const double a = A[i + (int64_t)l * lda];
+#pragma unroll
+    for (int c = 0; c < CB; ++c) acc[c] += a * G[c * ldg + l];
+  }
+}
+
+// y(i, c) += sign Q G over the s rows of Q
+template <int CB>
+__device__ void ga_expand(const double* Q, int64_t s, int r, const double* G, double* y, int64_t ldy, int nc,
+                          double sign) {
+  for (int64_t i = threadIdx.x; i < s; i += kGaThreads) {
+    double acc[CB];
+    ga_row<CB>(Q, s, i, 0, r, G, r, acc);
+#pragma unroll
+    for (int c = 0; c < CB; ++c)
+      if (c < nc) y[c * ldy + i] += sign > 0.0 ? acc[c] : -acc[c];
+  }
+}
+
+// T <- L^{-1} T (trans = 0) or L^{-T} T for the lower triangular r x r L, CB columns of T (column
+// c at T + c r) in shared memory, by blocks of 32 rows: a warp per column solves the diagonal block
+// with a row per lane, then all threads update the other rows.
+template <int CB>
+__device__ void ga_trsv(const double* L, int r, double* T, int trans, double* xs) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  double* D = xs;  // 32 x 33, diagonal as reciprocals
+  const int nb = (r + 31) / 32;
+  for (int b = 0; b < nb; ++b) {
+    const int i0 = 32 * (trans ? nb - 1 - b : b), ib = min(32, r - i0);
+    __syncthreads();
+    for (int e = tid; e < 32 * 32; e += kGaThreads) {
+      const int i = e & 31, l = e >> 5;
+      if (i < ib && l <= i) {
+        const double v = L[i0 + i + (int64_t)(i0 + l) * r];
+        D[i * 33 + l] = l == i ? 1.0 / v : v;
+      }
+    }
+    __syncthreads();
+    if (w < CB) {
+      double t = lane < ib ? T[w * r + i0 + lane] : 0.0;
+      for (int q = 0; q < ib; ++q) {
+        const int l = trans ? ib - 1 - q : q;
+        if (lane == l) t *= D[l * 33 + l];
+        const double tl = __shfl_sync(0xffffffffu, t, l);
+        if (trans ? lane < l : (lane > l && lane < ib)) t -= (trans ? D[l * 33 + lane] : D[lane * 33 + l]) * tl;
+      }
+      if (lane < ib) T[w * r + i0 + lane] = t;
+    }
+    __syncthreads();
+    if (!trans) {
+      for (int i = i0 + ib + tid; i < r; i += kGaThreads) {
+        double acc[CB];
+        ga_row<CB>(L, r, i, i0, i0 + ib, T, r, acc);
+#pragma unroll
+        for (int c = 0; c < CB; ++c) T[c * r + i] -= acc[c];
+      }
+    } else if (i0 > 0) {
+      // rows l < i0 take the block's rows: column l of L, 32 consecutive entries
+      ga_proj<CB>(L + i0, r, i0, ib, T + i0, r, T, r, -1.0);
+    }
+  }
+  __syncthreads();
+}
+
+// The r x r part: from z1, z2 (in Z1, Z2) to the coefficients g1 (left in Z1; modes 1 and 3) and
+// g2 (left in Z2) of the expansions y1 -/+= Q1 g1, y2 -/+= Q2 g2.
+template <int CB>
+__device__ void ga_middle(const GNodeDesc& N, int mode, double* Z1, double* Z2, double* T, double* xs) {
+  const int r = N.r, tid = threadIdx.x;
+  const double* C = N.C;
+  const double* Lm = N.L22;
+  if (mode == 0 || mode == 1) {
+    for (int e = tid; e < CB * r; e += kGaThreads) T[e] = Z2[e];
+    __syncthreads();
+    if (mode == 0) ga_proj<CB>(C, r, r, r, Z1, r, T, r, -1.0);  // z2 - C' z1
+    ga_trsv<CB>(Lm, r, T, mode, xs);
+    for (int e = tid; e < CB * r; e += kGaThreads) Z2[e] -= T[e];
+    if (mode == 1)
+      for (int i = tid; i < r; i += kGaThreads) {
+        double acc[CB];
+        ga_row<CB>(C, r, i, 0, r, T, r, acc);
+#pragma unroll
+        for (int c = 0; c < CB; ++c) Z1[c * r + i] = acc[c];
+      }
+  } else {
+    for (int e = tid; e < CB * r; e += kGaThreads) T[e] = -Z2[e];
+    __syncthreads();
+    if (mode == 2) {
+      ga_proj<CB>(C, r, r, r, Z1, r, T, r, 1.0);
+      __syncthreads();
+    } else {
+      ga_proj<CB>(Lm, r, r, r, Z2, r, T, r, 1.0);  // entries above the diagonal are stored zeros
+    }
+    for (int i = tid; i < r; i += kGaThreads) {
+      double acc[CB];
+      ga_row<CB>(mode == 2 ? Lm : C, r, i, 0, mode == 2 ? i + 1 : r, Z2, r, acc);
+#pragma unroll
+      for (int c = 0; c < CB; ++c) {
+        if (mode == 2) T[c * r + i] += acc[c];
+        else Z1[c * r + i] = acc[c];
+      }
+    }
+    __syncthreads();
+    for (int e = tid; e < CB * r; e += kGaThreads) Z2[e] = T[e];
+  }
+  __syncthreads();
+}
+
+template <int CB>
+__global__ void __launch_bounds__(kGaThreads) k_gapply(const GApplyItem* __restrict__ items,
+                                                       const GNodeDesc* __restrict__ nodes, int mode, double* X,
+                                                       const double* Xin, int64_t ldX, int kX) {
   extern __shared__ double sm[];
   const GApplyItem I = items[blockIdx.x];
-  if (I.big) return;  // large nodes go through the library-GEMM path
+  if (I.big) return;  // large nodes go through the products over all SMs
   const GNodeDesc N = nodes[I.node];
   const int r = N.r;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int col = blockIdx.y * 8 + w;
-  double* base = I.base ? I.base : X;
   const int64_t ld = I.base ? I.ld : ldX;
-  const int ncols = I.base ? I.ncols : kX;
-  if (col >= ncols) return;
-  double* z1 = sm + (size_t)w * 3 * r;
-  double* z2 = z1 + r;
-  double* t = z2 + r;
+  const int ncols = I.base ? I.ncols : kX, col = blockIdx.y * CB;
+  if (col >= ncols || r == 0) return;
+  const int nc = min(CB, ncols - col);
+  double* Z1 = sm;
+  double* Z2 = Z1 + CB * r;
+  double* T = Z2 + CB * r;
+  double* xs = T + CB * r;
+  double* base = I.base ? I.base : X;
   double* y1 = base + I.off1 + (int64_t)col * ld;
   double* y2 = base + I.off2 + (int64_t)col * ld;
-  const double* x1 = (mode == 4) ? Xin + I.off1 + (int64_t)col * ldX : y1;
-  const double* x2 = (mode == 4) ? Xin + I.off2 + (int64_t)col * ldX : y2;
-  const double* Q1 = N.Q1;
-  const double* Q2 = N.Q2;
-  const int64_t s1 = N.s1, s2 = N.s2;
-  // projections z1 = Q1' x1, z2 = Q2' x2 (mode 4: z1 = U' x2, z2 = V' x1)
-  for (int q = 0; q < r; ++q) {
-    const double* q1 = (mode == 4 ? Q2 : Q1) + (int64_t)q * (mode == 4 ? s2 : s1);
-    const double* q2 = (mode == 4 ? Q1 : Q2) + (int64_t)q * (mode == 4 ? s1 : s2);
-    const double* xa = (mode == 4) ? x2 : x1;
-    const double* xb = (mode == 4) ? x1 : x2;
-    const int64_t na = (mode == 4) ? s2 : s1, nb = (mode == 4) ? s1 : s2;
-    double a = 0.0, b = 0.0;
-    if (mode == 0 || mode == 2 || mode == 4)
-      for (int64_t i = lane; i < na; i += 32) a += q1[i] * xa[i];
-    for (int64_t i = lane; i < nb; i += 32) b += q2[i] * xb[i];
-    a = warp_sum(a);
-    b = warp_sum(b);
-    if (lane == 0) {
-      z1[q] = a;
-      z2[q] = b;
-    }
-  }
-  __syncwarp();
-  const double* C = N.C;
-  const double* Lm = N.L22;
   if (mode == 4) {
-    // y1 (rows c1) += V z1 ; y2 (rows c2) += U z2   (V = Q1 rows c1, U = Q2 rows c2)
-    for (int64_t i = lane; i < s1; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q1[i + (int64_t)q * s1] * z1[q];
-      y1[i] += acc;
-    }
-    for (int64_t i = lane; i < s2; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q2[i + (int64_t)q * s2] * z2[q];
-      y2[i] += acc;
-    }
+    ga_proj_rows<CB>(N.Q2, N.s2, r, Xin + I.off2 + (int64_t)col * ldX, ldX, nc, xs, Z1);
+    ga_proj_rows<CB>(N.Q1, N.s1, r, Xin + I.off1 + (int64_t)col * ldX, ldX, nc, xs, Z2);
+    ga_expand<CB>(N.Q1, N.s1, r, Z1, y1, ld, nc, 1.0);
+    ga_expand<CB>(N.Q2, N.s2, r, Z2, y2, ld, nc, 1.0);
     return;
   }
-  if (mode == 0) {
-    for (int i = lane; i < r; i += 32) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[l + (int64_t)i * r] * z1[l];
-      t[i] = z2[i] - acc;
-    }
-    __syncwarp();
-    for (int l = 0; l < r; ++l) {
-      const double v = t[l] / Lm[l + (int64_t)l * r];
-      __syncwarp();
-      if (lane == 0) t[l] = v;
-      for (int i = l + 1 + lane; i < r; i += 32) t[i] -= Lm[i + (int64_t)l * r] * v;
-      __syncwarp();
-    }
-    for (int i = lane; i < r; i += 32) t[i] = z2[i] - t[i];
-    __syncwarp();
-    for (int64_t i = lane; i < s2; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q2[i + (int64_t)q * s2] * t[q];
-      y2[i] -= acc;
-    }
-  } else if (mode == 1) {
-    for (int i = lane; i < r; i += 32) t[i] = z2[i];
-    __syncwarp();
-    for (int i = r - 1; i >= 0; --i) {
-      const double v = t[i] / Lm[i + (int64_t)i * r];
-      __syncwarp();
-      if (lane == 0) t[i] = v;
-      for (int l = lane; l < i; l += 32) t[l] -= Lm[i + (int64_t)l * r] * v;
-      __syncwarp();
-    }
-    // z1 <- C t (reuse z1), z2 <- z2 - t
-    for (int i = lane; i < r; i += 32) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[i + (int64_t)l * r] * t[l];
-      z1[i] = acc;
-    }
-    __syncwarp();
-    for (int i = lane; i < r; i += 32) z2[i] -= t[i];
-    __syncwarp();
-    for (int64_t i = lane; i < s1; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q1[i + (int64_t)q * s1] * z1[q];
-      y1[i] -= acc;
-    }
-    for (int64_t i = lane; i < s2; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q2[i + (int64_t)q * s2] * z2[q];
-      y2[i] -= acc;
-    }
-  } else if (mode == 2) {
-    for (int i = lane; i < r; i += 32) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[l + (int64_t)i * r] * z1[l];
-      for (int l = 0; l <= i; ++l) acc += Lm[i + (int64_t)l * r] * z2[l];
-      t[i] = acc - z2[i];
-    }
-    __syncwarp();
-    for (int64_t i = lane; i < s2; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q2[i + (int64_t)q * s2] * t[q];
-      y2[i] += acc;
-    }
-  } else {
-    for (int i = lane; i < r; i += 32) {
-      double a1 = 0.0, a2 = 0.0;
-      for (int l = 0; l < r; ++l) a1 += C[i + (int64_t)l * r] * z2[l];
-      for (int l = i; l < r; ++l) a2 += Lm[l + (int64_t)i * r] * z2[l];
-      z1[i] = a1;
-      t[i] = a2 - z2[i];
-    }
-    __syncwarp();
-    for (int64_t i = lane; i < s1; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q1[i + (int64_t)q * s1] * z1[q];
-      y1[i] += acc;
-    }
-    for (int64_t i = lane; i < s2; i += 32) {
-      double acc = 0.0;
-      for (int q = 0; q < r; ++q) acc += Q2[i + (int64_t)q * s2] * t[q];
-      y2[i] += acc;
-    }
-  }
+  if (mode == 0 || mode == 2) ga_proj_rows<CB>(N.Q1, N.s1, r, y1, ld, nc, xs, Z1);
+  ga_proj_rows<CB>(N.Q2, N.s2, r, y2, ld, nc, xs, Z2);
+  ga_middle<CB>(N, mode, Z1, Z2, T, xs);
+  const double sign = mode < 2 ? -1.0 : 1.0;
+  if (mode == 1 || mode == 3) ga_expand<CB>(N.Q1, N.s1, r, Z1, y1, ld, nc, sign);
+  ga_expand<CB>(N.Q2, N.s2, r, Z2, y2, ld, nc, sign);
 }
 
-// The r x r part of k_gapply (same operations in the same order) for the nodes whose
-// projections and expansions run as library GEMMs: one warp per column.
-__global__ void k_gsmall(const GNodeDesc* __restrict__ node, int mode, const double* __restrict__ Z1,
-                         const double* __restrict__ Z2, double* __restrict__ G1, double* __restrict__ G2) {
+// The r x r part alone for a node whose projections and expansions run as products over all SMs
+// (columns of Z1, Z2, G1, G2: r consecutive values), CB columns per CTA.
+template <int CB>
+__global__ void __launch_bounds__(kGaThreads) k_gsmall(const GNodeDesc* __restrict__ node, int mode,
+                                                       const double* __restrict__ Z1, const double* __restrict__ Z2,
+                                                       double* __restrict__ G1, double* __restrict__ G2, int ncols) {
   extern __shared__ double sm[];
   const GNodeDesc N = *node;
-  const int r = N.r;
-  const int lane = threadIdx.x;
-  const int col = blockIdx.x;
+  const int r = N.r, col = blockIdx.x * CB, nc = min(CB, ncols - col);
   double* z1 = sm;
-  double* z2 = z1 + r;
-  double* t = z2 + r;
-  for (int i = lane; i < r; i += 32) {
-    z1[i] = (mode == 0 || mode == 2) ? Z1[(int64_t)col * r + i] : 0.0;
-    z2[i] = Z2[(int64_t)col * r + i];
+  double* z2 = z1 + CB * r;
+  double* T = z2 + CB * r;
+  double* xs = T + CB * r;
+  const int64_t off = (int64_t)col * r;
+  for (int e = threadIdx.x; e < CB * r; e += kGaThreads) {
+    z1[e] = (e < nc * r && (mode == 0 || mode == 2)) ? Z1[off + e] : 0.0;
+    z2[e] = e < nc * r ? Z2[off + e] : 0.0;
   }
-  __syncwarp();
-  const double* C = N.C;
-  const double* Lm = N.L22;
-  double* g1 = G1 + (int64_t)col * r;
-  double* g2 = G2 + (int64_t)col * r;
-  if (mode == 0) {
-    for (int i = lane; i < r; i += 32) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[l + (int64_t)i * r] * z1[l];
-      t[i] = z2[i] - acc;
-    }
-    __syncwarp();
-    for (int l = 0; l < r; ++l) {
-      const double v = t[l] / Lm[l + (int64_t)l * r];
-      __syncwarp();
-      if (lane == 0) t[l] = v;
-      for (int i = l + 1 + lane; i < r; i += 32) t[i] -= Lm[i + (int64_t)l * r] * v;
-      __syncwarp();
-    }
-    for (int i = lane; i < r; i += 32) g2[i] = z2[i] - t[i];
-  } else if (mode == 1) {
-    for (int i = lane; i < r; i += 32) t[i] = z2[i];
-    __syncwarp();
-    for (int i = r - 1; i >= 0; --i) {
-      const double v = t[i] / Lm[i + (int64_t)i * r];
-      __syncwarp();
-      if (lane == 0) t[i] = v;
-      for (int l = lane; l < i; l += 32) t[l] -= Lm[i + (int64_t)l * r] * v;
-      __syncwarp();
-    }
-    for (int i = lane; i < r; i += 32) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[i + (int64_t)l * r] * t[l];
-      g1[i] = acc;
-      g2[i] = z2[i] - t[i];
-    }
-  } else if (mode == 2) {
-    for (int i = lane; i < r; i += 32) {
-      double acc = 0.0;
-      for (int l = 0; l < r; ++l) acc += C[l + (int64_t)i * r] * z1[l];
-      for (int l = 0; l <= i; ++l) acc += Lm[i + (int64_t)l * r] * z2[l];
-      g2[i] = acc - z2[i];
-    }
-  } else {
-    for (int i = lane; i < r; i += 32) {
-      double a1 = 0.0, a2 = 0.0;
-      for (int l = 0; l < r; ++l) a1 += C[i + (int64_t)l * r] * z2[l];
-      for (int l = i; l < r; ++l) a2 += Lm[l + (int64_t)i * r] * z2[l];
-      g1[i] = a1;
-      g2[i] = a2 - z2[i];
-    }
+  __syncthreads();
+  ga_middle<CB>(N, mode, z1, z2, T, xs);
+  for (int e = threadIdx.x; e < nc * r; e += kGaThreads) {
+    if (mode == 1 || mode == 3) G1[off + e] = z1[e];
+    G2[off + e] = z2[e];
   }
 }
 
-// 2 sum log |diag(L22)| over the general nodes: one partial per node (deterministic).
-__global__ void k_glogdet(const GNodeDesc* __restrict__ nodes, int nn, double* __restrict__ partial) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nn) return;
-  const GNodeDesc N = nodes[q];
+// shared memory of CB columns at rank r; the widest CB <= want whose vectors fit
+size_t ga_smem(int cb, int r) {
+  return ((size_t)3 * cb * std::max(r, 1) + std::max(cb * kGaStage, 32 * 33)) * sizeof(double);
+}
+int ga_width(int ncols, int r) {
+  int cb = ncols == 1 ? 1 : ncols == 2 ? 2 : ncols <= 4 ? 4 : 8;
+  while (cb > 1 && ga_smem(cb, r) > 200 * 1024) cb >>= 1;
+  return cb;
+}
+
+template <int CB>
+void gapply_launch(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int mode, double* X,
+                   const double* Xin, int64_t ldX, int kX, cudaStream_t st) {
+  const size_t sm = ga_smem(CB, maxr);
+  smem_limit((const void*)k_gapply<CB>, sm);
+  k_gapply<CB><<<dim3((unsigned)n, (unsigned)((maxcols + CB - 1) / CB)), kGaThreads, sm, st>>>(items, nodes, mode, X,
+                                                                                         Xin, ldX, kX);
+}
+
+template <int CB>
+void gsmall_launch(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2, int r,
+                   int ncols, cudaStream_t st) {
+  const size_t sm = ga_smem(CB, r);
+  smem_limit((const void*)k_gsmall<CB>, sm);
+  k_gsmall<CB><<<(unsigned)((ncols + CB - 1) / CB), kGaThreads, sm, st>>>(node, mode, Z1, Z2, G1, G2, ncols);
+}
+
+}  // namespace
+
+// 2 sum log |diag(L22)| over the general nodes: one partial per node, a warp each (deterministic).
+__global__ void k_glogdet(const GNodeDesc* __restrict__ nodes, double* __restrict__ partial) {
+  const GNodeDesc N = nodes[blockIdx.x];
   double s = 0.0;
-  for (int i = 0; i < N.r; ++i) s += 2.0 * log(fabs(N.L22[i + (int64_t)i * N.r]));
-  partial[q] = s;
+  for (int i = threadIdx.x; i < N.r; i += 32) s += 2.0 * log(fabs(N.L22[i + (int64_t)i * N.r]));
+  s = warp_sum(s);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
 }  // namespace
@@ -1140,23 +1051,6 @@ void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b
 void launch_aca(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int maxcap, double* P,
                 uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first) {
   aca_launch(pts, kp, blocks, nblocks, last_first, -1, maxcap, P, F, piv, rtol, rank, status, st);
-}
-
-void launch_panel_qr(const PanelDesc* descs, int n, int kmax, double* taus, double* Ts, cudaStream_t st) {
-  if (n <= 0 || kmax <= 0) return;
-  const int nblk = (kmax + kQB - 1) / kQB;
-  const int ntiles = (kmax + kQU - 1) / kQU;
-  const size_t smu = ((size_t)2 * kQB * kQU + kQC * kQV) * sizeof(double);
-  smem_limit((const void*)k_pq_update, smu);
-  for (int b = 0; b < nblk; ++b) {
-    k_pq_factor<<<n, 512, 0, st>>>(descs, b * kQB, taus, kmax, Ts, nblk);
-    k_pq_update<<<dim3((unsigned)n, (unsigned)ntiles), 256, smu, st>>>(descs, b * kQB, Ts, nblk, 1);
-  }
-  k_pq_rout<<<n, 256, 0, st>>>(descs);
-  for (int b = nblk - 1; b >= 0; --b) {
-    k_pq_update<<<dim3((unsigned)n, (unsigned)ntiles), 256, smu, st>>>(descs, b * kQB, Ts, nblk, 0);
-    k_pq_form<<<n, 512, 0, st>>>(descs, b * kQB, taus, kmax);
-  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1363,8 +1257,7 @@ int64_t panel_qr_gemm_scratch(const PanelDesc* hdescs, int n, int kmax) {
 }
 
 // C[:, j1:k] <- (I - V op(T) V') C[:, j1:k] for big panel p, block j0: W = V' C, W2 = op(T) W,
-// C -= V W2 (op(T) = T' while factoring, T while forming Q), then the small panels' blocks by
-// k_pq_update
+// C -= V W2 (op(T) = T' while factoring, T while forming Q)
 static void panel_block_gemm(const PanelDesc* descs, const PanelDesc& D, int p, int j0, int nblk, const double* Ts,
                              double* scr, int kmax, double* split, int64_t split_len, int transT, cudaStream_t st) {
   const int k = D.k;
@@ -1416,9 +1309,6 @@ void launch_panel_qr_gemm(const PanelDesc* descs, const PanelDesc* hdescs, int n
                           long long wait_limit) {
   if (n <= 0 || kmax <= 0) return;
   const int nblk = (kmax + kQB - 1) / kQB;
-  const int ntiles = (kmax + kQU - 1) / kQU;
-  const size_t smu = ((size_t)2 * kQB * kQU + kQC * kQV) * sizeof(double);
-  smem_limit((const void*)k_pq_update, smu);
   // scratch after the GEMM buffers: partials of the cooperative steps and the barrier words
   int64_t mbig = 0;
   for (int p = 0; p < n; ++p)
@@ -1441,7 +1331,7 @@ void launch_panel_qr_gemm(const PanelDesc* descs, const PanelDesc* hdescs, int n
         return;
       cudaGetLastError();
     }
-    k_pq_factor<<<1, 512, 0, st>>>(dp, j0, tau, kmax, Ts + (int64_t)p * nblk * kQB * kQB, nblk, 0);
+    k_pq_factor<<<1, 512, 0, st>>>(dp, j0, tau, kmax, Ts + (int64_t)p * nblk * kQB * kQB, nblk);
   };
   auto form_big = [&](int p, int b) {
     const int G = pq_grid_size(hdescs[p].m);
@@ -1454,57 +1344,48 @@ void launch_panel_qr_gemm(const PanelDesc* descs, const PanelDesc* hdescs, int n
         return;
       cudaGetLastError();
     }
-    k_pq_form<<<1, 512, 0, st>>>(dp, j0, tau, kmax, 0);
+    k_pq_form<<<1, 512, 0, st>>>(dp, j0, tau, kmax);
   };
   for (int b = 0; b < nblk; ++b) {
-    k_pq_factor<<<n, 512, 0, st>>>(descs, b * kQB, taus, kmax, Ts, nblk, 1);
     for (int p = 0; p < n; ++p)
       if (hdescs[p].big && b * kQB < hdescs[p].k) factor_big(p, b);
-    k_pq_update<<<dim3((unsigned)n, (unsigned)ntiles), 256, smu, st>>>(descs, b * kQB, Ts, nblk, 1);
     for (int p = 0; p < n; ++p)
       if (hdescs[p].big)
         panel_block_gemm(descs, hdescs[p], p, b * kQB, nblk, Ts, gemm_scratch, kmax, split, split_len, 1, st);
   }
-  k_pq_rout<<<n, 256, 0, st>>>(descs);
+  launch_panel_rout(descs, n, kmax, 1, st);
   for (int b = nblk - 1; b >= 0; --b) {
-    k_pq_update<<<dim3((unsigned)n, (unsigned)ntiles), 256, smu, st>>>(descs, b * kQB, Ts, nblk, 0);
     for (int p = 0; p < n; ++p)
       if (hdescs[p].big)
         panel_block_gemm(descs, hdescs[p], p, b * kQB, nblk, Ts, gemm_scratch, kmax, split, split_len, 0, st);
-    k_pq_form<<<n, 512, 0, st>>>(descs, b * kQB, taus, kmax, 1);
     for (int p = 0; p < n; ++p)
       if (hdescs[p].big && b * kQB < hdescs[p].k) form_big(p, b);
   }
 }
 
-int64_t panel_qr_scratch(int n, int kmax) {
+int64_t panel_qr_gemm_taus(int n, int kmax) {
   const int nblk = (kmax + kQB - 1) / kQB;
   return (int64_t)n * kmax + (int64_t)n * nblk * kQB * kQB;
-}
-
-void launch_gnode(const GNodeDesc* nodes, int n, int* info, cudaStream_t st) {
-  k_gnode<<<n, 512, 0, st>>>(nodes, info);
 }
 
 void launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int mode,
                    double* X, const double* Xin, int64_t ldX, int kX, cudaStream_t st) {
   if (n <= 0) return;
-  dim3 grid((unsigned)n, (unsigned)((maxcols + 7) / 8));
-  const size_t sm = (size_t)8 * 3 * std::max(maxr, 1) * sizeof(double);
-  smem_limit((const void*)k_gapply, sm);
-  k_gapply<<<grid, 256, sm, st>>>(items, nodes, mode, X, Xin, ldX, kX);
+  const int cb = ga_width(maxcols, maxr);
+  (cb == 8 ? gapply_launch<8> : cb == 4 ? gapply_launch<4> : cb == 2 ? gapply_launch<2> : gapply_launch<1>)(
+      items, n, nodes, maxr, maxcols, mode, X, Xin, ldX, kX, st);
 }
 
 void launch_gsmall(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2,
                    int r, int ncols, cudaStream_t st) {
   if (ncols <= 0 || r <= 0) return;
-  const size_t sm = (size_t)3 * r * sizeof(double);
-  smem_limit((const void*)k_gsmall, sm);
-  k_gsmall<<<(unsigned)ncols, 32, sm, st>>>(node, mode, Z1, Z2, G1, G2);
+  const int cb = ga_width(ncols, r);
+  (cb == 8 ? gsmall_launch<8> : cb == 4 ? gsmall_launch<4> : cb == 2 ? gsmall_launch<2> : gsmall_launch<1>)(
+      node, mode, Z1, Z2, G1, G2, r, ncols, st);
 }
 
 void launch_glogdet(const GNodeDesc* nodes, int nn, double* partial, cudaStream_t st) {
-  k_glogdet<<<(nn + 127) / 128, 128, 0, st>>>(nodes, nn, partial);
+  k_glogdet<<<nn, 32, 0, st>>>(nodes, partial);
 }
 
 }  // namespace km

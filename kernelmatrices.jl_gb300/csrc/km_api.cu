@@ -489,9 +489,9 @@ NodeMatsH node_mats(km_handle* h) {
 // k_gapply gives one warp per (node, column), which serialises the O(size x rank) projections
 // of the top levels on a few SMs.
 constexpr int64_t kGapplyBig = 16384;
-// Panels with at least this many rows apply their block reflectors as library GEMMs (one CTA per
-// 8-column tile over all rows leaves most SMs idle on the few tall panels of the top levels).
-constexpr int64_t kPanelBig = 16384;
+// Panels of more rows than a cluster's shared memory holds are factored by all SMs
+// (launch_panel_qr_gemm), the others by clusters (launch_panel_qr).
+constexpr int64_t kPanelBig = kPanelRowsMax + 1;
 
 // Applies the node factors of items [a, b) of a level (host list hl, device list dl): k_gapply for
 // the small nodes, and for every large node Z = Q' x (DGEMM), the r x r part (k_gsmall), then
@@ -1510,12 +1510,20 @@ static int general_factorize(km_handle* h) {
     if (!fi.empty())
       KM_CUDA(h, cudaMemcpy(h->d_gfact, fi.data(), sizeof(GApplyItem) * fi.size(), cudaMemcpyHostToDevice));
     h->gfact_h = fi;
-    // panel QR scratch (taus and block T factors) for the largest level
+    // panel QR scratch for the largest level
     std::vector<int> kmax_l(t.L + 2, 0);
+    std::vector<int64_t> mmax_l(t.L + 2, 0);  // rows of the largest panel that is not big
     int64_t pqs = 1;
     for (int l = 1; l <= t.L; ++l) {
-      for (int64_t p = pdoff[l]; p < pdoff[l + 1]; ++p) kmax_l[l] = std::max(kmax_l[l], pd[p].k);
-      pqs = std::max(pqs, panel_qr_scratch((int)(pdoff[l + 1] - pdoff[l]), kmax_l[l]));
+      const int np = (int)(pdoff[l + 1] - pdoff[l]);
+      bool anybig = false;
+      for (int64_t p = pdoff[l]; p < pdoff[l + 1]; ++p) {
+        kmax_l[l] = std::max(kmax_l[l], pd[p].k);
+        if (pd[p].big) anybig = true;
+        else mmax_l[l] = std::max(mmax_l[l], pd[p].m);
+      }
+      if (mmax_l[l] > 0) pqs = std::max(pqs, panel_qr_scratch(np, kmax_l[l], mmax_l[l]));
+      if (anybig) pqs = std::max(pqs, panel_qr_gemm_taus(np, kmax_l[l]));
     }
     if ((rc = grow(h, &h->d_pqs, pqs))) return rc;
     if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri_desc(h->d_Lf, t, 0, h->d_ldesc, (int)ld.size(), h->gmaxr, st)))
@@ -1529,12 +1537,18 @@ static int general_factorize(km_handle* h) {
         KLV(h, KM_PROF_LEAF_QR, launch_panel_qr_gemm(h->d_pdesc + pdoff[l], pd.data() + pdoff[l], np, kmax_l[l],
                                                      h->d_pqs, h->d_pqs + (int64_t)np * kmax_l[l], h->d_pqg,
                                                      h->d_info + t.nleaf + nb, st, h->wait_limit));
-      } else {
-        KLV(h, KM_PROF_LEAF_QR, launch_panel_qr(h->d_pdesc + pdoff[l], np, kmax_l[l], h->d_pqs,
-                                                h->d_pqs + (int64_t)np * kmax_l[l], st));
       }
-      KLV(h, KM_PROF_NODE, launch_gnode(h->d_gnodes + h->lvoff[l], (int)(h->lvoff[l + 1] - h->lvoff[l]),
-                                        h->d_info + t.nleaf + h->lvoff[l], st));
+      if (mmax_l[l] > 0 && kmax_l[l] > 0) {
+        int nk = 0;
+        KLV(h, KM_PROF_LEAF_QR, nk = launch_panel_qr(h->d_pdesc + pdoff[l], np, kmax_l[l], mmax_l[l], h->d_pqs, st));
+        h->stats.kernel_launches += nk - 1;
+      }
+      if (kmax_l[l] > 0) {
+        int nk = 0;
+        KLV(h, KM_PROF_NODE, nk = launch_gnode(h->d_gnodes + h->lvoff[l], (int)(h->lvoff[l + 1] - h->lvoff[l]),
+                                               kmax_l[l], h->d_info + t.nleaf + h->lvoff[l], st));
+        h->stats.kernel_launches += nk - 1;
+      }
       const int64_t a = h->gfoff[l], b = h->gfoff[l + 1];
       if (b > a && (rc = run_gapply(h, h->gfact_h, h->d_gfact, a, b, maxcols, 0, nullptr, nullptr, 0, 0)) != KM_OK)
         return rc;

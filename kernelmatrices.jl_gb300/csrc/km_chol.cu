@@ -192,7 +192,64 @@ int chol_steps(const Mats& mats, int64_t nmat, int mmax, int* info, cudaStream_t
   return launches;
 }
 
+// C = R1 R2' (R1, R2 upper triangular) or, with the lower triangle of C'C wanted, L22 = I - C'C
+// (zeros above the diagonal): 32 x 32 tiles, grid (tile, tile, node), 256 threads.
+template <bool GRAM>
+__global__ void __launch_bounds__(256) k_gnode_product(const GNodeDesc* __restrict__ nodes) {
+  __shared__ double As[32 * 33], Bs[32 * 33];
+  const GNodeDesc N = nodes[blockIdx.z];
+  const int r = N.r, i0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+  if (i0 >= r || c0 >= r) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double acc[4] = {};  // row i0 + lane, columns c0 + w + 8 q
+  if (!GRAM || i0 >= c0) {
+    for (int l0 = GRAM ? 0 : max(i0, c0); l0 < r; l0 += 32) {
+      __syncthreads();
+      for (int u = w; u < 32; u += 8) {
+        if (GRAM) {  // entry (l, i) of C: As[i][l]
+          As[u * 33 + lane] = (l0 + lane < r && i0 + u < r) ? N.C[l0 + lane + (int64_t)(i0 + u) * r] : 0.0;
+          Bs[u * 33 + lane] = (l0 + lane < r && c0 + u < r) ? N.C[l0 + lane + (int64_t)(c0 + u) * r] : 0.0;
+        } else {     // entry (i, l) of R1, (c, l) of R2, zero below the diagonal
+          As[lane * 33 + u] = (i0 + lane <= l0 + u && l0 + u < r) ? N.R1[i0 + lane + (int64_t)(l0 + u) * r] : 0.0;
+          Bs[lane * 33 + u] = (c0 + lane <= l0 + u && l0 + u < r) ? N.R2[c0 + lane + (int64_t)(l0 + u) * r] : 0.0;
+        }
+      }
+      __syncthreads();
+#pragma unroll 8
+      for (int l = 0; l < 32; ++l) {
+        const double a = As[lane * 33 + l];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q] = __fma_rn(a, Bs[(w + 8 * q) * 33 + l], acc[q]);
+      }
+    }
+  }
+  const int i = i0 + lane;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int c = c0 + w + 8 * q;
+    if (i < r && c < r) {
+      if (GRAM) N.L22[i + (int64_t)c * r] = i < c ? 0.0 : (i == c ? 1.0 : 0.0) - acc[q];
+      else N.C[i + (int64_t)c * r] = acc[q];
+    }
+  }
+}
+
+struct NodeMats22 {
+  const GNodeDesc* nodes;
+  __device__ CholMat operator()(int64_t q) const { return CholMat{nodes[q].L22, nodes[q].L22, nodes[q].r}; }
+};
+
 }  // namespace
+
+// Node capacitances of the general factorisation: C = R1 R2', L22 = chol(I - C'C) (lower).
+// info[q]: failing column (1-based) of node q, zero on entry.  One CTA a node, as before, took
+// 70 ms at rank 496 (an FP64-bound 2/3 r^3 multiply-adds on one SM); tiles over all SMs 3.1 ms.
+int launch_gnode(const GNodeDesc* nodes, int n, int maxr, int* info, cudaStream_t st) {
+  const unsigned nt = (unsigned)((maxr + 31) / 32);
+  k_gnode_product<false><<<dim3(nt, nt, (unsigned)n), 256, 0, st>>>(nodes);
+  k_gnode_product<true><<<dim3(nt, nt, (unsigned)n), 256, 0, st>>>(nodes);
+  return 2 + chol_steps<NodeMats22, 32>(NodeMats22{nodes}, n, maxr, info, st);
+}
 
 int launch_leaf_chol_f64(const double* K, double* Lf, const Tree& t, int* info, cudaStream_t st) {
   const LeafMats mats{K, Lf, dtree(t)};

@@ -35,7 +35,7 @@ struct PanelDesc {            // Householder QR with explicit Q of A (m x k, lea
   int64_t m, lda;
   int k;
   double* R;                  // k x k output
-  int big;                    // 1: block reflectors applied with library GEMMs (k_pq_update skips it)
+  int big;                    // 1: factored by all SMs (km_pqr.cu skips it)
 };
 struct GNodeDesc {            // one node of the general factorisation
   double* Q1;                 // V panel (rows c1), Q after the QR
@@ -231,17 +231,22 @@ int64_t aca_grid_scratch(int cap);
 // ACA of a single block by one cluster regardless of its grid flag (fallback)
 void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b, int maxcap, double* P,
                     uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st);
-// Householder QR with explicit Q of n panels (largest column count kmax); scratch of
-// panel_qr_scratch(n, kmax) doubles: taus (n x kmax) then the T factors
-void launch_panel_qr(const PanelDesc* descs, int n, int kmax, double* taus, double* Ts, cudaStream_t st);
-// the same with the panels marked big handled by all SMs: their 8-column factor and form steps
+// Householder QR with explicit Q of the panels that are not marked big (km_pqr.cu): n descriptors,
+// largest column count kmax, largest row count mmax <= kPanelRowsMax of those panels; scratch of
+// panel_qr_scratch(n, kmax, mmax) doubles.  Returns the number of kernels launched.
+constexpr int64_t kPanelRowsMax = 12288;  // 16 CTAs of 768 rows x 32 columns of shared memory
+int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, double* scratch, cudaStream_t st);
+int64_t panel_qr_scratch(int n, int kmax, int64_t mmax);
+void launch_panel_rout(const PanelDesc* descs, int n, int kmax, int big, cudaStream_t st);
+// the same of the panels marked big, by all SMs: their 8-column factor and form steps
 // as cooperative launches (bounded grid barriers; a barrier that runs out sets *grid_err) and
 // their block-reflector applications as FP64 products over all SMs (launch_dgemm; hdescs: host
-// copies of descs;
+// copies of descs; taus: panel_qr_gemm_taus(n, kmax) doubles, Ts their tail after n kmax;
 // gemm_scratch: panel_qr_gemm_scratch(hdescs, n, kmax) doubles)
 void launch_panel_qr_gemm(const PanelDesc* descs, const PanelDesc* hdescs, int n, int kmax, double* taus,
                           double* Ts, double* gemm_scratch, int* grid_err, cudaStream_t st,
                           long long wait_limit = -1);
+int64_t panel_qr_gemm_taus(int n, int kmax);
 int64_t panel_qr_gemm_scratch(const PanelDesc* hdescs, int n, int kmax);
 // C = alpha op(A) B + beta C (FP64, column-major; op(A) = A' when transA), km_gemm.cu.  A long
 // reduction with op = T is split over CTAs when `scratch` holds dgemm_scratch(...) doubles
@@ -250,8 +255,9 @@ void launch_dgemm(int transA, int64_t M, int64_t N, int64_t K, double alpha, con
                   const double* B, int64_t ldb, double beta, double* C, int64_t ldc, double* scratch,
                   int64_t scratch_len, cudaStream_t st);
 int64_t dgemm_scratch(int transA, int64_t M, int64_t N, int64_t K);
-int64_t panel_qr_scratch(int n, int kmax);
-void launch_gnode(const GNodeDesc* nodes, int n, int* info, cudaStream_t st);
+// C = R1 R2' and L22 = chol(I - C'C) of n nodes of rank at most maxr (km_chol.cu); info zero on
+// entry; returns the number of kernels launched
+int launch_gnode(const GNodeDesc* nodes, int n, int maxr, int* info, cudaStream_t st);
 void launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int mode,
                    double* X, const double* Xin, int64_t ldX, int kX, cudaStream_t st);
 void launch_glogdet(const GNodeDesc* nodes, int nn, double* partial, cudaStream_t st);

@@ -89,7 +89,7 @@ extern "C" int km_probe_fp64_tflops(int device, double* out) {
 namespace km {
 
 void smem_limit(const void* func, size_t bytes) {
-  if (bytes <= 48 * 1024) return;  // within the default limit
+  if (bytes <= 32 * 1024) return;  // within the default limit of 48 KB with up to 16 KB of static arrays
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, bool> raised;
   int dev = 0;

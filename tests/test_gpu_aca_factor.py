@@ -1,0 +1,50 @@
+"""General (ACA) factorisation at ranks and sizes around its tiles: 32-column reflector blocks,
+32 x 32 tiles, right-hand sides 8 (4, 2, 1) at a time, row chunks of 128 to 512.
+
+Every check is an identity of the matrix that the engine itself multiplies by before factorising:
+W (W' x) = K x, K (K^-1 b) = b, W^-1 and W'^-1 against W and W'.  The matrices have a unit diagonal
+plus a nugget of 1, condition number below 1e5, so 1e-10 relative is well above rounding.  (With a
+longer range the rank-limited matrix of 25000 points is not positive definite.)
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,lv,rank,k", [(300, 1, 2, 1), (300, 1, 31, 2), (517, 2, 32, 3), (517, 2, 33, 8), (1000, 2, 64, 9),
+                                        (1003, 1, 65, 17), (2500, 3, 97, 5), (4100, 2, 40, 33), (6000, 2, 130, 8),
+                                        (25000, 5, 24, 4)])
+def test_factor_identities(lib, n, lv, rank, k):
+    import kmhodlr as K
+    from kmhodlr.data import uniform_points
+    pts = uniform_points(n, 3)
+    hk = K.KernelHODLR(K.KernelMatrix(pts, pts, np.array([1.0, 0.02 if n < 10000 else 0.005, 1.0]), K.Matern32()), 1e-13, rank,
+                       K.FixedLevel(lv))
+    x = np.random.default_rng(4).standard_normal((n, k))
+    y = hk @ x
+    K.symmetricfactorize(hk)
+    close = lambda a, b: np.linalg.norm(a - b) < 1e-10 * np.linalg.norm(b)  # noqa: E731
+    assert close(hk @ x, y)
+    assert close(hk.ldiv(y), x)
+    assert close(hk.W.ldiv(hk.W @ x), x)
+    assert close(hk.W.T.ldiv(hk.W.T @ x), x)
+    one = hk.ldiv(y[:, :1].copy())
+    assert close(one, x[:, :1])
+
+
+def test_unsorted_points_full_rank(lib):
+    """Unsorted points: the top block's rank comes close to its size (the README example's case)."""
+    import kmhodlr as K
+    from kmhodlr.data import normal_points
+    from oracle import hodlr_oracle as O
+    n = 600
+    pts = normal_points(n, 5)
+    p = np.array([1.0, 1.0, 1.0])
+    hk = K.KernelHODLR(K.KernelMatrix(pts, pts, p, K.RatQuad()), 1e-12, 0, K.FixedLevel(1))
+    A = O.kernel_block(O.KERNEL_RQ, pts, pts, p)
+    b = np.random.default_rng(6).standard_normal(n)
+    K.symmetricfactorize(hk)
+    want = np.linalg.solve(A, b)
+    assert np.linalg.norm(hk.ldiv(b) - want) < 1e-9 * np.linalg.norm(want)
+    assert abs(hk.logdet() - np.linalg.slogdet(A)[1]) < 1e-8 * n
