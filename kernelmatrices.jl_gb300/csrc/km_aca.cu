@@ -866,6 +866,109 @@ __global__ void __launch_bounds__(kGaThreads) k_gapply(const GApplyItem* __restr
   ga_expand<CB>(N.Q2, N.s2, r, Z2, y2, ld, nc, sign);
 }
 
+// The same in three launches for few items: the projections and the expansions spread over (item,
+// columns, side and row chunk) CTAs, the r x r part in between.  Partial projections of item q,
+// side d, chunk h, column c start at part + (((2 q + d) nchunk + h) ncol + c) ldr; the
+// coefficients at coef + ((2 q + d) ncol + c) ldr (ncol: columns rounded up to CB, ldr: largest r).
+// Nodes of 4096 and 8192 rows with 8 right-hand sides: 4.1 and 8.1 ms by one CTA a node, @A@ and
+// @B@ ms spread.
+struct GSpread {
+  double* part;
+  double* coef;
+  int nchunk, rows, ncol, ldr;
+};
+
+template <int CB>
+__global__ void __launch_bounds__(kGaThreads) k_gproj(const GApplyItem* __restrict__ items,
+                                                      const GNodeDesc* __restrict__ nodes, int mode, const double* X,
+                                                      int64_t ldX, int kX, GSpread sp) {
+  extern __shared__ double sm[];
+  const GApplyItem I = items[blockIdx.x];
+  if (I.big) return;
+  const GNodeDesc N = nodes[I.node];
+  const int r = N.r, d = blockIdx.z & 1, h = blockIdx.z >> 1, col = blockIdx.y * CB;
+  const int ncols = I.base ? I.ncols : kX;
+  const bool first = mode == 4 ? d == 1 : d == 0;  // Q1 and the rows c1 (mode 4: z1 = U' x2)
+  if (col >= ncols || r == 0 || (d == 0 && (mode == 1 || mode == 3))) return;
+  const int64_t s = first ? N.s1 : N.s2, i0 = (int64_t)h * sp.rows;
+  if (i0 >= s) return;
+  const int64_t ld = I.base ? I.ld : ldX;
+  const double* x = (I.base ? I.base : X) + (first ? I.off1 : I.off2) + (int64_t)col * ld + i0;
+  double* Z = sm;
+  double* xs = Z + CB * r;
+  const int nc = min(CB, ncols - col), n = (int)min((int64_t)sp.rows, s - i0);
+  for (int e = threadIdx.x; e < CB * r; e += kGaThreads) Z[e] = 0.0;
+  for (int c = 0; c < CB; ++c)
+    for (int i = threadIdx.x; i < n; i += kGaThreads) xs[c * kGaStage + i] = c < nc ? x[c * ld + i] : 0.0;
+  __syncthreads();
+  ga_proj<CB>((first ? N.Q1 : N.Q2) + i0, s, r, n, xs, kGaStage, Z, r, 1.0);
+  __syncthreads();
+  double* out = sp.part + ((((int64_t)2 * blockIdx.x + d) * sp.nchunk + h) * sp.ncol + col) * sp.ldr;
+  for (int e = threadIdx.x; e < CB * r; e += kGaThreads) out[(int64_t)(e / r) * sp.ldr + e % r] = Z[e];
+}
+
+template <int CB>
+__global__ void __launch_bounds__(kGaThreads) k_gmid(const GApplyItem* __restrict__ items,
+                                                     const GNodeDesc* __restrict__ nodes, int mode, int kX,
+                                                     GSpread sp) {
+  extern __shared__ double sm[];
+  const GApplyItem I = items[blockIdx.x];
+  if (I.big) return;
+  const GNodeDesc N = nodes[I.node];
+  const int r = N.r, col = blockIdx.y * CB;
+  if (col >= (I.base ? I.ncols : kX) || r == 0) return;
+  double* z = sm;  // z1, z2, T
+  double* xs = z + 3 * CB * r;
+  for (int d = 0; d < 2; ++d) {
+    const int64_t s = (mode == 4 ? d == 1 : d == 0) ? N.s1 : N.s2;
+    const bool have = !(d == 0 && (mode == 1 || mode == 3));
+    const int nh = (int)((s + sp.rows - 1) / sp.rows);
+    const double* in = sp.part + (((int64_t)2 * blockIdx.x + d) * sp.nchunk * sp.ncol + col) * sp.ldr;
+    for (int e = threadIdx.x; e < CB * r; e += kGaThreads) {
+      double v = 0.0;
+      const double* p = in + (int64_t)(e / r) * sp.ldr + e % r;
+      if (have)
+        for (int h = 0; h < nh; ++h) v += p[(int64_t)h * sp.ncol * sp.ldr];
+      z[d * CB * r + e] = v;
+    }
+  }
+  __syncthreads();
+  if (mode != 4) ga_middle<CB>(N, mode, z, z + CB * r, z + 2 * CB * r, xs);
+  for (int d = 0; d < 2; ++d) {
+    double* out = sp.coef + (((int64_t)2 * blockIdx.x + d) * sp.ncol + col) * sp.ldr;
+    for (int e = threadIdx.x; e < CB * r; e += kGaThreads) out[(int64_t)(e / r) * sp.ldr + e % r] = z[d * CB * r + e];
+  }
+}
+
+template <int CB>
+__global__ void __launch_bounds__(kGaThreads) k_gexpand(const GApplyItem* __restrict__ items,
+                                                        const GNodeDesc* __restrict__ nodes, int mode, double* X,
+                                                        int64_t ldX, int kX, GSpread sp) {
+  extern __shared__ double G[];  // CB x r
+  const GApplyItem I = items[blockIdx.x];
+  if (I.big) return;
+  const GNodeDesc N = nodes[I.node];
+  const int r = N.r, d = blockIdx.z & 1, h = blockIdx.z >> 1, col = blockIdx.y * CB;
+  const int ncols = I.base ? I.ncols : kX;
+  if (col >= ncols || r == 0 || (d == 0 && (mode == 0 || mode == 2))) return;
+  const int64_t s = d == 0 ? N.s1 : N.s2, i0 = (int64_t)h * sp.rows;
+  if (i0 >= s) return;
+  const int64_t i1 = min(s, i0 + sp.rows), ld = I.base ? I.ld : ldX;
+  const int nc = min(CB, ncols - col);
+  const double* in = sp.coef + (((int64_t)2 * blockIdx.x + d) * sp.ncol + col) * sp.ldr;
+  for (int e = threadIdx.x; e < CB * r; e += kGaThreads) G[e] = in[(int64_t)(e / r) * sp.ldr + e % r];
+  __syncthreads();
+  double* y = (I.base ? I.base : X) + (d == 0 ? I.off1 : I.off2) + (int64_t)col * ld;
+  const double* Q = d == 0 ? N.Q1 : N.Q2;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += kGaThreads) {
+    double acc[CB];
+    ga_row<CB>(Q, s, i, 0, r, G, r, acc);
+#pragma unroll
+    for (int c = 0; c < CB; ++c)
+      if (c < nc) y[c * ld + i] += mode < 2 ? -acc[c] : acc[c];
+  }
+}
+
 // The r x r part alone for a node whose projections and expansions run as products over all SMs
 // (columns of Z1, Z2, G1, G2: r consecutive values), CB columns per CTA.
 template <int CB>
@@ -902,13 +1005,43 @@ int ga_width(int ncols, int r) {
   return cb;
 }
 
+// Shape of an application: how many columns a CTA takes and, when the items alone would not give
+// six CTAs an SM, how the rows are split so that the projections and expansions do (chunks of 64
+// to kGaStage rows, at most 64 of them, so that their sums stay a small part of the middle step).
+struct GShape {
+  int cb, cols, rows, nchunk;  // nchunk 0: one launch
+};
+GShape ga_shape(int n, int maxr, int maxcols, int64_t maxs) {
+  GShape g{ga_width(maxcols, maxr), 0, 0, 0};
+  g.cols = (maxcols + g.cb - 1) / g.cb;
+  const int64_t ctas = (int64_t)n * g.cols;
+  if (ctas >= 6 * 152) return g;
+  const int64_t want = std::min<int64_t>((6 * 152 + 2 * ctas - 1) / (2 * ctas), 64);
+  int64_t rows = std::max<int64_t>(64, ((maxs + want - 1) / want + 31) / 32 * 32);
+  g.rows = (int)std::min<int64_t>(rows, kGaStage);
+  g.nchunk = (int)((maxs + g.rows - 1) / g.rows);
+  return g;
+}
+
 template <int CB>
-void gapply_launch(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int mode, double* X,
-                   const double* Xin, int64_t ldX, int kX, cudaStream_t st) {
+void gapply_launch(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, const GShape& g, int mode,
+                   double* X, const double* Xin, int64_t ldX, int kX, double* scratch, cudaStream_t st) {
   const size_t sm = ga_smem(CB, maxr);
-  smem_limit((const void*)k_gapply<CB>, sm);
-  k_gapply<CB><<<dim3((unsigned)n, (unsigned)((maxcols + CB - 1) / CB)), kGaThreads, sm, st>>>(items, nodes, mode, X,
-                                                                                         Xin, ldX, kX);
+  if (g.nchunk == 0) {
+    smem_limit((const void*)k_gapply<CB>, sm);
+    k_gapply<CB><<<dim3((unsigned)n, (unsigned)g.cols), kGaThreads, sm, st>>>(items, nodes, mode, X, Xin, ldX, kX);
+    return;
+  }
+  const int ncol = g.cols * CB;
+  const GSpread sp{scratch, scratch + (int64_t)2 * n * g.nchunk * ncol * maxr, g.nchunk, g.rows, ncol, maxr};
+  const size_t sp1 = ((size_t)CB * maxr + CB * kGaStage) * sizeof(double), sp2 = (size_t)CB * maxr * sizeof(double);
+  smem_limit((const void*)k_gproj<CB>, sp1);
+  smem_limit((const void*)k_gmid<CB>, sm);
+  smem_limit((const void*)k_gexpand<CB>, sp2);
+  const dim3 wide((unsigned)n, (unsigned)g.cols, (unsigned)(2 * g.nchunk));
+  k_gproj<CB><<<wide, kGaThreads, sp1, st>>>(items, nodes, mode, mode == 4 ? Xin : X, ldX, kX, sp);
+  k_gmid<CB><<<dim3((unsigned)n, (unsigned)g.cols), kGaThreads, sm, st>>>(items, nodes, mode, kX, sp);
+  k_gexpand<CB><<<wide, kGaThreads, sp2, st>>>(items, nodes, mode, X, ldX, kX, sp);
 }
 
 template <int CB>
@@ -1368,12 +1501,20 @@ int64_t panel_qr_gemm_taus(int n, int kmax) {
   return (int64_t)n * kmax + (int64_t)n * nblk * kQB * kQB;
 }
 
-void launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int mode,
-                   double* X, const double* Xin, int64_t ldX, int kX, cudaStream_t st) {
-  if (n <= 0) return;
-  const int cb = ga_width(maxcols, maxr);
-  (cb == 8 ? gapply_launch<8> : cb == 4 ? gapply_launch<4> : cb == 2 ? gapply_launch<2> : gapply_launch<1>)(
-      items, n, nodes, maxr, maxcols, mode, X, Xin, ldX, kX, st);
+int64_t gapply_scratch(int n, int maxr, int maxcols, int64_t maxs) {
+  const GShape g = ga_shape(n, maxr, maxcols, maxs);
+  return (int64_t)2 * n * (g.nchunk > 0 ? g.nchunk + 1 : 0) * g.cols * g.cb * maxr;
+}
+
+int launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int64_t maxs, int mode,
+                  double* X, const double* Xin, int64_t ldX, int kX, double* scratch, cudaStream_t st) {
+  if (n <= 0 || maxcols <= 0) return 0;
+  const GShape g = ga_shape(n, maxr, maxcols, maxs);
+  (g.cb == 8   ? gapply_launch<8>
+   : g.cb == 4 ? gapply_launch<4>
+   : g.cb == 2 ? gapply_launch<2>
+               : gapply_launch<1>)(items, n, nodes, maxr, g, mode, X, Xin, ldX, kX, scratch, st);
+  return g.nchunk > 0 ? 3 : 1;
 }
 
 void launch_gsmall(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2,

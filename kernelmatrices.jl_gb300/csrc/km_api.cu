@@ -485,74 +485,73 @@ NodeMatsH node_mats(km_handle* h) {
 
 // ---- general (ACA) path -------------------------------------------------------------------
 
-// Nodes at least this large (rows of both children) apply their factor through library GEMMs:
-// k_gapply gives one warp per (node, column), which serialises the O(size x rank) projections
-// of the top levels on a few SMs.
+// Nodes at least this large (rows of both children) update the coarser panels of the factorisation
+// by FP64 products over all SMs (launch_dgemm): those updates have hundreds of columns.
 constexpr int64_t kGapplyBig = 16384;
 // Panels of more rows than a cluster's shared memory holds are factored by all SMs
 // (launch_panel_qr_gemm), the others by clusters (launch_panel_qr).
 constexpr int64_t kPanelBig = kPanelRowsMax + 1;
 
-// Applies the node factors of items [a, b) of a level (host list hl, device list dl): k_gapply for
-// the small nodes, and for every large node Z = Q' x (DGEMM), the r x r part (k_gsmall), then
-// y -= / += Q G (DGEMM).  Modes as in k_gapply: 0 W^{-1}, 1 W'^{-1}, 2 W, 3 W', 4 pre-factor
-// product (Q1 = V rows c1, Q2 = U rows c2; y1 += V U' x2, y2 += U V' x1).
+// Applies the node factors of items [a, b) of a level (host list hl, device list dl), modes as in
+// k_gapply: 0 W^{-1}, 1 W'^{-1}, 2 W, 3 W', 4 pre-factor product (Q1 = V rows c1, Q2 = U rows c2;
+// y1 += V U' x2, y2 += U V' x1).  Items marked big (panel updates of the factorisation, mode 0)
+// run one by one: Z = Q' x (DGEMM), the r x r part (k_gsmall), y -= Q G (DGEMM).
 static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyItem* dl, int64_t a, int64_t b,
-                      int maxcols, int mode, double* X, const double* Xin, int64_t ldX, int kX) {
+                      int mode, double* X, const double* Xin, int64_t ldX, int kX) {
   cudaStream_t st = h->stream;
   if (b <= a) return KM_OK;
-  KLV(h, KM_PROF_SWEEP, launch_gapply(dl + a, (int)(b - a), h->d_gnodes, h->gmaxr, maxcols, mode, X, Xin, ldX, kX, st));
-  int64_t need = 0, split = 0;
-  for (int64_t q = a; q < b; ++q)
-    if (hl[q].big) {
+  // scratch of the whole sweep, so that its levels do not regrow it one after the other
+  const std::vector<int64_t>& off = &hl == &h->gsolve_h ? h->lvoff : h->gfoff;
+  int maxr = 1, maxcols = 0;  // of this level, over the items that are not big
+  int64_t maxs = 1, need = 0, split = 0, room = 0;
+  for (int l = 1; l <= h->tree.L; ++l) {
+    int r1 = 1, c1 = 0;
+    int64_t s1 = 1, nd = 0, sp = 0;
+    for (int64_t q = off[l]; q < off[l + 1]; ++q) {
       const GNodeDesc& N = h->gnodes_h[hl[q].node];
       const int nc = hl[q].base ? hl[q].ncols : kX;
-      need = std::max<int64_t>(need, 4 * (int64_t)N.r * nc);
-      split = std::max(split, std::max(dgemm_scratch(1, N.r, nc, N.s1), dgemm_scratch(1, N.r, nc, N.s2)));
+      if (hl[q].big) {
+        nd = std::max<int64_t>(nd, 4 * (int64_t)N.r * nc);
+        sp = std::max(sp, std::max(dgemm_scratch(1, N.r, nc, N.s1), dgemm_scratch(1, N.r, nc, N.s2)));
+      } else {
+        r1 = std::max(r1, N.r);
+        c1 = std::max(c1, nc);
+        s1 = std::max(s1, std::max(N.s1, N.s2));
+      }
     }
-  if (need == 0) return KM_OK;
+    room = std::max(room, std::max(nd + sp, gapply_scratch((int)(off[l + 1] - off[l]), r1, c1, s1)));
+    if (off[l] == a) {
+      maxr = r1;
+      maxcols = c1;
+      maxs = s1;
+      need = nd;
+      split = sp;
+    }
+  }
   int rc;
-  if ((rc = grow(h, &h->d_gz, need + split)) != KM_OK) return rc;
-  const double one = 1.0, mone = -1.0;
-  for (int64_t q = a; q < b; ++q) {
+  if ((rc = grow(h, &h->d_gz, room)) != KM_OK) return rc;
+  int nk = 0;
+  if (maxcols > 0) {
+    KLV(h, KM_PROF_SWEEP, nk = launch_gapply(dl + a, (int)(b - a), h->d_gnodes, maxr, maxcols, maxs, mode, X, Xin, ldX,
+                                             kX, h->d_gz, st));
+    h->stats.kernel_launches += nk - 1;
+  }
+  for (int64_t q = a; q < b && need > 0; ++q) {
     const GApplyItem& I = hl[q];
     if (!I.big) continue;
     const GNodeDesc& N = h->gnodes_h[I.node];
-    const int r = N.r;
-    double* base = I.base ? I.base : X;
-    const int64_t ld = I.base ? I.ld : ldX;
-    const int nc = I.base ? I.ncols : kX;
+    const int r = N.r, nc = I.ncols;
     if (r <= 0 || nc <= 0) continue;
-    double* y1 = base + I.off1;
-    double* y2 = base + I.off2;
-    const double* x1 = (mode == 4) ? Xin + I.off1 : y1;
-    const double* x2 = (mode == 4) ? Xin + I.off2 : y2;
     double* Z1 = h->d_gz;
     double* Z2 = Z1 + (int64_t)r * nc;
     double* G1 = Z2 + (int64_t)r * nc;
     double* G2 = G1 + (int64_t)r * nc;
-    const int64_t s1 = N.s1, s2 = N.s2;
     double* spl = G2 + (int64_t)r * nc;  // partial products of the split Q' x reductions
-    auto gemm_t = [&](const double* Q, int64_t s, const double* x, double* Z) {  // Z = Q' x
-      launch_dgemm(1, r, nc, s, 1.0, Q, s, x, ld, 0.0, Z, r, spl, split, st);
-    };
-    auto gemm_n = [&](const double* Q, int64_t s, const double* G, double* y, const double* alpha) {  // y += a Q G
-      launch_dgemm(0, s, nc, r, *alpha, Q, s, G, r, 1.0, y, ld, nullptr, 0, st);
-    };
-    const GNodeDesc* dN = h->d_gnodes + I.node;
     KLV(h, KM_PROF_SWEEP, {
-      if (mode == 4) {
-        gemm_t(N.Q2, s2, x2, Z1);  // U' x2
-        gemm_t(N.Q1, s1, x1, Z2);  // V' x1
-        gemm_n(N.Q1, s1, Z1, y1, &one);
-        gemm_n(N.Q2, s2, Z2, y2, &one);
-      } else {
-        if (mode == 0 || mode == 2) gemm_t(N.Q1, s1, x1, Z1);
-        gemm_t(N.Q2, s2, x2, Z2);
-        launch_gsmall(dN, mode, Z1, Z2, G1, G2, r, nc, st);
-        if (mode == 1 || mode == 3) gemm_n(N.Q1, s1, G1, y1, mode == 1 ? &mone : &one);
-        gemm_n(N.Q2, s2, G2, y2, (mode == 0 || mode == 1) ? &mone : &one);
-      }
+      launch_dgemm(1, r, nc, N.s1, 1.0, N.Q1, N.s1, I.base + I.off1, I.ld, 0.0, Z1, r, spl, split, st);
+      launch_dgemm(1, r, nc, N.s2, 1.0, N.Q2, N.s2, I.base + I.off2, I.ld, 0.0, Z2, r, spl, split, st);
+      launch_gsmall(h->d_gnodes + I.node, mode, Z1, Z2, G1, G2, r, nc, st);
+      launch_dgemm(0, N.s2, nc, r, -1.0, N.Q2, N.s2, G2, r, 1.0, I.base + I.off2, I.ld, nullptr, 0, st);
     });
   }
   return check_launch(h, "factor application");
@@ -566,7 +565,7 @@ int general_fwd(km_handle* h, double* X, int k) {  // X <- W^{-1} X
   for (int l = 1; l <= t.L; ++l) {
     const int64_t a = h->lvoff[l], b = h->lvoff[l + 1];
     int rc;
-    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, k, 0, X, X, t.n, k)) != KM_OK) return rc;
+    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, 0, X, X, t.n, k)) != KM_OK) return rc;
   }
   return check_launch(h, "general fwd");
 }
@@ -577,7 +576,7 @@ int general_bwd(km_handle* h, double* X, int k) {  // X <- W'^{-1} X
   for (int l = t.L; l >= 1; --l) {
     const int64_t a = h->lvoff[l], b = h->lvoff[l + 1];
     int rc;
-    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, k, 1, X, X, t.n, k)) != KM_OK) return rc;
+    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, 1, X, X, t.n, k)) != KM_OK) return rc;
   }
   if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 1, X, 1, t.n, 0, X, 1, t.n, 0, k, st)))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
@@ -590,7 +589,7 @@ int general_mul(km_handle* h, double* X, int k) {  // X <- W X
   for (int l = t.L; l >= 1; --l) {
     const int64_t a = h->lvoff[l], b = h->lvoff[l + 1];
     int rc;
-    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, k, 2, X, X, t.n, k)) != KM_OK) return rc;
+    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, 2, X, X, t.n, k)) != KM_OK) return rc;
   }
   if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 2, X, 1, t.n, 0, X, 1, t.n, 0, k, st)))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular kernel");
@@ -605,7 +604,7 @@ int general_mul_t(km_handle* h, double* X, int k) {  // X <- W' X
   for (int l = 1; l <= t.L; ++l) {
     const int64_t a = h->lvoff[l], b = h->lvoff[l + 1];
     int rc;
-    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, k, 3, X, X, t.n, k)) != KM_OK) return rc;
+    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, 3, X, X, t.n, k)) != KM_OK) return rc;
   }
   return check_launch(h, "general mul_t");
 }
@@ -619,7 +618,7 @@ int general_matvec(km_handle* h, const double* X, double* Y, int k) {
   for (int l = 1; l <= t.L; ++l) {
     const int64_t a = h->lvoff[l], b = h->lvoff[l + 1];
     int rc;
-    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, k, 4, Y, X, t.n, k)) != KM_OK) return rc;
+    if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, 4, Y, X, t.n, k)) != KM_OK) return rc;
   }
   return check_launch(h, "general matvec");
 }
@@ -1425,7 +1424,7 @@ static int aca_assemble(km_handle* h, const double* pts, bool dev, const Tree& t
     N.s2 = b.nro;
     N.r = rq;
     o += (int64_t)rq * rq;
-    items[q] = GApplyItem{q, 0, b.col0, b.row0, 0, nullptr, (b.nro + b.ncl >= kGapplyBig) ? 1 : 0};
+    items[q] = GApplyItem{q, 0, b.col0, b.row0, 0, nullptr, 0};
   }
   h->gnodes_h = nodes;
   h->gsolve_h = items;
@@ -1467,7 +1466,6 @@ static int general_factorize(km_handle* h) {
     std::vector<GApplyItem> fi;
     h->gfoff.assign(t.L + 2, 0);
     std::vector<int64_t> pdoff(t.L + 2, 0);
-    int maxcols = 1;
     for (int l = 1; l <= t.L; ++l) {
       pdoff[l] = (int64_t)pd.size();
       h->gfoff[l] = (int64_t)fi.size();
@@ -1490,7 +1488,6 @@ static int general_factorize(km_handle* h) {
           const int64_t ldp = first ? bp.ncl : bp.nro;
           fi.push_back(GApplyItem{q, h->brank[qp], b.col0 - side0, b.row0 - side0, ldp, panel,
                                   (b.nro + b.ncl >= kGapplyBig) ? 1 : 0});
-          maxcols = std::max(maxcols, h->brank[qp]);
         }
       }
     }
@@ -1550,7 +1547,7 @@ static int general_factorize(km_handle* h) {
         h->stats.kernel_launches += nk - 1;
       }
       const int64_t a = h->gfoff[l], b = h->gfoff[l + 1];
-      if (b > a && (rc = run_gapply(h, h->gfact_h, h->d_gfact, a, b, maxcols, 0, nullptr, nullptr, 0, 0)) != KM_OK)
+      if (b > a && (rc = run_gapply(h, h->gfact_h, h->d_gfact, a, b, 0, nullptr, nullptr, 0, 0)) != KM_OK)
         return rc;
     }
   }

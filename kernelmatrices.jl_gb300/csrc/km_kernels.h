@@ -258,8 +258,11 @@ int64_t dgemm_scratch(int transA, int64_t M, int64_t N, int64_t K);
 // C = R1 R2' and L22 = chol(I - C'C) of n nodes of rank at most maxr (km_chol.cu); info zero on
 // entry; returns the number of kernels launched
 int launch_gnode(const GNodeDesc* nodes, int n, int maxr, int* info, cudaStream_t st);
-void launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int mode,
-                   double* X, const double* Xin, int64_t ldX, int kX, cudaStream_t st);
+// Applies the factors of n items (nodes of rank at most maxr and at most maxs rows a side) to at
+// most maxcols columns each; scratch of gapply_scratch(...) doubles; returns the kernels launched.
+int launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int64_t maxs, int mode,
+                  double* X, const double* Xin, int64_t ldX, int kX, double* scratch, cudaStream_t st);
+int64_t gapply_scratch(int n, int maxr, int maxcols, int64_t maxs);
 void launch_glogdet(const GNodeDesc* nodes, int nn, double* partial, cudaStream_t st);
 // the r x r part of k_gapply for one node and ncols columns: from the projections Z1 = Q1' x1,
 // Z2 = Q2' x2 (r x ncols each; mode 4 is not handled here) to the expansion coefficients G1, G2

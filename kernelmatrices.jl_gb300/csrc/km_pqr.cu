@@ -29,8 +29,8 @@ constexpr int kPB = 32;          // columns of a reflector block
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kRowsMax = 768;    // rows of a block that one CTA holds (32 x 769 doubles)
-constexpr int kVtcRows = 512;    // rows of one V' C partial product
-constexpr int kApplyRows = 256;  // rows of one update CTA
+constexpr int kVtcRows = 512;    // most rows of one V' C partial product
+constexpr int kApplyRows = 256;  // most rows of one update CTA
 
 // Sums v[0..4) over the warp; lanes 8 b (b = 0..3) return the sum of v[2 b1 + b0] with b1, b0 the
 // lane's bits 4 and 3.
@@ -176,11 +176,11 @@ __device__ __forceinline__ double v_entry(const double* A, int64_t lda, int i, i
 // Wp[panel][chunk][c][p] = sum over the chunk's rows of V[i, p] C[i, c], c counted from the first
 // trailing column j1: grid (panel, column tile of 32, row chunk).
 __global__ void __launch_bounds__(kThreads) k_pqr_vtc(const PanelDesc* __restrict__ descs, int j0, double* __restrict__ Wp,
-                                                      int kmax, int nchunk) {
+                                                      int kmax, int nchunk, int rows) {
   __shared__ double Vs[32 * 33], Cs[32 * 33];
   const PanelDesc D = descs[blockIdx.x];
   const int j1 = j0 + kPB, nt = D.k - j1, c0 = blockIdx.y * 32, M = (int)D.m - j0;
-  const int r0 = blockIdx.z * kVtcRows, r1 = min(M, r0 + kVtcRows);
+  const int r0 = blockIdx.z * rows, r1 = min(M, r0 + rows);
   if (D.big || c0 >= nt || r0 >= M) return;
   const double* V = D.A + (int64_t)j0 * D.lda + j0;
   const double* C = D.A + (int64_t)(j1 + c0) * D.lda + j0;
@@ -211,14 +211,15 @@ __global__ void __launch_bounds__(kThreads) k_pqr_vtc(const PanelDesc* __restric
 // transT = 1 while factoring (op(T) = T'), 0 while forming Q.
 __global__ void __launch_bounds__(kThreads) k_pqr_apply(const PanelDesc* __restrict__ descs, int j0,
                                                         const double* __restrict__ Wp, const double* __restrict__ Ts,
-                                                        int nblk, int kmax, int nchunk, int transT) {
+                                                        int nblk, int kmax, int nchunk, int vrows, int rows,
+                                                        int transT) {
   __shared__ double Vs[32 * 33], W[32 * 33], W2[32 * 33], Tm[32 * 33];
   const PanelDesc D = descs[blockIdx.x];
   const int j1 = j0 + kPB, nt = D.k - j1, c0 = blockIdx.y * 32, M = (int)D.m - j0;
-  const int r0 = blockIdx.z * kApplyRows, r1 = min(M, r0 + kApplyRows);
+  const int r0 = blockIdx.z * rows, r1 = min(M, r0 + rows);
   if (D.big || c0 >= nt || r0 >= M) return;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int nch = (M + kVtcRows - 1) / kVtcRows;
+  const int nch = (M + vrows - 1) / vrows;
   const double* Tin = Ts + ((int64_t)blockIdx.x * nblk + j0 / kPB) * 2 * kPB * kPB;
   for (int u = w; u < 32; u += kWarps) {
     double s = 0.0;
@@ -277,11 +278,11 @@ __global__ void k_pqr_rout(const PanelDesc* __restrict__ descs, int big) {
 // The block's own columns of Q: zeros above row j0, E - V (T V_top') below; grid (panel, row
 // chunk), rows counted from the top of the panel.  A CTA reads V in its own rows only.
 __global__ void __launch_bounds__(kThreads) k_pqr_form(const PanelDesc* __restrict__ descs, int j0,
-                                                       const double* __restrict__ Ts, int nblk) {
+                                                       const double* __restrict__ Ts, int nblk, int rows) {
   __shared__ double Vs[32 * 33], W2[32 * 33];
   const PanelDesc D = descs[blockIdx.x];
   const int m = (int)D.m, M = m - j0;
-  const int r0 = blockIdx.y * kApplyRows, r1 = min(m, r0 + kApplyRows);
+  const int r0 = blockIdx.y * rows, r1 = min(m, r0 + rows);
   if (D.big || j0 >= D.k || r0 >= m) return;
   const int jb = min(kPB, D.k - j0);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -311,9 +312,17 @@ __global__ void __launch_bounds__(kThreads) k_pqr_form(const PanelDesc* __restri
 
 }  // namespace
 
+// rows of a CTA when `others` CTAs share a row range of mmax: the most that still give four CTAs an
+// SM, at least 64 (an update CTA repeats the 32 x 32 x 32 product with T)
+static int pqr_rows(int64_t others, int64_t mmax, int most) {
+  const int64_t chunks = std::max<int64_t>(1, (4 * 152 + others - 1) / others);
+  const int64_t rows = ((mmax + chunks - 1) / chunks + 31) / 32 * 32;
+  return (int)std::min<int64_t>(std::max<int64_t>(rows, 64), most);
+}
+
 // T factors (two kPB x kPB values per block) and the partial products of one block
 int64_t panel_qr_scratch(int n, int kmax, int64_t mmax) {
-  const int64_t nblk = (kmax + kPB - 1) / kPB, nchunk = (mmax + kVtcRows - 1) / kVtcRows;
+  const int64_t nblk = (kmax + kPB - 1) / kPB, nchunk = (mmax + 63) / 64;
   return n * nblk * 2 * kPB * kPB + n * nchunk * std::max(kmax, 1) * kPB;
 }
 
@@ -323,8 +332,8 @@ void launch_panel_rout(const PanelDesc* descs, int n, int kmax, int big, cudaStr
 
 int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, double* scratch, cudaStream_t st) {
   if (n <= 0 || kmax <= 0) return 0;
-  const int nblk = (kmax + kPB - 1) / kPB, nchunk = (int)((mmax + kVtcRows - 1) / kVtcRows);
-  const int napply = (int)((mmax + kApplyRows - 1) / kApplyRows);
+  const int nblk = (kmax + kPB - 1) / kPB;
+  auto chunks = [&](int rows) { return (unsigned)((mmax + rows - 1) / rows); };
   double* Ts = scratch;
   double* Wp = Ts + (int64_t)n * nblk * 2 * kPB * kPB;
   // CTAs per panel: enough for the rows to fit, then as many as keep a CTA per SM and 128 rows or
@@ -336,6 +345,16 @@ int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, doubl
                                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
   (void)wide;
   int launches = 0;
+  const int frows = pqr_rows(n, mmax, kApplyRows);
+  auto apply = [&](int j0, int nt, int transT) {
+    const unsigned tiles = (unsigned)((nt + 31) / 32);
+    const int vrows = pqr_rows((int64_t)n * tiles, mmax, kVtcRows), arows = pqr_rows((int64_t)n * tiles, mmax, kApplyRows);
+    const int nchunk = (int)chunks(vrows);
+    k_pqr_vtc<<<dim3((unsigned)n, tiles, (unsigned)nchunk), kThreads, 0, st>>>(descs, j0, Wp, kmax, nchunk, vrows);
+    k_pqr_apply<<<dim3((unsigned)n, tiles, chunks(arows)), kThreads, 0, st>>>(descs, j0, Wp, Ts, nblk, kmax, nchunk,
+                                                                              vrows, arows, transT);
+    launches += 2;
+  };
   for (int b = 0; b < nblk; ++b) {
     const int j0 = b * kPB;
     const int M = (int)mmax - j0;
@@ -355,25 +374,13 @@ int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, doubl
     cudaLaunchKernelEx(&cfg, k_pqr_factor, descs, j0, Ts, nblk, rs);
     ++launches;
     const int nt = kmax - j0 - kPB;
-    if (nt > 0) {
-      const unsigned tiles = (unsigned)((nt + 31) / 32);
-      k_pqr_vtc<<<dim3((unsigned)n, tiles, (unsigned)nchunk), kThreads, 0, st>>>(descs, j0, Wp, kmax, nchunk);
-      k_pqr_apply<<<dim3((unsigned)n, tiles, (unsigned)napply), kThreads, 0, st>>>(descs, j0, Wp, Ts, nblk, kmax,
-                                                                                   nchunk, 1);
-      launches += 2;
-    }
+    if (nt > 0) apply(j0, nt, 1);
   }
   launch_panel_rout(descs, n, kmax, 0, st);
   for (int b = nblk - 1; b >= 0; --b) {
     const int j0 = b * kPB, nt = kmax - j0 - kPB;
-    if (nt > 0) {
-      const unsigned tiles = (unsigned)((nt + 31) / 32);
-      k_pqr_vtc<<<dim3((unsigned)n, tiles, (unsigned)nchunk), kThreads, 0, st>>>(descs, j0, Wp, kmax, nchunk);
-      k_pqr_apply<<<dim3((unsigned)n, tiles, (unsigned)napply), kThreads, 0, st>>>(descs, j0, Wp, Ts, nblk, kmax,
-                                                                                   nchunk, 0);
-      launches += 2;
-    }
-    k_pqr_form<<<dim3((unsigned)n, (unsigned)napply), kThreads, 0, st>>>(descs, j0, Ts, nblk);
+    if (nt > 0) apply(j0, nt, 0);
+    k_pqr_form<<<dim3((unsigned)n, chunks(frows)), kThreads, 0, st>>>(descs, j0, Ts, nblk, frows);
     ++launches;
   }
   return launches + 1;
