@@ -105,9 +105,10 @@ __device__ bool grid_barrier(GridBar gb) {
 // few lanes are active: the chains bound the kernel.  One CTA per block ran a 512 x 512 block of
 // rank 496 (the README example: unsorted points, tolerance 1e-12) in 147 ms.  Split over 16 SMs a
 // slice holds 32 entries, and where a slice has at most 64 the multiplies, which do not wait for
-// one another, go to the quarters that the subtractions leave idle: 25.9 ms.  The 4096-point blocks
-// of a 2^14 matrix went from 191 to 25.8 ms, its 8192-point block (every SM in both forms; before
-// with seven barriers a step, searches by one thread and unbatched loads) from 74 to 29 ms.
+// one another, go to the quarters that the subtractions leave idle.  The slices of the first columns
+// stay in shared memory (L2 latency had doubled the chains' time): 20.6 ms.  The 4096-point blocks
+// of a 2^14 matrix went from 191 to 21.4 ms, its 8192-point block (every SM in both forms; before
+// with seven barriers a step, searches by one thread and unbatched loads) from 74 to 21.8 ms.
 // ---------------------------------------------------------------------------------------------
 namespace {
 
@@ -251,54 +252,73 @@ __device__ void aca_publish(AcaShared& S, AcaRec* out, AcaRec r) {
   }
 }
 
-// Residual entries e in [lo, hi) of a row or column: out[e] = k(e) - sum_j coef[j] M[e, j], one
+// A CTA's slices of the earlier columns of U or V: the first `kept` columns in shared memory
+// (column j at s + j n), every column in global memory (entry e at g + e + j ld, lo <= e < lo + n).
+struct AcaSlice {
+  double* s;
+  int kept, n;
+  const double* g;
+  int64_t ld, lo;
+};
+
+// Residual entries of the slice of a row or column: out[e] = k(e) - sum_j coef[j] M[e, j], one
 // multiply and one subtract per j in order; returns the thread's candidate among those not in
-// `used`.  role: this warp's number, rotated between the clusters so that the subtraction warps
+// `used`.  keep: where to put a copy (entry e - lo) or null.  role: this warp's number, rotated between the clusters so that the subtraction warps
 // of co-resident CTAs fall on different quarters of the SM.
 template <typename Eval>
-__device__ AcaRec aca_residual(Eval&& eval, const double* M, int64_t ld, int64_t lo, int64_t hi, double* out,
-                               const uint8_t* used, const double* coef, int nj, double* prod, int role) {
+__device__ AcaRec aca_residual(Eval&& eval, const AcaSlice& M, double* out, double* keep, const uint8_t* used,
+                               const double* coef, int nj, double* prod, int role) {
   AcaRec r{0, LLONG_MAX, LLONG_MAX, 0.0, 0.0};
   const int lane = threadIdx.x & 31;
-  if (hi - lo > kAcaSplit) {
-    for (int64_t e = lo + role * 32 + lane; e < hi; e += kAcaThreads) {
-      double v = eval(e);
+  if (M.n > kAcaSplit) {
+    for (int e = role * 32 + lane; e < M.n; e += kAcaThreads) {
+      double v = eval(M.lo + e);
+      const int js = min(nj, M.kept);
       int j = 0;
+#pragma unroll 8
+      for (; j < js; ++j) v = __dsub_rn(v, __dmul_rn(coef[j], M.s[j * M.n + e]));
+      const double* g = M.g + M.lo + e;
       for (; j + 8 <= nj; j += 8) {
         double m[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) m[q] = M[e + (int64_t)(j + q) * ld];
+        for (int q = 0; q < 8; ++q) m[q] = g[(int64_t)(j + q) * M.ld];
 #pragma unroll
         for (int q = 0; q < 8; ++q) v = __dsub_rn(v, __dmul_rn(coef[j + q], m[q]));
       }
-      for (; j < nj; ++j) v = __dsub_rn(v, __dmul_rn(coef[j], M[e + (int64_t)j * ld]));
-      out[e] = v;
-      aca_offer(r, v, e, used[e]);
+      for (; j < nj; ++j) v = __dsub_rn(v, __dmul_rn(coef[j], g[(int64_t)j * M.ld]));
+      out[M.lo + e] = v;
+      if (keep) keep[e] = v;
+      aca_offer(r, v, M.lo + e, used[M.lo + e]);
     }
     return r;
   }
-  const int nc = hi - lo > 32 ? 2 : 1;             // subtraction warps: roles 0 .. nc-1
+  const int nc = M.n > 32 ? 2 : 1;                 // subtraction warps: roles 0 .. nc-1
   const int np = (kAcaThreads / 128) * (4 - nc);   // multiply warps: roles with role % 4 >= nc
-  const int64_t e = lo + role * 32 + lane;
-  const bool mine = role < nc && e < hi;
-  double v = mine ? eval(e) : 0.0;
+  const int e = role * 32 + lane;
+  const bool mine = role < nc && e < M.n;
+  double v = mine ? eval(M.lo + e) : 0.0;
   const int nchunk = (nj + kAcaChunk - 1) / kAcaChunk;
   for (int t = 0; t <= nchunk; ++t) {
     if ((role & 3) >= nc) {
       if (t < nchunk) {
         double* buf = prod + (t & 1) * kAcaChunk * kAcaSplit;
-        const int jn = min(kAcaChunk, nj - t * kAcaChunk);
+        const int j0 = t * kAcaChunk, jn = min(kAcaChunk, nj - j0);
         const int pw = (role >> 2) * (4 - nc) + (role & 3) - nc;
-#pragma unroll 4
-        for (int it = pw; it < jn * nc; it += np) {
-          const int jj = it / nc, h = it - jj * nc;
-          const int64_t ee = lo + h * 32 + lane;
-          const int j = t * kAcaChunk + jj;
-          if (ee < hi) buf[jj * kAcaSplit + h * 32 + lane] = __dmul_rn(coef[j], M[ee + (int64_t)j * ld]);
+        if (j0 + jn <= M.kept) {
+          for (int it = pw; it < jn * nc; it += np) {
+            const int jj = it / nc, ee = (it - jj * nc) * 32 + lane;
+            if (ee < M.n) buf[jj * kAcaSplit + ee] = __dmul_rn(coef[j0 + jj], M.s[(j0 + jj) * M.n + ee]);
+          }
+        } else {
+#pragma unroll 8
+          for (int it = pw; it < jn * nc; it += np) {
+            const int jj = it / nc, ee = (it - jj * nc) * 32 + lane;
+            if (ee < M.n) buf[jj * kAcaSplit + ee] = __dmul_rn(coef[j0 + jj], M.g[M.lo + ee + (j0 + jj) * M.ld]);
+          }
         }
       }
     } else if (mine && t > 0) {
-      const double* buf = prod + ((t - 1) & 1) * kAcaChunk * kAcaSplit + role * 32 + lane;
+      const double* buf = prod + ((t - 1) & 1) * kAcaChunk * kAcaSplit + e;
       const int jn = min(kAcaChunk, nj - (t - 1) * kAcaChunk);
 #pragma unroll 8
       for (int jj = 0; jj < jn; ++jj) v = __dsub_rn(v, buf[jj * kAcaSplit]);
@@ -306,15 +326,32 @@ __device__ AcaRec aca_residual(Eval&& eval, const double* M, int64_t ld, int64_t
     __syncthreads();
   }
   if (mine) {
-    out[e] = v;
-    aca_offer(r, v, e, used[e]);
+    out[M.lo + e] = v;
+    if (keep) keep[e] = v;
+    aca_offer(r, v, M.lo + e, used[M.lo + e]);
   }
   return r;
 }
 
+// 4 lanes' parts of sum_e M[e, j] x[e] over the slice
+__device__ __forceinline__ double aca_dot(const AcaSlice& M, int j, const double* x, int p) {
+  double a = 0.0;
+  if (j < M.kept) {
+    const double* m = M.s + j * M.n;
+#pragma unroll 8
+    for (int e = p; e < M.n; e += 4) a += m[e] * x[e];
+  } else {
+    const double* m = M.g + M.lo + (int64_t)j * M.ld;
+#pragma unroll 8
+    for (int e = p; e < M.n; e += 4) a += m[e] * x[e];
+  }
+  return a;
+}
+
+// store: shared memory of `room` doubles for the slices of the first columns.
 // The whole approximation; false if a barrier ran out (every CTA of the team then leaves).
 template <typename Team>
-__device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, const double* __restrict__ pts,
+__device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, double* store, int64_t room, int turn, const double* __restrict__ pts,
                         const KParams& kp, const AcaBlock& B, double* P, uint8_t* F, int* __restrict__ piv,
                         double rtol, int* __restrict__ rank_out, int* __restrict__ status) {
   const int G = team.size(), g = team.rank();
@@ -336,6 +373,9 @@ __device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, c
   const int64_t rs = (nro + G - 1) / G, cs = (ncl + G - 1) / G;
   const int64_t r_lo = min(nro, g * rs), r_hi = min(nro, r_lo + rs);
   const int64_t c_lo = min(ncl, g * cs), c_hi = min(ncl, c_lo + cs);
+  const int rn = (int)(r_hi - r_lo), cn = (int)(c_hi - c_lo);
+  const int kept = (int)min((int64_t)cap, room / (rs + cs));
+  const AcaSlice Us{store, kept, rn, U, nro, r_lo}, Vs{store + (int64_t)kept * rs, kept, cn, V, ncl, c_lo};
   const double* xr = pts + 2 * B.row0;
   const double* xc = pts + 2 * B.col0;
   for (int64_t i = r_lo + tid; i < r_hi; i += kAcaThreads) urow[i] = 0;
@@ -355,7 +395,7 @@ __device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, c
   // first row not all zero (factorizations.jl:24-30)
   int64_t ri = 0;
   for (;;) {
-    aca_publish(S, team.mine(0), aca_residual(row_of(ri), V, ncl, c_lo, c_hi, V, ucol, coef, 0, prod, role));
+    aca_publish(S, team.mine(0), aca_residual(row_of(ri), Vs, V, nullptr, ucol, coef, 0, prod, role));
     if (!team.barrier()) return false;
     aca_combine(team, S, 0, ncl);
     if (S.win.key != 0 || ri + 1 >= maxsz) break;
@@ -381,9 +421,15 @@ __device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, c
         }
       }
       for (int j = tid; j < frnk; j += kAcaThreads) coef[j] = __ldcg(V + cj + (int64_t)j * ncl);
-      for (int64_t c = c_lo + tid; c < c_hi; c += kAcaThreads) row[c] = __ddiv_rn(row[c], cv);
+      double* rkeep = frnk < kept ? Vs.s + frnk * cn : nullptr;
+      double* ckeep = frnk < kept ? Us.s + frnk * rn : nullptr;
+      for (int c = tid; c < cn; c += kAcaThreads) {
+        const double v = __ddiv_rn(row[c_lo + c], cv);
+        row[c_lo + c] = v;
+        if (rkeep) rkeep[c] = v;
+      }
       __syncthreads();
-      const AcaRec rr = aca_residual(col_of(cj), U, nro, r_lo, r_hi, col, urow, coef, frnk, prod, role);
+      const AcaRec rr = aca_residual(col_of(cj), Us, col, ckeep, urow, coef, frnk, prod, role);
       __syncthreads();
       // this CTA's parts of the dots with the earlier columns and (entry frnk) of the squared
       // norms: 4 lanes per column, so that a warp reduces 8 columns by two shuffle steps
@@ -391,12 +437,8 @@ __device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, c
         const int j = j0 + (tid >> 2), p = tid & 3;
         double a = 0.0, b = 0.0;
         if (j <= frnk) {
-          const double* uj = U + (int64_t)j * nro;
-          const double* vj = V + (int64_t)j * ncl;
-#pragma unroll 4
-          for (int64_t i = r_lo + p; i < r_hi; i += 4) a += uj[i] * col[i];
-#pragma unroll 4
-          for (int64_t c = c_lo + p; c < c_hi; c += 4) b += vj[c] * row[c];
+          a = aca_dot(Us, j, ckeep ? ckeep : col + r_lo, p);
+          b = aca_dot(Vs, j, rkeep ? rkeep : row + c_lo, p);
         }
         if (j0 + (w << 3) <= frnk) {
           a += __shfl_xor_sync(0xffffffffu, a, 1);
@@ -471,8 +513,7 @@ __device__ bool aca_run(const Team& team, AcaShared& S, double* dsm, int turn, c
       for (int j = tid; j < frnk; j += kAcaThreads) coef[j] = __ldcg(U + ri + (int64_t)j * nro);
       __syncthreads();
       if (tid == 0 && ri >= r_lo && ri < r_hi) urow[ri] = 1;
-      aca_publish(S, team.mine(0), aca_residual(row_of(ri), V, ncl, c_lo, c_hi, V + (int64_t)frnk * ncl, ucol, coef, frnk, prod,
-                                     role));
+      aca_publish(S, team.mine(0), aca_residual(row_of(ri), Vs, V + (int64_t)frnk * ncl, nullptr, ucol, coef, frnk, prod, role));
       if (!team.barrier()) return false;
       aca_combine(team, S, 0, ncl);
     }
@@ -1068,7 +1109,8 @@ __global__ void k_glogdet(const GNodeDesc* __restrict__ nodes, double* __restric
 __global__ void __launch_bounds__(kAcaThreads) k_aca(const double* __restrict__ pts, KParams kp,
                                                      const AcaBlock* __restrict__ blocks, int nblocks, int last_first,
                                                      double* P, uint8_t* F, int* __restrict__ piv, double rtol,
-                                                     int* __restrict__ rank_out, int* __restrict__ status, int only) {
+                                                     int* __restrict__ rank_out, int* __restrict__ status, int only,
+                                                     int dyn) {
   extern __shared__ double dsm[];
   __shared__ AcaShared S;
   const int cid = (int)(blockIdx.x / cg::this_cluster().num_blocks());
@@ -1076,24 +1118,27 @@ __global__ void __launch_bounds__(kAcaThreads) k_aca(const double* __restrict__ 
   const AcaBlock B = blocks[bid];
   if (only < 0 && B.grid) return;  // compressed by k_aca_grid (the whole cluster leaves)
   const ClusterTeam team{&S, dsm + B.cap + 2 * kAcaChunk * kAcaSplit, B.cap + 1};
-  aca_run(team, S, dsm, cid, pts, kp, B, P, F, piv, rtol, rank_out + bid, status + bid);
+  const int fixed = 3 * B.cap + 2 + 2 * kAcaChunk * kAcaSplit;
+  aca_run(team, S, dsm, dsm + fixed, dyn - fixed, cid, pts, kp, B, P, F, piv, rtol, rank_out + bid, status + bid);
 }
 
 __global__ void __launch_bounds__(kAcaThreads) k_aca_grid(const double* __restrict__ pts, KParams kp,
                                                           const AcaBlock* __restrict__ blocks, int bidx, double* P,
                                                           uint8_t* F, int* __restrict__ piv, double rtol,
                                                           int* __restrict__ rank_out, int* __restrict__ status,
-                                                          double* scr, GridBar gb) {
+                                                          double* scr, GridBar gb, int dyn) {
   extern __shared__ double dsm[];
   __shared__ AcaShared S;
   const AcaBlock B = blocks[bidx];
   const GridTeam team{gb, reinterpret_cast<AcaRec*>(scr), scr + 3 * gridDim.x * (sizeof(AcaRec) / sizeof(double)),
                       B.cap + 1};
-  aca_run(team, S, dsm, 0, pts, kp, B, P, F, piv, rtol, rank_out + bidx, status + bidx);
+  const int fixed = B.cap + 2 * kAcaChunk * kAcaSplit;
+  aca_run(team, S, dsm, dsm + fixed, dyn - fixed, 0, pts, kp, B, P, F, piv, rtol, rank_out + bidx, status + bidx);
   if (blockIdx.x == 0 && threadIdx.x == 0 && *gb.err) status[bidx] = 3;
 }
 
 constexpr int kAcaGridMaxCtas = 152 * 2;
+constexpr size_t kAcaSmem = 208 * 1024;  // dynamic shared memory of a CTA that has its SM to itself
 
 // records, partial dots and (last) the barrier words of up to kAcaGridMaxCtas CTAs, in doubles
 static int64_t aca_grid_words_at(int G, int cap) {
@@ -1109,18 +1154,19 @@ bool launch_aca_grid(const double* pts, KParams kp, const AcaBlock* blocks, int 
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (!coop) return false;
-  const size_t sm = ((size_t)std::max(cap, 1) + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
+  const size_t sm = kAcaSmem;  // one CTA an SM: whatever the fixed arrays leave holds slices
   smem_limit((const void*)k_aca_grid, sm);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aca_grid, kAcaThreads, sm) != cudaSuccess || per < 1) {
     cudaGetLastError();
     return false;
   }
   const int G = std::min(nsm, kAcaGridMaxCtas);
+  int dyn = (int)(sm / sizeof(double));
   unsigned* words = reinterpret_cast<unsigned*>(scratch + aca_grid_words_at(G, cap));
   if (cudaMemsetAsync(words, 0, 4 * sizeof(unsigned), st) != cudaSuccess) return false;
   GridBar gb{words, words + 1, reinterpret_cast<volatile int*>(words + 2), wait_limit};
   void* args[] = {(void*)&pts, (void*)&kp, (void*)&blocks, (void*)&b, (void*)&P, (void*)&F, (void*)&piv,
-                  (void*)&rtol, (void*)&rank, (void*)&status, (void*)&scratch, (void*)&gb};
+                  (void*)&rtol, (void*)&rank, (void*)&status, (void*)&scratch, (void*)&gb, (void*)&dyn};
   if (cudaLaunchCooperativeKernel((const void*)k_aca_grid, dim3(G), dim3(kAcaThreads), args, sm, st) !=
       cudaSuccess) {
     cudaGetLastError();
@@ -1157,9 +1203,13 @@ static int aca_cluster(size_t sm) {
 static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int last_first, int only,
                        int maxcap, double* P, uint8_t* F, int* piv, double rtol, int* rank, int* status,
                        cudaStream_t st) {
-  const size_t sm = ((size_t)3 * std::max(maxcap, 1) + 2 + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
-  smem_limit((const void*)k_aca, sm);
-  const int cs = aca_cluster(sm);
+  // the fixed arrays, then this CTA's share of an SM for slices when the CTAs fit at most three to
+  // an SM (more, and the shared memory is worth more as L1 cache)
+  size_t sm = ((size_t)3 * std::max(maxcap, 1) + 2 + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
+  smem_limit((const void*)k_aca, kAcaSmem);
+  const int cs = aca_cluster(kAcaSmem);
+  const int per = ((only >= 0 ? 1 : nblocks) * cs + 151) / 152;
+  if (per <= 3) sm = std::max(sm, kAcaSmem / per);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((only >= 0 ? 1 : nblocks) * cs));
   cfg.blockDim = dim3(kAcaThreads);
@@ -1170,7 +1220,8 @@ static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, in
   at[0].val.clusterDim = {(unsigned)cs, 1, 1};
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_aca, pts, kp, blocks, nblocks, last_first, P, F, piv, rtol, rank, status, only);
+  cudaLaunchKernelEx(&cfg, k_aca, pts, kp, blocks, nblocks, last_first, P, F, piv, rtol, rank, status, only,
+                     (int)(sm / sizeof(double)));
 }
 
 void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b, int maxcap, double* P,
