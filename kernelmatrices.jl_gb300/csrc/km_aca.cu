@@ -1106,7 +1106,7 @@ __global__ void k_glogdet(const GNodeDesc* __restrict__ nodes, double* __restric
 
 }  // namespace
 
-__global__ void __launch_bounds__(kAcaThreads) k_aca(const double* __restrict__ pts, KParams kp,
+__global__ void __launch_bounds__(kAcaThreads, 3) k_aca(const double* __restrict__ pts, KParams kp,
                                                      const AcaBlock* __restrict__ blocks, int nblocks, int last_first,
                                                      double* P, uint8_t* F, int* __restrict__ piv, double rtol,
                                                      int* __restrict__ rank_out, int* __restrict__ status, int only,

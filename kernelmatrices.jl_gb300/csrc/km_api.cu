@@ -1818,7 +1818,8 @@ static int factorize_launches(km_handle* h) {
       if (fwd) cudaEventRecord(h->xev[1], h->side);
       for (int l = 1; l <= t.L; ++l) {
         KLV(h, KM_PROF_NODE, launch_node_factor<double>(h->d_R, h->d_SinvT, r, l, t, h->d_Ct, h->d_L22, h->d_Eref,
-                                                        h->d_Etau, h->d_info + t.nleaf, st));
+                                                        h->d_Etau, h->d_info + t.nleaf, st, h->node_cluster_max,
+                                                        (int)std::min<int64_t>(h->wait_limit, INT32_MAX)));
         side_level(h, l);
         {
           const NodeMatsH nm = node_mats(h);

@@ -343,7 +343,8 @@ __global__ void __launch_bounds__(leaf_qr_threads<T>()) k_leaf_formq(T* __restri
 }
 
 // ---------------------------------------------------------------------------------------------
-// Node factorisation, one CTA (1024 threads) per node of level l.  Given the children's R factors
+// Node factorisation in float pairs (the FP64 form is in km_node64.cu), one CTA (1024 threads) per
+// node of level l.  Given the children's R factors
 // (slots c1, c2) and Sc = chol(S) (lower):
 //   T1 = R1 Sc^{-T}, T2 = R2 Sc^{-T}   (upper triangular)
 //   Ct = T1 T2'                        (= R1 S^{-1} R2')
@@ -737,182 +738,6 @@ __global__ void __launch_bounds__(1024) k_node_factor(T* __restrict__ R, const T
     }
 }
 
-// FP64 variant: thread per output entry, 256 threads.  The FP64 pipe (2 DFMA/clk/SM) bounds
-// this kernel, and with few warps per CTA it keeps that pipe busier than the warp-item mapping
-// of k_node_factor.
-__global__ void __launch_bounds__(256) k_node_factor_f64(double* __restrict__ R, const double* __restrict__ SinvT,
-                                                     int r, int level, int L, int64_t nleaf,
-                                                     int64_t cbase, int64_t nbase, double* __restrict__ Ct_out,
-                                                     double* __restrict__ L22_out, double* __restrict__ Eref,
-                                                     double* __restrict__ Etau, int* __restrict__ info) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  double* sm = reinterpret_cast<double*>(smraw);
-  __shared__ double red[32];
-  __shared__ double sh[2];
-  const int ld = r + 1;
-  double* X0 = sm;
-  double* X1 = X0 + r * ld;
-  double* X2 = X1 + r * ld;
-  double* X3 = X2 + r * ld;
-  const int64_t k = blockIdx.x;
-  const int64_t node = nbase + k;  // node index within all nodes (level-major)
-  const double* R1 = R + (cbase + 2 * k) * (int64_t)r * r;
-  const double* R2 = R + (cbase + 2 * k + 1) * (int64_t)r * r;
-  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nth >> 5;
-  // load: X0 = Sc^{-T} (upper), X1 = R1, X2 = R2   (element (i,c) at i + c*ld)
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    X0[i + c * ld] = SinvT[e];
-    X1[i + c * ld] = R1[e];
-    X2[i + c * ld] = R2[e];
-  }
-  __syncthreads();
-  // T1 = R1 Sc^{-T} -> X3 (upper x upper: entries l in [i, c])
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    double acc = double(0.0);
-    if (i <= c) {
-#pragma unroll 4
-      for (int l = i; l <= c; ++l) acc += X1[i + l * ld] * X0[l + c * ld];
-    }
-    X3[i + c * ld] = acc;
-  }
-  __syncthreads();
-  // T2 = R2 Sc^{-T} -> X1
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    double acc = double(0.0);
-    if (i <= c) {
-#pragma unroll 4
-      for (int l = i; l <= c; ++l) acc += X2[i + l * ld] * X0[l + c * ld];
-    }
-    X1[i + c * ld] = acc;
-  }
-  __syncthreads();
-  // Ct = T1 T2' -> X0 ; Ct[i][c] = sum_{l >= max(i,c)} T1[i][l] T2[c][l]
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    double acc = double(0.0);
-#pragma unroll 4
-    for (int l = max(i, c); l < r; ++l) acc += X3[i + l * ld] * X1[c + l * ld];
-    X0[i + c * ld] = acc;
-  }
-  __syncthreads();
-  // H = I - Ct' Ct -> X3 (lower triangle)
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    if (i >= c) {
-      double acc = double(0.0);
-#pragma unroll 4
-      for (int l = 0; l < r; ++l) acc += X0[l + i * ld] * X0[l + c * ld];
-      X3[i + c * ld] = double(i == c ? 1.0 : 0.0) - acc;
-    }
-  }
-  __syncthreads();
-  // L22 = chol(H) in place (lower)
-  int bad = 0;
-  for (int j = 0; j < r; ++j) {
-    const double d = X3[j + j * ld];
-    const bool ok = d > 0.0;
-    if (!ok && bad == 0) bad = j + 1;
-    const double sd = ok ? sqrt(d) : double(1.0);
-    __syncthreads();
-    for (int i = j + 1 + tid; i < r; i += nth) X3[i + j * ld] /= sd;
-    if (tid == 0) X3[j + j * ld] = sd;
-    __syncthreads();
-    const int wdt = r - j - 1;
-    for (int e = tid; e < wdt * wdt; e += nth) {
-      const int i = j + 1 + e % wdt, c = j + 1 + e / wdt;
-      if (i >= c) X3[i + c * ld] -= X3[i + j * ld] * X3[c + j * ld];
-    }
-    __syncthreads();
-  }
-  if (tid == 0 && bad) info[node] = bad;
-  // store Ct and L22
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    Ct_out[node * (int64_t)r * r + e] = X0[i + c * ld];
-    L22_out[node * (int64_t)r * r + e] = (i >= c) ? X3[i + c * ld] : double(0.0);
-  }
-  if (level >= L) return;
-  __syncthreads();
-  // reload R1 -> X1 (X2 still holds R2)
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    X1[i + c * ld] = R1[e];
-  }
-  __syncthreads();
-  // B = R2 - Ct' R1 -> X2 (column c of R1 has entries l <= c)
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    double acc = double(0.0);
-#pragma unroll 4
-    for (int l = 0; l <= c; ++l) acc += X0[l + i * ld] * X1[l + c * ld];
-    X2[i + c * ld] -= acc;
-  }
-  __syncthreads();
-  // B <- L22^{-1} B, row by row with the whole CTA
-  for (int i = 0; i < r; ++i) {
-    const double inv = double(1.0) / X3[i + i * ld];
-    for (int c = tid; c < r; c += nth) X2[i + c * ld] *= inv;
-    __syncthreads();
-    const int rows = r - i - 1;
-    for (int e = tid; e < rows * r; e += nth) {
-      const int ii = i + 1 + e % rows, c = e / rows;
-      X2[ii + c * ld] -= X3[ii + i * ld] * X2[i + c * ld];
-    }
-    __syncthreads();
-  }
-  // structured Householder QR of [X1 (upper r x r) ; X2 (r x r)]:
-  // reflector j acts on row j of the top and all r rows of the bottom.
-  for (int j = 0; j < r; ++j) {
-    double part = double(0.0);
-    for (int i = tid; i < r; i += nth) part += X2[i + j * ld] * X2[i + j * ld];
-    part = warp_sum_t(part);
-    if (lane == 0) red[w] = part;
-    __syncthreads();
-    if (tid == 0) {
-      double sig = double(0.0);
-      for (int q = 0; q < nw; ++q) sig += red[q];
-      const double alpha = X1[j + j * ld];
-      double tj = double(0.0), beta = alpha, scal = double(0.0);
-      if (sig != 0.0) {
-        const double nrm = sqrt(alpha * alpha + sig);
-        beta = alpha >= 0.0 ? -nrm : nrm;
-        tj = (beta - alpha) / beta;
-        scal = double(1.0) / (alpha - beta);
-      }
-      X1[j + j * ld] = beta;
-      sh[0] = scal;
-      sh[1] = tj;
-      Etau[node * (int64_t)r + j] = tj;
-    }
-    __syncthreads();
-    const double scal = sh[0], tj = sh[1];
-    if (tj != 0.0) {
-      // scaled reflector column v = X2[:, j] * scal is formed on the fly; each warp updates
-      // whole columns c > j
-      for (int c = j + 1 + w; c < r; c += nw) {
-        double acc = double(0.0);
-        for (int i = lane; i < r; i += 32) acc += X2[i + j * ld] * X2[i + c * ld];
-        acc = (warp_sum_t(acc) * scal + X1[j + c * ld]) * tj;
-        if (lane == 0) X1[j + c * ld] -= acc;
-        const double f = acc * scal;
-        for (int i = lane; i < r; i += 32) X2[i + c * ld] -= f * X2[i + j * ld];
-      }
-    }
-    __syncthreads();
-    for (int i = tid; i < r; i += nth) X2[i + j * ld] *= scal;
-    __syncthreads();
-  }
-  double* Rn = R + (nleaf + node) * (int64_t)r * r;
-  for (int e = tid; e < r * r; e += nth) {
-    const int i = e % r, c = e / r;
-    Rn[e] = (i <= c) ? X1[i + c * ld] : double(0.0);
-    Eref[node * (int64_t)r * r + e] = X2[i + c * ld];
-  }
-}
-
 // Sc^{-T} (upper triangular) from the landmark Cholesky factor Sc (lower): X = Sc^{-1} by forward
 // substitution on all r columns at once, one CTA with Sc and the right-hand sides in shared
 // memory.  At step l the columns j <= l take x[l][j] = b[l][j] / Sc[l][l], then the rows i > l of
@@ -1063,20 +888,21 @@ static int sm_count() {
   return v;
 }
 
-// CTAs per node of the float-pair node kernel: the largest of 8, 4, 2 with nodes x csize <= the
-// SM count and at least one such cluster schedulable (checked once per size and device), else 1.
-// max_cs (the handle's setting) and KM_NODE_CLUSTER=1, 2, 4 or 8 cap it (1 gives the one-CTA
-// form).
-static int node_cluster_size(const void* fn, int64_t nodes, int threads, size_t smem, int max_cs) {
+// CTAs per node of the node kernels (form 0: FP64, 1: float pairs): the largest of 8, 4, 2 with
+// nodes x csize <= the SM count and at least one such cluster schedulable (checked once per form,
+// size and device), else 1.  max_cs (the handle's setting) and KM_NODE_CLUSTER=1, 2, 4 or 8 cap it
+// (1 gives the one-CTA form).
+static int node_cluster_size(int form, const void* fn, int64_t nodes, int threads, size_t smem, int max_cs) {
   static const int cap = [] {
     const char* e = std::getenv("KM_NODE_CLUSTER");
     const int v = e ? std::atoi(e) : 8;
     return v >= 8 ? 8 : v >= 4 ? 4 : v >= 2 ? 2 : 1;
   }();
   constexpr int kDevMax = 64;
-  // per device and size 1, 2, 4, 8: 0 unknown, 1 schedulable, -1 not (handles on several host
+  // per form, device and size 1, 2, 4, 8: 0 unknown, 1 schedulable, -1 not (handles on several host
   // threads may ask at once; a repeated query gives the same answer)
-  static std::atomic<int> ok[kDevMax][4];
+  static std::atomic<int> ok_of[2][kDevMax][4];
+  auto& ok = ok_of[form];
   const int nsm = sm_count();
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevMax) return 1;
@@ -1108,20 +934,26 @@ static int node_cluster_size(const void* fn, int64_t nodes, int threads, size_t 
 template <typename T>
 void launch_node_factor(T* R, const T* SinvT, int r, int level, const Tree& t, T* Ct, T* L22, T* Eref,
                         T* Etau, int* info, cudaStream_t st, int max_cluster, int wait_limit) {
-  const int64_t cbase = (level == 1) ? 0 : t.nleaf + t.node_off[level - 1];
-  const int64_t nbase = t.node_off[level];
   if constexpr (std::is_same<T, double>::value) {
-    const size_t sm = (size_t)4 * r * (r + 1) * sizeof(double);
-    smem_limit((const void*)k_node_factor_f64, sm);
-    k_node_factor_f64<<<(unsigned)t.nodes_at(level), 256, sm, st>>>(
-        reinterpret_cast<double*>(R), reinterpret_cast<const double*>(SinvT), r, level, t.L, t.nleaf, cbase, nbase,
-        reinterpret_cast<double*>(Ct), reinterpret_cast<double*>(L22), reinterpret_cast<double*>(Eref),
-        reinterpret_cast<double*>(Etau), info);
+    const size_t sm = node_f64_smem(r);
+    smem_limit(node_f64_kernel(), sm);
+    const int64_t nodes = t.nodes_at(level);
+    const int cs = node_cluster_size(0, node_f64_kernel(), nodes, 256, sm, max_cluster);
+    if (cs > 1) {
+      const cudaError_t prior = cudaPeekAtLastError();
+      if (launch_node_f64(R, SinvT, r, level, t, Ct, L22, Eref, Etau, info, cs, wait_limit, st) == cudaSuccess) return;
+      // the cluster launch was refused (nothing ran): one CTA per node instead; an error from
+      // before this launch stays for the caller
+      if (prior == cudaSuccess) cudaGetLastError();
+    }
+    launch_node_f64(R, SinvT, r, level, t, Ct, L22, Eref, Etau, info, 1, wait_limit, st);
   } else {
+    const int64_t cbase = (level == 1) ? 0 : t.nleaf + t.node_off[level - 1];
+    const int64_t nbase = t.node_off[level];
     const size_t sm = ((size_t)4 * r * (r + 1) + 3 * r) * sizeof(T) + (size_t)(r + 1) * sizeof(int);
     smem_limit((const void*)k_node_factor<T>, sm);
     const int64_t nodes = t.nodes_at(level);
-    const int cs = node_cluster_size((const void*)k_node_factor<T>, nodes, 1024, sm, max_cluster);
+    const int cs = node_cluster_size(1, (const void*)k_node_factor<T>, nodes, 1024, sm, max_cluster);
     if (cs > 1) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(nodes * cs));

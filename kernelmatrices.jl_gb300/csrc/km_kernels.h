@@ -127,6 +127,11 @@ template <typename T>
 // the first poll, the test of the timeout path); a wait that gives up sets info = -1
 void launch_node_factor(T* R, const T* SinvT, int r, int level, const Tree& t, T* Ct, T* L22, T* Eref, T* Etau,
                         int* info, cudaStream_t st, int max_cluster = 8, int wait_limit = -1);
+// FP64 node kernel (km_node64.cu) with cs CTAs per node; its shared memory and address
+cudaError_t launch_node_f64(double* R, const double* SinvT, int r, int level, const Tree& t, double* Ct, double* L22,
+                            double* Eref, double* Etau, int* info, int cs, int wait_limit, cudaStream_t st);
+size_t node_f64_smem(int r);
+const void* node_f64_kernel();
 template <typename T>
 void launch_leaf_formq(T* Pan, const T* tau, int r, const Tree& t, cudaStream_t st);
 template <typename T>

@@ -58,11 +58,16 @@ __device__ __forceinline__ double reduce4(double (&v)[4], int lane) {
 // (dlarfg: beta = -sign(alpha) ||.||).  The parts alternate between two buffers, so one barrier a
 // column is enough.
 __global__ void __launch_bounds__(kThreads) k_pqr_factor(const PanelDesc* __restrict__ descs, int j0,
-                                                         double* __restrict__ Ts, int nblk, int rs) {
+                                                         double* __restrict__ Ts, int nblk, int rs, int CS) {
   extern __shared__ double P[];
   __shared__ double part[2][kPB], top[2][kPB], tot[kPB], trow[kPB], T[kPB * kPB], G[kPB], refl[3];
-  cg::cluster_group cl = cg::this_cluster();
-  const int CS = (int)cl.num_blocks(), g = (int)cl.block_rank();
+  // (a panel of one CTA is a plain launch: no cluster operations)
+  const int g = (int)(blockIdx.x % CS);
+  auto team_sync = [&]() {
+    if (CS == 1) __syncthreads();
+    else cg::this_cluster().sync();
+  };
+  auto at = [&](double* p, int q) { return CS == 1 ? p : cg::this_cluster().map_shared_rank(p, q); };
   const PanelDesc D = descs[blockIdx.x / CS];
   if (D.big || j0 >= D.k) return;  // the whole cluster leaves
   const int jb = min(kPB, D.k - j0), M = (int)D.m - j0;
@@ -95,18 +100,18 @@ __global__ void __launch_bounds__(kThreads) k_pqr_factor(const PanelDesc* __rest
     }
     const bool own = j >= lo && j < lo + n;
     if (own && tid < jb) tp[tid] = P[tid * ldp + j - lo];
-    cl.sync();
+    team_sync();
     {
       // 8 lanes per column add the CTAs' parts
       const int c = tid >> 3, p = tid & 7;
       double s = 0.0;
       if (c < jb)
-        for (int q = p; q < CS; q += 8) s += cl.map_shared_rank(pt, q)[c];
+        for (int q = p; q < CS; q += 8) s += at(pt, q)[c];
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (p == 0 && c < jb) {
         tot[c] = s;
-        trow[c] = cl.map_shared_rank(tp, j / rs)[c];
+        trow[c] = at(tp, j / rs)[c];
       }
     }
     __syncthreads();
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(kThreads) k_pqr_factor(const PanelDesc* __rest
       out[kPB * kPB + e] = z;
     }
   }
-  cl.sync();  // no CTA leaves while another may still read its parts
+  team_sync();  // no CTA leaves while another may still read its parts
 }
 
 // Entry (i, p) of the block's V, rows counted from j0
@@ -370,8 +375,8 @@ int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, doubl
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim = {(unsigned)cs, 1, 1};
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_pqr_factor, descs, j0, Ts, nblk, rs);
+    cfg.numAttrs = cs > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k_pqr_factor, descs, j0, Ts, nblk, rs, cs);
     ++launches;
     const int nt = kmax - j0 - kPB;
     if (nt > 0) apply(j0, nt, 1);
