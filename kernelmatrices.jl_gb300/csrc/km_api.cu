@@ -424,11 +424,12 @@ bool run_launch(km_handle* h, int cls, F&& f) {
 #define KL(h, cls, expr) run_launch(h, cls, [&]() -> bool { return (expr); })
 #define KLV(h, cls, expr) run_launch(h, cls, [&]() -> bool { expr; return true; })
 
-// FP64 leaf Cholesky, d_K into d_Lf; false if a leaf is too large
-bool leaf_chol_f64(km_handle* h) {
+// FP64 leaf Cholesky, d_K into d_Lf, and with r > 0 the leaf panels L^{-1} Phi, d_Phi into d_Q;
+// false if a leaf is too large
+bool leaf_chol_f64(km_handle* h, int r) {
   int n = 0;
-  const bool ok = KL(h, KM_PROF_LEAF_CHOL,
-                     (n = launch_leaf_chol_f64(h->d_K, h->d_Lf, h->tree, h->d_info, h->stream)) > 0);
+  const bool ok = KL(h, KM_PROF_LEAF_CHOL, (n = launch_leaf_chol_f64(h->d_K, h->d_Lf, h->d_Phi, h->d_Q, r, h->tree,
+                                                                     h->d_info, h->stream)) > 0);
   h->stats.kernel_launches += n - 1;
   return ok;
 }
@@ -1445,7 +1446,7 @@ static int general_factorize(km_handle* h) {
   int rc;
   timer_start(h);
   KM_CUDA(h, cudaMemsetAsync(h->d_info, 0, sizeof(int) * (t.nleaf + nb + 1), st));  // + grid-barrier word
-  if (!leaf_chol_f64(h))
+  if (!leaf_chol_f64(h, 0))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the leaf Cholesky kernel");
   if (nb > 0) {
     // leaf triangular solves of every panel (invapply!, src/HODLR/src/utils.jl:54-65)
@@ -1771,7 +1772,7 @@ static int factorize_launches(km_handle* h) {
     }
     if (fwd) aux_fwd_leaf<ff>(h);
   } else if (!(h->mixed ? KL(h, KM_PROF_LEAF_CHOL, launch_leaf_chol<ff>(h->d_K, P<ff>(h->d_Lf), t, h->d_info, st))
-                        : leaf_chol_f64(h))) {
+                        : leaf_chol_f64(h, leaf_chol_f64_solves(t) ? r : 0))) {
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the leaf Cholesky kernel");
   }
   // A = L^{-1} Phi on every leaf, then Householder QR of each leaf panel
@@ -1807,9 +1808,11 @@ static int factorize_launches(km_handle* h) {
     }
     if (fwd) aux_fwd_nodes<ff>(h);
   } else {
-    KM_CUDA(h, cudaMemcpyAsync(h->d_Q, h->d_Phi, sizeof(double) * t.n * r, cudaMemcpyDeviceToDevice, st));
-    if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 0, h->d_Q, r, 0, 1, h->d_Q, r, 0, 1, r, st)))
-      return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
+    if (!leaf_chol_f64_solves(t)) {
+      KM_CUDA(h, cudaMemcpyAsync(h->d_Q, h->d_Phi, sizeof(double) * t.n * r, cudaMemcpyDeviceToDevice, st));
+      if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 0, h->d_Q, r, 0, 1, h->d_Q, r, 0, 1, r, st)))
+        return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
+    }
     if (fwd) aux_fwd_leaf<double>(h);
     if (t.L > 0) {
       KLV(h, KM_PROF_LEAF_QR, launch_leaf_qr<double>(h->d_Q, r, t, h->d_tauleaf, h->d_R, st));

@@ -6,7 +6,9 @@
 // leaf left 2 leaves of 500 points on 2 SMs for 7.2 ms and 64 leaves of 469 on 64 SMs for 6.1 ms.
 // Here a step solves the rows below its NB x NB diagonal block (k_chol_panel), then updates the
 // trailing triangle in 32 x 32 tiles, one CTA each, the first of which also factors the next
-// diagonal block (k_chol_update).  Measured: 2 leaves of 500
+// diagonal block (k_chol_update).  The Nystrom panel rides along: A = L^{-1} Phi by the same steps
+// on the r columns of Phi (a separate solve kernel took 1.6 ms for 256 leaves of 256 points, rank 72,
+// a third of it in 32-step substitutions with one useful lane at a time).  Measured: 2 leaves of 500
 // 7.21 -> 1.84 ms, 64 of 469 6.14 -> 3.5 ms, 256 of 256 2.85 -> 2.19 ms.
 //
 // Every element sees the operations of the blocked right-looking algorithm in the same order
@@ -14,6 +16,7 @@
 // division by its pivot; a trailing element takes one fused multiply-add chain per step,
 // subtracted once.  The factor's bits do not depend on the number of CTAs.
 #include <algorithm>
+#include <climits>
 
 #include "km_kernels.h"
 
@@ -29,118 +32,178 @@ struct CholMat {
   const double* in;
   double* out;
   int m;
+  const double* pin;  // r columns of length m to be solved with the factor (read at step 0, then
+  double* pout;       // from pout; leading dimension m): A = L^{-1} Phi
 };
 
 struct LeafMats {
   const double* K;
   double* Lf;
+  const double* Phi;
+  double* A;
+  int r;
   DTree t;
   __device__ CholMat operator()(int64_t j) const {
-    const int64_t off = d_leaf_koff(t, j);
-    return CholMat{K + off, Lf + off, d_leaf_size(t, j)};
+    const int64_t off = d_leaf_koff(t, j), s = d_leaf_start(t, j) * r;
+    return CholMat{K + off, Lf + off, d_leaf_size(t, j), Phi + s, A + s};
   }
 };
 
-// Cholesky factor of the NB x NB diagonal block at column k0 by one warp, a row per lane in
-// registers: the pivot and the multipliers travel by shuffles, no barrier (about 8 us at NB = 32,
-// a chain of NB square roots and divisions).  d: row `lane` of the block, columns <= lane.
+// Cholesky factor of the NB x NB diagonal block at column k0, entries in D (row-major, leading
+// dimension NB + 1, lower triangle), by 4 warps, lane = row.  Warp w updates the columns c = w mod 4
+// (each quarter of the SM has its own FP64 pipe); the warp of the next column updates it first and
+// forms its square root and divisions while the others are still updating: one barrier a column.
+// The loops stay rolled: with the block in registers of one warp the unrolled code, run once,
+// waited for its own instructions (58 us for 32 columns, now @D@ us: NB times a square root, a
+// division and an update).
 template <int NB>
-__device__ void chol_diag(double (&d)[NB], const CholMat& M, int k0, int* __restrict__ info) {
-  const int lane = threadIdx.x & 31, m = M.m, kb = min(NB, m - k0);
-  int bad = 0;
-#pragma unroll
-  for (int j = 0; j < NB; ++j) {
-    if (j < kb) {
-      const double p = __shfl_sync(0xffffffffu, d[j], j);
-      const bool ok = p > 0.0;
-      if (!ok && bad == 0) bad = k0 + j + 1;
-      const double sd = ok ? sqrt(p) : 1.0;
-      d[j] = lane == j ? sd : d[j] / sd;
-#pragma unroll
-      for (int c = j + 1; c < NB; ++c) d[c] = __fma_rn(-d[j], __shfl_sync(0xffffffffu, d[j], c), d[c]);
+__device__ void chol_diag(double* D, const CholMat& M, int k0, int* __restrict__ info) {
+  constexpr int LD = NB + 1;
+  __shared__ int first_bad;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m = M.m, kb = min(NB, m - k0);
+  // column j (updated value y of row `lane`) into its final form
+  auto finish = [&](int j, double y) {
+    const double p = __shfl_sync(0xffffffffu, y, j);
+    const bool ok = p > 0.0;
+    if (!ok && lane == 0) atomicMin(&first_bad, k0 + j + 1);
+    const double sd = ok ? sqrt(p) : 1.0;
+    // (a zero numerator in an idle lane would send the warp through the slow division)
+    const bool below = lane > j && lane < kb;
+    const double x = below ? y : 1.0;
+    const double v = x / sd;
+    if (below || lane == j) D[lane * LD + j] = below ? v : sd;
+  };
+  if (threadIdx.x == 0) first_bad = INT_MAX;
+  __syncthreads();
+  if (w == 0) finish(0, lane < kb ? D[lane * LD] : 0.0);
+  __syncthreads();
+  for (int j = 0; j < kb; ++j) {
+    const bool live = lane >= j && lane < kb;
+    const double x = live ? D[lane * LD + j] : 0.0;
+    if (w == (j & 3) && live) M.out[(int64_t)(k0 + j) * m + k0 + lane] = x;
+    int c = j + 1 + ((w - j - 1) & 3);
+    if (c == j + 1 && c < kb) {
+      finish(c, lane >= c && lane < kb ? __fma_rn(-x, D[c * LD + j], D[lane * LD + c]) : 0.0);
+      c += 4;
     }
+    for (; c < kb; c += 4)
+      if (lane >= c && lane < kb) D[lane * LD + c] = __fma_rn(-x, D[c * LD + j], D[lane * LD + c]);
+    __syncthreads();
   }
-  if (lane < kb) {
-#pragma unroll
-    for (int c = 0; c < NB; ++c)
-      if (c <= lane) M.out[(int64_t)(k0 + c) * m + k0 + lane] = d[c];
-  }
-  if (lane == 0 && bad && *info == 0) *info = bad;
+  if (threadIdx.x == 0 && first_bad != INT_MAX && *info == 0) *info = first_bad;
 }
 
 template <typename Mats, int NB>
-__global__ void __launch_bounds__(32) k_chol_first(Mats mats, int* __restrict__ info) {
-  const CholMat M = mats(blockIdx.x);
-  const int lane = threadIdx.x, kb = min(NB, M.m);
-  double d[NB];
-#pragma unroll
-  for (int c = 0; c < NB; ++c) d[c] = (c <= lane && lane < kb) ? M.in[(int64_t)c * M.m + lane] : 0.0;
-  chol_diag<NB>(d, M, 0, info + blockIdx.x);
-}
-
-// Rows below the diagonal block at column k0: x D' = a, grid (matrix, row chunk), a row per thread.
-template <typename Mats, int NB>
-__global__ void __launch_bounds__(128) k_chol_panel(Mats mats, int k0) {
+__global__ void __launch_bounds__(128) k_chol_first(Mats mats, int* __restrict__ info) {
   __shared__ double D[NB * (NB + 1)];
+  const CholMat M = mats(blockIdx.x);
+  const int lane = threadIdx.x & 31, kb = min(NB, M.m);
+  for (int c = threadIdx.x >> 5; c < kb; c += 4)
+    if (lane >= c && lane < kb) D[lane * (NB + 1) + c] = M.in[(int64_t)c * M.m + lane];
+  __syncthreads();
+  chol_diag<NB>(D, M, 0, info + blockIdx.x);
+}
+
+// Rows below the diagonal block at column k0: x D' = a, and the block's rows of the r solved columns
+// (their transposes are rows of the same kind): grid (matrix, 32-row chunk; the first `nrow` chunks
+// below the block, then those of the columns), 4 warps, lane = row.  Warp l mod 4 finishes column
+// l; every warp updates every fourth column, so the warp that finishes column l + 1 is the one that
+// updated it: one barrier a column.  The rows of the factor divide by the pivot, the solved columns
+// multiply by its reciprocal, as the triangular solve kernel does.
+template <typename Mats, int NB>
+__global__ void __launch_bounds__(128) k_chol_panel(Mats mats, int k0, int nrow, int r) {
+  __shared__ double D[NB * (NB + 1)], V[32 * (NB + 1)], inv[NB];
   constexpr int LD = NB + 1;
   const CholMat M = mats(blockIdx.x);
-  const int m = M.m, row0 = k0 + NB + (int)(blockIdx.y * blockDim.x);
-  if (row0 >= m) return;  // the block has all NB columns: rows exist below it
-  const double* src = k0 == 0 ? M.in : M.out;
-  const int i = row0 + threadIdx.x;
-  double v[NB];
-#pragma unroll
-  for (int c = 0; c < NB; ++c) v[c] = i < m ? src[(int64_t)(k0 + c) * m + i] : 0.0;
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    const int r = e % NB, c = e / NB;
-    if (r >= c) D[r * LD + c] = M.out[(int64_t)(k0 + c) * m + k0 + r];
+  const int m = M.m, kb = min(NB, m - k0);
+  const bool solve = (int)blockIdx.y >= nrow;
+  const int row0 = solve ? ((int)blockIdx.y - nrow) * 32 : k0 + NB + (int)blockIdx.y * 32;
+  if (kb <= 0 || (!solve && row0 >= m)) return;  // (rows below the block: it has all NB columns)
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = row0 + lane;
+  double* v = V + lane * LD;
+  if (solve) {
+    const double* src = k0 == 0 ? M.pin : M.pout;
+    for (int q = w; q < 32; q += 4)
+      if (lane < kb) V[q * LD + lane] = row0 + q < r ? src[(int64_t)(row0 + q) * m + k0 + lane] : 1.0;
+    if (w == 0 && lane < kb) inv[lane] = 1.0 / M.out[(int64_t)(k0 + lane) * m + k0 + lane];
+  } else {
+    const double* src = k0 == 0 ? M.in : M.out;
+    for (int c = w; c < NB; c += 4) v[c] = i < m ? src[(int64_t)(k0 + c) * m + i] : 1.0;
   }
+  for (int c = w; c < kb; c += 4)
+    if (lane >= c && lane < kb) D[lane * LD + c] = M.out[(int64_t)(k0 + c) * m + k0 + lane];
   __syncthreads();
-  if (i >= m) return;
-#pragma unroll
-  for (int l = 0; l < NB; ++l) {
-    v[l] /= D[l * LD + l];
-#pragma unroll
-    for (int c = l + 1; c < NB; ++c) v[c] = __fma_rn(-v[l], D[c * LD + l], v[c]);
+  if (w == 0) v[0] = solve ? __dmul_rn(v[0], inv[0]) : v[0] / D[0];
+  __syncthreads();
+  for (int l = 0; l < kb; ++l) {
+    const double x = v[l];
+    if (w == (l & 3) && !solve && i < m) M.out[(int64_t)(k0 + l) * m + i] = x;
+    int c = l + 1 + ((w - l - 1) & 3);
+    if (c == l + 1 && c < kb) {  // the next column first
+      const double y = __fma_rn(-x, D[c * LD + l], v[c]);
+      v[c] = solve ? __dmul_rn(y, inv[c]) : y / D[c * LD + c];
+      c += 4;
+    }
+    for (; c < kb; c += 4) v[c] = __fma_rn(-x, D[c * LD + l], v[c]);
+    __syncthreads();
   }
-#pragma unroll
-  for (int c = 0; c < NB; ++c) M.out[(int64_t)(k0 + c) * m + i] = v[c];
+  if (solve)
+    for (int q = w; q < 32; q += 4)
+      if (lane < kb && row0 + q < r) M.pout[(int64_t)(row0 + q) * m + k0 + lane] = V[q * LD + lane];
 }
 
-// Trailing update A[i, c] -= sum_l P[i, l] P[c, l] of one 32 x 32 tile, P the step's panel rows:
-// grid (tile of the lower triangle, matrix), 128 threads with 2 x 4 outputs each.  The CTA of the
-// first tile goes on to factor the next diagonal block, which lies inside it.
+// Trailing update of one 32 x 32 tile: A[i, c] -= sum_l P[i, l] P[c, l] of the lower triangle (P the
+// step's panel rows), or A[i, q] -= sum_l P[i, l] X[l, q] of the solved columns (X their rows of the
+// step): grid (tile; the ntri tiles of the triangle, then row tiles x column tiles, matrix), 128
+// threads with 2 x 4 outputs each.  The CTA of the first tile goes on to factor the next diagonal
+// block, which lies inside it.
 template <typename Mats, int NB>
-__global__ void __launch_bounds__(128) k_chol_update(Mats mats, int k0, int* __restrict__ info) {
+__global__ void __launch_bounds__(128) k_chol_update(Mats mats, int k0, int ntri, int nb, int r, int* __restrict__ info) {
   __shared__ double Pi[kTile * (NB + 1)], Pc[kTile * (NB + 1)];
   constexpr int LD = NB + 1;
   const CholMat M = mats(blockIdx.y);
   const int m = M.m, r0 = k0 + NB, mr = m - r0;
-  int bi = (int)((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
-  while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
-  while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
-  const int bc = blockIdx.x - bi * (bi + 1) / 2;
+  const bool solve = (int)blockIdx.x >= ntri;
+  int bi, bc;
+  if (solve) {
+    bc = ((int)blockIdx.x - ntri) / nb;
+    bi = (int)blockIdx.x - ntri - bc * nb;
+  } else {
+    bi = (int)((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
+    while (bi * (bi + 1) / 2 > (int)blockIdx.x) --bi;
+    while ((bi + 1) * (bi + 2) / 2 <= (int)blockIdx.x) ++bi;
+    bc = blockIdx.x - bi * (bi + 1) / 2;
+  }
   if (bi * kTile >= mr) return;
-  const int i0 = r0 + bi * kTile, c0 = r0 + bc * kTile;
-  const double* src = k0 == 0 ? M.in : M.out;
+  const int i0 = r0 + bi * kTile, c0 = solve ? bc * kTile : r0 + bc * kTile;
+  const int clim = solve ? r : m;
+  const double* src = solve ? (k0 == 0 ? M.pin : M.pout) : (k0 == 0 ? M.in : M.out);
+  double* dst = solve ? M.pout : M.out;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   for (int l = w; l < NB; l += 4) {
     const double* col = M.out + (int64_t)(k0 + l) * m;
     Pi[lane * LD + l] = i0 + lane < m ? col[i0 + lane] : 0.0;
-    Pc[lane * LD + l] = c0 + lane < m ? col[c0 + lane] : 0.0;
+    if (!solve) Pc[lane * LD + l] = c0 + lane < m ? col[c0 + lane] : 0.0;
   }
+  if (solve)
+    for (int q = w; q < kTile; q += 4)
+      if (lane < NB) Pc[q * LD + lane] = c0 + q < r ? M.pout[(int64_t)(c0 + q) * m + k0 + lane] : 0.0;
   const int ti = tid & 15, tc = tid >> 4;
+  // columns tc + 8 q: those beyond the last, and the half of a diagonal tile above the diagonal
+  // (rows below 16, columns from 16 on), are left out
+  const int nq = min(4, (clim - c0 + 7) / 8);
+  const bool diag = !solve && bi == bc;
   double a[2][4];
 #pragma unroll
   for (int p = 0; p < 2; ++p)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = i0 + ti + 16 * p, c = c0 + tc + 8 * q;
-      a[p][q] = (i < m && i >= c) ? src[(int64_t)c * m + i] : 0.0;
+      a[p][q] = (i < m && c < clim && (solve || i >= c)) ? src[(int64_t)c * m + i] : 0.0;
     }
   __syncthreads();
   double acc[2][4] = {};
-#pragma unroll 8
+#pragma unroll 4
   for (int l = 0; l < NB; ++l) {
     double x[2], y[4];
 #pragma unroll
@@ -148,17 +211,19 @@ __global__ void __launch_bounds__(128) k_chol_update(Mats mats, int k0, int* __r
 #pragma unroll
     for (int q = 0; q < 4; ++q) y[q] = Pc[(tc + 8 * q) * LD + l];
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[p][q] = __fma_rn(x[p], y[q], acc[p][q]);
+    for (int q = 0; q < 4; ++q)
+      if (q < nq) {
+        if (!(diag && q >= 2)) acc[0][q] = __fma_rn(x[0], y[q], acc[0][q]);
+        acc[1][q] = __fma_rn(x[1], y[q], acc[1][q]);
+      }
   }
 #pragma unroll
   for (int p = 0; p < 2; ++p)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = i0 + ti + 16 * p, c = c0 + tc + 8 * q;
-      a[p][q] -= acc[p][q];
-      if (i < m && i >= c) M.out[(int64_t)c * m + i] = a[p][q];
+      a[p][q] = __dsub_rn(a[p][q], acc[p][q]);
+      if (i < m && c < clim && (solve || i >= c)) dst[(int64_t)c * m + i] = a[p][q];
     }
   if (blockIdx.x > 0) return;
   __syncthreads();
@@ -168,26 +233,25 @@ __global__ void __launch_bounds__(128) k_chol_update(Mats mats, int k0, int* __r
     for (int q = 0; q < 4; ++q)
       if (tc + 8 * q < NB) Pi[(ti + 16 * p) * LD + tc + 8 * q] = a[p][q];
   __syncthreads();
-  if (w > 0) return;
-  const int kb = min(NB, mr);
-  double d[NB];
-#pragma unroll
-  for (int c = 0; c < NB; ++c) d[c] = (c <= lane && lane < kb) ? Pi[lane * LD + c] : 0.0;
-  chol_diag<NB>(d, M, r0, info + blockIdx.y);
+  chol_diag<NB>(Pi, M, r0, info + blockIdx.y);
 }
 
 template <typename Mats, int NB>
-int chol_steps(const Mats& mats, int64_t nmat, int mmax, int* info, cudaStream_t st) {
+int chol_steps(const Mats& mats, int64_t nmat, int mmax, int r, int* info, cudaStream_t st) {
   int launches = 1;
-  k_chol_first<Mats, NB><<<(unsigned)nmat, 32, 0, st>>>(mats, info);
-  for (int k0 = 0; k0 + NB < mmax; k0 += NB) {
-    const int rows = mmax - k0 - NB, nb = (rows + kTile - 1) / kTile;
-    // one warp per CTA while that gives at most four CTAs an SM, so that the rows of few matrices
-    // are solved by many SMs
-    const int nt = nmat * ((rows + 31) / 32) <= 4 * 152 ? 32 : 128;
-    k_chol_panel<Mats, NB><<<dim3((unsigned)nmat, (unsigned)((rows + nt - 1) / nt)), nt, 0, st>>>(mats, k0);
-    k_chol_update<Mats, NB><<<dim3((unsigned)(nb * (nb + 1) / 2), (unsigned)nmat), 128, 0, st>>>(mats, k0, info);
-    launches += 2;
+  k_chol_first<Mats, NB><<<(unsigned)nmat, 128, 0, st>>>(mats, info);
+  for (int k0 = 0; k0 < mmax; k0 += NB) {
+    const int rows = std::max(mmax - k0 - NB, 0), nb = (rows + kTile - 1) / kTile, nr = (r + 31) / 32;
+    if (nb + nr > 0) {
+      k_chol_panel<Mats, NB><<<dim3((unsigned)nmat, (unsigned)(nb + nr)), 128, 0, st>>>(mats, k0, nb, r);
+      ++launches;
+    }
+    if (nb > 0) {
+      const int ntri = nb * (nb + 1) / 2;
+      k_chol_update<Mats, NB><<<dim3((unsigned)(ntri + nb * nr), (unsigned)nmat), 128, 0, st>>>(mats, k0, ntri, nb, r,
+                                                                                               info);
+      ++launches;
+    }
   }
   return launches;
 }
@@ -236,7 +300,7 @@ __global__ void __launch_bounds__(256) k_gnode_product(const GNodeDesc* __restri
 
 struct NodeMats22 {
   const GNodeDesc* nodes;
-  __device__ CholMat operator()(int64_t q) const { return CholMat{nodes[q].L22, nodes[q].L22, nodes[q].r}; }
+  __device__ CholMat operator()(int64_t q) const { return CholMat{nodes[q].L22, nodes[q].L22, nodes[q].r, nullptr, nullptr}; }
 };
 
 }  // namespace
@@ -248,18 +312,28 @@ int launch_gnode(const GNodeDesc* nodes, int n, int maxr, int* info, cudaStream_
   const unsigned nt = (unsigned)((maxr + 31) / 32);
   k_gnode_product<false><<<dim3(nt, nt, (unsigned)n), 256, 0, st>>>(nodes);
   k_gnode_product<true><<<dim3(nt, nt, (unsigned)n), 256, 0, st>>>(nodes);
-  return 2 + chol_steps<NodeMats22, 32>(NodeMats22{nodes}, n, maxr, info, st);
+  return 2 + chol_steps<NodeMats22, 32>(NodeMats22{nodes}, n, maxr, 0, info, st);
 }
 
-int launch_leaf_chol_f64(const double* K, double* Lf, const Tree& t, int* info, cudaStream_t st) {
-  const LeafMats mats{K, Lf, dtree(t)};
+// block widths and size limit of the shared-memory panel (m + NB) x (NB + 1) of the one-CTA kernel
+// that float pairs use: a wider block at the same size would round differently
+static int leaf_chol_width(int64_t m) {
+  for (int64_t nb : {32, 16, 8})
+    if ((m + nb) * (nb + 1) * (int64_t)sizeof(double) <= 200 * 1024) return (int)nb;
+  return 0;
+}
+
+bool leaf_chol_f64_solves(const Tree& t) { return leaf_chol_width(t.max_leaf) == 32; }
+
+int launch_leaf_chol_f64(const double* K, double* Lf, const double* Phi, double* A, int r, const Tree& t, int* info,
+                         cudaStream_t st) {
+  const LeafMats mats{K, Lf, Phi, A, r, dtree(t)};
   const int m = (int)t.max_leaf;
-  // block widths and size limit of the shared-memory panel (m + NB) x (NB + 1) of the one-CTA
-  // kernel that float pairs use: a wider block at the same size would round differently
-  auto fits = [&](int64_t nb) { return (m + nb) * (nb + 1) * (int64_t)sizeof(double) <= 200 * 1024; };
-  if (fits(32)) return chol_steps<LeafMats, 32>(mats, t.nleaf, m, info, st);
-  if (fits(16)) return chol_steps<LeafMats, 16>(mats, t.nleaf, m, info, st);
-  if (fits(8)) return chol_steps<LeafMats, 8>(mats, t.nleaf, m, info, st);
+  switch (leaf_chol_width(m)) {
+    case 32: return chol_steps<LeafMats, 32>(mats, t.nleaf, m, r, info, st);
+    case 16: return chol_steps<LeafMats, 16>(mats, t.nleaf, m, 0, info, st);
+    case 8: return chol_steps<LeafMats, 8>(mats, t.nleaf, m, 0, info, st);
+  }
   return 0;
 }
 

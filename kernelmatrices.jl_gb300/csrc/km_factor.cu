@@ -889,8 +889,9 @@ static int sm_count() {
 }
 
 // CTAs per node of the node kernels (form 0: FP64, 1: float pairs): the largest of 8, 4, 2 with
-// nodes x csize <= the SM count and at least one such cluster schedulable (checked once per form,
-// size and device), else 1.  max_cs (the handle's setting) and KM_NODE_CLUSTER=1, 2, 4 or 8 cap it
+// nodes x csize <= the SM count and as many such clusters schedulable at once (asked once per form,
+// size and device: clusters do not straddle the groups that SMs come in, so 16 of 8 may not fit
+// 152 SMs), else 1.  max_cs (the handle's setting) and KM_NODE_CLUSTER=1, 2, 4 or 8 cap it
 // (1 gives the one-CTA form).
 static int node_cluster_size(int form, const void* fn, int64_t nodes, int threads, size_t smem, int max_cs) {
   static const int cap = [] {
@@ -899,17 +900,18 @@ static int node_cluster_size(int form, const void* fn, int64_t nodes, int thread
     return v >= 8 ? 8 : v >= 4 ? 4 : v >= 2 ? 2 : 1;
   }();
   constexpr int kDevMax = 64;
-  // per form, device and size 1, 2, 4, 8: 0 unknown, 1 schedulable, -1 not (handles on several host
-  // threads may ask at once; a repeated query gives the same answer)
-  static std::atomic<int> ok_of[2][kDevMax][4];
-  auto& ok = ok_of[form];
+  // per form, device, size 1, 2, 4, 8 and whether a CTA takes more than half an SM's shared memory:
+  // clusters at once, 0 unknown, -1 none (handles on several host threads may ask at once; a
+  // repeated query gives the same answer)
+  static std::atomic<int> room[2][kDevMax][4][2];
   const int nsm = sm_count();
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevMax) return 1;
   const int top = std::min(cap, max_cs);
   for (int cs = top, lg = top >= 8 ? 3 : top == 4 ? 2 : top == 2 ? 1 : 0; cs > 1; cs >>= 1, --lg) {
     if (nodes * cs > nsm) continue;
-    if (ok[dev][lg].load() == 0) {
+    std::atomic<int>& n = room[form][dev][lg][smem > 113 * 1024];
+    if (n.load() == 0) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)cs);
       cfg.blockDim = dim3((unsigned)threads);
@@ -924,9 +926,9 @@ static int node_cluster_size(int form, const void* fn, int64_t nodes, int thread
       int nclusters = 0;
       const cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, fn, &cfg);
       if (e != cudaSuccess) cudaGetLastError();  // clear the query's error; the size is not used
-      ok[dev][lg].store((e == cudaSuccess && nclusters > 0) ? 1 : -1);
+      n.store((e == cudaSuccess && nclusters > 0) ? nclusters : -1);
     }
-    if (ok[dev][lg].load() > 0) return cs;
+    if (n.load() >= nodes) return cs;
   }
   return 1;
 }

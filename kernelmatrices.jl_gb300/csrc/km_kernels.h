@@ -96,7 +96,11 @@ template <typename T>
 bool launch_leaf_chol(const double* K, T* Lf, const Tree& t, int* info, cudaStream_t st);
 // FP64 leaf Cholesky over all SMs (km_chol.cu): lower triangles of Lf only; info zero on entry.
 // Returns the number of kernels launched, 0 if a leaf is too large.
-int launch_leaf_chol_f64(const double* K, double* Lf, const Tree& t, int* info, cudaStream_t st);
+// With r > 0 also A = L^{-1} Phi for the leaf panels (m x r, column-major), for trees where
+// leaf_chol_f64_solves (the block width is that of the triangular solve kernel).
+int launch_leaf_chol_f64(const double* K, double* Lf, const double* Phi, double* A, int r, const Tree& t, int* info,
+                         cudaStream_t st);
+bool leaf_chol_f64_solves(const Tree& t);
 template <typename T>
 bool launch_leaf_tri(const T* Lf, const Tree& t, int op, T* Bptr, int64_t bmul, int64_t bld, int bld_is_m, T* Xptr,
                      int64_t xmul, int64_t xld, int xld_is_m, int ncols, cudaStream_t st);

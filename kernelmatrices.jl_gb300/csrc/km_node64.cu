@@ -10,16 +10,20 @@
 // 65 k such instructions, so one CTA per node took 1.05 ms whatever the level, and the levels
 // with fewer nodes than SMs left the others idle.  Here a node is a cluster of up to 8 CTAs:
 //   products       (column, 32-row chunk) items over all warps of the cluster; T1, T2 and Ct are
-//                  stored into every CTA's shared memory, H = I - Ct'Ct (lower half only) into CTA 0
-//   Cholesky       CTA 0, in dataflow order over (column, chunk) items: the square root of a column
-//                  and the divisions of its chunks run on different quarters
-//   L22^{-1} B     every CTA on its own columns c = rank, rank + CTAs, ...
+//                  stored into every CTA's shared memory; column c of H = I - Ct'Ct (lower half
+//                  only) and of B = R2 - Ct'R1 belongs to CTA c mod CTAs
+//   Cholesky       by columns in dataflow order, (column, chunk) items: a chunk takes the earlier
+//                  columns as they arrive, the chunk with the pivot publishes its square root, and
+//                  every chunk divides by it and goes to all CTAs with asynchronous stores that
+//                  complete a barrier there (no fence, no cluster barrier)
+//   L22^{-1} B     every CTA on its own columns, a step per row
 //   QR             a warp owns its columns; the warp of column j + 1 applies reflector j to that
-//                  column first, forms reflector j + 1 and sends it to every CTA with asynchronous
-//                  stores that complete a barrier there (no fence, no cluster barrier), then applies
+//                  column first, forms reflector j + 1 and sends it in the same way, then applies
 //                  reflector j to its other columns, four at a time so that their dot products
-//                  share the additions over the lanes
-// Rank 72, time per level: 1.05 ms -> @A@ ms with 8 CTAs a node (up to 19 nodes), @B@ ms with one.
+//                  share the additions over the lanes.  One warp per quarter of the SM where the
+//                  column chain bounds it (several CTAs a node), two where the FP64 pipe does.
+// Rank 72, time per level: 1.05 ms -> @A@ ms with 8 CTAs a node, @B@ ms with one.  (Cholesky in CTA 0
+// alone, where its chunks compete for four quarters, took 286 k cycles against @C@ k.)
 //
 // Every number is formed by the operations of the one-CTA kernel in the same order (dot products by
 // row chunks of 32 and a butterfly over the lanes, updates one fused multiply-add at a time), so the
@@ -62,7 +66,7 @@ __device__ __forceinline__ bool bar_try(unsigned bar, int cs) {
   if (cs > 1)
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar)
@@ -70,7 +74,7 @@ __device__ __forceinline__ bool bar_try(unsigned bar, int cs) {
   else
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar)
@@ -120,6 +124,13 @@ __device__ __forceinline__ double reduce4(double (&v)[4], int lane) {
   return s;
 }
 
+// d > 0, d != 0 on the bits: an FP64 comparison would take the FP64 pipe for 65 cycles
+__device__ __forceinline__ bool positive(double d) {
+  const long long b = __double_as_longlong(d);
+  return b > 0 && b <= 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool nonzero(double d) { return (__double_as_longlong(d) << 1) != 0; }
+
 __device__ __forceinline__ double butterfly(double s) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
@@ -136,18 +147,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
                                                               int wait_limit) {
   extern __shared__ __align__(16) double sm[];
   const int ld = r + 1;
-  double* X0 = sm;            // Sc^{-T}, then Ct
+  double* X0 = sm;            // Sc^{-T}, then Ct; then G: L22^{-1} B, the updated columns, the reflectors
   double* X1 = X0 + r * ld;   // R1, then T2, then the own columns of R1 (of R_N in the end)
-  double* X2 = X1 + r * ld;   // R2; own columns: B, L22^{-1} B, the updated columns; sent reflectors
-  double* X3 = X2 + r * ld;   // T1, then H and L22
+  double* X2 = X1 + r * ld;   // R2, then the own columns of B
+  double* X3 = X2 + r * ld;   // T1, then the own columns of H, then L22
   double* va = X3 + r * ld;   // pivots of L22, then the betas
   double* vb = va + r;        // reflector scales
   double* vc = vb + r;        // reflector taus
   double* vi = vc + r;        // 1 / L22[j][j] (not va: another CTA's betas may arrive during the solve)
   unsigned long long* bars = reinterpret_cast<unsigned long long*>(vi + r);  // reflector j has arrived
-  volatile int* fl = reinterpret_cast<volatile int*>(bars + r);              // 3 r: chunk (c, s) of L22 is final
-  volatile int* fd = fl + 3 * r;                                             // r: pivot of column c is known
-  __shared__ int sh_bad;
+  unsigned long long* cols = bars + r;  // 3 r: chunk s of column c of L22 (entry 3 c + s) has arrived
+  volatile int* fd = reinterpret_cast<volatile int*>(cols + 3 * r);  // r: pivot of an own column is known
+  __shared__ int sh_bad[8];   // of CTA 0: first non-positive pivot found by each CTA
+  __shared__ int my_bad;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int rank = (int)(blockIdx.x % cs);
   const int64_t k = blockIdx.x / cs, node = nbase + k;
@@ -163,14 +175,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
       X1[i + c * ld] = R1[e];
       X2[i + c * ld] = R2[e];
     }
-  for (int e = tid; e < 4 * r; e += kThreads) fl[e] = 0;
-  if (tid == 0) sh_bad = r + 1;
-  for (int j = tid; j < r; j += kThreads) {
-    const unsigned b = smem_u32(bars + j);
+  for (int e = tid; e < r; e += kThreads) fd[e] = 0;
+  if (tid == 0) my_bad = r + 1;
+  // one CTA: a barrier completes by the arrival of the warp that formed the reflector or chunk;
+  // several: by the bytes it sends (entry 4 j: reflector j, 4 j + 1 + s: chunk s of column j)
+  for (int e = tid; e < 4 * r; e += kThreads) {
+    const int j = e >> 2, s = (e & 3) - 1;
+    const int n = s < 0 ? r + 3 : min(r, 32 * s + 32) - max(j, 32 * s);  // values
+    if (n <= 0) continue;
+    const unsigned b = smem_u32(s < 0 ? bars + j : cols + 3 * j + s);
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-    if (cs == 1) continue;  // completed by the arrival of the warp that formed reflector j
+    if (cs == 1) continue;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((r + 3) * 8) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(n * 8) : "memory");
   }
   cluster_barrier(cs);
   // T1 = R1 Sc^{-T} -> X3, T2 = R2 Sc^{-T} -> X1 (upper triangular), Ct = T1 T2' -> X0
@@ -198,10 +215,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
     }
   }
   cluster_barrier(cs);
-  // H = I - Ct' Ct -> X3 of CTA 0, lower triangle: columns p and r - 1 - p together hold r + 1
+  // H = I - Ct' Ct -> X3 of the column's CTA, lower triangle: columns p and r - 1 - p together hold r + 1
   // entries, so consecutive lanes take consecutive entries of such a pair
   {
-    double* H = cs == 1 ? X3 : cg::this_cluster().map_shared_rank(X3, 0u);
     const int npair = (r + 1) / 2;
     for (int e = rank * kThreads + tid; e < npair * (r + 1); e += cs * kThreads) {
       const int p = e / (r + 1), u = e - p * (r + 1);
@@ -209,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
       const int c = u < r - p ? p : r - 1 - p, i = u < r - p ? p + u : r - 1 - p + (u - (r - p));
       double acc = 0.0;
       for (int l = 0; l < r; ++l) acc = __fma_rn(X0[l + i * ld], X0[l + c * ld], acc);
+      double* H = cs == 1 ? X3 : cg::this_cluster().map_shared_rank(X3, (unsigned)(c % cs));
       H[i + c * ld] = __dsub_rn(i == c ? 1.0 : 0.0, acc);
     }
   }
@@ -230,13 +247,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
     }
   }
   cluster_barrier(cs);
-  // L22 = chol(H) in CTA 0, items (column c, chunk s) in column order, round robin over the warps.
-  // An item takes the contributions of columns k < c as their chunks become final; the chunk that
-  // holds the pivot publishes its square root, and every chunk of the column divides by it.
-  if (rank == 0) {
-    bool dead = false;  // after one expired wait this warp stops waiting
+  // L22 = chol(H): chunks s of the own columns in column order, round robin over the warps.  A wait
+  // that gives up marks the node with info = -1; the warp then stops waiting and carries on, so
+  // that everything is sent.
+  bool dead = false;
+  auto give_up = [&]() {
+    if (lane == 0) info[node] = -1;
+    dead = true;
+  };
+  {
     int at = 0;
-    for (int c = 0; c < r; ++c) {
+    for (int c = rank; c < r; c += cs) {
       const int pc = c >> 5;
       for (int s = pc; s < nch; ++s, ++at) {
         if (at % kWarps != w) continue;
@@ -245,16 +266,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
         double v = live ? X3[i + c * ld] : 0.0;
         int k0 = 0;
         while (k0 < c) {
-          int spins = 0;
-          while (!dead && (wait_limit == 0 || fl[3 * k0 + s] == 0 || fl[3 * k0 + pc] == 0))
-            if (++spins > lim) {
-              if (lane == 0) info[node] = -1;
-              dead = true;
-            }
+          // chunk s of the column, and chunk pc for the multiplier L22[c][k]
+          if (!dead && !bar_wait(smem_u32(cols + 3 * k0 + pc), wait_limit, cs)) give_up();
+          if (s != pc && !dead && !bar_wait(smem_u32(cols + 3 * k0 + s), wait_limit, cs)) give_up();
           int k1 = k0 + 1;
-          if (dead) k1 = c;
-          while (k1 < c && fl[3 * k1 + s] != 0 && fl[3 * k1 + pc] != 0) ++k1;
-          __threadfence_block();
+          while (k1 < c && (dead || (bar_try(smem_u32(cols + 3 * k1 + pc), cs) &&
+                                     (s == pc || bar_try(smem_u32(cols + 3 * k1 + s), cs)))))
+            ++k1;
           if (live)
             for (int kk = k0; kk < k1; ++kk) v = __fma_rn(-X3[i + kk * ld], X3[c + kk * ld], v);
           k0 = k1;
@@ -262,38 +280,55 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
         double sd;
         if (s == pc) {
           const double d = __shfl_sync(0xffffffffu, v, c & 31);
-          const bool ok = d > 0.0;
-          if (!ok && lane == 0) atomicMin(&sh_bad, c + 1);
+          const bool ok = positive(d);
+          if (!ok && lane == 0) atomicMin(&my_bad, c + 1);
           sd = ok ? sqrt(d) : 1.0;
-          if (lane == 0) va[c] = sd;
-          __threadfence_block();
-          __syncwarp();
-          if (lane == 0) fd[c] = 1;
+          if (s + 1 < nch) {
+            if (lane == 0) va[c] = sd;
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) fd[c] = 1;
+          }
         } else {
           int spins = 0;
           while (!dead && (wait_limit == 0 || fd[c] == 0))
-            if (++spins > lim) {
-              if (lane == 0) info[node] = -1;
-              dead = true;
-            }
+            if (++spins > lim) give_up();
           __threadfence_block();
           sd = va[c];
         }
-        const double x = i == c ? sd : v / sd;
-        if (live) X3[i + c * ld] = x;
-        __threadfence_block();
-        __syncwarp();
-        if (lane == 0) fl[3 * c + s] = 1;
-        if (live && cs > 1) {
-          cg::cluster_group cl = cg::this_cluster();
-          for (int d = 1; d < cs; ++d) *cl.map_shared_rank(X3 + i + c * ld, (unsigned)d) = x;
+        // (a zero numerator in an idle lane would send the warp through the slow division)
+        const double x = i == c ? sd : (live ? v : 1.0) / sd;
+        if (cs == 1) {
+          if (live) X3[i + c * ld] = x;
+          __threadfence_block();
+          __syncwarp();
+          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(cols + 3 * c + s)) : "memory");
+        } else if (live) {
+          // the CTA of the next column first
+          const unsigned to = smem_u32(X3 + i + c * ld), bar = smem_u32(cols + 3 * c + s);
+          for (int u = 1, d = rank; u <= cs; ++u) {
+            d = d + 1 == cs ? 0 : d + 1;
+            st_async(at_rank(to, d), x, at_rank(bar, d));
+          }
         }
       }
     }
-    __syncthreads();
-    if (tid == 0 && sh_bad <= r && info[node] == 0) info[node] = sh_bad;
+  }
+  // all of L22 has arrived (also after a wait that gave up: everything is sent)
+  for (int c = w; c < r; c += kWarps)
+    for (int q = c >> 5; q < nch; ++q)
+      if (!bar_wait(smem_u32(cols + 3 * c + q), -1, cs) && lane == 0) info[node] = -1;
+  __syncthreads();
+  if (tid == 0) {
+    int* to = cs == 1 ? sh_bad : cg::this_cluster().map_shared_rank(sh_bad, 0u);
+    to[rank] = my_bad;
   }
   cluster_barrier(cs);
+  if (rank == 0 && tid == 0) {
+    int bad = r + 1;
+    for (int d = 0; d < cs; ++d) bad = min(bad, sh_bad[d]);
+    if (bad <= r && info[node] == 0) info[node] = bad;
+  }
   for (int q = w; q < nown; q += kWarps) {
     const int c = rank + cs * q;
     for (int i = lane; i < r; i += 32) {
@@ -302,25 +337,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
       L22_out[e] = i >= c ? X3[i + c * ld] : 0.0;
     }
   }
-  if (level >= L) return;  // (no CTA touches another's memory after the barrier above)
-  // B <- L22^{-1} B, row by row on the own columns
+  if (level >= L) return;  // (no CTA touches another's memory from here on)
+  // G = L22^{-1} B -> X0 (own columns), row by row: a thread keeps to one column and every
+  // 256 / nown-th row, scales the row's entry for itself, and the first of them stores it
   for (int i = tid; i < r; i += kThreads) vi[i] = 1.0 / X3[i + i * ld];
   __syncthreads();
-  for (int i = 0; i < r; ++i) {
-    const double inv = vi[i];
-    for (int lc = tid; lc < nown; lc += kThreads) X2[i + (rank + cs * lc) * ld] *= inv;
-    __syncthreads();
-    const int rows = r - i - 1;
-    for (int e = tid; e < rows * nown; e += kThreads) {
-      const int lc = e / rows, ii = i + 1 + e - lc * rows, c = rank + cs * lc;
-      X2[ii + c * ld] = __fma_rn(-X3[ii + i * ld], X2[i + c * ld], X2[ii + c * ld]);
+  {
+    const int per = kThreads / nown, off = tid / nown, c = rank + cs * (tid - off * nown);
+    double* b = X2 + c * ld;
+    for (int i = 0; i < r; ++i) {
+      if (off < per) {
+        const double x = __dmul_rn(b[i], vi[i]);
+        if (off == 0) X0[i + c * ld] = x;
+        for (int ii = i + 1 + off; ii < r; ii += per) b[ii] = __fma_rn(-X3[ii + i * ld], x, b[ii]);
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
-  // Householder QR of [X1 (upper) ; X2] by columns: warp w of CTA `rank` owns the columns
-  // c = rank + cs (w + 8 t)
-  const int mine = rank + cs * w, step = cs * kWarps;
-  const int last = mine >= r ? -1 : mine + (r - 1 - mine) / step * step;  // largest own column
+  // Householder QR of [X1 (upper) ; X0] by columns: warp w < qw of CTA `rank` owns the columns
+  // c = rank + cs (w + qw t)
+  const int qw = cs == 1 ? kWarps : 4;
+  const int mine = rank + cs * w, step = cs * qw;
+  const int last = w >= qw || mine >= r ? -1 : mine + (r - 1 - mine) / step * step;  // largest own column
   auto rows3 = [&](const double* col, double (&x)[3]) {
 #pragma unroll
     for (int s = 0; s < 3; ++s) x[s] = 32 * s + lane < r ? col[32 * s + lane] : 0.0;
@@ -333,27 +371,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
                  s2 = __shfl_sync(0xffffffffu, t, 16);
     const double sig = __dadd_rn(__dadd_rn(s0, s1), s2), alpha = X1[c + c * ld];
     double beta = alpha, q = 0.0;
-    if (sig != 0.0) {
+    if (nonzero(sig)) {
       const double nrm = sqrt(__fma_rn(alpha, alpha, sig));
-      beta = alpha >= 0.0 ? -nrm : nrm;
+      beta = __double_as_longlong(alpha) >= 0 || !nonzero(alpha) ? -nrm : nrm;  // alpha >= 0
       // lane 1: tau = (beta - alpha) / beta; the others: scale = 1 / (alpha - beta)
       const double d = __dsub_rn(lane == 1 ? beta : alpha, lane == 1 ? alpha : beta);
       q = __ddiv_rn(lane == 1 ? d : 1.0, lane == 1 ? beta : d);
     }
-    const unsigned bar = smem_u32(bars + c), col = smem_u32(X2 + c * ld);
+    const unsigned bar = smem_u32(bars + c), col = smem_u32(X0 + c * ld);
     const double mineq = lane == 2 ? beta : q;  // lane 0 scale, 1 tau, 2 beta
     double* mineto = (lane == 0 ? vb : lane == 1 ? vc : va) + c;
     const unsigned slot = smem_u32(mineto);
     if (cs == 1) {
 #pragma unroll
       for (int s = 0; s < 3; ++s)
-        if (32 * s + lane < r) X2[32 * s + lane + c * ld] = x[s];
+        if (32 * s + lane < r) X0[32 * s + lane + c * ld] = x[s];
       if (lane < 3) *mineto = mineq;
       __threadfence_block();
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
     }
-    for (int d = 0; d < cs && cs > 1; ++d) {
+    for (int u = 1, d = rank; u <= cs && cs > 1; ++u) {  // the CTA of the next column first
+      d = d + 1 == cs ? 0 : d + 1;
       const unsigned rb = at_rank(bar, d), rc = at_rank(col, d);
 #pragma unroll
       for (int s = 0; s < 3; ++s)
@@ -362,26 +401,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
     }
     if (lane == 1) Etau[node * (int64_t)r + c] = q;
   };
-  if (mine == 0) {
+  if (mine == 0 && w < qw) {
     double x[3];
-    rows3(X2, x);
+    rows3(X0, x);
     reflect(0, x);
   }
-  bool dead = false;
   for (int j = 0; j < last; ++j) {
-    if (!dead && !bar_wait(smem_u32(bars + j), wait_limit, cs)) {
-      if (lane == 0) info[node] = -1;
-      dead = true;
-    }
+    if (!dead && !bar_wait(smem_u32(bars + j), wait_limit, cs)) give_up();
     const double tau = vc[j], scal = vb[j];
     double v[3];
-    rows3(X2 + j * ld, v);
+    rows3(X0 + j * ld, v);
     const int first = j < mine ? mine : mine + ((j - mine) / step + 1) * step;  // own columns > j
     int c0 = first;
     if (first == j + 1) {  // the next reflector's column
       double x[3];
-      rows3(X2 + first * ld, x);
-      if (tau != 0.0) {
+      rows3(X0 + first * ld, x);
+      if (nonzero(tau)) {
         double a = __fma_rn(v[0], x[0], 0.0);
         a = __fma_rn(v[1], x[1], a);
         a = __fma_rn(v[2], x[2], a);
@@ -395,13 +430,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
       reflect(first, x);
       c0 += step;
     }
-    if (tau == 0.0) continue;
+    if (!nonzero(tau)) continue;
     for (; c0 < r; c0 += 4 * step) {
       double x[4][3], a[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int c = min(c0 + u * step, last);
-        rows3(X2 + c * ld, x[u]);
+        rows3(X0 + c * ld, x[u]);
       }
       const int nu = (last - c0) / step + 1;  // columns of this group (4 or fewer)
 #pragma unroll
@@ -424,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
       for (int u = 0; u < 4; ++u) {
         const double fu = __shfl_sync(0xffffffffu, f, (u >> 1) * 16 + (u & 1) * 8);
         if (u < nu) {
-          double* col = X2 + (c0 + u * step) * ld;
+          double* col = X0 + (c0 + u * step) * ld;
 #pragma unroll
           for (int s = 0; s < 3; ++s)
             if (32 * s + lane < r) col[32 * s + lane] = __fma_rn(-fu, v[s], x[u][s]);
@@ -440,18 +475,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
   }
   __syncthreads();
   double* Rn = R + (nleaf + node) * (int64_t)r * r;
-  for (int c = mine; c < r; c += step) {
+  for (int c = mine; c <= last; c += step) {
     const double scal = vb[c], beta = va[c];
     for (int i = lane; i < r; i += 32) {
       const int64_t e = i + (int64_t)c * r;
       Rn[e] = i < c ? X1[i + c * ld] : (i == c ? beta : 0.0);
-      Eref[node * (int64_t)r * r + e] = __dmul_rn(X2[i + c * ld], scal);
+      Eref[node * (int64_t)r * r + e] = __dmul_rn(X0[i + c * ld], scal);
     }
   }
 }
 
 size_t node_f64_smem(int r) {
-  return ((size_t)4 * r * (r + 1) + 5 * r) * sizeof(double) + (size_t)4 * r * sizeof(int);
+  return ((size_t)4 * r * (r + 1) + 8 * r) * sizeof(double) + (size_t)r * sizeof(int);
 }
 
 cudaError_t launch_node_f64(double* R, const double* SinvT, int r, int level, const Tree& t, double* Ct, double* L22,
