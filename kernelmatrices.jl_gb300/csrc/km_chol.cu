@@ -64,7 +64,9 @@ __device__ void chol_diag(double* D, const CholMat& M, int k0, int* __restrict__
   // column j (updated value y of row `lane`) into its final form
   auto finish = [&](int j, double y) {
     const double p = __shfl_sync(0xffffffffu, y, j);
-    const bool ok = p > 0.0;
+    // p > 0 on the bits (an FP64 comparison is one more instruction of the FP64 pipe on the chain)
+    const long long pb = __double_as_longlong(p);
+    const bool ok = pb > 0 && pb <= 0x7ff0000000000000ll;
     if (!ok && lane == 0) atomicMin(&first_bad, k0 + j + 1);
     const double sd = ok ? sqrt(p) : 1.0;
     // (a zero numerator in an idle lane would send the warp through the slow division)
@@ -77,17 +79,23 @@ __device__ void chol_diag(double* D, const CholMat& M, int k0, int* __restrict__
   __syncthreads();
   if (w == 0) finish(0, lane < kb ? D[lane * LD] : 0.0);
   __syncthreads();
+  auto update = [&](int c, int j) {
+    if (lane >= c && lane < kb) D[lane * LD + c] = __fma_rn(-D[lane * LD + j], D[c * LD + j], D[lane * LD + c]);
+  };
   for (int j = 0; j < kb; ++j) {
     const bool live = lane >= j && lane < kb;
-    const double x = live ? D[lane * LD + j] : 0.0;
-    if (w == (j & 3) && live) M.out[(int64_t)(k0 + j) * m + k0 + lane] = x;
-    int c = j + 1 + ((w - j - 1) & 3);
-    if (c == j + 1 && c < kb) {
-      finish(c, lane >= c && lane < kb ? __fma_rn(-x, D[c * LD + j], D[lane * LD + c]) : 0.0);
-      c += 4;
+    if (w == (j & 3) && live) M.out[(int64_t)(k0 + j) * m + k0 + lane] = D[lane * LD + j];
+    const int c = j + 1 + ((w - j - 1) & 3);
+    if (c == j + 1) {
+      // next column first; this warp's other columns take column j in the next step
+      if (c < kb)
+        finish(c, lane >= c && lane < kb ? __fma_rn(-D[lane * LD + j], D[c * LD + j], D[lane * LD + c]) : 0.0);
+    } else {
+      for (int q = c; q < kb; q += 4) {
+        if (j > 0 && c == j + 4) update(q, j - 1);
+        update(q, j);
+      }
     }
-    for (; c < kb; c += 4)
-      if (lane >= c && lane < kb) D[lane * LD + c] = __fma_rn(-x, D[c * LD + j], D[lane * LD + c]);
     __syncthreads();
   }
   if (threadIdx.x == 0 && first_bad != INT_MAX && *info == 0) *info = first_bad;
@@ -138,13 +146,22 @@ __global__ void __launch_bounds__(128) k_chol_panel(Mats mats, int k0, int nrow,
   for (int l = 0; l < kb; ++l) {
     const double x = v[l];
     if (w == (l & 3) && !solve && i < m) M.out[(int64_t)(k0 + l) * m + i] = x;
-    int c = l + 1 + ((w - l - 1) & 3);
-    if (c == l + 1 && c < kb) {  // the next column first
-      const double y = __fma_rn(-x, D[c * LD + l], v[c]);
-      v[c] = solve ? __dmul_rn(y, inv[c]) : y / D[c * LD + c];
-      c += 4;
+    const int c = l + 1 + ((w - l - 1) & 3);
+    if (c == l + 1) {
+      // next column first; this warp's other columns take column l in the next step
+      if (c < kb) {
+        const double y = __fma_rn(-x, D[c * LD + l], v[c]);
+        v[c] = solve ? __dmul_rn(y, inv[c]) : y / D[c * LD + c];
+      }
+    } else {
+      const bool two = l > 0 && c == l + 4;
+      const double xp = two ? v[l - 1] : 0.0;
+      for (int q = c; q < kb; q += 4) {
+        double y = v[q];
+        if (two) y = __fma_rn(-xp, D[q * LD + l - 1], y);
+        v[q] = __fma_rn(-x, D[q * LD + l], y);
+      }
     }
-    for (; c < kb; c += 4) v[c] = __fma_rn(-x, D[c * LD + l], v[c]);
     __syncthreads();
   }
   if (solve)
