@@ -561,7 +561,7 @@ static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyIte
 int general_fwd(km_handle* h, double* X, int k) {  // X <- W^{-1} X
   const Tree& t = h->tree;
   cudaStream_t st = h->stream;
-  if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 0, X, 1, t.n, 0, X, 1, t.n, 0, k, st)))
+  if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_solve_f64(h->d_Lf, t, 0, X, t.n, k, st)))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
   for (int l = 1; l <= t.L; ++l) {
     const int64_t a = h->lvoff[l], b = h->lvoff[l + 1];
@@ -579,7 +579,7 @@ int general_bwd(km_handle* h, double* X, int k) {  // X <- W'^{-1} X
     int rc;
     if ((rc = run_gapply(h, h->gsolve_h, h->d_gsolve, a, b, 1, X, X, t.n, k)) != KM_OK) return rc;
   }
-  if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 1, X, 1, t.n, 0, X, 1, t.n, 0, k, st)))
+  if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_solve_f64(h->d_Lf, t, 1, X, t.n, k, st)))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
   return check_launch(h, "general bwd");
 }
@@ -641,8 +641,10 @@ static bool leaf_solve(km_handle* h, int op, T* X, int k) {
   cudaStream_t st = h->stream;
   if constexpr (std::is_same<T, ff>::value) {
     if (use_tri_blk(h, k)) return KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri_blk(P<ff>(h->d_Lf), t, op, X, t.n, k, st));
+    return KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<ff>(P<ff>(h->d_Lf), t, op, X, 1, t.n, 0, X, 1, t.n, 0, k, st));
+  } else {
+    return KL(h, KM_PROF_LEAF_TRI, launch_leaf_solve_f64(h->d_Lf, t, op, X, t.n, k, st));
   }
-  return KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<T>(P<T>(h->d_Lf), t, op, X, 1, t.n, 0, X, 1, t.n, 0, k, st));
 }
 
 template <typename T>
@@ -1448,6 +1450,7 @@ static int general_factorize(km_handle* h) {
   KM_CUDA(h, cudaMemsetAsync(h->d_info, 0, sizeof(int) * (t.nleaf + nb + 1), st));  // + grid-barrier word
   if (!leaf_chol_f64(h, 0))
     return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the leaf Cholesky kernel");
+  KLV(h, KM_PROF_OTHER, launch_leaf_diaginv(h->d_Lf, t, st));
   if (nb > 0) {
     // leaf triangular solves of every panel (invapply!, src/HODLR/src/utils.jl:54-65)
     std::vector<LeafDesc> ld;
@@ -1721,7 +1724,8 @@ static void aux_fwd_leaf(km_handle* h) {
     job->ok = use_tri_blk(h, job->k) ? launch_leaf_tri_blk(P<ff>(h->d_Lf), t, 0, X, t.n, job->k, ax)
                          : launch_leaf_tri<ff>(P<ff>(h->d_Lf), t, 0, X, 1, t.n, 0, X, 1, t.n, 0, job->k, ax);
   } else {
-    job->ok = launch_leaf_tri<double>(h->d_Lf, t, 0, X, 1, t.n, 0, X, 1, t.n, 0, job->k, ax);
+    launch_leaf_diaginv(h->d_Lf, t, ax);
+    job->ok = launch_leaf_solve_f64(h->d_Lf, t, 0, X, t.n, job->k, ax);
   }
   h->stats.kernel_launches += 2;
 }
@@ -1813,10 +1817,13 @@ static int factorize_launches(km_handle* h) {
       if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<double>(h->d_Lf, t, 0, h->d_Q, r, 0, 1, h->d_Q, r, 0, 1, r, st)))
         return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
     }
+    // the inverses of the leaf factors' diagonal blocks are for the solves only: off the main stream
     if (fwd) aux_fwd_leaf<double>(h);
+    else if (t.L == 0) KLV(h, KM_PROF_OTHER, launch_leaf_diaginv(h->d_Lf, t, st));
     if (t.L > 0) {
       KLV(h, KM_PROF_LEAF_QR, launch_leaf_qr<double>(h->d_Q, r, t, h->d_tauleaf, h->d_R, st));
       side_begin(h);
+      if (!fwd) launch_leaf_diaginv(h->d_Lf, t, h->side);
       launch_leaf_formq<double>(h->d_Q, h->d_tauleaf, r, t, h->side);
       if (fwd) cudaEventRecord(h->xev[1], h->side);
       for (int l = 1; l <= t.L; ++l) {

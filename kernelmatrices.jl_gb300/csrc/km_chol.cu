@@ -54,7 +54,7 @@ struct LeafMats {
 // (each quarter of the SM has its own FP64 pipe); the warp of the next column updates it first and
 // forms its square root and divisions while the others are still updating: one barrier a column.
 // The loops stay rolled: with the block in registers of one warp the unrolled code, run once,
-// waited for its own instructions (58 us for 32 columns, now @D@ us: NB times a square root, a
+// waited for its own instructions (58 us for 32 columns, now 36 us: NB times a square root, a
 // division and an update).
 template <int NB>
 __device__ void chol_diag(double* D, const CholMat& M, int k0, int* __restrict__ info) {

@@ -10,6 +10,7 @@
 // where a and b are the sums of phi and dphi of the siblings along the leaf's path to the root.
 // The sums travel through the tree sweeps with 2r-long vectors [phi ; dphi].
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "km_kernels.h"
@@ -609,10 +610,13 @@ __global__ void k_eval_dphi2(const double* __restrict__ pts, const double* __res
 // uq = ceil(r / 4), accumulates the 4 x 8 block q = u + uq a, c = c0 + v + g b (strided, so that
 // the shared-memory reads of a warp fall in distinct banks).  The leaf rows go in chunks of 32:
 // A_mat (r x 32) and X (8g x 32) are staged in shared memory as T along i with a padded stride;
-// rows past the leaf are zeros.  grid (nleaf, 3, ceil(k / 8g)), block uq g.
+// rows past the leaf are zeros.  grid (nleaf, 3, ceil(k / 8g)), block uq g.  With PARTS > 1 (few
+// leaves: g = 1) PARTS threads share a 4 x 8 block, each taking every PARTS-th row, and their sums
+// are added in order: 2 leaves of 500 points, 25 columns, rank 32 took 0.70 ms on 6 CTAs of one
+// warp, now 0.13 ms.  block uq g PARTS.
 constexpr int kPjK = 32, kPjS = kPjK + 1, kPjMaxG = 10, kPjMaxU = (kMaxNysRank + 3) / 4;
 
-template <typename T>
+template <typename T, int PARTS>
 __global__ void __launch_bounds__(kPjMaxU * kPjMaxG, 2)
     k_leaf_proj3(const T* __restrict__ Phi, const T* __restrict__ dPhi2, int r, DTree t, const T* __restrict__ X,
                  int64_t ldx, double* __restrict__ VP, int k, int g) {
@@ -629,7 +633,7 @@ __global__ void __launch_bounds__(kPjMaxU * kPjMaxG, 2)
   const int c0 = blockIdx.z * 8 * g;
   const int ncol = min(8 * g, k - c0);
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int u = tid % uq, v = tid / uq;
+  const int u = tid % uq, v = tid / uq % g, part = tid / (uq * g);
   acc_t<T> acc[4][8] = {};
   for (int i0 = 0; i0 < m; i0 += kPjK) {
     const int rows = min(kPjK, m - i0);
@@ -644,7 +648,7 @@ __global__ void __launch_bounds__(kPjMaxU * kPjMaxG, 2)
     }
     __syncthreads();
 #pragma unroll 2
-    for (int i = 0; i < kPjK; ++i) {
+    for (int i = part; i < kPjK; i += PARTS) {
       T av[4], xv[8];
 #pragma unroll
       for (int a = 0; a < 4; ++a) av[a] = As[(u + uq * a) * kPjS + i];
@@ -656,6 +660,25 @@ __global__ void __launch_bounds__(kPjMaxU * kPjMaxG, 2)
         for (int b = 0; b < 8; ++b) acc[a][b] += av[a] * xv[b];
     }
   }
+  if constexpr (PARTS > 1) {
+    // sums of the parts, 4 x 8 values per thread of part 0 (over the staged operands)
+    T* sums = As;
+    for (int p = 1; p < PARTS; ++p) {
+      __syncthreads();
+      if (part == p)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 8; ++b) sums[(a * 8 + b) * uq * g + v * uq + u] = accv(acc[a][b]);
+      __syncthreads();
+      if (part == 0)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int b = 0; b < 8; ++b) acc[a][b] += sums[(a * 8 + b) * uq * g + v * uq + u];
+    }
+    if (part > 0) return;
+  }
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -665,33 +688,51 @@ __global__ void __launch_bounds__(kPjMaxU * kPjMaxG, 2)
     }
 }
 
+// a == b for finite doubles, without the FP64 pipe (its comparisons take 65 cycles a warp)
+__device__ __forceinline__ bool same_value(double a, double b) {
+  const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
+  return x == y || ((x | y) << 1) == 0;
+}
+
 // VP[(leaf k + c) W + 3r + q] = sum over the leaf's points x_i equal to landmark p_q (coordinate by
 // coordinate) of X[i][c]: the projection on the nugget derivative dK_2(X, P) = [x == p], a
-// 0/1 matrix with at most one entry per row for distinct points.  Thread q scans the leaf once;
-// a landmark with several equal points (repeated points) rescans it per column, in order.
-// grid nleaf, block 32 ceil(r / 32).
-__global__ void k_nugget_proj(const double* __restrict__ pts, const double* __restrict__ lnd, int r, DTree t,
-                              const double* __restrict__ X, int64_t ldx, double* __restrict__ VP, int k) {
-  const int q = threadIdx.x;
-  if (q >= r) return;
+// 0/1 matrix with at most one entry per row for distinct points.  The (point, landmark) pairs are
+// compared by all threads; a landmark with several equal points (repeated points) rescans the leaf
+// per column, in order.  grid (nleaf, parts of the columns), block 256.
+__global__ void __launch_bounds__(256) k_nugget_proj(const double* __restrict__ pts, const double* __restrict__ lnd,
+                                                     int r, DTree t, const double* __restrict__ X, int64_t ldx,
+                                                     double* __restrict__ VP, int k) {
+  __shared__ double px[kMaxNysRank], py[kMaxNysRank];
+  __shared__ int first[kMaxNysRank], cnt[kMaxNysRank];
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   const int64_t s = d_leaf_start(t, leaf);
   const int W = 4 * r;
-  const double px = lnd[2 * q], py = lnd[2 * q + 1];
-  int first = -1, cnt = 0;
-  for (int i = 0; i < m; ++i)
-    if (pts[2 * (s + i)] == px && pts[2 * (s + i) + 1] == py) {
-      if (first < 0) first = i;
-      ++cnt;
-    }
-  for (int c = 0; c < k; ++c) {
+  for (int q = threadIdx.x; q < r; q += blockDim.x) {
+    px[q] = lnd[2 * q];
+    py[q] = lnd[2 * q + 1];
+    first[q] = INT_MAX;
+    cnt[q] = 0;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < m; i += blockDim.x) {
+    const double x = pts[2 * (s + i)], y = pts[2 * (s + i) + 1];
+    for (int q = 0; q < r; ++q)
+      if (same_value(x, px[q]) && same_value(y, py[q])) {
+        atomicMin(&first[q], i);
+        atomicAdd(&cnt[q], 1);
+      }
+  }
+  __syncthreads();
+  const int per = (k + gridDim.y - 1) / gridDim.y, ca = blockIdx.y * per, ce = min(k, ca + per);
+  for (int e = threadIdx.x; e < (ce - ca) * r; e += blockDim.x) {
+    const int q = e % r, c = ca + e / r;
     double v = 0.0;
-    if (cnt == 1) {
-      v = X[(int64_t)c * ldx + s + first];
-    } else if (cnt > 1) {
-      for (int i = first; i < m; ++i)
-        if (pts[2 * (s + i)] == px && pts[2 * (s + i) + 1] == py) v += X[(int64_t)c * ldx + s + i];
+    if (cnt[q] == 1) {
+      v = X[(int64_t)c * ldx + s + first[q]];
+    } else if (cnt[q] > 1) {
+      for (int i = first[q]; i < m; ++i)
+        if (same_value(pts[2 * (s + i)], px[q]) && same_value(pts[2 * (s + i) + 1], py[q])) v += X[(int64_t)c * ldx + s + i];
     }
     VP[(leaf * k + c) * W + 3 * r + q] = v;
   }
@@ -970,16 +1011,26 @@ void launch_eval_dphi2(const double* pts, const double* lnd, const float* P3, co
 template <typename T>
 void launch_leaf_proj3(const T* Phi, const T* dPhi2, int r, const Tree& t, const T* X, int64_t ldx, double* VP, int k,
                        cudaStream_t st) {
-  const int g = std::min(kPjMaxG, (k + 7) / 8), uq = (r + 3) / 4;
+  const int uq = (r + 3) / 4;
+  int g = std::min(kPjMaxG, (k + 7) / 8);
+  constexpr int kParts = 8;
+  const bool few = t.nleaf * 3 * ((k + 8 * g - 1) / (8 * g)) < 2 * 152 && uq * kParts <= kPjMaxU * kPjMaxG;
+  if (few) g = 1;
   dim3 grid((unsigned)t.nleaf, 3u, (unsigned)((k + 8 * g - 1) / (8 * g)));
-  const size_t sm = (size_t)(4 * uq + 8 * g) * kPjS * sizeof(T);
-  smem_limit((const void*)k_leaf_proj3<T>, sm);
-  k_leaf_proj3<T><<<grid, uq * g, sm, st>>>(Phi, dPhi2, r, dtree(t), X, ldx, VP, k, g);
+  const size_t sm = std::max((size_t)(4 * uq + 8 * g) * kPjS, (size_t)32 * uq * g) * sizeof(T);
+  if (few) {
+    smem_limit((const void*)k_leaf_proj3<T, kParts>, sm);
+    k_leaf_proj3<T, kParts><<<grid, uq * g * kParts, sm, st>>>(Phi, dPhi2, r, dtree(t), X, ldx, VP, k, g);
+  } else {
+    smem_limit((const void*)k_leaf_proj3<T, 1>, sm);
+    k_leaf_proj3<T, 1><<<grid, uq * g, sm, st>>>(Phi, dPhi2, r, dtree(t), X, ldx, VP, k, g);
+  }
 }
 
 void launch_nugget_proj(const double* pts, const double* lnd, int r, const Tree& t, const double* X, int64_t ldx,
                         double* VP, int k, cudaStream_t st) {
-  k_nugget_proj<<<(unsigned)t.nleaf, 32 * ((r + 31) / 32), 0, st>>>(pts, lnd, r, dtree(t), X, ldx, VP, k);
+  const unsigned parts = (unsigned)std::max<int64_t>(1, std::min<int64_t>((k + 7) / 8, 2 * 152 / t.nleaf));
+  k_nugget_proj<<<dim3((unsigned)t.nleaf, parts), 256, 0, st>>>(pts, lnd, r, dtree(t), X, ldx, VP, k);
 }
 
 void launch_proj_total(double* VP, int W, int64_t nleaf, int k, cudaStream_t st) {

@@ -104,6 +104,10 @@ bool leaf_chol_f64_solves(const Tree& t);
 template <typename T>
 bool launch_leaf_tri(const T* Lf, const Tree& t, int op, T* Bptr, int64_t bmul, int64_t bld, int bld_is_m, T* Xptr,
                      int64_t xmul, int64_t xld, int xld_is_m, int ncols, cudaStream_t st);
+// FP64 leaf solves L x = b (op 0), L' x = b (op 1) in place on k columns (ld ldx) with the inverses of
+// the 32 x 32 diagonal blocks that launch_leaf_diaginv leaves in their upper triangles
+void launch_leaf_diaginv(double* Lf, const Tree& t, cudaStream_t st);
+bool launch_leaf_solve_f64(const double* Lf, const Tree& t, int op, double* X, int64_t ldx, int k, cudaStream_t st);
 template <typename T>
 void launch_leaf_qr(T* Pan, int r, const Tree& t, T* tau, T* Rout, cudaStream_t st);
 // Mixed form on the tensor cores (km_leaf_tc.cu): blocked Cholesky of the augmented leaf matrices

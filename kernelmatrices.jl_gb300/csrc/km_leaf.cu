@@ -7,6 +7,9 @@
 // sides staged in shared memory; the triangular solves are blocked by 32 rows so that the
 // dependency chain is a 32-step shuffle solve per block and the bulk of the work is an
 // independent multiply-add update (FP64 throughput bound).
+#include <algorithm>
+#include <type_traits>
+
 #include "km_kernels.h"
 
 namespace km {
@@ -64,17 +67,41 @@ __device__ void leaf_tri_body(const T* __restrict__ L, int m, int op, const T* B
       // update of the remaining rows with the solved block: items of (row, 4 columns), so that
       // each loaded L entry feeds 4 multiply-adds and all threads stay busy as the remaining
       // rows shrink
-      const int R = (op == 0) ? m - (i0 + ib) : i0;
-      const int r0 = (op == 0) ? i0 + ib : 0;
+      if (op == 1) {
+        // rows i < i0 take L[i0 + l, i]: along l in memory, so 32 x 32 tiles go through shared
+        // memory (over D, which this block has finished with); items of (row, 2 columns)
+        for (int r0 = 0; r0 < i0; r0 += 32) {
+          for (int e = tid; e < 32 * 32; e += blockDim.x) {
+            const int l = e & 31, i = e >> 5;
+            if (l < ib) D[l * 33 + i] = L[(int64_t)(r0 + i) * m + i0 + l];
+          }
+          __syncthreads();
+          for (int e = tid; e < 32 * ((nc + 1) >> 1); e += blockDim.x) {
+            const int i = e & 31, cb = 2 * (e >> 5);
+            const T* xc = xs + cb * m + i0;
+            acc_t<T> acc[2] = {};
+            const int c2 = cb + 1 < nc ? m : 0;
+#pragma unroll 4
+            for (int l = 0; l < ib; ++l) {
+              const T a = D[l * 33 + i];
+              acc[0] += a * xc[l];
+              acc[1] += a * xc[c2 + l];
+            }
+            xs[cb * m + r0 + i] -= accv(acc[0]);
+            if (c2) xs[cb * m + m + r0 + i] -= accv(acc[1]);
+          }
+          __syncthreads();
+        }
+        continue;
+      }
+      const int R = m - (i0 + ib);
+      const int r0 = i0 + ib;
       const int ng = (nc + 3) >> 2;
       for (int e = tid; e < R * ng; e += blockDim.x) {
         const int g = e / R, i = r0 + (e - g * R), cb = 4 * g;
         const T* xc = xs + cb * m + i0;
         acc_t<T> acc[4] = {};
-        auto ld = [&](int l) {
-          return (op == 0) ? L[(int64_t)(i0 + l) * m + i]   // L[i, i0 + l]
-                           : L[(int64_t)i * m + i0 + l];    // L[i0 + l, i]
-        };
+        auto ld = [&](int l) { return L[(int64_t)(i0 + l) * m + i]; };  // L[i, i0 + l]
         int l = 0;
         for (; l + 3 < ib; l += 4) {  // four entries loaded ahead of their multiply-adds
           const T a0 = ld(l), a1 = ld(l + 1), a2 = ld(l + 2), a3 = ld(l + 3);
@@ -167,35 +194,43 @@ __global__ void __launch_bounds__(256) k_leaf_tri_desc(const double* __restrict_
 // Q_leaf' y (proj) and y += sign * Q_leaf g (expand) with the explicit leaf bases Q (m x r,
 // column-major at start*r).  grid = (nleaf, ceil(k / 16)), block 256.
 // ---------------------------------------------------------------------------------------------
-// VP[leaf][c] = Q_leaf' y_c for a chunk of up to 16 columns.  The leaf is processed in chunks of
-// 64 rows: Q (64 x r, padded rows) and y (16 x 64) are staged in shared memory, then thread t
-// owns basis column q = t % r and the columns of group t / r, with up to 6 accumulators.
+// VP[leaf][c] = Q_leaf' y_c for a chunk of up to 16 columns and the basis columns q0 .. q0 + rq - 1.
+// The leaf is processed in chunks of 64 rows: Q (64 x rq, padded rows) and y (16 x 64) are staged in
+// shared memory, then thread t owns basis column t % rq and the columns of group t / rq, with up to
+// 6 accumulators; where there are at least twice as many groups as columns, the groups of a column
+// share its rows and their sums are added in order at the end.  Few leaves split the basis columns
+// over CTAs: 2 leaves of 500 points, 25 columns, rank 32 took 250 us on 4 CTAs, now 40 us.
 constexpr int kProjRows = 64;
+constexpr int kProjCols = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_leaf_qproj(const T* __restrict__ Q, int r, DTree t, const T* __restrict__ Y,
-                                                    int64_t ldy, T* __restrict__ VP, int k) {
+                                                    int64_t ldy, T* __restrict__ VP, int k, int rq) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int ldq = r + 1;
-  T* qs = reinterpret_cast<T*>(smraw);   // kProjRows x (r + 1): element (i, q) at i * ldq + q
-  T* ys = qs + kProjRows * ldq;           // 16 x kProjRows
+  const int q0 = blockIdx.z * rq;
+  if (r - q0 < rq) rq = r - q0;
+  const int ldq = rq + 1;
+  T* qs = reinterpret_cast<T*>(smraw);   // kProjRows x (rq + 1): element (i, q) at i * ldq + q
+  T* ys = qs + kProjRows * ldq;           // kProjCols x kProjRows
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   const int64_t s = d_leaf_start(t, leaf);
-  const int c0 = blockIdx.y * 16;
-  const int nc = min(16, k - c0);
+  const int c0 = blockIdx.y * kProjCols;
+  const int nc = min(kProjCols, k - c0);
   const int tid = threadIdx.x;
-  const int G = blockDim.x / r;                 // column groups (>= 3 for r <= 80)
-  const int q = tid % r, g = tid / r;
-  const int cper = (nc + G - 1) / G;            // <= 6
-  const int cb = g * cper, ce = min(nc, cb + cper);
-  const bool active = g < G;
+  const int G = blockDim.x / rq;                // groups (>= 3 for rq <= 80)
+  const int q = tid % rq, g = tid / rq;
+  const int parts = max(1, G / nc);             // row parts of a column
+  const int cper = parts > 1 ? 1 : (nc + G - 1) / G;  // <= 6
+  const int part = parts > 1 ? g / nc : 0;
+  const int cb = parts > 1 ? g % nc : g * cper, ce = min(nc, cb + cper);
+  const bool active = g < G && part < parts;
   acc_t<T> acc[6] = {};
-  const T* Ql = Q + s * r;
+  const T* Ql = Q + s * r + (int64_t)q0 * m;
   for (int i0 = 0; i0 < m; i0 += kProjRows) {
     const int rows = min(kProjRows, m - i0);
     __syncthreads();
-    for (int e = tid; e < rows * r; e += blockDim.x) {
+    for (int e = tid; e < rows * rq; e += blockDim.x) {
       const int qq = e / rows, i = e - qq * rows;
       qs[i * ldq + qq] = Ql[(int64_t)qq * m + i0 + i];
     }
@@ -204,62 +239,213 @@ __global__ void __launch_bounds__(256) k_leaf_qproj(const T* __restrict__ Q, int
       ys[c * kProjRows + i] = Y[(int64_t)(c0 + c) * ldy + s + i0 + i];
     }
     __syncthreads();
-    if (active) {
-      for (int i = 0; i < rows; ++i) {
+    // cper columns a thread, unrolled for that number (a multiply-add that is switched off still
+    // takes its pipe); a last group with fewer columns repeats its last one
+    auto dots = [&](auto count) {
+      constexpr int CP = decltype(count)::value;
+      int at[CP];
+#pragma unroll
+      for (int j = 0; j < CP; ++j) at[j] = min(cb + j, nc - 1) * kProjRows;
+      for (int i = part; i < rows; i += parts) {
         const T a = qs[i * ldq + q];
 #pragma unroll
-        for (int j = 0; j < 6; ++j)
-          if (cb + j < ce) acc[j] += a * ys[(cb + j) * kProjRows + i];
+        for (int j = 0; j < CP; ++j) acc[j] += a * ys[at[j] + i];
       }
+    };
+    if (active) switch (cper) {
+        case 1: dots(std::integral_constant<int, 1>{}); break;
+        case 2: dots(std::integral_constant<int, 2>{}); break;
+        case 3: dots(std::integral_constant<int, 3>{}); break;
+        case 4: dots(std::integral_constant<int, 4>{}); break;
+        default: dots(std::integral_constant<int, 6>{});
+      }
+  }
+  if (parts > 1) {
+    __syncthreads();
+    T* sums = qs;  // part x column x rq (at most 256 values)
+    if (active) sums[(part * nc + cb) * rq + q] = accv(acc[0]);
+    __syncthreads();
+    if (active && part == 0) {
+      acc_t<T> tot = sums[cb * rq + q];
+      for (int p = 1; p < parts; ++p) tot += sums[(p * nc + cb) * rq + q];
+      VP[(leaf * k + c0 + cb) * r + q0 + q] = accv(tot);
     }
+    return;
   }
   if (active)
 #pragma unroll
     for (int j = 0; j < 6; ++j)
-      if (cb + j < ce) VP[(leaf * k + c0 + cb + j) * r + q] = accv(acc[j]);
+      if (cb + j < ce) VP[(leaf * k + c0 + cb + j) * r + q0 + q] = accv(acc[j]);
 }
 
-// y_c += sign * Q_leaf g_c for a chunk of up to 16 columns: thread per leaf row, the chunk's
-// coefficients g (16 x r) in shared memory, one accumulator per column; Q is read once.
-template <typename T>
-__global__ void __launch_bounds__(256) k_leaf_qexpand(const T* __restrict__ Q, int r, DTree t, const T* __restrict__ VG,
-                                                      T* __restrict__ Y, int64_t ldy, int k, double sign) {
+// y_c += sign * Q_leaf g_c for a chunk of up to CB columns and 128 rows: thread per leaf row, the
+// chunk's coefficients g (CB x r) in shared memory, one accumulator per column; Q is read once
+// per chunk.
+constexpr int kExpRows = 128;
+
+template <typename T, int CB>
+__global__ void __launch_bounds__(kExpRows) k_leaf_qexpand(const T* __restrict__ Q, int r, DTree t,
+                                                           const T* __restrict__ VG, T* __restrict__ Y, int64_t ldy,
+                                                           int k, double sign) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  T* gs = reinterpret_cast<T*>(smraw);  // 16 x r
+  T* gs = reinterpret_cast<T*>(smraw);  // CB x r
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   const int64_t s = d_leaf_start(t, leaf);
-  const int c0 = blockIdx.y * 16;
-  const int nc = min(16, k - c0);
+  const int c0 = blockIdx.y * CB;
+  const int nc = min(CB, k - c0);
   for (int e = threadIdx.x; e < nc * r; e += blockDim.x) gs[e] = VG[(leaf * k + c0) * r + e];
   __syncthreads();
   const T* Ql = Q + s * r;
   const bool add = sign > 0.0;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    acc_t<T> acc[16] = {};
-    int q = 0;
-    for (; q + 1 < r; q += 2) {  // two basis entries loaded ahead of their multiply-adds
-      const T a0 = Ql[(int64_t)q * m + i], a1 = Ql[(int64_t)(q + 1) * m + i];
+  const int i = blockIdx.z * kExpRows + threadIdx.x;
+  if (i >= m) return;
+  acc_t<T> acc[CB] = {};
+  int q = 0;
+  for (; q + 3 < r; q += 4) {  // four basis entries loaded ahead of their multiply-adds
+    T a[4];
 #pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c < nc) {
-          acc[c] += a0 * gs[c * r + q];
-          acc[c] += a1 * gs[c * r + q + 1];
-        }
-    }
-    for (; q < r; ++q) {
-      const T a = Ql[(int64_t)q * m + i];
+    for (int u = 0; u < 4; ++u) a[u] = Ql[(int64_t)(q + u) * m + i];
 #pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c < nc) acc[c] += a * gs[c * r + q];
-    }
-#pragma unroll
-    for (int c = 0; c < 16; ++c)
+    for (int c = 0; c < CB; ++c)
       if (c < nc) {
-        T* y = Y + (int64_t)(c0 + c) * ldy + s + i;
-        *y = add ? *y + accv(acc[c]) : *y - accv(acc[c]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[c] += a[u] * gs[c * r + q + u];
       }
   }
+  for (; q < r; ++q) {
+    const T a = Ql[(int64_t)q * m + i];
+#pragma unroll
+    for (int c = 0; c < CB; ++c)
+      if (c < nc) acc[c] += a * gs[c * r + q];
+  }
+#pragma unroll
+  for (int c = 0; c < CB; ++c)
+    if (c < nc) {
+      T* y = Y + (int64_t)(c0 + c) * ldy + s + i;
+      *y = add ? *y + accv(acc[c]) : *y - accv(acc[c]);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// FP64 leaf solves L x = b (op 0) and L' x = b (op 1) by 32-row blocks with the inverses of the
+// diagonal blocks: x_q = X_q (b_q - L_{q,<q} x_{<q}).  A substitution inside a block is 32 steps of
+// one useful lane each; with X_q it is a product whose rows a and 31 - a of two columns share a
+// lane: 33 FP64 instructions for 2 columns instead of 128, and no chain.  X_q (strictly lower part)
+// lives in the block's upper triangle of Lf, which nothing else uses.
+// Measured: 128 leaves of 312 points, 32 right-hand sides 0.67 -> 0.54 ms; 2 leaves of 500, one right-hand
+// side 270 -> 205 us.
+// ---------------------------------------------------------------------------------------------
+
+// X_q of every diagonal block: grid (nleaf, blocks), 4 warps, lane = column of X; warp i mod 4 keeps
+// the rows i; row l is finished by its warp, then subtracted from the rows below.
+__global__ void __launch_bounds__(128) k_leaf_diaginv(double* __restrict__ Lf, DTree t) {
+  __shared__ double D[32 * 33], X[32 * 33], inv[32];
+  const int64_t leaf = blockIdx.x;
+  const int m = d_leaf_size(t, leaf), i0 = blockIdx.y * 32;
+  if (i0 >= m) return;
+  const int ib = min(32, m - i0), lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* L = Lf + d_leaf_koff(t, leaf) + (int64_t)i0 * m + i0;
+  for (int c = w; c < ib; c += 4)
+    if (lane >= c && lane < ib) D[lane * 33 + c] = L[(int64_t)c * m + lane];
+  for (int i = w; i < 32; i += 4) X[i * 33 + lane] = i == lane ? 1.0 : 0.0;
+  if (w == 0 && lane < ib) inv[lane] = 1.0 / L[(int64_t)lane * m + lane];
+  __syncthreads();
+  for (int l = 0; l < ib; ++l) {
+    if (w == (l & 3)) X[l * 33 + lane] *= inv[l];
+    __syncthreads();
+    const double x = X[l * 33 + lane];
+    for (int i = l + 1 + ((w - l - 1) & 3); i < ib; i += 4) X[i * 33 + lane] -= D[i * 33 + l] * x;
+  }
+  __syncthreads();
+  for (int i = w; i < ib; i += 4)  // X[i][l], l < i, at row l of column i
+    if (lane < i) L[(int64_t)i * m + lane] = X[i * 33 + lane];
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_leaf_solve(const double* __restrict__ Lf, DTree t, int op,
+                                                    double* __restrict__ Xg, int64_t ldx, int k) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double* xs = reinterpret_cast<double*>(smraw);  // NC x m
+  const int64_t leaf = blockIdx.x;
+  const int m = d_leaf_size(t, leaf);
+  const double* L = Lf + d_leaf_koff(t, leaf);
+  double* D = xs + NC * m;                        // 32 x 33
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int c0 = blockIdx.y * NC, nc = min(NC, k - c0);
+  double* X = Xg + d_leaf_start(t, leaf) + (int64_t)c0 * ldx;
+  for (int c = 0; c < nc; ++c)
+    for (int i = tid; i < m; i += 256) xs[c * m + i] = X[(int64_t)c * ldx + i];
+  const int nblk = (m + 31) / 32;
+  for (int q = 0; q < nblk; ++q) {
+    const int i0 = 32 * (op == 0 ? q : nblk - 1 - q), ib = min(32, m - i0);
+    __syncthreads();
+    // op 0: D[a][l] = X_q[a][l], l <= a; op 1: D[a][l] = X_q[31 - l][31 - a], the transpose with rows
+    // and columns reversed, again lower triangular (rows beyond the block are zero)
+    for (int i = w; i < 32; i += 8) {
+      double v = 0.0;
+      if (i < ib && lane <= i) {
+        const double e = L[(int64_t)(i0 + i) * m + i0 + lane];
+        v = lane == i ? 1.0 / e : e;
+      }
+      if (lane <= i) D[op == 0 ? i * 33 + lane : (31 - lane) * 33 + 31 - i] = v;
+    }
+    __syncthreads();
+    for (int c = 2 * w; c < nc; c += 16) {
+      double* b0 = xs + c * m + i0;
+      double* b1 = c + 1 < nc ? b0 + m : b0;
+      double first = 0.0, acc = 0.0;
+      for (int u = 0; u <= 32; ++u) {
+        const bool one = u <= lane;
+        if (u == lane + 1) {
+          first = acc;
+          acc = 0.0;
+        }
+        const int row = one ? lane : 31 - lane, l = one ? u : u - lane - 1;
+        const int i = op == 0 ? l : 31 - l;
+        const double b = i < ib ? (one ? b0 : b1)[i] : 0.0;
+        acc += D[row * 33 + l] * b;
+      }
+      const double second = acc;
+      __syncwarp();
+      const int ra = op == 0 ? lane : 31 - lane, rb = 31 - ra;
+      if (ra < ib) b0[ra] = first;
+      __syncwarp();
+      if (c + 1 < nc && rb < ib) b1[rb] = second;
+    }
+    __syncthreads();
+    const int R = op == 0 ? m - (i0 + ib) : i0, r0 = op == 0 ? i0 + ib : 0;
+    constexpr int CG = NC < 4 ? NC : 4;
+    const int ng = (nc + CG - 1) / CG;
+    for (int e = tid; e < R * ng; e += 256) {
+      const int g = e / R, i = r0 + (e - g * R), cb = CG * g;
+      const double* xc = xs + cb * m + i0;
+      const double* a = op == 0 ? L + (int64_t)i0 * m + i : L + (int64_t)i * m + i0;
+      const int64_t sa = op == 0 ? m : 1;
+      double acc[CG] = {};
+      int l = 0;
+      for (; l + 7 < ib; l += 8) {  // eight entries loaded ahead of their multiply-adds
+        double av[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) av[u] = a[(l + u) * sa];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+          for (int j = 0; j < CG; ++j)
+            if (cb + j < nc) acc[j] += av[u] * xc[j * m + l + u];
+      }
+      for (; l < ib; ++l)
+#pragma unroll
+        for (int j = 0; j < CG; ++j)
+          if (cb + j < nc) acc[j] += a[l * sa] * xc[j * m + l];
+#pragma unroll
+      for (int j = 0; j < CG; ++j)
+        if (cb + j < nc) xs[(cb + j) * m + i] -= acc[j];
+    }
+  }
+  __syncthreads();
+  for (int c = 0; c < nc; ++c)
+    for (int i = tid; i < m; i += 256) X[(int64_t)c * ldx + i] = xs[c * m + i];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -314,18 +500,58 @@ bool launch_leaf_tri_desc(const double* Lf, const Tree& t, int op, const LeafDes
 template <typename T>
 void launch_leaf_proj(const T* Q, const T*, int r, const Tree& t, const T* Y, int64_t ldy, T* VP, int k,
                       cudaStream_t st) {
-  dim3 grid((unsigned)t.nleaf, (unsigned)((k + 15) / 16));
-  const size_t sm = ((size_t)kProjRows * (r + 1) + 16 * kProjRows) * sizeof(T);
+  const unsigned chunks = (unsigned)((k + kProjCols - 1) / kProjCols);
+  // basis columns of a CTA: halved while the CTAs do not fill the SMs twice (the right-hand sides
+  // are then staged once per part)
+  int parts = 1;
+  while (t.nleaf * chunks * parts < 2 * 152 && r >= 16 * parts) parts *= 2;
+  const int rq = (r + parts - 1) / parts;
+  dim3 grid((unsigned)t.nleaf, chunks, (unsigned)((r + rq - 1) / rq));
+  const size_t sm = std::max<size_t>((size_t)kProjRows * (rq + 1) + kProjCols * kProjRows, 256) * sizeof(T);
   smem_limit((const void*)k_leaf_qproj<T>, sm);
-  k_leaf_qproj<T><<<grid, 256, sm, st>>>(Q, r, dtree(t), Y, ldy, VP, k);
+  k_leaf_qproj<T><<<grid, 256, sm, st>>>(Q, r, dtree(t), Y, ldy, VP, k, rq);
+}
+
+template <typename T, int CB>
+static void expand_launch(const T* Q, int r, const Tree& t, const T* VG, T* Y, int64_t ldy, int k, double sign,
+                          cudaStream_t st) {
+  dim3 grid((unsigned)t.nleaf, (unsigned)((k + CB - 1) / CB), (unsigned)((t.max_leaf + kExpRows - 1) / kExpRows));
+  k_leaf_qexpand<T, CB><<<grid, kExpRows, (size_t)CB * r * sizeof(T), st>>>(Q, r, dtree(t), VG, Y, ldy, k, sign);
 }
 
 template <typename T>
 void launch_leaf_expand(const T* Q, const T*, int r, const Tree& t, const T* VG, T* Y, int64_t ldy, int k,
                         double sign, cudaStream_t st) {
-  dim3 grid((unsigned)t.nleaf, (unsigned)((k + 15) / 16));
-  const size_t sm = (size_t)16 * r * sizeof(T);
-  k_leaf_qexpand<T><<<grid, 256, sm, st>>>(Q, r, dtree(t), VG, Y, ldy, k, sign);
+  // 16 columns a CTA reads Q least often; 4 where 16 would leave SMs without a CTA
+  const int64_t rows = (t.max_leaf + kExpRows - 1) / kExpRows;
+  if (k <= 4 || t.nleaf * rows * ((k + 15) / 16) < 4 * 152)
+    expand_launch<T, 4>(Q, r, t, VG, Y, ldy, k, sign, st);
+  else
+    expand_launch<T, 16>(Q, r, t, VG, Y, ldy, k, sign, st);
+}
+
+void launch_leaf_diaginv(double* Lf, const Tree& t, cudaStream_t st) {
+  k_leaf_diaginv<<<dim3((unsigned)t.nleaf, (unsigned)((t.max_leaf + 31) / 32)), 128, 0, st>>>(Lf, dtree(t));
+}
+
+template <int NC>
+static bool solve_launch(const double* Lf, const Tree& t, int op, double* X, int64_t ldx, int k, cudaStream_t st) {
+  const size_t sm = ((size_t)NC * t.max_leaf + 32 * 33) * sizeof(double);
+  if (sm > 200 * 1024) return false;
+  smem_limit((const void*)k_leaf_solve<NC>, sm);
+  k_leaf_solve<NC><<<dim3((unsigned)t.nleaf, (unsigned)((k + NC - 1) / NC)), 256, sm, st>>>(Lf, dtree(t), op, X, ldx, k);
+  return true;
+}
+
+bool launch_leaf_solve_f64(const double* Lf, const Tree& t, int op, double* X, int64_t ldx, int k, cudaStream_t st) {
+  // widest column chunk that still gives about four CTAs an SM (a CTA reads its leaf's factor once)
+  auto ctas = [&](int nc) { return t.nleaf * (int64_t)((k + nc - 1) / nc); };
+  const int64_t want = 4 * 152;
+  if (k > 8 && ctas(16) >= want && solve_launch<16>(Lf, t, op, X, ldx, k, st)) return true;
+  if (k > 4 && ctas(8) >= want && solve_launch<8>(Lf, t, op, X, ldx, k, st)) return true;
+  if (k > 2 && ctas(4) >= want && solve_launch<4>(Lf, t, op, X, ldx, k, st)) return true;
+  if (k > 1 && solve_launch<2>(Lf, t, op, X, ldx, k, st)) return true;
+  return solve_launch<1>(Lf, t, op, X, ldx, k, st);
 }
 
 template bool launch_leaf_tri<double>(const double*, const Tree&, int, double*, int64_t, int64_t, int, double*,

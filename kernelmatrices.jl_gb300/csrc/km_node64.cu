@@ -22,8 +22,8 @@
 //                  reflector j to its other columns, four at a time so that their dot products
 //                  share the additions over the lanes.  One warp per quarter of the SM where the
 //                  column chain bounds it (several CTAs a node), two where the FP64 pipe does.
-// Rank 72, time per level: 1.05 ms -> @A@ ms with 8 CTAs a node, @B@ ms with one.  (Cholesky in CTA 0
-// alone, where its chunks compete for four quarters, took 286 k cycles against @C@ k.)
+// Rank 72, time per level: 1.05 ms -> 0.34 ms with 8 CTAs a node, 0.75 ms with one.  (Cholesky in CTA 0
+// alone, where its chunks compete for four quarters, took 286 k cycles against 168 k.)
 //
 // Every number is formed by the operations of the one-CTA kernel in the same order (dot products by
 // row chunks of 32 and a butterfly over the lanes, updates one fused multiply-add at a time), so the
