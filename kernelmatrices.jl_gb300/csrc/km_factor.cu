@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "km_cluster.cuh"
 #include "km_kernels.h"
 
 namespace km {
@@ -343,9 +344,8 @@ __global__ void __launch_bounds__(leaf_qr_threads<T>()) k_leaf_formq(T* __restri
 }
 
 // ---------------------------------------------------------------------------------------------
-// Node factorisation in float pairs (the FP64 form is in km_node64.cu), one CTA (1024 threads) per
-// node of level l.  Given the children's R factors
-// (slots c1, c2) and Sc = chol(S) (lower):
+// Node factorisation in float pairs (the FP64 form is in km_node64.cu), one CTA or a cluster of 2, 4 or 8
+// CTAs per node of level l.  Given the children's R factors (slots c1, c2) and Sc = chol(S) (lower):
 //   T1 = R1 Sc^{-T}, T2 = R2 Sc^{-T}   (upper triangular)
 //   Ct = T1 T2'                        (= R1 S^{-1} R2')
 //   L22 = chol(I - Ct' Ct)
@@ -353,33 +353,24 @@ __global__ void __launch_bounds__(leaf_qr_threads<T>()) k_leaf_formq(T* __restri
 //              reflector j is e_j on top plus a dense bottom part, kept in Eref[:, j])
 // Outputs per node: Ct, L22 (lower), Eref (r x r), Etau (r), R_N into slot N.
 //
-// Work mapping: the products are split into (column c, 32-row chunk s) items, one warp per
-// item, lane = row, so that no index needs a division by r and the warps stay converged; sums
-// use the Dot2 accumulator (km_ff.cuh).  The Cholesky runs in dataflow order over columns (one
-// warp per column, shared-memory flags instead of block barriers), L22^{-1} B is then solved by
-// blocks of 8 rows with all threads, and the QR is a dataflow pipeline in which each warp owns
-// four columns and forms their reflectors itself.
-// Shared memory: four r x (r+1) matrices, three r-vectors and r + 1 flags.
-//
-// Cluster form (csize = 2, 4 or 8 CTAs per node, 1-D thread-block clusters): on levels with fewer
-// nodes than SMs the product phases (T1, T2, Ct, H, B) are split by columns over the CTAs of the
-// node's cluster, CTA `rank` taking columns rank, rank + csize, ...  Every CTA loads the inputs;
-// T1, T2 and Ct are all-gathered by storing each column into every CTA's shared memory
-// (distributed shared memory), H and B are stored into CTA 0 only, and cluster barriers separate
-// the phases (they also make sure that every CTA has started before the first remote store and
-// that no CTA exits while others still write to it).  CTA 0 then runs the Cholesky, the solve,
-// the QR and the stores alone; the other CTAs return.  With csize = 1 the kernel is the
-// one-CTA form (block barriers, local stores).
+// Products: (column, 32-row chunk) or entry items over the threads, sums in the Dot2 accumulator
+// (km_ff.cuh).  In a cluster every CTA loads the inputs and takes the columns rank, rank + csize, ... of
+// T1 and Ct, which go into every CTA's shared memory, and the rows of T2 that it needs itself; H goes to
+// CTA 0, the columns of B to the others.  Cluster barriers separate the phases (they also make sure that
+// every CTA has started before the first remote store and that no CTA exits while others write to it).
+// Cholesky: one warp factors panels of 4 columns in registers, other warps apply them; a panel's chain of
+// square roots and reciprocals (about 450 cycles a column) bounds it, so that its warp has its quarter of
+// the SM to itself.  L22^{-1} B follows one panel behind, in the same CTA or in the other CTAs of the
+// cluster, which get every panel in one bulk copy; CTA 0 collects the result.
+// QR (CTA 0): a dataflow pipeline in which each warp owns four columns and forms their reflectors itself.
+// Rank 72, cycles of a node: 265 k with one CTA (was 425 k with a warp per Cholesky column, flags between
+// them, and the solve after it), 134 k with 8 (was 245 k).
+// Shared memory: four r x 82 matrices, three r-vectors, barriers, flags and the list of H's entries.
 // ---------------------------------------------------------------------------------------------
 // Iteration bound of a spin wait on a shared-memory flag (a few tens of cycles per iteration:
 // well above any legitimate wait inside one node, far below a watchdog).  The spin does not
 // sleep: a sleeping waiter wakes too late for the column-to-column handoff.
 constexpr int kWaitLimit = 1 << 22;
-
-template <typename T>
-__device__ __forceinline__ T sel(bool p, T a) {
-  return p ? a : T(0.0);
-}
 
 // v into the same shared-memory location as p in every CTA of the cluster (locally if csize = 1)
 template <typename T>
@@ -408,8 +399,77 @@ __device__ __forceinline__ void node_barrier(int csize) {
   else cg::this_cluster().sync();
 }
 
+// up to 96 registers a thread (with 1024 threads some values went to local memory); warps for 80 QR columns
+constexpr int kNodeThreads = 640;
+constexpr int kPanel = 4;    // columns of L22 factored at a time
+// columns of the shared-memory matrices lie this far apart: above the largest rank (80), a constant, so
+// that addresses are immediates, and 16 bytes times an odd number, so that two neighbours of a column
+// are one load and the lanes' loads from 8 columns hit different banks
+constexpr int kNodeLd = 82;
+
+constexpr int kPivotRow = 81;  // (row 81 of a column is free)
+
+struct __align__(16) ffpair {
+  ff a, b;
+};
+// elements l and l + 1 (l even) of a column
+__device__ __forceinline__ ffpair two(const ff* p) { return *reinterpret_cast<const ffpair*>(p); }
+
+// The kPanel = 4 columns c0 .. c0 + 3 of L22 by one warp, element (i, c) at X[i + c kNodeLd]: the rows
+// from the chunk of c0 down in its lanes, NC chunks of 32.  The columns hold their accumulators, all
+// earlier panels applied.  The reciprocal pivot of column c goes to X[kPivotRow + c kNodeLd], into bad
+// the first column (from 1) whose pivot is not positive.
+template <int NC>
+__device__ __forceinline__ void chol_panel(ff* X, int r, int c0, int lane, int& bad) {
+  constexpr int ld = kNodeLd;
+  const int i0 = (c0 & ~31) + lane;
+  ffacc v[4][NC];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int s = 0; s < NC; ++s) {
+      const int i = i0 + 32 * s, c = c0 + j;
+      v[j][s] = (i >= c && i < r && c < r) ? X[i + c * ld] : ff(0.f, 0.f);
+    }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int c = c0 + j;
+    if (c >= r) break;
+    const ff d = shfl_idx(accv(v[j][0]), c & 31);
+    if (!(d > 0.0) && bad == 0) bad = c + 1;
+    const ff sd = d > 0.0 ? sqrt(d) : ff(1.0);
+    const ff inv = ff_recip(sd);
+    ff x[NC];
+#pragma unroll
+    for (int s = 0; s < NC; ++s) {
+      const int i = i0 + 32 * s;
+      x[s] = accv(v[j][s]) * inv;
+      if (i == c) x[s] = sd;
+      if (i >= c && i < r) X[i + c * ld] = x[s];
+    }
+    if (lane == 0) X[kPivotRow + c * ld] = inv;
+#pragma unroll
+    for (int q = j + 1; q < 4; ++q) {
+      const ff m = shfl_idx(x[0], (c0 + q) & 31);
+#pragma unroll
+      for (int s = 0; s < NC; ++s) v[q][s] -= x[s] * m;
+    }
+  }
+}
+
+// Entry (i, c), i >= c, number e of a lower triangle of order r: columns p and r - 1 - p together hold
+// r + 1 entries, so consecutive threads take consecutive entries of such a pair, and every part of the
+// numbering has early and late columns.  False for the second half of the middle column of an odd r.
+__device__ __forceinline__ bool lower_entry(int e, int r, int& i, int& c) {
+  const int p = e / (r + 1), u = e - p * (r + 1);
+  if (u >= r - p && 2 * p == r - 1) return false;
+  c = u < r - p ? p : r - 1 - p;
+  i = u < r - p ? p + u : r - 1 - p + (u - (r - p));
+  return true;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(1024) k_node_factor(T* __restrict__ R, const T* __restrict__ SinvT,
+__global__ void __launch_bounds__(kNodeThreads) k_node_factor(T* __restrict__ R, const T* __restrict__ SinvT,
                                                      int r, int level, int L, int64_t nleaf,
                                                      int64_t cbase, int64_t nbase, T* __restrict__ Ct_out,
                                                      T* __restrict__ L22_out, T* __restrict__ Eref,
@@ -417,7 +477,7 @@ __global__ void __launch_bounds__(1024) k_node_factor(T* __restrict__ R, const T
                                                      int csize, int wait_limit) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
-  const int ld = r + 1;
+  constexpr int ld = kNodeLd;
   // polls of a flag before a wait gives up; wait_limit 0: every wait gives up at its first poll,
   // as if its flag were never set (the test of the timeout path)
   const int lim = wait_limit < 0 ? kWaitLimit : wait_limit;
@@ -425,10 +485,13 @@ __global__ void __launch_bounds__(1024) k_node_factor(T* __restrict__ R, const T
   T* X1 = X0 + r * ld;
   T* X2 = X1 + r * ld;
   T* X3 = X2 + r * ld;
-  T* va = X3 + r * ld;  // r values: sqrt(d_j), then the reflector betas
-  T* vb = va + r;       // r values: 1 / L22[j][j], then the reflector scales
+  T* va = X3 + r * ld;  // r values: the reflector betas
+  T* vb = va + r;       // r values: the reflector scales
   T* vc = vb + r;       // r values: the reflector taus
-  int* flags = reinterpret_cast<int*>(vc + r);  // r + 1 ints: column published / first bad pivot
+  const int np = (r + kPanel - 1) / kPanel;  // panels of L22
+  unsigned long long* pbar = reinterpret_cast<unsigned long long*>(vc + r);  // np: a panel of L22 has arrived
+  int* flags = reinterpret_cast<int*>(pbar + np);  // r ints: reflector published
+  unsigned short* tab = reinterpret_cast<unsigned short*>(flags + r);  // entries of H by columns: row | column << 8
   const int64_t k = blockIdx.x / csize;
   const int rank = (int)(blockIdx.x % csize);  // rank in the node's cluster (1-D clusters)
   const int64_t node = nbase + k;  // node index within all nodes (level-major)
@@ -436,187 +499,303 @@ __global__ void __launch_bounds__(1024) k_node_factor(T* __restrict__ R, const T
   const T* R2 = R + (cbase + 2 * k + 1) * (int64_t)r * r;
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nth >> 5;
   const int nch = (r + 31) >> 5;   // 32-row chunks per column (r <= 96)
-  // product items of this CTA: (column c = rank + csize * lc, 32-row chunk s)
-  const int nitems = ((r - rank + csize - 1) / csize) * nch;
-  for (int e = tid; e <= r; e += nth) flags[e] = (e < r) ? 0 : r + 1;
-  // load: X0 = Sc^{-T} (upper), X1 = R1, X2 = R2   (element (i,c) at i + c*ld)
-  for (int c = w; c < r; c += nw)
-    for (int i = lane; i < r; i += 32) {
-      const int e = i + c * r;
-      X0[i + c * ld] = SinvT[e];
-      X1[i + c * ld] = R1[e];
-      X2[i + c * ld] = R2[e];
-    }
-  node_barrier(csize);
-  // T1 = R1 Sc^{-T} -> X3: T1[i][c] = sum_{l = i..c} R1[i][l] Sinv[l][c]
-  for (int q = w; q < nitems; q += nw) {
-    const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane, ii = min(i, r - 1);
-    acc_t<T> a0{}, a1{};
-    int l = 32 * s;
-    for (; l + 1 <= c; l += 2) {
-      a0 += sel(l >= i, X1[ii + l * ld]) * X0[l + c * ld];
-      a1 += sel(l + 1 >= i, X1[ii + (l + 1) * ld]) * X0[l + 1 + c * ld];
-    }
-    if (l <= c) a0 += sel(l >= i, X1[ii + l * ld]) * X0[l + c * ld];
-    if (i < r) put_all(X3 + i + c * ld, accv(a0) + accv(a1), csize);
-  }
-  node_barrier(csize);
-  // T2 = R2 Sc^{-T} -> X1
-  for (int q = w; q < nitems; q += nw) {
-    const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane, ii = min(i, r - 1);
-    acc_t<T> a0{}, a1{};
-    int l = 32 * s;
-    for (; l + 1 <= c; l += 2) {
-      a0 += sel(l >= i, X2[ii + l * ld]) * X0[l + c * ld];
-      a1 += sel(l + 1 >= i, X2[ii + (l + 1) * ld]) * X0[l + 1 + c * ld];
-    }
-    if (l <= c) a0 += sel(l >= i, X2[ii + l * ld]) * X0[l + c * ld];
-    if (i < r) put_all(X1 + i + c * ld, accv(a0) + accv(a1), csize);
-  }
-  node_barrier(csize);
-  // Ct = T1 T2' -> X0: Ct[i][c] = sum_{l >= max(i, c)} T1[i][l] T2[c][l]
-  for (int q = w; q < nitems; q += nw) {
-    const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane, ii = min(i, r - 1);
-    acc_t<T> a0{}, a1{};
-    int l = max(32 * s, c);
-    for (; l + 1 < r; l += 2) {
-      a0 += sel(l >= i, X3[ii + l * ld]) * X1[c + l * ld];
-      a1 += sel(l + 1 >= i, X3[ii + (l + 1) * ld]) * X1[c + (l + 1) * ld];
-    }
-    if (l < r) a0 += sel(l >= i, X3[ii + l * ld]) * X1[c + l * ld];
-    if (i < r) put_all(X0 + i + c * ld, accv(a0) + accv(a1), csize);
-  }
-  node_barrier(csize);
-  // H = I - Ct' Ct -> X3 of CTA 0 (lower triangle); CTA 0 reloads R1 into X1 for the QR meanwhile
-  if (level < L && rank == 0)
+  const bool solve = level < L;
+  // own columns of T1 and Ct (rows of T2) c = rank + csize lc, in items (lc, 32-row chunk s)
+  const int nitems = (r - rank + csize - 1) / csize * nch;
+  // own columns of B: c = cfirst + cstep lc; in a cluster CTA 0 has none, it factors H
+  const int cstep = csize > 1 ? csize - 1 : 1, cfirst = csize > 1 ? rank - 1 : 0;
+  const int nown = cfirst < 0 ? 0 : (r - cfirst + cstep - 1) / cstep;
+  // upper triangle of an r x r matrix, zero below, with all loads of a warp in flight
+  auto load = [&](T* X, const T* G, bool own) {
+    constexpr int kC = (80 + kNodeThreads / 32 - 1) / (kNodeThreads / 32);
+    T t[kC][3];
+#pragma unroll
+    for (int a = 0; a < kC; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const int c = w + nw * a, i = lane + 32 * b;
+        t[a][b] = (i <= c && c < r && (!own || c % cstep == cfirst)) ? G[i + c * r] : T(0.0);
+      }
+#pragma unroll
+    for (int a = 0; a < kC; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const int c = w + nw * a, i = lane + 32 * b;
+        if (i < r && c < r) X[i + c * ld] = t[a][b];
+      }
+  };
+  for (int e = tid; e < r; e += nth) flags[e] = 0;
+  if (rank == 0)
     for (int c = w; c < r; c += nw)
-      for (int i = lane; i < r; i += 32) X1[i + c * ld] = R1[i + c * r];
-  for (int q = w; q < nitems; q += nw) {
-    const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane, ii = min(i, r - 1);
-    if (32 * s + 31 < c) continue;
-    acc_t<T> a0{}, a1{};
-    int l = 0;
-    for (; l + 1 < r; l += 2) {
-      a0 += X0[l + ii * ld] * X0[l + c * ld];
-      a1 += X0[l + 1 + ii * ld] * X0[l + 1 + c * ld];
+      for (int i = c + lane; i < r; i += 32) tab[c * r - c * (c - 1) / 2 + i - c] = (unsigned short)(i | c << 8);
+  if (csize > 1 && solve)
+    for (int e = tid; e < np; e += nth) {
+      const unsigned b = smem_u32(pbar + e), n = min(kPanel, r - kPanel * e) * ld * sizeof(T);
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(n) : "memory");
     }
-    if (l < r) a0 += X0[l + ii * ld] * X0[l + c * ld];
-    if (i < r && i >= c) put_rank0(X3 + i + c * ld, (i == c ? T(1.0) : T(0.0)) - (accv(a0) + accv(a1)), csize);
-  }
-  // B = R2 - Ct' R1 -> X2 of CTA 0 (column c of R1 has entries l <= c; R1 read from global memory)
-  if (level < L)
-    for (int q = w; q < nitems; q += nw) {
-      const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane, ii = min(i, r - 1);
-      const T* r1 = R1 + (int64_t)c * r;
-      acc_t<T> a0{}, a1{};
-      int l = 0;
-      for (; l + 1 <= c; l += 2) {
-        a0 += X0[l + ii * ld] * r1[l];
-        a1 += X0[l + 1 + ii * ld] * r1[l + 1];
-      }
-      if (l <= c) a0 += X0[l + ii * ld] * r1[l];
-      if (i < r) put_rank0(X2 + i + c * ld, X2[i + c * ld] - (accv(a0) + accv(a1)), csize);
-    }
+  // X0 = Sc^{-T}, X1 = R1, X2 = R2, all upper triangular   (element (i,c) at i + c*ld)
+  load(X0, SinvT, false);
+  load(X1, R1, false);
+  load(X2, R2, false);
   node_barrier(csize);
-  if (rank != 0) return;  // the rest runs in CTA 0; no CTA touches another's memory after the barrier
-  // L22 = chol(H) by columns in dataflow order.  Warp w owns columns w, w + nw, ... and finishes
-  // them in increasing order: column c accumulates the contributions of columns k < c as soon as
-  // each is published (flag[k] set after its values are in shared memory), then takes its pivot
-  // and publishes itself; vc[c] keeps the reciprocal pivot.  No block barrier inside the loop.
-  // Waits are bounded; a wait that runs out marks the node with info = -1 (reported as a
-  // timeout) and the kernel carries on.
-  int bad = 0;
-  {
-    volatile int* vflag = flags;
-    int known = 0;           // columns 0 .. known-1 are published (as seen by this warp)
-    bool timed_out = false;  // after one expired wait this warp stops waiting
-    for (int c = w; c < r; c += nw) {
-      acc_t<T> v[3];
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int i = 32 * s + lane;
-        v[s] = (i >= c && i < r) ? X3[i + c * ld] : T(0.0);
-      }
-      for (int k = 0; k < c; ++k) {
-        if (k >= known && !timed_out) {
-          int spins = 0;
-          // a warp more than two columns behind the pivot it waits for is off the critical
-          // chain: it naps between polls, so that its polls do not take issue slots from the
-          // warp that forms the next column
-          const bool nap = c - k > 2;
-          while (wait_limit == 0 || vflag[k] == 0) {
-            if (++spins > lim) {
-              if (lane == 0) info[node] = -1;
-              timed_out = true;
-              break;
-            }
-            if (nap) __nanosleep(32);
-          }
-          __threadfence_block();
-          known = k + 1;
-          while (known < c && vflag[known] != 0) ++known;
-          __threadfence_block();
-        }
-        const T lck = X3[c + k * ld];
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-          if (32 * s + 31 < c) continue;
-          const int i = 32 * s + lane;
-          if (i >= c && i < r) v[s] -= X3[i + k * ld] * lck;
-        }
-      }
-      const int cs = c >> 5;
-      const T d = shfl_idx(accv(cs == 0 ? v[0] : (cs == 1 ? v[1] : v[2])), c & 31);
-      if (!(d > 0.0) && bad == 0) bad = c + 1;
-      const T sd = d > 0.0 ? sqrt(d) : T(1.0);
-      const T inv = ff_recip(sd);
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        const int i = 32 * s + lane;
-        if (i == c) X3[i + c * ld] = sd;
-        else if (i > c && i < r) X3[i + c * ld] = accv(v[s]) * inv;
-      }
-      if (lane == 0) vc[c] = inv;
-      __threadfence_block();
-      __syncwarp();
-      if (lane == 0) vflag[c] = 1;
+  // T1 = R1 Sc^{-T} -> X3 of every CTA: T1[i][c] = sum_{l = i..c} R1[i][l] Sinv[l][c]
+  // (in all products a0 takes the first, third, ... term, a1 the second, fourth, ...)
+  auto upper = [&](const T* A, int s, int c) {
+    const T *a = A + min(32 * s + lane, r - 1), *x = X0 + c * ld;
+    acc_t<T> a0{}, a1{};
+    int l = 32 * s;
+#pragma unroll 2
+    for (; l + 1 <= c; l += 2) {
+      const ffpair v = two(x + l);
+      a0 += a[l * ld] * v.a;
+      a1 += a[(l + 1) * ld] * v.b;
     }
+    if (l <= c) a0 += a[l * ld] * x[l];
+    return accv(a0) + accv(a1);
+  };
+  for (int q = w; q < nitems; q += nw) {
+    const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane;
+    if (32 * s > c) continue;
+    const T v = upper(X1, s, c);
+    if (i < r) put_all(X3 + i + c * ld, v, csize);
   }
   __syncthreads();
-  // B' = L22^{-1} B (element (i, c) at X2[i + c * ld]) by blocks of 8 rows: the rows of a block
-  // take the contributions of all earlier rows (one output per thread, a dot product over the
-  // solved rows), then a thread per column solves them with the 8 x 8 diagonal block.
-  if (level < L)
-    for (int k0 = 0; k0 < r; k0 += 8) {
-      const int kb = min(8, r - k0);
-      if (k0 > 0) {
-        for (int e = tid; e < kb * r; e += nth) {
-          const int jj = e % kb, c = e / kb;
-          acc_t<T> acc = X2[k0 + jj + c * ld];
-          for (int q = 0; q < k0; ++q) acc -= X3[k0 + jj + q * ld] * X2[q + c * ld];
-          X2[k0 + jj + c * ld] = accv(acc);
-        }
-        __syncthreads();
+  // T2' = (R2 Sc^{-T})' -> X1 (T2[i][c] at c + i ld), own rows only: the other CTAs need no part of them
+  for (int q = w; q < nitems; q += nw) {
+    const int lc = q / nch, s = q - lc * nch;
+    if (csize == 1) {  // a column of all rows: even work for the lanes
+      const int c = lc, i = 32 * s + lane;
+      if (32 * s > c) continue;
+      const T v = upper(X2, s, c);
+      if (i < r) X1[c + i * ld] = v;
+    } else {
+      const int i = rank + csize * lc, c = 32 * s + lane;
+      if (c < i || c >= r) continue;
+      const T *a = X2 + i, *x = X0 + c * ld;
+      acc_t<T> a0{}, a1{};
+      int l = i & ~1;
+#pragma unroll 2
+      for (; l + 1 <= c; l += 2) {
+        const ffpair v = two(x + l);
+        a0 += a[l * ld] * v.a;
+        a1 += a[(l + 1) * ld] * v.b;
       }
-      if (tid < r) {
-        T y[8];
+      if (l <= c) a0 += a[l * ld] * x[l];
+      X1[c + i * ld] = accv(a0) + accv(a1);
+    }
+  }
+  node_barrier(csize);
+  // Ct = T1 T2' -> X0 of every CTA: Ct[i][c] = sum_{l >= max(i, c)} T1[i][l] T2[c][l]
+  for (int q = w; q < nitems; q += nw) {
+    const int lc = q / nch, s = q - lc * nch, c = rank + csize * lc, i = 32 * s + lane;
+    const T *a = X3 + min(i, r - 1), *x = X1 + c * ld;
+    acc_t<T> a0{}, a1{};
+    int l = max(32 * s, c);
+    const bool odd = l & 1;
+    if (odd) {
+      a1 += a[l * ld] * x[l];  // (the two sums change places)
+      ++l;
+    }
+#pragma unroll 2
+    for (; l + 1 < r; l += 2) {
+      const ffpair v = two(x + l);
+      a0 += a[l * ld] * v.a;
+      a1 += a[(l + 1) * ld] * v.b;
+    }
+    if (l < r) a0 += a[l * ld] * x[l];
+    const T u = odd ? accv(a1) : accv(a0), v = odd ? accv(a0) : accv(a1);
+    if (i < r) put_all(X0 + i + c * ld, u + v, csize);
+  }
+  node_barrier(csize);
+  // R1 into X1 again: the own columns for B, all of them in CTA 0 for the QR
+  if (solve) load(X1, R1, rank != 0);
+  // H = I - Ct' Ct -> X3 of CTA 0, lower triangle; B costs as much as H, and CTA 0 has no part of B
+  const int nh = (r + 1) / 2 * (r + 1), h0 = solve ? min(nh, (2 * nh + csize - 1) / csize) : (nh + csize - 1) / csize;
+  const int hs = csize > 1 ? (nh - h0 + csize - 2) / (csize - 1) : 0;
+  const int hbeg = rank ? h0 + (rank - 1) * hs : 0, hend = min(nh, hbeg + (rank ? hs : h0));
+  for (int e = hbeg + tid; e < hend; e += nth) {
+    int i, c;
+    if (!lower_entry(e, r, i, c)) continue;
+    const T *x = X0 + i * ld, *y = X0 + c * ld;
+    acc_t<T> a0{}, a1{};
+    int l = 0;
+#pragma unroll 2
+    for (; l + 1 < r; l += 2) {
+      const ffpair u = two(x + l), v = two(y + l);
+      a0 += u.a * v.a;
+      a1 += u.b * v.b;
+    }
+    if (l < r) a0 += x[l] * y[l];
+    put_rank0(X3 + i + c * ld, (i == c ? T(1.0) : T(0.0)) - (accv(a0) + accv(a1)), csize);
+  }
+  // B = R2 - Ct' R1 -> X2, own columns (column c of R1 has entries l <= c), from the last thread down:
+  // the upper threads of a cluster's CTA have no entry of H
+  if (solve) {
+    __syncthreads();
+    for (int e = nth - 1 - tid; e < nown * r; e += nth) {
+      const int lc = e / r, i = e - lc * r, c = cfirst + cstep * lc;
+      const T *x = X0 + i * ld, *y = X1 + c * ld;
+      acc_t<T> a0{}, a1{};
+      int l = 0;
+#pragma unroll 2
+      for (; l + 1 <= c; l += 2) {
+        const ffpair u = two(x + l), v = two(y + l);
+        a0 += u.a * v.a;
+        a1 += u.b * v.b;
+      }
+      if (l <= c) a0 += x[l] * y[l];
+      X2[i + c * ld] = X2[i + c * ld] - (accv(a0) + accv(a1));
+    }
+  }
+  node_barrier(csize);
+  if (rank != 0 && !solve) return;  // (no CTA touches another's memory from here on)
+  // L22 = chol(H) in CTA 0 by panels of 4 columns and B' = L22^{-1} B by the CTAs that own its columns
+  // (element (i, c) at X2[i + c * ld]), one panel behind.  In step p
+  //   in CTA 0 four other warps on the SM quarter of warp 0 apply panel p - 1 to panel p, a column each,
+  //   then warp 0 factors it and copies it to the other CTAs;
+  //   warps 1 to 3, a thread per own column, take panel p - 2 in the rows of panel p - 1, solve these
+  //   and hand them to CTA 0;
+  //   the other warps apply panel p - 1 to the entries of H behind panel p and panel p - 2 to the rows
+  //   of B from panel p on; (Next to seven busy warps warp 0 would take 7500 cycles for a panel, alone
+  //   it takes 1400 to 2000.)
+  // An unfinished entry of H or B is its accumulator.  Rows of B are renormalised when all rows before
+  // their block of 8 are in.
+  {
+    const int wid = w < 4 ? -1 : rank ? w - 4 : (w & 3) ? 3 * (w >> 2) + (w & 3) - 4 : -1;
+    const int nwk = rank ? nw - 4 : 3 * (nw / 4 - 1), id = 32 * wid + lane, nid = 32 * nwk;
+    int bad = 0;
+    bool dead = false;
+    for (int p = rank ? 1 : 0; p < np + (solve ? 1 : 0); ++p) {
+      const int c0 = kPanel * p, k0 = c0 - kPanel, q0 = k0 - kPanel;  // panels p, p - 1, p - 2
+      if (rank && !dead && !bar_wait(smem_u32(pbar + p - 1), wait_limit, csize)) {
+        if (lane == 0) info[node] = -1;
+        dead = true;
+      }
+      if (rank == 0 && p > 0 && p < np && !(w & 3) && w <= 4 * kPanel) {
+        const int c = c0 + (w >> 2) - 1;
+        if (w > 0 && c < r) {
+          const T *a = X3 + k0 * ld, *b = a + c;
+          T *col = X3 + c * ld, m[kPanel];
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          if (jj < kb) {
-            acc_t<T> acc = X2[k0 + jj + tid * ld];
+          for (int q = 0; q < kPanel; ++q) m[q] = b[q * ld];
+          acc_t<T> v[3];
 #pragma unroll
-            for (int q = 0; q < jj; ++q) acc -= X3[k0 + jj + (k0 + q) * ld] * y[q];
-            y[jj] = accv(acc) * vc[k0 + jj];
-            X2[k0 + jj + tid * ld] = y[jj];
+          for (int s = 0; s < 3; ++s) {
+            const int i = min(32 * s + lane, r - 1);
+            v[s] = col[i];
+            if (32 * s + 31 < c) continue;
+#pragma unroll
+            for (int q = 0; q < kPanel; ++q) v[s] -= a[i + q * ld] * m[q];
+          }
+#pragma unroll
+          for (int s = 0; s < 3; ++s)
+            if (32 * s + lane >= c && 32 * s + lane < r) col[32 * s + lane] = T(v[s].s, v[s].c);
+        }
+        asm volatile("bar.sync 1, 160;" ::: "memory");  // (warps 0, 4, 8, 12, 16)
+      }
+      if (w == 0) {
+        if (rank == 0 && p < np) switch (nch - (c0 >> 5)) {
+            case 1: chol_panel<1>(X3, r, c0, lane, bad); break;
+            case 2: chol_panel<2>(X3, r, c0, lane, bad); break;
+            default: chol_panel<3>(X3, r, c0, lane, bad);
+          }
+        if (rank == 0 && p < np && csize > 1 && solve) {
+          // the panel with its reciprocal pivots to the other CTAs, a copy each
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane > 0 && lane < csize) {
+            const unsigned src = smem_u32(X3 + c0 * ld), n = min(kPanel, r - c0) * ld * sizeof(T);
+            copy_to_rank(at_rank(src, lane), src, n, at_rank(smem_u32(pbar + p), lane));
+          }
+        }
+      } else if (w < 4) {
+        if (solve && p > 0 && tid - 32 < nown) {
+          T* b = X2 + (cfirst + cstep * (tid - 32)) * ld;
+          const T* l = X3 + k0;
+          T y[kPanel];
+          acc_t<T> acc[kPanel];
+#pragma unroll
+          for (int j = 0; j < kPanel; ++j) acc[j] = b[min(k0 + j, r - 1)];
+          if (p >= 2) {
+#pragma unroll
+            for (int q = 0; q < kPanel; ++q) y[q] = b[q0 + q];
+#pragma unroll
+            for (int j = 0; j < kPanel; ++j) {
+              if ((k0 & 7) && k0 > kPanel) acc[j] = accv(acc[j]);
+#pragma unroll
+              for (int q = 0; q < kPanel; ++q) acc[j] -= l[j + (q0 + q) * ld] * y[q];
+              if (!(k0 & 7)) acc[j] = accv(acc[j]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < kPanel; ++j) {
+            if (k0 + j >= r) break;
+#pragma unroll
+            for (int q = 0; q < j; ++q) acc[j] -= l[j + (k0 + q) * ld] * y[q];
+            y[j] = accv(acc[j]) * l[kPivotRow - k0 + (k0 + j) * ld];
+          }
+#pragma unroll
+          for (int j = 0; j < kPanel; ++j)
+            if (k0 + j < r) {
+              b[k0 + j] = y[j];
+              if (csize > 1) put_rank0(b + k0 + j, y[j], csize);
+            }
+        }
+      } else if (wid >= 0) {
+        const int cc = c0 + kPanel;
+        if (rank == 0 && p > 0 && cc < r) {
+          for (int e = cc * r - cc * (cc - 1) / 2 + id; e < r * (r + 1) / 2; e += nid) {
+            const int i = tab[e] & 255, c = tab[e] >> 8;
+            const T *a = X3 + i + k0 * ld, *b = X3 + c + k0 * ld;
+            acc_t<T> v = X3[i + c * ld];
+#pragma unroll
+            for (int q = 0; q < kPanel; ++q) v -= a[q * ld] * b[q * ld];
+            X3[i + c * ld] = T(v.s, v.c);
+          }
+        }
+        if (nown > 0 && solve && p >= 2 && c0 < r) {
+          // two columns at a time, which share the loads of L22
+          const int m = r - c0, dl = nid / m, di = nid - dl * m;
+          int lc = id / m, i = id - lc * m;
+          while (2 * lc < nown) {
+            T* b0 = X2 + (cfirst + cstep * 2 * lc) * ld + q0;
+            T* b1 = 2 * lc + 1 < nown ? b0 + cstep * ld : b0;
+            const T* l = X3 + c0 + i + q0 * ld;
+            acc_t<T> u = b0[2 * kPanel + i], v = b1[2 * kPanel + i];
+#pragma unroll
+            for (int q = 0; q < kPanel; q += 2) {
+              const ffpair x = two(b0 + q), y = two(b1 + q);
+              const T l0 = l[q * ld], l1 = l[(q + 1) * ld];
+              u -= l0 * x.a;
+              v -= l0 * y.a;
+              u -= l1 * x.b;
+              v -= l1 * y.b;
+            }
+            b0[2 * kPanel + i] = T(u.s, u.c);
+            if (b1 != b0) b1[2 * kPanel + i] = T(v.s, v.c);
+            i += di;
+            lc += dl;
+            if (i >= m) {
+              i -= m;
+              ++lc;
+            }
           }
         }
       }
       __syncthreads();
     }
-  // a warp's first non-positive pivot; the smallest over the warps is written below
-  if (lane == 0 && bad) atomicMin(flags + r, bad);
-  __syncthreads();
-  if (tid == 0 && flags[r] < r + 1 && info[node] == 0) info[node] = flags[r];
+    if (tid == 0 && bad && info[node] == 0) info[node] = bad;
+    if (csize > 1 && solve) {
+      // after a wait that gave up: all panels have arrived (all are sent), so that nothing is on its way
+      // to this CTA when it leaves
+      if (dead)
+        for (int p = 0; p < np; ++p) bar_wait(smem_u32(pbar + p), -1, csize);
+      node_barrier(csize);
+      if (rank != 0) return;
+    }
+  }
   // store Ct and L22
   for (int c = w; c < r; c += nw)
     for (int i = lane; i < r; i += 32) {
@@ -634,8 +813,6 @@ __global__ void __launch_bounds__(1024) k_node_factor(T* __restrict__ R, const T
   // X2[:, j], beta, scale and tau into va, vb, vc, then flag[j]).  No block barrier inside the
   // loop; three of four handoffs stay inside a warp.  The betas and the scaling of the reflector
   // columns are applied in the output loop.
-  for (int e = tid; e < r; e += nth) flags[e] = 0;  // reused: the Cholesky waits ended at the barrier above
-  __syncthreads();
   const int gq = lane & 7, grp = lane >> 3;
   const int rpl = (r + 7) >> 3;  // rows per lane (<= 10 for r <= 80)
   auto gsum = [&](T x) {
@@ -952,14 +1129,15 @@ void launch_node_factor(T* R, const T* SinvT, int r, int level, const Tree& t, T
   } else {
     const int64_t cbase = (level == 1) ? 0 : t.nleaf + t.node_off[level - 1];
     const int64_t nbase = t.node_off[level];
-    const size_t sm = ((size_t)4 * r * (r + 1) + 3 * r) * sizeof(T) + (size_t)(r + 1) * sizeof(int);
+    const size_t sm = ((size_t)4 * r * kNodeLd + 3 * r + (r + kPanel - 1) / kPanel) * sizeof(T) + (size_t)r * sizeof(int) +
+                      (size_t)r * (r + 1) / 2 * sizeof(unsigned short);
     smem_limit((const void*)k_node_factor<T>, sm);
     const int64_t nodes = t.nodes_at(level);
-    const int cs = node_cluster_size(1, (const void*)k_node_factor<T>, nodes, 1024, sm, max_cluster);
+    const int cs = node_cluster_size(1, (const void*)k_node_factor<T>, nodes, kNodeThreads, sm, max_cluster);
     if (cs > 1) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)(nodes * cs));
-      cfg.blockDim = dim3(1024);
+      cfg.blockDim = dim3(kNodeThreads);
       cfg.dynamicSmemBytes = sm;
       cfg.stream = st;
       cudaLaunchAttribute at[1];
@@ -978,7 +1156,7 @@ void launch_node_factor(T* R, const T* SinvT, int r, int level, const Tree& t, T
       if (prior == cudaSuccess) cudaGetLastError();
     }
     {
-      k_node_factor<T><<<(unsigned)nodes, 1024, sm, st>>>(R, SinvT, r, level, t.L, t.nleaf, cbase, nbase, Ct, L22,
+      k_node_factor<T><<<(unsigned)nodes, kNodeThreads, sm, st>>>(R, SinvT, r, level, t.L, t.nleaf, cbase, nbase, Ct, L22,
                                                           Eref, Etau, info, 1, wait_limit);
     }
   }

@@ -30,6 +30,7 @@
 // factor's bits do not depend on the cluster size.
 #include <cooperative_groups.h>
 
+#include "km_cluster.cuh"
 #include "km_kernels.h"
 
 namespace km {
@@ -41,55 +42,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kSpin = 1 << 22;     // polls of a shared-memory flag before a wait gives up
-constexpr long long kWaitCycles = 1ll << 28;  // clock cycles before a barrier wait gives up (0.13 s)
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// the address of shared-memory location `a` in CTA `rank` of the cluster
-__device__ __forceinline__ unsigned at_rank(unsigned a, int rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-
-__device__ __forceinline__ void st_async(unsigned addr, double v, unsigned bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
-               "l"(__double_as_longlong(v)), "r"(bar)
-               : "memory");
-}
-
-// Cluster instructions (mapa, st.async, cluster-scope waits) are for launches with a cluster
-// dimension only: in a plain launch the node kernel's st.async raised an illegal instruction.  A
-// one-CTA node therefore stores locally and arrives on the barrier itself.
-__device__ __forceinline__ bool bar_try(unsigned bar, int cs) {
-  unsigned ok;
-  if (cs > 1)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar)
-        : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar)
-        : "memory");
-  return ok != 0;
-}
-
-// Waits for phase 0 of the barrier; false if it gave up (after wait_limit tries, < 0: kWaitCycles)
-__device__ __forceinline__ bool bar_wait(unsigned bar, int wait_limit, int cs) {
-  const long long t0 = clock64();
-  int n = 0;
-  while (wait_limit == 0 || !bar_try(bar, cs))
-    if (wait_limit >= 0 ? ++n > wait_limit : clock64() - t0 > kWaitCycles) return false;
-  return true;
-}
 
 // v into the same location of every CTA (local store if the cluster is one CTA)
 __device__ __forceinline__ void put_all(double* p, double v, int cs) {
