@@ -629,9 +629,8 @@ T* P(double* p) {
   return reinterpret_cast<T*>(p);
 }
 
-// The block solve re-reads a leaf's factor for every chunk of 4 right-hand sides; from 32
-// columns on (the probe blocks of the gradient) the substitution kernel's wider chunks win.
-static bool use_tri_blk(const km_handle* h, int64_t k) { return h->leaf_tc && k < 32; }
+// the factor of the tensor-core stage: its leaves are solved with the inverses of its diagonal blocks
+static bool use_tri_blk(const km_handle* h) { return h->leaf_tc; }
 
 // Leaf solve L x = b (op 0) or L' x = b (op 1) on k columns in place: by 64-row blocks with the
 // diagonal-block inverses the tensor-core leaf stage keeps, else by substitution.
@@ -640,7 +639,7 @@ static bool leaf_solve(km_handle* h, int op, T* X, int k) {
   const Tree& t = h->tree;
   cudaStream_t st = h->stream;
   if constexpr (std::is_same<T, ff>::value) {
-    if (use_tri_blk(h, k)) return KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri_blk(P<ff>(h->d_Lf), t, op, X, t.n, k, st));
+    if (use_tri_blk(h)) return KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri_blk(P<ff>(h->d_Lf), t, op, X, t.n, k, st));
     return KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<ff>(P<ff>(h->d_Lf), t, op, X, 1, t.n, 0, X, 1, t.n, 0, k, st));
   } else {
     return KL(h, KM_PROF_LEAF_TRI, launch_leaf_solve_f64(h->d_Lf, t, op, X, t.n, k, st));
@@ -1721,7 +1720,7 @@ static void aux_fwd_leaf(km_handle* h) {
   T* X = reinterpret_cast<T*>(job->X);
   if constexpr (std::is_same<T, ff>::value) {
     launch_to_ff(job->X, X, t.n * job->k, ax);
-    job->ok = use_tri_blk(h, job->k) ? launch_leaf_tri_blk(P<ff>(h->d_Lf), t, 0, X, t.n, job->k, ax)
+    job->ok = use_tri_blk(h) ? launch_leaf_tri_blk(P<ff>(h->d_Lf), t, 0, X, t.n, job->k, ax)
                          : launch_leaf_tri<ff>(P<ff>(h->d_Lf), t, 0, X, 1, t.n, 0, X, 1, t.n, 0, job->k, ax);
   } else {
     launch_leaf_diaginv(h->d_Lf, t, ax);
