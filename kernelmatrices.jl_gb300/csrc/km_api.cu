@@ -646,6 +646,8 @@ static bool leaf_solve(km_handle* h, int op, T* X, int k) {
   }
 }
 
+// (The sweep kernels may start early: an ordinary kernel comes before each sweep, and the node matrices
+// were final when that one started.)
 template <typename T>
 int nested_fwd_t(km_handle* h, T* X, int k) {  // X <- W^{-1} X
   const Tree& t = h->tree;
@@ -655,8 +657,8 @@ int nested_fwd_t(km_handle* h, T* X, int k) {  // X <- W^{-1} X
   if (t.L == 0) return check_launch(h, "fwd");
   NodeMatsH nm = node_mats(h);
   KLV(h, KM_PROF_LEAF_REFL, launch_leaf_proj<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, X, t.n, P<T>(h->d_VP), k, st));
-  for (int l = 1; l <= t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_FWD_, st));
-  for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_FWD_, st));
+  for (int l = 1; l <= t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_FWD_, st, true));
+  for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_FWD_, st, true));
   KLV(h, KM_PROF_LEAF_REFL, launch_leaf_expand<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, P<T>(h->d_VG), X, t.n, k, -1.0, st));
   return check_launch(h, "fwd");
 }
@@ -675,8 +677,8 @@ int nested_bwd_t(km_handle* h, T* X, int k, bool after_fwd = false) {  // X <- W
       KLV(h, KM_PROF_LEAF_REFL, launch_slot_sub<T>(P<T>(h->d_VP), P<T>(h->d_VG), t.nleaf * (int64_t)k * h->r, st));
     else
       KLV(h, KM_PROF_LEAF_REFL, launch_leaf_proj<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, X, t.n, P<T>(h->d_VP), k, st));
-    for (int l = 1; l < t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_PROJ_, st));
-    for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_BWD_, st));
+    for (int l = 1; l < t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_PROJ_, st, true));
+    for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_BWD_, st, true));
     KLV(h, KM_PROF_LEAF_REFL, launch_leaf_expand<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, P<T>(h->d_VG), X, t.n, k, -1.0, st));
   }
   if (!leaf_solve<T>(h, 1, X, k)) return fail(h, KM_ERR_UNSUPPORTED, "leaf too large for the triangular solve kernel");
@@ -690,8 +692,8 @@ int nested_mul_t_(km_handle* h, T* X, int k) {  // X <- W X
   if (t.L > 0) {
     NodeMatsH nm = node_mats(h);
     KLV(h, KM_PROF_LEAF_REFL, launch_leaf_proj<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, X, t.n, P<T>(h->d_VP), k, st));
-    for (int l = 1; l < t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_PROJ_, st));
-    for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_MUL_, st));
+    for (int l = 1; l < t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_PROJ_, st, true));
+    for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_MUL_, st, true));
     KLV(h, KM_PROF_LEAF_REFL, launch_leaf_expand<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, P<T>(h->d_VG), X, t.n, k, 1.0, st));
   }
   if (!KL(h, KM_PROF_LEAF_TRI, launch_leaf_tri<T>(P<T>(h->d_Lf), t, 2, X, 1, t.n, 0, X, 1, t.n, 0, k, st)))
@@ -708,8 +710,8 @@ int nested_mult_t(km_handle* h, T* X, int k) {  // X <- W' X
   if (t.L == 0) return check_launch(h, "mul_t");
   NodeMatsH nm = node_mats(h);
   KLV(h, KM_PROF_LEAF_REFL, launch_leaf_proj<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, X, t.n, P<T>(h->d_VP), k, st));
-  for (int l = 1; l <= t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_MULT_, st));
-  for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_MULT_, st));
+  for (int l = 1; l <= t.L; ++l) KLV(h, KM_PROF_SWEEP, launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_MULT_, st, true));
+  for (int l = t.L; l >= 1; --l) KLV(h, KM_PROF_SWEEP, launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_MULT_, st, true));
   KLV(h, KM_PROF_LEAF_REFL, launch_leaf_expand<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, P<T>(h->d_VG), X, t.n, k, 1.0, st));
   return check_launch(h, "mul_t");
 }
@@ -1745,7 +1747,7 @@ static void aux_fwd_nodes(km_handle* h) {
       launch_up<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VD), k, UP_FWD_, ax);
     }
     for (int l = t.L; l >= 1; --l)
-      launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_FWD_, ax);
+      launch_down<T>(t, nm, l, P<T>(h->d_VP), P<T>(h->d_VG), P<T>(h->d_VD), k, DN_FWD_, ax, true);
     launch_leaf_expand<T>(P<T>(h->d_Q), P<T>(h->d_tauleaf), h->r, t, P<T>(h->d_VG), X, t.n, k, -1.0, ax);
     h->stats.kernel_launches += 2 + 2 * t.L;
   }

@@ -162,10 +162,11 @@ template <typename T>
 void launch_slot_sub(T* VP, const T* VG, int64_t count, cudaStream_t st);
 enum { DN_FWD_ = 0, DN_BWD_ = 1, DN_MUL_ = 2, DN_MULT_ = 3 };
 template <typename T>
-void launch_up(const Tree& t, const NodeMatsH& h, int level, T* VP, T* VD, int k, int mode, cudaStream_t st);
+void launch_up(const Tree& t, const NodeMatsH& h, int level, T* VP, T* VD, int k, int mode, cudaStream_t st,
+               bool early = false);
 template <typename T>
 void launch_down(const Tree& t, const NodeMatsH& h, int level, const T* VP, T* VG, const T* VD, int k, int mode,
-                 cudaStream_t st);
+                 cudaStream_t st, bool early = false);
 template <typename T>
 void launch_leaf_proj(const T* Qref, const T* tau, int r, const Tree& t, const T* Y, int64_t ldy, T* VP, int k,
                       cudaStream_t st);
