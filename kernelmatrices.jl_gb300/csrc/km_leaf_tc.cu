@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kLcDiagThreads) k_lc_diag(ff* __restrict__ Lf,
   __syncthreads();
   // L in the lower triangle of the diagonal block; the strictly lower part of X = D^{-1} in its
   // (otherwise unused) strictly upper triangle, X[i][c] at row c0 + c, column c0 + i, for the
-  // block solves of k_leaf_tri_blk (X's diagonal is 1 / D_ii, recomputed there the same way)
+  // block solves of k_leaf_tri_few and k_leaf_tri_wide (X's diagonal is 1 / D_ii, recomputed there the same way)
   for (int e = tid; e < nb * nb; e += NT) {
     const int i = e % nb, c = e / nb;
     if (i >= c) Lf[koff + (int64_t)(c0 + c) * m + c0 + i] = D[i * LD + c];
@@ -605,96 +605,89 @@ static int64_t lc_rp_max(const Tree& t, int r) { return lc_rows_padded(t.max_lea
 // that both steps are block products spread over all threads: no sequential chain over rows
 // (the substitution of k_leaf_tri runs one warp per column through each block).  After x_q the
 // remaining rows are updated at once (right-looking).  Same arithmetic as the TC stage's own
-// block column products, which use the same inverses.  The block of NC = 4 right-hand sides
-// lives in shared memory (narrow chunks keep several CTAs per leaf and SM in flight); grid
-// (nleaf, ceil(k / NC)), block 256.
+// block column products, which use the same inverses.
+//
+// Few columns, 4 a CTA: reading L bounds it.  Thread (row i of a 64 x 64 tile, part g) multiplies the
+// tile's columns g, g + 4, ...; a tile that lies along the rows in memory goes from memory to the
+// registers of these threads, one that lies across goes through shared memory, and the next tile is on
+// its way meanwhile.  The four parts are added in shared memory.  With four loads in flight a thread, row
+// by row, 256 leaves of 256 took 230 us for 16 columns, now 146; 512 leaves of 256 100 us for one, now 50.
+// grid (nleaf, ceil(k / 4)), block 256.
 // ---------------------------------------------------------------------------------------------
-template <int NC>
-__global__ void __launch_bounds__(256) k_leaf_tri_blk(const ff* __restrict__ Lf, DTree t, int op,
-                                                      ff* __restrict__ X, int64_t ldx, int k) {
+constexpr int kTfCols = 4, kTwLd = kLcNB + 1;
+
+__global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ Lf, DTree t, int op, ff* __restrict__ X,
+                                                      int64_t ldx, int k) {
   extern __shared__ __align__(16) unsigned char lc_smem_s[];
-  constexpr int LD = kLcNB + 1;
   const int64_t leaf = blockIdx.x;
-  const int m = d_leaf_size(t, leaf);
-  const int64_t s = d_leaf_start(t, leaf), koff = d_leaf_koff(t, leaf);
-  const int c0 = blockIdx.y * NC, nc = min(NC, k - c0);
-  const int tid = threadIdx.x;
-  ff* xs = reinterpret_cast<ff*>(lc_smem_s);  // NC x m, column c at xs[c * m]
-  ff* Xq = xs + NC * m;                       // 64 x 65, X_q[i][c] at Xq[i * LD + c]
-  for (int e = tid; e < NC * m; e += blockDim.x) {
-    const int c = e / m, i = e - c * m;
-    xs[e] = c < nc ? X[(int64_t)(c0 + c) * ldx + s + i] : ff(0.0);
-  }
-  const int nbk = (m + kLcNB - 1) / kLcNB;
-  for (int step = 0; step < nbk; ++step) {
-    const int q = op == 0 ? step : nbk - 1 - step;
-    const int b0 = kLcNB * q, nb = min(kLcNB, m - b0);
-    __syncthreads();
-    for (int e = tid; e < kLcNB * kLcNB; e += blockDim.x) {
-      const int i = e / kLcNB, c = e - i * kLcNB;
-      ff v(0.0);
-      if (i < nb && c < nb) {
-        if (c < i) v = Lf[koff + (int64_t)(b0 + i) * m + b0 + c];
-        else if (c == i) v = ff(1.0) / Lf[koff + (int64_t)(b0 + i) * m + b0 + i];
-      }
-      Xq[i * LD + c] = v;
-    }
-    __syncthreads();
-    // x_q = X_q y_q (op 0) or X_q' y_q (op 1): thread (row i, columns g, g + 4, ...)
-    const int i = tid & (kLcNB - 1), g = tid >> 6;
-    ff res[NC / 4];
+  const int m = d_leaf_size(t, leaf), nbk = (m + kLcNB - 1) / kLcNB, mp = nbk * kLcNB;
+  const int64_t s = d_leaf_start(t, leaf);
+  const ff* L = Lf + d_leaf_koff(t, leaf);
+  const int c0 = blockIdx.y * kTfCols, nc = min(kTfCols, k - c0);
+  const int tid = threadIdx.x, fast = tid & 63, g = tid >> 6;
+  ff* xs = reinterpret_cast<ff*>(lc_smem_s);  // kTfCols x mp, column c at xs[c mp], zero below row m
+  ff* red = xs + kTfCols * mp;                // part, column, row: 4 x kTfCols x 64
+  ff* T = red + 4 * kTfCols * kLcNB;          // 64 x 65, element (l, row) at T[l kTwLd + row]
+  for (int c = 0; c < nc; ++c)
+    for (int i = tid; i < mp; i += 256) xs[c * mp + i] = i < m ? X[(int64_t)(c0 + c) * ldx + s + i] : ff(0.0);
+  // tile (block q, rows of block b): L[b rows][q columns] (op 0) or its transpose, b == q: the inverse.
+  // In memory L runs along the rows, the inverse (upper triangle) across, for op 1 the other way round.
+  ff pre[16];
+  auto fetch = [&](int q, int b) {
+    const bool across = (b == q) == (op == 0);
+    const int col0 = kLcNB * (across ? b : q) + g, row = kLcNB * (across ? q : b) + fast;
+    const int cols = row < m ? m - col0 : 0;  // columns col0, col0 + 4, ... below this many
+    const ff* p = L + (int64_t)col0 * m + row;
 #pragma unroll
-    for (int u = 0; u < NC / 4; ++u) {
-      const int col = g + 4 * u;
-      acc_t<ff> a{};
-      if (col < nc && i < nb) {
-        const ff* y = xs + col * m + b0;
-        if (op == 0)
-          for (int c = 0; c < nb; ++c) a += Xq[i * LD + c] * y[c];
-        else
-          for (int c = 0; c < nb; ++c) a += Xq[c * LD + i] * y[c];
-      }
-      res[u] = accv(a);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < NC / 4; ++u) {
-      const int col = g + 4 * u;
-      if (col < nc && i < nb) xs[col * m + b0 + i] = res[u];
-    }
-    __syncthreads();
-    // remaining rows: op 0 rows below the block, op 1 rows above it
-    const int r0 = op == 0 ? b0 + nb : 0, r1 = op == 0 ? m : b0;
-    for (int row = r0 + tid; row < r1; row += blockDim.x) {
-      acc_t<ff> a[NC] = {};
-      int l = 0;
-      for (; l + 3 < nb; l += 4) {  // four entries of L loaded ahead of their multiply-adds
-        ff lv[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          lv[u] = op == 0 ? Lf[koff + (int64_t)(b0 + l + u) * m + row] : Lf[koff + (int64_t)row * m + b0 + l + u];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int c = 0; c < NC; ++c)
-            if (c < nc) a[c] += lv[u] * xs[c * m + b0 + l + u];
-      }
-      for (; l < nb; ++l) {
-        const ff lv = op == 0 ? Lf[koff + (int64_t)(b0 + l) * m + row] : Lf[koff + (int64_t)row * m + b0 + l];
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-          if (c < nc) a[c] += lv * xs[c * m + b0 + l];
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (c < nc) xs[c * m + row] -= accv(a[c]);
-    }
-  }
+    for (int u = 0; u < 16; ++u, p += 4 * m) pre[u] = 4 * u < cols ? *p : ff(0.0);
+  };
+  fetch(op == 0 ? 0 : nbk - 1, op == 0 ? 0 : nbk - 1);
   __syncthreads();
-  for (int e = tid; e < nc * m; e += blockDim.x) {
-    const int c = e / m, i = e - c * m;
-    X[(int64_t)(c0 + c) * ldx + s + i] = xs[e];
+  for (int step = 0; step < nbk; ++step) {
+    const int q = op == 0 ? step : nbk - 1 - step, left = nbk - step;
+    for (int v = 0; v < left; ++v) {
+      const int b = op == 0 ? q + v : q - v;
+      ff cur[16];  // columns g + 4 u of row `fast` of the tile
+#pragma unroll
+      for (int u = 0; u < 16; ++u) cur[u] = pre[u];
+      if (v == 0) {  // a triangle, its diagonal the reciprocal (fast <= column or row g + 4 u)
+        ff d(1.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+          if (fast == g + 4 * u && kLcNB * q + fast < m) d = cur[u];
+        d = ff(1.0) / d;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) cur[u] = fast < g + 4 * u ? cur[u] : fast == g + 4 * u ? d : ff(0.0);
+      }
+      if ((v == 0) == (op == 0)) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) T[fast * kTwLd + g + 4 * u] = cur[u];
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 16; ++u) cur[u] = T[(g + 4 * u) * kTwLd + fast];
+      }
+      if (v + 1 < left) fetch(q, op == 0 ? b + 1 : b - 1);
+      else if (left > 1) fetch(op == 0 ? q + 1 : q - 1, op == 0 ? q + 1 : q - 1);
+      for (int c = 0; c < nc; ++c) {
+        const ff* x = xs + c * mp + kLcNB * q + g;
+        acc_t<ff> a{};
+#pragma unroll
+        for (int u = 0; u < 16; ++u) a += cur[u] * x[4 * u];
+        red[(g * kTfCols + c) * kLcNB + fast] = accv(a);
+      }
+      __syncthreads();
+      if (g < nc) {
+        const ff* p = red + g * kLcNB + fast;
+        constexpr int sp = kTfCols * kLcNB;
+        const ff sum = (p[0] + p[sp]) + (p[2 * sp] + p[3 * sp]);
+        ff* out = xs + g * mp + kLcNB * b + fast;
+        *out = v == 0 ? sum : *out - sum;
+      }
+      __syncthreads();
+    }
   }
+  for (int c = 0; c < nc; ++c)
+    for (int i = tid; i < m; i += 256) X[(int64_t)(c0 + c) * ldx + s + i] = xs[c * mp + i];
 }
 
 // The same solves for many right-hand sides, 12 columns a CTA: 64 x 64 tiles of L (or L'), and of the
@@ -704,7 +697,7 @@ __global__ void __launch_bounds__(256) k_leaf_tri_blk(const ff* __restrict__ Lf,
 // kernel (12 instructions a multiply-add).  512 leaves of 488, 72 columns: the substitution of
 // k_leaf_tri took 4.4 ms, this 2.8 ms; the FP32 floor is 1.5 ms.  The chunks of a leaf are neighbours in
 // the grid and find its tiles in L2.  grid nleaf ceil(k / 12), block 256.
-constexpr int kTwCols = 12, kTwLd = kLcNB + 1;
+constexpr int kTwCols = 12;
 
 __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__ Lf, DTree t, int op, ff* __restrict__ X,
                                                           int64_t ldx, int k) {
@@ -739,12 +732,15 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
   auto put = [&](int q, int b) {
     const bool across = (b == q) == (op == 0);
     if (b == q) {
-      const bool below = kLcNB * q + fast < m;
+      ff d(1.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (fast == slow + 4 * u && kLcNB * q + fast < m) d = pre[u];
+      d = ff(1.0) / d;
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const int sl = slow + 4 * u;  // kept: l <= i (op 0) or l >= i (op 1), fast <= sl for both
-        T[across ? fast * kTwLd + sl : sl * kTwLd + fast] =
-            fast > sl ? ff(0.0) : fast == sl && below ? ff(1.0) / pre[u] : pre[u];
+        T[across ? fast * kTwLd + sl : sl * kTwLd + fast] = fast < sl ? pre[u] : fast == sl ? d : ff(0.0);
       }
     } else {
       ff* to = across ? T + fast * kTwLd + slow : T + slow * kTwLd + fast;
@@ -790,24 +786,19 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
     for (int j = lane; j < m; j += 32) X[(int64_t)(c0 + c) * ldx + s + j] = xs[c * mp + j];
 }
 
-template <int NC>
-static bool tri_blk_launch(const ff* Lf, const Tree& t, int op, ff* X, int64_t ldx, int k, cudaStream_t st) {
-  const size_t sm = ((size_t)NC * t.max_leaf + (size_t)kLcNB * (kLcNB + 1)) * sizeof(ff);
-  if (sm > 200 * 1024) return false;
-  smem_limit((const void*)k_leaf_tri_blk<NC>, sm);
-  k_leaf_tri_blk<NC><<<dim3((unsigned)t.nleaf, (unsigned)((k + NC - 1) / NC)), 256, sm, st>>>(Lf, dtree(t), op, X,
-                                                                                              ldx, k);
-  return true;
-}
-
-// from this many columns on the wide form is faster
-constexpr int kTriWideMin = 32;
-
 bool launch_leaf_tri_blk(const ff* Lf, const Tree& t, int op, ff* X, int64_t ldx, int k, cudaStream_t st) {
   if (k <= 0) return true;
   if (t.max_leaf > kLcMaxLeaf || (op != 0 && op != 1)) return false;
-  if (k < kTriWideMin) return tri_blk_launch<4>(Lf, t, op, X, ldx, k, st);
   const int64_t mp = (t.max_leaf + kLcNB - 1) / kLcNB * kLcNB;
+  // 12 columns a CTA take as long as 2.1 chunks of 4 columns (256 leaves of 256: 81 us against 31, 50, 90,
+  // 124 us for 1, 4, 8, 12 columns; 16 columns 155 against 146, 24 columns 156 against 220)
+  if (2 * ((k + kTwCols - 1) / kTwCols) >= (k + kTfCols - 1) / kTfCols) {
+    const size_t sm = ((size_t)kTfCols * mp + (size_t)4 * kTfCols * kLcNB + (size_t)kLcNB * kTwLd) * sizeof(ff);
+    smem_limit((const void*)k_leaf_tri_few, sm);
+    k_leaf_tri_few<<<dim3((unsigned)t.nleaf, (unsigned)((k + kTfCols - 1) / kTfCols)), 256, sm, st>>>(Lf, dtree(t), op, X,
+                                                                                                    ldx, k);
+    return true;
+  }
   const size_t sm = ((size_t)kTwCols * mp + (size_t)kLcNB * kTwLd) * sizeof(ff);
   smem_limit((const void*)k_leaf_tri_wide, sm);
   k_leaf_tri_wide<<<(unsigned)(t.nleaf * ((k + kTwCols - 1) / kTwCols)), 256, sm, st>>>(Lf, dtree(t), op, X, ldx, k);

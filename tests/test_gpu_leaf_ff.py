@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,lv,r,k", [(140, 1, 32, 33), (300, 1, 64, 36), (510, 1, 3, 32), (513, 1, 33, 37), (514, 1, 80, 72),
                                       (1024, 1, 72, 48), (1027, 1, 31, 35), (2048, 1, 65, 33), (2052, 1, 40, 34),
-                                      (3001, 4, 72, 73), (4500, 3, 17, 64)])
+                                      (3001, 4, 72, 73), (4500, 3, 17, 64), (140, 1, 32, 1), (513, 1, 33, 2), (514, 1, 60, 4),
+                                      (1280, 1, 40, 5), (1000, 2, 72, 13), (2045, 1, 80, 3), (2048, 1, 20, 16)])
 def test_solve(lib, n, lv, r, k):
     import kmhodlr as K
     from kmhodlr.data import uniform_points
