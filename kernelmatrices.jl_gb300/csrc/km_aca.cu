@@ -911,8 +911,7 @@ __global__ void __launch_bounds__(kGaThreads) k_gapply(const GApplyItem* __restr
 // columns, side and row chunk) CTAs, the r x r part in between.  Partial projections of item q,
 // side d, chunk h, column c start at part + (((2 q + d) nchunk + h) ncol + c) ldr; the
 // coefficients at coef + ((2 q + d) ncol + c) ldr (ncol: columns rounded up to CB, ldr: largest r).
-// Nodes of 4096 and 8192 rows with 8 right-hand sides: 4.1 and 8.1 ms by one CTA a node, @A@ and
-// @B@ ms spread.
+// (One CTA a node took 4.1 and 8.1 ms for nodes of 4096 and 8192 rows with 8 right-hand sides.)
 struct GSpread {
   double* part;
   double* coef;

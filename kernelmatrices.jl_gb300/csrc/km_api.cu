@@ -955,13 +955,14 @@ int derivative_apply(km_handle* h, int j, const double* X, double* Y, int k) {
     if ((rc = grow(h, &h->d_GB, t.nleaf * 2 * r * k))) return rc;
     KLV(h, KM_PROF_LEAF_APPLY, launch_dbeta<ff>(P<ff>(h->d_SinvF), P<ff>(h->d_M2F), r, h->d_GG, t.nleaf * (int64_t)k,
                                                 P<ff>(h->d_GB), st));
-    KLV(h, KM_PROF_LEAF_APPLY, launch_leaf_dnys_apply<ff>(P<ff>(h->d_dKf), P<ff>(h->d_Phif), P<ff>(h->d_dPhif), h->d_Sc,
-                                                          h->d_Sj, r, t, X, t.n, h->d_GG, Y, t.n, k, st,
-                                                          P<ff>(h->d_GB)));
+    KLV(h, KM_PROF_LEAF_APPLY, launch_leaf_dnys_apply<ff>(P<ff>(h->d_dKf), P<ff>(h->d_Phif), P<ff>(h->d_dPhif), r, t, X,
+                                                          t.n, Y, t.n, k, st, P<ff>(h->d_GB)));
+  } else {
+    // the projections in d_GP have been summed: their place takes the landmark coefficients
+    KLV(h, KM_PROF_LEAF_APPLY, launch_dbeta_solve(h->d_Sc, h->d_Sj, r, h->d_GG, t.nleaf * (int64_t)k, h->d_GP, st));
+    KLV(h, KM_PROF_LEAF_APPLY, launch_leaf_dnys_apply<double>(h->d_dK, h->d_Phi, h->d_dPhi, r, t, X, t.n, Y, t.n, k, st,
+                                                              h->d_GP));
   }
-  else
-    KLV(h, KM_PROF_LEAF_APPLY, launch_leaf_dnys_apply<double>(h->d_dK, h->d_Phi, h->d_dPhi, h->d_Sc, h->d_Sj, r, t, X,
-                                                              t.n, h->d_GG, Y, t.n, k, st));
   return check_launch(h, "derivative");
 }
 

@@ -88,82 +88,116 @@ __device__ __forceinline__ void load8(const double* p, double (&v)[8]) {
   }
 }
 
-// y_leaf = dK_leaf x + dPhi beta1 + Phi beta2, beta1 = S^{-1} a, beta2 = S^{-1}(b - Sj beta1),
-// [a ; b] = VG[leaf][col], for a chunk of 8 columns.  The betas are solved in FP64 (one warp per
-// column), then x and the betas are staged in shared memory as T and each thread owns leaf rows
-// with 8 accumulators, so every matrix entry read feeds 8 multiply-adds.
-// grid (nleaf, ceil(k/8)), block 256.
+// beta[pair] = [beta1 ; beta2], beta1 = S^{-1} a, beta2 = S^{-1}(b - Sj beta1), [a ; b] = VG[pair], for every
+// (leaf, column) pair in FP64: a warp per pair, forward and backward substitutions with Sc = chol(S) and
+// the reciprocals of its diagonal (a division in each of the 4 r steps of the chain took three quarters
+// of it).  grid ceil(npairs / 4), block 128.
+__global__ void __launch_bounds__(128) k_dbeta_solve(const double* __restrict__ Sc, const double* __restrict__ Sj, int r,
+                                                     const double* __restrict__ VG, int64_t npairs,
+                                                     double* __restrict__ beta) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double* rd = reinterpret_cast<double*>(smraw);  // r: 1 / Sc[l][l]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* b1 = rd + r + w * 2 * r;
+  double* b2 = b1 + r;
+  for (int l = threadIdx.x; l < r; l += 128) rd[l] = 1.0 / Sc[(int64_t)l * r + l];
+  __syncthreads();
+  const int64_t pair = (int64_t)blockIdx.x * 4 + w;
+  if (pair >= npairs) return;
+  for (int i = lane; i < 2 * r; i += 32) b1[i] = VG[pair * 2 * r + i];
+  __syncwarp();
+  for (int pass = 0; pass < 2; ++pass) {
+    double* v = pass == 0 ? b1 : b2;
+    if (pass == 1) {  // b2 <- b2 - Sj b1
+      for (int i = lane; i < r; i += 32) {
+        double a = 0.0;
+        for (int l = 0; l < r; ++l) a += Sj[i + (int64_t)l * r] * b1[l];
+        b2[i] -= a;
+      }
+      __syncwarp();
+    }
+    // v <- S^{-1} v = Sc^{-T} Sc^{-1} v
+    for (int l = 0; l < r; ++l) {
+      const double vl = v[l] * rd[l];
+      __syncwarp();
+      if (lane == 0) v[l] = vl;
+      for (int i = l + 1 + lane; i < r; i += 32) v[i] -= Sc[(int64_t)l * r + i] * vl;
+      __syncwarp();
+    }
+    for (int i = r - 1; i >= 0; --i) {
+      const double vi = v[i] * rd[i];
+      __syncwarp();
+      if (lane == 0) v[i] = vi;
+      for (int l = lane; l < i; l += 32) v[l] -= Sc[i + (int64_t)l * r] * vi;
+      __syncwarp();
+    }
+  }
+  for (int i = lane; i < 2 * r; i += 32) beta[pair * 2 * r + i] = b1[i];
+}
+
+// y_leaf = dK_leaf x + dPhi beta1 + Phi beta2 for a chunk of 8 columns, the betas from k_dbeta or
+// k_dbeta_solve.  x and the betas are staged in shared memory as T.  Float pairs: each thread owns leaf
+// rows with 8 accumulators, so every matrix entry read feeds 8 multiply-adds (grid.z 1, block 256).
+// FP64, bound by its pipe: items (row, 4 columns) over blockIdx.z and the threads, so that a leaf of one
+// row more than the block costs no second pass of a lone warp (32 leaves of 257, 48 landmarks, 25 columns:
+// 457 us with the float-pair form's mapping and the betas solved in every CTA, now 193 and 77 for the betas).
+// grid (nleaf, ceil(k/8), parts), block 128.
 template <typename T>
 __global__ void __launch_bounds__(256) k_leaf_dnys_apply(const T* __restrict__ dKl, const T* __restrict__ Phi,
-                                                         const T* __restrict__ dPhi, const double* __restrict__ Sc,
-                                                         const double* __restrict__ Sj, int r, DTree t,
+                                                         const T* __restrict__ dPhi, int r, DTree t,
                                                          const double* __restrict__ X, int64_t ldx,
-                                                         const double* __restrict__ VG, double* __restrict__ Y,
-                                                         int64_t ldy, int k, const T* __restrict__ betas) {
+                                                         double* __restrict__ Y, int64_t ldy, int k,
+                                                         const T* __restrict__ betas) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   const int64_t s = d_leaf_start(t, leaf);
   const int c0 = blockIdx.y * 8;
   const int nc = min(8, k - c0);
-  double* bd = reinterpret_cast<double*>(smraw);  // 8 x 3r : beta1 | beta2 | (spare), FP64
-  T* xs = reinterpret_cast<T*>(bd + 8 * 3 * r);   // m x 8 (16-byte aligned)
-  T* bs = xs + 8 * m;                              // 2r x 8 : beta1 rows, then beta2 rows
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T* xs = reinterpret_cast<T*>(smraw);   // m x 8
+  T* bs = xs + 8 * m;                    // 2r x 8 : beta1 rows, then beta2 rows
   for (int e = threadIdx.x; e < 8 * m; e += blockDim.x) {  // row l of the chunk at xs[8 l]
     const int c = e / m, i = e % m;
     xs[8 * i + c] = c < nc ? from_double<T>(X[(int64_t)(c0 + c) * ldx + s + i]) : T(0.0);
   }
-  if (betas) {  // coefficients formed by k_dbeta
-    for (int e = threadIdx.x; e < 8 * 2 * r; e += blockDim.x) {
-      const int c = e / (2 * r), i = e % (2 * r);
-      bs[8 * i + c] = c < nc ? betas[(leaf * k + c0 + c) * 2 * r + i] : T(0.0);
-    }
-  } else if (w < nc) {
-    double* b1 = bd + w * 3 * r;
-    double* b2 = b1 + r;
-    const double* g = VG + (leaf * k + c0 + w) * 2 * r;
-    for (int i = lane; i < r; i += 32) {
-      b1[i] = g[i];
-      b2[i] = g[r + i];
-    }
-    __syncwarp();
-    for (int pass = 0; pass < 2; ++pass) {
-      double* v = pass == 0 ? b1 : b2;
-      if (pass == 1) {
-        // b2 <- b2 - Sj b1
-        for (int i = lane; i < r; i += 32) {
-          double a = 0.0;
-          for (int l = 0; l < r; ++l) a += Sj[i + (int64_t)l * r] * b1[l];
-          b2[i] -= a;
-        }
-        __syncwarp();
-      }
-      // v <- S^{-1} v = Sc^{-T} Sc^{-1} v
-      for (int l = 0; l < r; ++l) {
-        const double vl = v[l] / Sc[(int64_t)l * r + l];
-        __syncwarp();
-        if (lane == 0) v[l] = vl;
-        for (int i = l + 1 + lane; i < r; i += 32) v[i] -= Sc[(int64_t)l * r + i] * vl;
-        __syncwarp();
-      }
-      for (int i = r - 1; i >= 0; --i) {
-        const double vi = v[i] / Sc[(int64_t)i * r + i];
-        __syncwarp();
-        if (lane == 0) v[i] = vi;
-        for (int l = lane; l < i; l += 32) v[l] -= Sc[i + (int64_t)l * r] * vi;
-        __syncwarp();
-      }
-    }
-    for (int i = lane; i < 2 * r; i += 32) bs[8 * i + w] = from_double<T>(b1[i]);  // row i at bs[8 i]
-  } else if (w < 8) {
-    for (int i = lane; i < 2 * r; i += 32) bs[8 * i + w] = T(0.0);
+  for (int e = threadIdx.x; e < 8 * 2 * r; e += blockDim.x) {
+    const int c = e / (2 * r), i = e % (2 * r);
+    bs[8 * i + c] = c < nc ? betas[(leaf * k + c0 + c) * 2 * r + i] : T(0.0);
   }
   __syncthreads();
   const T* K = dKl + d_leaf_koff(t, leaf);
   const T* P = Phi + s * r;
   const T* dP = dPhi + s * r;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
+  if constexpr (std::is_same<T, double>::value) {
+    for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < (nc > 4 ? 2 : 1) * m; e += gridDim.z * blockDim.x) {
+      const int h = e >= m ? 4 : 0, i = e >= m ? e - m : e;
+      double acc[4] = {};
+      auto add = [&](double a, const double* v) {
+        const double2 u = *reinterpret_cast<const double2*>(v), w = *reinterpret_cast<const double2*>(v + 2);
+        acc[0] += a * u.x;
+        acc[1] += a * u.y;
+        acc[2] += a * w.x;
+        acc[3] += a * w.y;
+      };
+      int l = 0;
+      for (; l + 3 < m; l += 4) {
+        double a[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = K[i + (int64_t)(l + u) * m];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) add(a[u], xs + 8 * (l + u) + h);
+      }
+      for (; l < m; ++l) add(K[i + (int64_t)l * m], xs + 8 * l + h);
+#pragma unroll 2
+      for (int q = 0; q < r; ++q) {
+        add(dP[i + (int64_t)q * m], bs + 8 * q + h);
+        add(P[i + (int64_t)q * m], bs + 8 * (r + q) + h);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (h + c < nc) Y[(int64_t)(c0 + h + c) * ldy + s + i] = acc[c];
+    }
+  } else for (int i = threadIdx.x; i < m; i += blockDim.x) {
     T acc[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[c] = T(0.0);
@@ -347,25 +381,31 @@ void launch_leaf_phiT(const double* Phi, int r, const Tree& t, const double* X, 
 }
 
 template <typename T>
-void launch_leaf_dnys_apply(const T* dKl, const T* Phi, const T* dPhi, const double* Sc, const double* Sj, int r,
-                            const Tree& t, const double* X, int64_t ldx, const double* VG, double* Y, int64_t ldy,
-                            int k, cudaStream_t st, const T* betas) {
-  dim3 grid((unsigned)t.nleaf, (unsigned)((k + 7) / 8));
-  const size_t sm = (size_t)8 * 3 * r * sizeof(double) + ((size_t)8 * t.max_leaf + 8 * 2 * r) * sizeof(T);
+void launch_leaf_dnys_apply(const T* dKl, const T* Phi, const T* dPhi, int r, const Tree& t, const double* X, int64_t ldx,
+                            double* Y, int64_t ldy, int k, cudaStream_t st, const T* betas) {
+  const bool f64 = std::is_same<T, double>::value;
+  const unsigned nth = f64 ? 128 : 256, parts = f64 ? (unsigned)((2 * t.max_leaf + nth - 1) / nth) : 1u;
+  dim3 grid((unsigned)t.nleaf, (unsigned)((k + 7) / 8), parts);
+  const size_t sm = ((size_t)8 * t.max_leaf + 8 * 2 * r) * sizeof(T);
   smem_limit((const void*)k_leaf_dnys_apply<T>, sm);
-  k_leaf_dnys_apply<T><<<grid, 256, sm, st>>>(dKl, Phi, dPhi, Sc, Sj, r, dtree(t), X, ldx, VG, Y, ldy, k, betas);
+  k_leaf_dnys_apply<T><<<grid, nth, sm, st>>>(dKl, Phi, dPhi, r, dtree(t), X, ldx, Y, ldy, k, betas);
+}
+
+void launch_dbeta_solve(const double* Sc, const double* Sj, int r, const double* VG, int64_t npairs, double* beta,
+                        cudaStream_t st) {
+  if (npairs <= 0) return;
+  k_dbeta_solve<<<(unsigned)((npairs + 3) / 4), 128, (size_t)9 * r * sizeof(double), st>>>(Sc, Sj, r, VG, npairs, beta);
 }
 
 template void launch_leaf_dphiT<double>(const double*, const double*, int, const Tree&, const double*, int64_t,
                                         double*, int, cudaStream_t);
 template void launch_leaf_dphiT<ff>(const ff*, const ff*, int, const Tree&, const double*, int64_t, double*, int,
                                     cudaStream_t);
-template void launch_leaf_dnys_apply<double>(const double*, const double*, const double*, const double*,
-                                             const double*, int, const Tree&, const double*, int64_t,
-                                             const double*, double*, int64_t, int, cudaStream_t, const double*);
-template void launch_leaf_dnys_apply<ff>(const ff*, const ff*, const ff*, const double*, const double*, int,
-                                         const Tree&, const double*, int64_t, const double*, double*, int64_t, int,
-                                         cudaStream_t, const ff*);
+template void launch_leaf_dnys_apply<double>(const double*, const double*, const double*, int, const Tree&,
+                                             const double*, int64_t, double*, int64_t, int, cudaStream_t,
+                                             const double*);
+template void launch_leaf_dnys_apply<ff>(const ff*, const ff*, const ff*, int, const Tree&, const double*, int64_t,
+                                         double*, int64_t, int, cudaStream_t, const ff*);
 
 // ---------------------------------------------------------------------------------------------
 // Second-derivative product of the stochastic Hessian (Deriv2mul, src/HODLR/src/utils.jl:157-177)

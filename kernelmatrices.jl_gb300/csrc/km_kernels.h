@@ -184,9 +184,10 @@ template <typename T>
 void launch_leaf_dphiT(const T* Phi, const T* dPhi, int r, const Tree& t, const double* X, int64_t ldx, double* VP,
                        int k, cudaStream_t st);
 template <typename T>
-void launch_leaf_dnys_apply(const T* dKl, const T* Phi, const T* dPhi, const double* Sc, const double* Sj, int r,
-                            const Tree& t, const double* X, int64_t ldx, const double* VG, double* Y, int64_t ldy,
-                            int k, cudaStream_t st, const T* betas = nullptr);
+void launch_leaf_dnys_apply(const T* dKl, const T* Phi, const T* dPhi, int r, const Tree& t, const double* X, int64_t ldx,
+                            double* Y, int64_t ldy, int k, cudaStream_t st, const T* betas);
+void launch_dbeta_solve(const double* Sc, const double* Sj, int r, const double* VG, int64_t npairs, double* beta,
+                        cudaStream_t st);
 // C = A op(B), r x r FP64 (op = transpose when transB)
 // second-derivative product of the stochastic Hessian (km_grad.cu)
 void launch_leaf_phi4T(const double* Phi, const double* Phi3, int r, const Tree& t, const double* X, int64_t ldx,
