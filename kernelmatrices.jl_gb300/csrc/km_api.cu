@@ -880,7 +880,7 @@ int fetch_info_async(km_handle* h, int64_t count) {
 // The leaf pivot status in info[0 .. count): PosDefException for the first failing leaf.
 int check_info_words(km_handle* h, const int* info, int64_t count, const char* what) {
   for (int64_t i = 0; i < count; ++i) {
-    if (info[i] < 0) return fail(h, KM_ERR_TIMEOUT, "a bounded wait of the tensor-core leaf update ran out");
+    if (info[i] < 0) return fail(h, KM_ERR_TIMEOUT, "a bounded wait of the leaf kernels ran out");
     if (info[i] != 0) {
       char buf[160];
       snprintf(buf, sizeof buf, "PosDefException: %s %lld is not positive definite (pivot %d)",
@@ -1792,7 +1792,8 @@ static int factorize_launches(km_handle* h) {
       if (fwd) aux_fwd_leaf<ff>(h);
     }
     if (t.L > 0) {
-      KLV(h, KM_PROF_LEAF_QR, launch_leaf_qr<ff>(P<ff>(h->d_Q), r, t, P<ff>(h->d_tauleaf), P<ff>(h->d_R), st));
+      KLV(h, KM_PROF_LEAF_QR, launch_leaf_qr<ff>(P<ff>(h->d_Q), r, t, P<ff>(h->d_tauleaf), P<ff>(h->d_R), h->d_info,
+                                                   (int)std::min<int64_t>(h->wait_limit, INT32_MAX), st));
       side_begin(h);
       launch_leaf_formq<ff>(P<ff>(h->d_Q), P<ff>(h->d_tauleaf), r, t, h->side);
       if (fwd) cudaEventRecord(h->xev[1], h->side);
@@ -1823,7 +1824,8 @@ static int factorize_launches(km_handle* h) {
     if (fwd) aux_fwd_leaf<double>(h);
     else if (t.L == 0) KLV(h, KM_PROF_OTHER, launch_leaf_diaginv(h->d_Lf, t, st));
     if (t.L > 0) {
-      KLV(h, KM_PROF_LEAF_QR, launch_leaf_qr<double>(h->d_Q, r, t, h->d_tauleaf, h->d_R, st));
+      KLV(h, KM_PROF_LEAF_QR, launch_leaf_qr<double>(h->d_Q, r, t, h->d_tauleaf, h->d_R, h->d_info,
+                                                       (int)std::min<int64_t>(h->wait_limit, INT32_MAX), st));
       side_begin(h);
       if (!fwd) launch_leaf_diaginv(h->d_Lf, t, h->side);
       launch_leaf_formq<double>(h->d_Q, h->d_tauleaf, r, t, h->side);

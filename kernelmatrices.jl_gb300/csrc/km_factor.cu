@@ -160,148 +160,166 @@ __global__ void __launch_bounds__(NT) k_leaf_chol(const double* __restrict__ K, 
 // v = x/(alpha-beta); a zero column x gives tau = 0 (H = I).  One CTA per leaf; the panel is
 // copied to shared memory when it fits.
 // ---------------------------------------------------------------------------------------------
-// One CTA per leaf.  With float pairs it has 1024 threads: the panel (up to 200 KB of shared
-// memory) admits one CTA per SM, so the CTA takes all the warps the SM can hold to hide the
-// latency of the float-pair dot products.  The FP64 kernel is bound by the FP64 pipe and keeps
-// 256 threads (and the registers that go with them).
+// Iteration bound of a spin wait on a shared-memory flag (a few tens of cycles per iteration:
+// well above any legitimate wait inside one leaf or node, far below a watchdog).  The waiter of the
+// critical column does not sleep: it would wake too late for the column-to-column handoff.
+constexpr int kWaitLimit = 1 << 22;
+
+// Householder QR of the leaf panels (m x r, in place: R above, the scaled reflectors below), a CTA per
+// leaf, in dataflow order: of the NW warps warp w owns the columns w, w + NW, ...; reflector j + 1 is formed
+// by the warp that owns its column as soon as it has applied reflector j to it, before its other columns,
+// and published with a flag (the unscaled column; scale and tau in sc, ta).  The reflectors are scaled at
+// the end.  Waits are bounded; one that runs out marks the leaf with info = -1 and the warp carries on.
+// With two block barriers a column and one thread forming the reflector between them (same operations,
+// same order) 256 panels of 256 x 72 took 636 us in float pairs and 1.64 ms in FP64, 512 of 488 x 72
+// 2.35 ms in float pairs; now 527 us, 1.42 ms and 1.91 ms.  FP64 has a quarter of the warps: one warp fills a
+// quarter of its pipe.  grid nleaf, block 32 NW.
 template <typename T>
-constexpr int leaf_qr_threads() { return std::is_same<T, double>::value ? 256 : 1024; }
+constexpr int leaf_qr_warps() { return std::is_same<T, double>::value ? 8 : 32; }
 
 template <typename T, bool SMEM>
-__global__ void __launch_bounds__(leaf_qr_threads<T>()) k_leaf_qr(T* __restrict__ Pan, int r, DTree t,
-                                                                 T* __restrict__ tau, T* __restrict__ Rout) {
+__global__ void __launch_bounds__(32 * leaf_qr_warps<T>()) k_leaf_qr(T* __restrict__ Pan, int r, DTree t,
+                                                                    T* __restrict__ tau, T* __restrict__ Rout,
+                                                                    int* __restrict__ info, int wait_limit) {
+  constexpr int NW = leaf_qr_warps<T>(), NT = 32 * NW;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
-  __shared__ T red[32];
-  __shared__ T sh_tau;
+  __shared__ T red[32], sc[kMaxNysRank], ta[kMaxNysRank];
+  __shared__ volatile int flag[kMaxNysRank];
+  const int lim = wait_limit < 0 ? kWaitLimit : wait_limit;
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
-  const int64_t s = d_leaf_start(t, leaf);
-  T* G = Pan + s * r;
+  T* G = Pan + d_leaf_start(t, leaf) * r;
   T* A = SMEM ? sm : G;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  if (SMEM) {
-    for (int64_t e = tid; e < (int64_t)m * r; e += blockDim.x) sm[e] = G[e];
-    __syncthreads();
-  }
   const int kmax = min(m, r);
-  // Two barriers a column: (1) thread 0 forms reflector j from alpha = a[j][j] and the norm of
-  // the rest of column j, which the warp that last updated that column left in sh_sig, while the
-  // other threads scale the previous reflector; (2) one warp per column c > j applies H_j with
-  // the unscaled vector x = a[j+1:, j] (v = scal x), and the warp of column j + 1 then leaves the
-  // norm of its rows below j + 1 for the next step.
-  __shared__ T sh_sig, sh_scal;
-  if (kmax > 0) {  // norm of column 0 below its first row
+  for (int e = tid; e < r; e += NT) flag[e] = 0;
+  if (SMEM)
+    for (int e = tid; e < m * r; e += NT) sm[e] = G[e];
+  __syncthreads();
+  // reflector j from alpha = a[j][j] and sig, the squared norm below it (all lanes alike): one division
+  // forms tau = (beta - alpha) / beta in lane 1 and scale = 1 / (alpha - beta) in the others
+  auto reflect = [&](int j, T sig) {
+    T* aj = A + (int64_t)j * m;
+    const T alpha = aj[j];
+    T tj = T(0.0), beta = alpha, scal = T(0.0);
+    if (sig != 0.0) {
+      const T nrm = sqrt(alpha * alpha + sig);
+      beta = alpha >= 0.0 ? -nrm : nrm;
+      const T num = lane == 1 ? beta - alpha : T(1.0), den = lane == 1 ? beta : alpha - beta;
+      const T q = num / den;
+      tj = shfl_idx(q, 1);
+      scal = shfl_idx(q, 0);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      aj[j] = beta;
+      sc[j] = scal;
+      ta[j] = tj;
+      tau[leaf * r + j] = tj;
+    }
+    __threadfence_block();
+    __syncwarp();
+    if (lane == 0) flag[j] = 1;
+  };
+  {  // norm of column 0 below its first row
     T part = T(0.0);
-    for (int i = 1 + tid; i < m; i += blockDim.x) part += A[i] * A[i];
+    for (int i = 1 + tid; i < m; i += NT) part += A[i] * A[i];
     part = warp_sum_t(part);
     if (lane == 0) red[w] = part;
     __syncthreads();
-    if (w == 0) {
-      T v = lane < (int)(blockDim.x >> 5) ? red[lane] : T(0.0);
-      v = warp_sum_t(v);
-      if (lane == 0) sh_sig = v;
-    }
+    if (w == 0) reflect(0, warp_sum_t(lane < NW ? red[lane] : T(0.0)));
   }
-  T prev_scal = T(0.0);
-  for (int j = 0; j < kmax; ++j) {
-    T* aj = A + (int64_t)j * m;
-    __syncthreads();
-    if (j > 0) {  // the previous reflector's vector, scaled in place (nobody reads it this phase)
-      T* ap = A + (int64_t)(j - 1) * m;
-      for (int i = j + tid; i < m; i += blockDim.x) ap[i] *= prev_scal;
-    }
-    if (tid == 0) {
-      const T sig = sh_sig;
-      const T alpha = aj[j];
-      T tj = T(0.0), beta = alpha, scal = T(0.0);
-      if (sig != 0.0) {
-        const T nrm = sqrt(alpha * alpha + sig);
-        beta = alpha >= 0.0 ? -nrm : nrm;
-        tj = (beta - alpha) / beta;
-        scal = T(1.0) / (alpha - beta);
+  bool timed_out = false;
+  const int last = w < r ? w + (r - 1 - w) / NW * NW : -1;
+  for (int j = 0; j < min(kmax, last); ++j) {
+    if (!timed_out) {
+      int spins = 0;
+      // the warp of the next reflector polls; the others leave it the issue slots
+      const unsigned nap = (j + 1) % NW == w ? 0 : (j + 2) % NW == w ? 32 : 256;
+      while (wait_limit == 0 || flag[j] == 0) {
+        if (++spins > lim) {
+          if (lane == 0) info[leaf] = -1;
+          timed_out = true;
+          break;
+        }
+        if (nap) __nanosleep(nap);
       }
-      aj[j] = beta;
-      sh_scal = scal;
-      sh_tau = tj;
-      tau[leaf * r + j] = tj;
     }
-    __syncthreads();
-    const T scal = sh_scal, tj = sh_tau;
-    prev_scal = scal;
-    if (tj != 0.0) {
-      // apply H_j = I - tau v v' to columns c > j, v = scal x.  Float pairs (32 warps): a warp
-      // takes the columns c and c + nwarps together, two independent dot products and updates in
-      // flight; FP64 (8 warps, bound by the FP64 pipe): one column a warp
-      constexpr bool kPair = std::is_same<T, ff>::value;
-      const int nwarps = (int)(blockDim.x >> 5);
-      for (int c = j + 1 + w; c < r; c += (kPair ? 2 : 1) * nwarps) {
-        const int c2 = c + nwarps;
-        const bool two = kPair && c2 < r;
-        T* ac = A + (int64_t)c * m;
-        T* ac2 = A + (int64_t)(two ? c2 : c) * m;
-        T acc = T(0.0), acc2 = T(0.0);
-        for (int i = j + 1 + lane; i < m; i += 32) {
-          const T x = aj[i];
-          acc += x * ac[i];
-          if (two) acc2 += x * ac2[i];
-        }
-        acc = (warp_sum_t(acc) * scal + ac[j]) * tj;
-        if (two) acc2 = (warp_sum_t(acc2) * scal + ac2[j]) * tj;
-        if (lane == 0) {
-          ac[j] -= acc;
-          if (two) ac2[j] -= acc2;
-        }
-        const T f = acc * scal, f2 = acc2 * scal;
-        if (c == j + 1) {  // the next column: its norm below row j + 1 on the way
-          T nrm = T(0.0);
-          for (int i = j + 1 + lane; i < m; i += 32) {
-            const T x = aj[i];
-            const T v = ac[i] - f * x;
-            ac[i] = v;
-            if (i > j + 1) nrm += v * v;
-            if (two) ac2[i] -= f2 * x;
-          }
-          nrm = warp_sum_t(nrm);
-          if (lane == 0) sh_sig = nrm;
-        } else {
-          for (int i = j + 1 + lane; i < m; i += 32) {
-            const T x = aj[i];
-            ac[i] -= f * x;
-            if (two) ac2[i] -= f2 * x;
-          }
-        }
-      }
-    } else if (j + 1 < kmax && w == 0) {  // H_j = I: the next column's norm as it stands
-      T* an = A + (int64_t)(j + 1) * m;
+    __threadfence_block();
+    const T scal = sc[j], tj = ta[j];
+    const T* aj = A + (int64_t)j * m;
+    int c = j < w ? w : w + ((j - w) / NW + 1) * NW;  // own columns > j
+    if (c == j + 1) {
+      T* ac = A + (int64_t)c * m;
       T nrm = T(0.0);
-      for (int i = j + 2 + lane; i < m; i += 32) nrm += an[i] * an[i];
-      nrm = warp_sum_t(nrm);
-      if (lane == 0) sh_sig = nrm;
+      if (tj != 0.0) {
+        T acc = T(0.0);
+        for (int i = j + 1 + lane; i < m; i += 32) acc += aj[i] * ac[i];
+        acc = (warp_sum_t(acc) * scal + ac[j]) * tj;
+        __syncwarp();
+        if (lane == 0) ac[j] -= acc;
+        const T f = acc * scal;
+        for (int i = j + 1 + lane; i < m; i += 32) {
+          const T v = ac[i] - f * aj[i];
+          ac[i] = v;
+          if (i > j + 1) nrm += v * v;
+        }
+        __syncwarp();
+      } else {
+        for (int i = j + 2 + lane; i < m; i += 32) nrm += ac[i] * ac[i];
+      }
+      if (c < kmax) reflect(c, warp_sum_t(nrm));
+      c += NW;
+    }
+    if (tj == 0.0) continue;
+    // float pairs: two columns at a time, two independent dot products and updates in flight
+    constexpr int NC = std::is_same<T, ff>::value ? 2 : 1;
+    for (; c <= last; c += NC * NW) {
+      const bool two = NC == 2 && c + NW <= last;
+      T* ac = A + (int64_t)c * m;
+      T* ac2 = two ? ac + (int64_t)NW * m : ac;
+      T acc = T(0.0), acc2 = T(0.0);
+      for (int i = j + 1 + lane; i < m; i += 32) {
+        const T x = aj[i];
+        acc += x * ac[i];
+        if (two) acc2 += x * ac2[i];
+      }
+      acc = (warp_sum_t(acc) * scal + ac[j]) * tj;
+      if (two) acc2 = (warp_sum_t(acc2) * scal + ac2[j]) * tj;
+      __syncwarp();
+      if (lane == 0) {
+        ac[j] -= acc;
+        if (two) ac2[j] -= acc2;
+      }
+      const T f = acc * scal, f2 = acc2 * scal;
+      for (int i = j + 1 + lane; i < m; i += 32) {
+        const T x = aj[i];
+        ac[i] -= f * x;
+        if (two) ac2[i] -= f2 * x;
+      }
     }
   }
   __syncthreads();
-  if (kmax > 0) {  // the last reflector's vector
-    T* ap = A + (int64_t)(kmax - 1) * m;
-    for (int i = kmax + tid; i < m; i += blockDim.x) ap[i] *= prev_scal;
+  for (int j = w; j < kmax; j += NW) {
+    T* aj = A + (int64_t)j * m;
+    const T scal = sc[j];
+    for (int i = j + 1 + lane; i < m; i += 32) aj[i] *= scal;
   }
   __syncthreads();
-  for (int j = kmax + tid; j < r; j += blockDim.x) tau[leaf * r + j] = T(0.0);
-  for (int e = tid; e < r * r; e += blockDim.x) {
+  for (int j = kmax + tid; j < r; j += NT) tau[leaf * r + j] = T(0.0);
+  for (int e = tid; e < r * r; e += NT) {
     const int i = e % r, c = e / r;
     Rout[leaf * (int64_t)r * r + e] = (i <= c && i < m) ? A[(int64_t)c * m + i] : T(0.0);
   }
-  if (SMEM) {
-    __syncthreads();
-    for (int64_t e = tid; e < (int64_t)m * r; e += blockDim.x) G[e] = sm[e];
-  }
+  if (SMEM)
+    for (int e = tid; e < m * r; e += NT) G[e] = sm[e];
 }
-
 
 // Explicit leaf basis Q = H_0 ... H_{r-1} [I; 0] in place of the reflectors (LAPACK dorg2r).
 // Runs on the side stream, overlapped with the node levels (only the solves need Q).
 template <typename T, bool SMEM>
-__global__ void __launch_bounds__(leaf_qr_threads<T>()) k_leaf_formq(T* __restrict__ Pan, const T* __restrict__ tau,
+__global__ void __launch_bounds__(32 * leaf_qr_warps<T>()) k_leaf_formq(T* __restrict__ Pan, const T* __restrict__ tau,
                                                                      int r, DTree t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);
@@ -367,10 +385,6 @@ __global__ void __launch_bounds__(leaf_qr_threads<T>()) k_leaf_formq(T* __restri
 // them, and the solve after it), 134 k with 8 (was 245 k).
 // Shared memory: four r x 82 matrices, three r-vectors, barriers, flags and the list of H's entries.
 // ---------------------------------------------------------------------------------------------
-// Iteration bound of a spin wait on a shared-memory flag (a few tens of cycles per iteration:
-// well above any legitimate wait inside one node, far below a watchdog).  The spin does not
-// sleep: a sleeping waiter wakes too late for the column-to-column handoff.
-constexpr int kWaitLimit = 1 << 22;
 
 // v into the same shared-memory location as p in every CTA of the cluster (locally if csize = 1)
 template <typename T>
@@ -1033,13 +1047,14 @@ bool launch_leaf_chol(const double* K, T* Lf, const Tree& t, int* info, cudaStre
 }
 
 template <typename T>
-void launch_leaf_qr(T* Pan, int r, const Tree& t, T* tau, T* Rout, cudaStream_t st) {
+void launch_leaf_qr(T* Pan, int r, const Tree& t, T* tau, T* Rout, int* info, int wait_limit, cudaStream_t st) {
+  const unsigned nth = 32 * leaf_qr_warps<T>();
   const size_t sm = (size_t)t.max_leaf * r * sizeof(T);
   if (sm <= 200 * 1024) {
     smem_limit((const void*)k_leaf_qr<T, true>, sm);
-    k_leaf_qr<T, true><<<(unsigned)t.nleaf, leaf_qr_threads<T>(), sm, st>>>(Pan, r, dtree(t), tau, Rout);
+    k_leaf_qr<T, true><<<(unsigned)t.nleaf, nth, sm, st>>>(Pan, r, dtree(t), tau, Rout, info, wait_limit);
   } else {
-    k_leaf_qr<T, false><<<(unsigned)t.nleaf, leaf_qr_threads<T>(), 0, st>>>(Pan, r, dtree(t), tau, Rout);
+    k_leaf_qr<T, false><<<(unsigned)t.nleaf, nth, 0, st>>>(Pan, r, dtree(t), tau, Rout, info, wait_limit);
   }
 }
 
@@ -1392,9 +1407,9 @@ void launch_leaf_formq(T* Pan, const T* tau, int r, const Tree& t, cudaStream_t 
   const size_t sm = (size_t)t.max_leaf * r * sizeof(T);
   if (sm <= 200 * 1024) {
     smem_limit((const void*)k_leaf_formq<T, true>, sm);
-    k_leaf_formq<T, true><<<(unsigned)t.nleaf, leaf_qr_threads<T>(), sm, st>>>(Pan, tau, r, dtree(t));
+    k_leaf_formq<T, true><<<(unsigned)t.nleaf, 32 * leaf_qr_warps<T>(), sm, st>>>(Pan, tau, r, dtree(t));
   } else {
-    k_leaf_formq<T, false><<<(unsigned)t.nleaf, leaf_qr_threads<T>(), 0, st>>>(Pan, tau, r, dtree(t));
+    k_leaf_formq<T, false><<<(unsigned)t.nleaf, 32 * leaf_qr_warps<T>(), 0, st>>>(Pan, tau, r, dtree(t));
   }
 }
 
@@ -1421,8 +1436,8 @@ template void launch_node_finalize<ff>(const ff*, const ff*, const ff*, const ff
                                        ff*, ff*, ff*, ff*, cudaStream_t);
 
 template bool launch_leaf_chol<ff>(const double*, ff*, const Tree&, int*, cudaStream_t);
-template void launch_leaf_qr<double>(double*, int, const Tree&, double*, double*, cudaStream_t);
-template void launch_leaf_qr<ff>(ff*, int, const Tree&, ff*, ff*, cudaStream_t);
+template void launch_leaf_qr<double>(double*, int, const Tree&, double*, double*, int*, int, cudaStream_t);
+template void launch_leaf_qr<ff>(ff*, int, const Tree&, ff*, ff*, int*, int, cudaStream_t);
 template void launch_node_factor<double>(double*, const double*, int, int, const Tree&, double*, double*, double*,
                                          double*, int*, cudaStream_t, int, int);
 template void launch_node_factor<ff>(ff*, const ff*, int, int, const Tree&, ff*, ff*, ff*, ff*, int*, cudaStream_t,

@@ -109,7 +109,7 @@ bool launch_leaf_tri(const T* Lf, const Tree& t, int op, T* Bptr, int64_t bmul, 
 void launch_leaf_diaginv(double* Lf, const Tree& t, cudaStream_t st);
 bool launch_leaf_solve_f64(const double* Lf, const Tree& t, int op, double* X, int64_t ldx, int k, cudaStream_t st);
 template <typename T>
-void launch_leaf_qr(T* Pan, int r, const Tree& t, T* tau, T* Rout, cudaStream_t st);
+void launch_leaf_qr(T* Pan, int r, const Tree& t, T* tau, T* Rout, int* info, int wait_limit, cudaStream_t st);
 // Mixed form on the tensor cores (km_leaf_tc.cu): blocked Cholesky of the augmented leaf matrices
 // [K_j; Phi_j'] giving Lf_j (float pairs) and A_j = L_j^{-1} Phi_j in place of G (= the float-pair
 // Phi, m x r per leaf).  Lf holds the float-pair leaf matrices (lower triangles) on entry.  Step
