@@ -37,7 +37,6 @@ constexpr int kLcTileN = 64;           // columns of a tile (MMA N)
 constexpr int kLcTcThreads = 512;      // 16 warps: warp w reads tensor-memory lanes 32 (w % 4) .. + 31,
                                        // columns 16 (w / 4) .. + 15 of a tile
 constexpr int kLcDiagThreads = 512;
-constexpr int kLcDiagCols = kLcNB * kLcNB / kLcDiagThreads;  // trailing-update columns a thread
 constexpr int kLcProbeThreads = 256;
 constexpr uint32_t kLcTmemCols = 512;  // kSlices x kLcTileN = 448 accumulator columns
 constexpr uint32_t kATileBytes = kLcTileM * kLcNB * 2;  // one slice of a 128-row tile
@@ -114,7 +113,9 @@ __device__ __forceinline__ void lc_tile_values(uint32_t tl, int j0, int erow, co
 // Diagonal block: grid = nleaf, block = kLcDiagThreads, dynamic shared memory 2 x 64 x 65 float
 // pairs.  D = chol(B) and X = D^{-1} for the block B = rows / columns [c0, c0 + nb) of the
 // matrix being factored (row j of X is finalised at step j, then rows i > j subtract L_ij X_j);
-// beyond nb both are the identity.  Writes D to Lf and the slices of the rows of X (64 rows,
+// beyond nb both are the identity.  The chain of square roots and reciprocals bounds it: with two block
+// barriers a column 256 leaves took 118 us a block, by panels of 4 columns (the same operations on every
+// entry in the same order) 77 us.  Writes D to Lf and the slices of the rows of X (64 rows,
 // the canonical layout) with their exponents.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kLcDiagThreads) k_lc_diag(ff* __restrict__ Lf, DTree t, int c0,
@@ -124,7 +125,6 @@ __global__ void __launch_bounds__(kLcDiagThreads) k_lc_diag(ff* __restrict__ Lf,
   constexpr int LD = kLcNB + 1;
   ff* D = reinterpret_cast<ff*>(lc_smem_d);
   ff* X = D + kLcNB * LD;
-  __shared__ int sbad;
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   if (c0 >= m) return;
@@ -142,40 +142,115 @@ __global__ void __launch_bounds__(kLcDiagThreads) k_lc_diag(ff* __restrict__ Lf,
     D[i * LD + c] = v;
     X[i * LD + c] = ff(i == c ? 1.0 : 0.0);
   }
-  if (tid == 0) sbad = 0;
+  // Panels of 4 columns.  In step p the four warps of one SM quarter apply panel p - 1 to panel p, a
+  // column each, and warp 0 factors panel p in registers; warps 1 and 2, a thread per column of X, apply
+  // the rows of panel p - 2 to those of panel p - 1 and finish these; the other warps apply panel p - 1 to
+  // the columns of D behind panel p and the rows of panel p - 2 of X to its rows from panel p on.
+  __shared__ ff srinv[kLcNB];
+  constexpr int kP = 4;
+  const int w = tid >> 5, lane = tid & 31, np = (nb + kP - 1) / kP;
+  // the workers: warps 3, 5, 6, 7, 9, 10, 11, 13, 14, 15
+  const int wi = (w & 3) == 0 || w < 3 ? -1 : w == 3 ? 0 : 3 * (w >> 2) - 3 + (w & 3), nwi = 10;
+  int bad = 0;
   __syncthreads();
-  // two barriers a column: every thread forms the pivot from D[j][j] (left in place until the
-  // end, the factor's diagonal goes to sdiag) and scales its share of column j and of row j of X;
-  // then the trailing update
-  __shared__ ff sdiag[kLcNB];
-  for (int j = 0; j < nb; ++j) {
-    const ff d = D[j * LD + j];
-    const bool ok = d > 0.0;
-    const ff sd = ok ? sqrt(d) : ff(1.0);
-    const ff rinv = ff(1.0) / sd;
-    if (!ok && tid == 0 && sbad == 0) sbad = c0 + j + 1;
-    for (int i = j + 1 + tid; i < nb; i += NT) D[i * LD + j] = ff(D[i * LD + j] * rinv);
-    for (int c = tid; c <= j; c += NT) X[j * LD + c] = ff(X[j * LD + c] * rinv);
-    if (tid == 0) sdiag[j] = sd;
-    __syncthreads();
-    // trailing lower triangle of D (i >= c > j) and rows i > j of X (columns c <= j): thread
-    // (row i = tid % 64, columns kLcDiagCols g .. + kLcDiagCols - 1 with g = tid / 64), the row's
-    // pivot-column entry loaded once
-    for (int e = tid; e < kLcNB * (kLcNB / kLcDiagCols); e += NT) {
-      const int i = e & (kLcNB - 1), g = e / kLcNB;
-      if (i > j && i < nb) {
-        const ff lij = D[i * LD + j];
+  for (int p = 0; p <= np; ++p) {
+    const int c0p = kP * p, k0 = c0p - kP, q0 = k0 - kP;  // panels p, p - 1, p - 2
+    if ((w & 3) == 0 && p < np) {
+      const int c = c0p + (w >> 2);
+      if (p > 0 && c < nb) {
+        ff v[2];
 #pragma unroll
-        for (int c = kLcDiagCols * g; c < kLcDiagCols * g + kLcDiagCols; ++c) {
-          if (c <= j) X[i * LD + c] -= lij * X[j * LD + c];
-          else if (c <= i) D[i * LD + c] -= lij * D[c * LD + j];
+        for (int s = 0; s < 2; ++s) v[s] = D[(lane + 32 * s) * LD + c];
+#pragma unroll
+        for (int k = k0; k < k0 + kP; ++k) {
+          const ff mc = D[c * LD + k];
+#pragma unroll
+          for (int s = 0; s < 2; ++s) v[s] -= D[(lane + 32 * s) * LD + k] * mc;
+        }
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+          if (lane + 32 * s >= c && lane + 32 * s < nb) D[(lane + 32 * s) * LD + c] = v[s];
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");  // (warps 0, 4, 8, 12)
+      if (w == 0) {
+        ff v[kP][2];
+#pragma unroll
+        for (int j = 0; j < kP; ++j)
+#pragma unroll
+          for (int s = 0; s < 2; ++s) v[j][s] = D[(lane + 32 * s) * LD + min(c0p + j, kLcNB - 1)];
+        const bool upper = c0p < 32;  // the pivots' half of the rows
+#pragma unroll
+        for (int j = 0; j < kP; ++j) {
+          const int cj = c0p + j;
+          if (cj >= nb) break;
+          const ff d = shfl_idx(upper ? v[j][0] : v[j][1], cj & 31);
+          const bool ok = d > 0.0;
+          const ff sd = ok ? sqrt(d) : ff(1.0);
+          const ff rinv = ff(1.0) / sd;
+          if (!ok && bad == 0) bad = c0 + cj + 1;
+          ff x[2];
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const int i = lane + 32 * s;
+            x[s] = ff(v[j][s] * rinv);
+            if (i == cj) D[i * LD + cj] = sd;
+            else if (i > cj && i < nb) D[i * LD + cj] = x[s];
+          }
+          if (lane == 0) srinv[cj] = rinv;
+#pragma unroll
+          for (int q = j + 1; q < kP; ++q) {
+            const ff mc = shfl_idx(upper ? x[0] : x[1], (c0p + q) & 31);
+#pragma unroll
+            for (int s = 0; s < 2; ++s) v[q][s] -= x[s] * mc;
+          }
         }
       }
+    } else if (w == 1 || w == 2) {
+      const int c = tid - 32;
+      if (p > 0) {
+        ff a[kP], y[kP];
+#pragma unroll
+        for (int j = 0; j < kP; ++j) a[j] = X[min(k0 + j, kLcNB - 1) * LD + c];
+        if (p > 1)
+#pragma unroll
+          for (int k = q0; k < q0 + kP; ++k) {
+            const ff x = X[k * LD + c];
+            if (c <= k)
+#pragma unroll
+              for (int j = 0; j < kP; ++j) a[j] -= D[min(k0 + j, kLcNB - 1) * LD + k] * x;
+          }
+#pragma unroll
+        for (int j = 0; j < kP; ++j) {
+          if (k0 + j >= nb) break;
+#pragma unroll
+          for (int q = 0; q < j; ++q)
+            if (c <= k0 + q) a[j] -= D[(k0 + j) * LD + k0 + q] * y[q];
+          y[j] = ff(a[j] * srinv[k0 + j]);
+          if (c <= k0 + j) X[(k0 + j) * LD + c] = y[j];
+        }
+      }
+    } else if (wi >= 0) {
+      if (p > 0)
+        for (int c = c0p + kP + wi; c < nb; c += nwi)
+          for (int i = (c & 32) + lane; i < nb; i += 32) {
+            if (i < c) continue;
+            ff v = D[i * LD + c];
+#pragma unroll
+            for (int k = k0; k < k0 + kP; ++k) v -= D[i * LD + k] * D[c * LD + k];
+            D[i * LD + c] = v;
+          }
+      if (p > 1)
+        for (int i = c0p + wi; i < nb; i += nwi)
+          for (int c = lane; c < q0 + kP; c += 32) {
+            ff v = X[i * LD + c];
+#pragma unroll
+            for (int k = q0; k < q0 + kP; ++k)
+              if (c <= k) v -= D[i * LD + k] * X[k * LD + c];
+            X[i * LD + c] = v;
+          }
     }
     __syncthreads();
   }
-  for (int j = tid; j < nb; j += NT) D[j * LD + j] = sdiag[j];
-  __syncthreads();
   // L in the lower triangle of the diagonal block; the strictly lower part of X = D^{-1} in its
   // (otherwise unused) strictly upper triangle, X[i][c] at row c0 + c, column c0 + i, for the
   // block solves of k_leaf_tri_few and k_leaf_tri_wide (X's diagonal is 1 / D_ii, recomputed there the same way)
@@ -184,7 +259,7 @@ __global__ void __launch_bounds__(kLcDiagThreads) k_lc_diag(ff* __restrict__ Lf,
     if (i >= c) Lf[koff + (int64_t)(c0 + c) * m + c0 + i] = D[i * LD + c];
     else Lf[koff + (int64_t)(c0 + c) * m + c0 + i] = X[c * LD + i];
   }
-  if (tid == 0 && sbad != 0 && info[leaf] == 0) info[leaf] = sbad;
+  if (tid == 0 && bad != 0 && info[leaf] == 0) info[leaf] = bad;
   // rows of X: four threads per row, 16 columns each
   uint16_t* dst = xsl + leaf * (int64_t)(kSlices * kLcNB * kLcNB);
   for (int rr = tid >> 2; rr < kLcNB; rr += NT >> 2) {
