@@ -646,7 +646,7 @@ __global__ void k_eval_dphi2(const double* __restrict__ pts, const double* __res
 // VP[(leaf k + c) W + mat r + q] = sum_i A_mat[i][q] X[i][c]: the projections phi = Phi_l' x_c,
 // dphi_0 = dPhi_0,l' x_c and dphi_1 = dPhi_1,l' x_c (W = 4r; the nugget block mat = 3 comes from
 // k_nugget_proj), one small GEMM per (leaf, matrix), register-tiled.  A CTA takes the r rows of
-// matrix mat = blockIdx.y and 8g columns (g <= 10); thread (u, v) = (tid % uq, tid / uq),
+// matrix mat = blockIdx.y and 8g columns (g <= 5); thread (u, v) = (tid % uq, tid / uq),
 // uq = ceil(r / 4), accumulates the 4 x 8 block q = u + uq a, c = c0 + v + g b (strided, so that
 // the shared-memory reads of a warp fall in distinct banks).  The leaf rows go in chunks of 32:
 // A_mat (r x 32) and X (8g x 32) are staged in shared memory as T along i with a padded stride;
@@ -654,10 +654,10 @@ __global__ void k_eval_dphi2(const double* __restrict__ pts, const double* __res
 // leaves: g = 1) PARTS threads share a 4 x 8 block, each taking every PARTS-th row, and their sums
 // are added in order: 2 leaves of 500 points, 25 columns, rank 32 took 0.70 ms on 6 CTAs of one
 // warp, now 0.13 ms.  block uq g PARTS.
-constexpr int kPjK = 32, kPjS = kPjK + 1, kPjMaxG = 10, kPjMaxU = (kMaxNysRank + 3) / 4;
+constexpr int kPjK = 32, kPjS = kPjK + 1, kPjMaxG = 5, kPjMaxU = (kMaxNysRank + 3) / 4;
 
 template <typename T, int PARTS>
-__global__ void __launch_bounds__(kPjMaxU * kPjMaxG, 2)
+__global__ void __launch_bounds__(PARTS > 1 ? 200 : kPjMaxU * kPjMaxG, PARTS > 1 ? 2 : 4)
     k_leaf_proj3(const T* __restrict__ Phi, const T* __restrict__ dPhi2, int r, DTree t, const T* __restrict__ X,
                  int64_t ldx, double* __restrict__ VP, int k, int g) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -912,6 +912,16 @@ __global__ void __launch_bounds__(256) k_landmark(const double* __restrict__ VP,
   }
 }
 
+// two neighbours in 16-byte-aligned shared memory with one load
+template <typename T>
+struct __align__(16) Two {
+  T x, y;
+};
+template <typename T>
+__device__ __forceinline__ Two<T> load2(const T* p) {
+  return *reinterpret_cast<const Two<T>*>(p);
+}
+
 __device__ __forceinline__ double twice(double x) { return x + x; }
 __device__ __forceinline__ ff twice(ff x) { return ff(x.hi + x.hi, x.lo + x.lo); }
 
@@ -921,7 +931,9 @@ __device__ __forceinline__ ff twice(ff x) { return ff(x.hi + x.hi, x.lo + x.lo);
 // its leaf (numbered row by row): the tile
 // of G from 32-column chunks of X staged in shared memory (thread (tx, ty) takes rows tx and
 // columns ty + 8 q), the derivative entries evaluated in registers (dkernel3 / dkernel3_ff, one
-// distance and one exponential for the three), off-diagonal entries counted twice.
+// distance and one exponential for the three), off-diagonal entries counted twice.  512 leaves of 488, 73
+// columns in float pairs: 3.56 ms with a load for every operand and a full last row tile, now 3.33; FP32
+// issue bounds it (12 instructions a multiply-add, about 400 an entry for the derivatives).
 // grid (nleaf, S), block (32, 8).
 template <typename T>
 __global__ void __launch_bounds__(256) k_leaf_dk_gram(const double* __restrict__ pts, const float* __restrict__ P3,
@@ -932,8 +944,11 @@ __global__ void __launch_bounds__(256) k_leaf_dk_gram(const double* __restrict__
   const int m = d_leaf_size(t, leaf);
   const int64_t s = d_leaf_start(t, leaf);
   const int nt = (m + 31) / 32;
-  __shared__ T xr[32][33];
-  __shared__ T xc[32][33];
+  // two columns of the chunk are one 16-byte load; the odd number of 16 bytes a row keeps the lanes' loads
+  // in different banks
+  constexpr int LD = 34;
+  __shared__ __align__(16) T xr[32][LD];
+  __shared__ __align__(16) T xc[32][LD];
   __shared__ double red[8][3];
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
   const T wp = from_double<T>(p > 0 ? 1.0 / (double)p : 0.0), w_a = from_double<T>(wa);
@@ -946,29 +961,49 @@ __global__ void __launch_bounds__(256) k_leaf_dk_gram(const double* __restrict__
   }
   for (; ti < nt;) {
     {
-      const int i = ti * 32 + tx;
+      // thread (tx, ty) takes entry (bi 32 + tx, ba 32 + ty + 8 q); a last row tile of few rows lies on the
+      // q side, where rows past the leaf cost nothing
+      const bool swap = ti == nt - 1 && tj < ti && m - 32 * ti <= 16;
+      const int bi = swap ? tj : ti, ba = swap ? ti : tj, nq = min(4, (m - 32 * ba + 7) >> 3);
+      const int i = bi * 32 + tx;
       acc_t<T> sp[4] = {}, sa[4] = {};
       for (int c0 = 0; c0 <= p; c0 += 32) {
         __syncthreads();
         for (int e = tid; e < 32 * 32; e += 256) {
           const int cq = e >> 5, rq = e & 31;  // column cq of the chunk, row rq of the tile
           const int c = c0 + cq;
-          const int ri = ti * 32 + rq, rj = tj * 32 + rq;
+          const int ri = bi * 32 + rq, rj = ba * 32 + rq;
           xr[rq][cq] = (c <= p && ri < m) ? X[(int64_t)c * n + s + ri] : T(0.0);
           xc[rq][cq] = (c <= p && rj < m) ? X[(int64_t)c * n + s + rj] : T(0.0);
         }
         __syncthreads();
         const int cend = min(32, p - c0);  // probe columns of this chunk; column p (alpha) apart
-        for (int cq = 0; cq < cend; ++cq) {
-          const T a = xr[tx][cq];
+        auto products = [&](auto count) {
+          constexpr int NQ = decltype(count)::value;
+          int cq = 0;
+          for (; cq + 1 < cend; cq += 2) {
+            const Two<T> a = load2(&xr[tx][cq]);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) sp[q] += a * xc[ty + 8 * q][cq];
-        }
-        if (p - c0 < 32) {
-          const T a = xr[tx][p - c0];
+            for (int q = 0; q < NQ; ++q) {
+              const Two<T> b = load2(&xc[ty + 8 * q][cq]);
+              sp[q] += a.x * b.x;
+              sp[q] += a.y * b.y;
+            }
+          }
+          if (cq < cend) {
+            const T a = xr[tx][cq];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) sa[q] += a * xc[ty + 8 * q][p - c0];
-        }
+            for (int q = 0; q < NQ; ++q) sp[q] += a * xc[ty + 8 * q][cq];
+          }
+          if (p - c0 < 32) {
+            const T a = xr[tx][p - c0];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) sa[q] += a * xc[ty + 8 * q][p - c0];
+          }
+        };
+        if (nq > 2) products(std::integral_constant<int, 4>());
+        else if (nq == 2) products(std::integral_constant<int, 2>());
+        else products(std::integral_constant<int, 1>());
       }
       double xi = 0.0, yi = 0.0;
       f3 x3i{}, y3i{};
@@ -982,10 +1017,10 @@ __global__ void __launch_bounds__(256) k_leaf_dk_gram(const double* __restrict__
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int a = tj * 32 + ty + 8 * q;
-        if (i < m && a < m && i >= a) {
+        const int a = ba * 32 + ty + 8 * q;
+        if (i < m && a < m && (swap || i >= a)) {
           T gv = T(accv(sp[q]) * wp) + T(accv(sa[q]) * w_a);
-          if (i > a) gv = twice(gv);
+          if (i != a) gv = twice(gv);
           if constexpr (std::is_same<T, ff>::value) {
             f3 x3a, y3a;
             load_p3(P3, s + a, x3a, y3a);
@@ -1052,9 +1087,12 @@ template <typename T>
 void launch_leaf_proj3(const T* Phi, const T* dPhi2, int r, const Tree& t, const T* X, int64_t ldx, double* VP, int k,
                        cudaStream_t st) {
   const int uq = (r + 3) / 4;
-  int g = std::min(kPjMaxG, (k + 7) / 8);
+  // columns in equal CTAs of at most 40: several CTAs an SM, one loading while another multiplies (512 leaves
+  // of 488, rank 72, 73 columns in float pairs: 2.45 ms with 80 a CTA, 2.33 with 40)
+  const int nz = (k + 39) / 40;
+  int g = ((k + nz - 1) / nz + 7) / 8;
   constexpr int kParts = 8;
-  const bool few = t.nleaf * 3 * ((k + 8 * g - 1) / (8 * g)) < 2 * 152 && uq * kParts <= kPjMaxU * kPjMaxG;
+  const bool few = t.nleaf * 3 * ((k + 79) / 80) < 2 * 152;
   if (few) g = 1;
   dim3 grid((unsigned)t.nleaf, 3u, (unsigned)((k + 8 * g - 1) / (8 * g)));
   const size_t sm = std::max((size_t)(4 * uq + 8 * g) * kPjS, (size_t)32 * uq * g) * sizeof(T);
