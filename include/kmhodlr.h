@@ -472,7 +472,7 @@ int km_profile_get(km_handle* h, int cls, double* total_ms, int64_t* launches);
 /* ---- diagnostics ------------------------------------------------------------------------- */
 
 /* Number of polls after which a bounded device-side wait of this handle's kernels gives up: the
- * dataflow flags and barriers of the node factorisation and the grid barriers of the ACA and tall
+ * dataflow flags and barriers of the leaf QR and the node factorisation and the grid barriers of the ACA and tall
  * panel-QR kernels.  polls < 0 restores the defaults (well above any legitimate wait); 0 makes
  * every such wait give up at its first poll, as if the flag it waits for were never set.  A wait
  * that gives up ends its kernel early and the call returns KM_ERR_TIMEOUT; the handle stays
