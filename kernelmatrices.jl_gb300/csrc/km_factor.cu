@@ -172,10 +172,10 @@ constexpr int kWaitLimit = 1 << 22;
 // the end.  Waits are bounded; one that runs out marks the leaf with info = -1 and the warp carries on.
 // With two block barriers a column and one thread forming the reflector between them (same operations,
 // same order) 256 panels of 256 x 72 took 636 us in float pairs and 1.64 ms in FP64, 512 of 488 x 72
-// 2.35 ms in float pairs; now 527 us, 1.42 ms and 1.91 ms.  FP64 has a quarter of the warps: one warp fills a
-// quarter of its pipe.  grid nleaf, block 32 NW.
+// 2.35 ms in float pairs; now 527 us, 1.42 ms and 1.91 ms.  FP64 has
+// half of the warps (64 panels of 469 x 72: 1.76, 1.07, 0.97, 0.95 ms with 4, 8, 12, 16).  grid nleaf, block 32 NW.
 template <typename T>
-constexpr int leaf_qr_warps() { return std::is_same<T, double>::value ? 8 : 32; }
+constexpr int leaf_qr_warps() { return std::is_same<T, double>::value ? 16 : 32; }
 
 template <typename T, bool SMEM>
 __global__ void __launch_bounds__(32 * leaf_qr_warps<T>()) k_leaf_qr(T* __restrict__ Pan, int r, DTree t,
@@ -224,11 +224,14 @@ __global__ void __launch_bounds__(32 * leaf_qr_warps<T>()) k_leaf_qr(T* __restri
   };
   {  // norm of column 0 below its first row
     T part = T(0.0);
-    for (int i = 1 + tid; i < m; i += NT) part += A[i] * A[i];
+    // (in FP64 the sums of 8 warps, also with 16: the order of the additions fixes the factor's bits)
+    constexpr int NS = std::is_same<T, double>::value ? 8 : NW;
+    if (w < NS)
+      for (int i = 1 + tid; i < m; i += 32 * NS) part += A[i] * A[i];
     part = warp_sum_t(part);
     if (lane == 0) red[w] = part;
     __syncthreads();
-    if (w == 0) reflect(0, warp_sum_t(lane < NW ? red[lane] : T(0.0)));
+    if (w == 0) reflect(0, warp_sum_t(lane < NS ? red[lane] : T(0.0)));
   }
   bool timed_out = false;
   const int last = w < r ? w + (r - 1 - w) / NW * NW : -1;
