@@ -462,6 +462,11 @@ static void launch_sweep(void (*fn)(P...), dim3 grid, int nth, size_t sm, cudaSt
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = early ? 1 : 0;
+  const cudaError_t prior = cudaPeekAtLastError();
+  if (cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...) == cudaSuccess || !early) return;
+  // an early start was refused (nothing ran): an ordinary launch; an error from before stays for the caller
+  if (prior == cudaSuccess) cudaGetLastError();
+  cfg.numAttrs = 0;
   cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
 }
 
