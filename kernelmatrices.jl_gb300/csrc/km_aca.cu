@@ -1053,6 +1053,7 @@ struct GShape {
 };
 GShape ga_shape(int n, int maxr, int maxcols, int64_t maxs) {
   GShape g{ga_width(maxcols, maxr), 0, 0, 0};
+  if (n <= 0 || maxcols <= 0) return g;  // (a level without items, or with big ones only)
   g.cols = (maxcols + g.cb - 1) / g.cb;
   const int64_t ctas = (int64_t)n * g.cols;
   if (ctas >= 6 * 152) return g;
