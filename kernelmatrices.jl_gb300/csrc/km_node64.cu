@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
   // 256 / nown-th row, scales the row's entry for itself, and the first of them stores it
   for (int i = tid; i < r; i += kThreads) vi[i] = 1.0 / X3[i + i * ld];
   __syncthreads();
-  {
+  if (nown > 0) {  // (a CTA of a rank below the cluster size may own no column)
     const int per = kThreads / nown, off = tid / nown, c = rank + cs * (tid - off * nown);
     double* b = X2 + c * ld;
     for (int i = 0; i < r; ++i) {

@@ -105,3 +105,26 @@ def test_wait_runs_out_then_the_handle_recovers(lib, r):
     assert np.array_equal(solve(h), solve(fresh))
     lib.km_destroy(h)
     lib.km_destroy(fresh)
+
+
+@pytest.mark.parametrize("n,lv,r", [(160, 3, 2), (331, 4, 3), (332, 3, 4), (500, 4, 5), (700, 4, 6), (701, 3, 7),
+                                    (333, 3, 8), (400, 3, 9)])
+def test_ranks_below_the_cluster_size(lib, n, lv, r):
+    """With 8 CTAs a node and fewer columns than that, some CTAs own no column.  The factor's
+    identities to 1e-12 times the condition number (below 1e3 with a nugget of 1), and the oracle."""
+    import kmhodlr as K
+    from kmhodlr.data import uniform_points
+    from oracle import hodlr_oracle as O
+    pts = uniform_points(n, 11)
+    p = np.array([1.0, 0.05, 1.0])
+    b = np.random.default_rng(12).standard_normal((n, 3))
+    hk = K.KernelHODLR(K.KernelMatrix(pts, pts, p, K.Matern32()), 0.0, r, K.FixedLevel(lv), nystrom=True)
+    y = hk @ b
+    K.symmetricfactorize(hk)
+    ok = O.build_hodlr(O.KernelMatrix(pts, pts, p, O.KERNEL_MATERN32), 0.0, r, O.FixedLevel(lv), nystrom=True)
+    O.symmetricfactorize(ok)
+    close = lambda a, c: np.linalg.norm(a - c) < 1e-9 * np.linalg.norm(c)  # noqa: E731
+    assert close(hk.ldiv(b), O.hodlr_ldiv(ok, b))
+    assert close(hk.ldiv(y), b) and close(hk @ b, y)
+    assert close(hk.W.ldiv(hk.W @ b), b) and close(hk.W.T.ldiv(hk.W.T @ b), b)
+    assert abs(hk.logdet() - O.hodlr_logdet(ok)) < 1e-9 * n
