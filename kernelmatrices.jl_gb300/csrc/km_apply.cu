@@ -106,6 +106,8 @@ __device__ __forceinline__ void stage_wait() {
 // run, and waits for the one before it only when it needs that one's vectors.  The launch and the
 // staging of the node matrices (final before the sweep began) thus overlap the level before: a level of
 // a one-column sweep took 10 to 14 us, of which 5 were these.  (Both do nothing in an ordinary launch.)
+// The vectors VP, VD and VG are plain pointers in these kernels: the one in front still writes them while
+// this one runs, which __restrict__ and the read-only loads it permits rule out.
 __device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -114,7 +116,7 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 // or from shared memory in a staged launch.
 template <typename T, bool STAGE>
 __global__ void __launch_bounds__(512) k_up(NodeMats<T> nm, int level, int L, int64_t cslot0, int64_t nslot0,
-                                            int64_t node0, T* __restrict__ VP, T* __restrict__ VD, int k, int mode, int kcb) {
+                                            int64_t node0, T* VP, T* VD, int k, int mode, int kcb) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* z = reinterpret_cast<T*>(smraw);   // kcb x 2r : [z1 ; z2] per column
   const int r = nm.r, r2 = 2 * r;
@@ -221,8 +223,8 @@ __global__ void __launch_bounds__(512) k_up(NodeMats<T> nm, int level, int L, in
 
 template <typename T, bool STAGE>
 __global__ void __launch_bounds__(512) k_down(NodeMats<T> nm, int level, int L, int64_t cslot0, int64_t nslot0,
-                                              int64_t node0, const T* __restrict__ VP, T* __restrict__ VG,
-                                              const T* __restrict__ VD, int k, int mode, int kcb) {
+                                              int64_t node0, const T* VP, T* VG, const T* VD, int k, int mode,
+                                              int kcb) {
   extern __shared__ __align__(16) unsigned char smraw[];
   T* g = reinterpret_cast<T*>(smraw);   // kcb x r  (parent coefficient)
   const int r = nm.r, r2 = 2 * r;

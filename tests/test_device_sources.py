@@ -1,0 +1,28 @@
+"""Promises that the device code must not make, read off its source (no GPU, no compiler)."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "kernelmatrices.jl_gb300" / "csrc"
+
+
+def kernels(text):
+    """(name, parameters, body) of every __global__ function of a source."""
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^;{]*?\)\s+)?(\w+)\(", text):
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[i], 0)
+            i += 1
+        depth, j = 1, text.index("{", i) + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[j], 0)
+            j += 1
+        yield m.group(1), text[m.end():i - 1], text[i:j]
+
+
+def test_kernels_that_start_early_do_not_restrict_their_vectors():
+    """__restrict__ promises that nobody else writes the vectors while the kernel runs, and allows loads by the
+    read-only path; the kernel in front of one that starts early still does."""
+    early = [(name, args) for f in CSRC.glob("*.cu") for name, args, body in kernels(f.read_text())
+             if "wait_for_previous()" in body or "griddepcontrol.wait" in body]
+    assert {name for name, _ in early} == {"k_up", "k_down"}
+    assert [name for name, args in early if "__restrict__" in args] == []
