@@ -1366,6 +1366,8 @@ static int aca_assemble(km_handle* h, const double* pts, bool dev, const Tree& t
     KM_CUDA(h, cudaMemsetAsync(h->d_bstatus, 0, sizeof(int) * nb, st));
   }
   KLV(h, KM_PROF_EVAL, launch_eval_leaves(h->d_pts, t, h->kp, -1, h->d_K, st));
+  // (now: setting a kernel attribute, as the first ACA launch of a process does, drops a pending error)
+  if ((rc = check_launch(h, "leaf evaluation")) != KM_OK) return rc;
   if (nb > 0)
     KLV(h, KM_PROF_ACA, launch_aca(h->d_pts, h->kp, h->d_blk, nb, maxcap, h->d_panels, h->d_flags, h->d_piv, tol,
                                    h->d_brank, h->d_bstatus, st, 1));
