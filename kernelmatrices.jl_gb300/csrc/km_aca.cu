@@ -16,7 +16,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <atomic>
 #include <climits>
 
 #include "km_kernels.h"
@@ -1175,31 +1174,6 @@ bool launch_aca_grid(const double* pts, KParams kp, const AcaBlock* blocks, int 
   return true;
 }
 
-// CTAs per cluster of k_aca: 16 where clusters of that size can be scheduled, else 8
-static int aca_cluster(size_t sm) {
-  static std::atomic<int> known{0};
-  int v = known.load();
-  if (v == 0) {
-    v = 8;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(kAcaThreads);
-    cfg.dynamicSmemBytes = sm;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim = {16, 1, 1};
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaFuncSetAttribute((const void*)k_aca, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, (const void*)k_aca, &cfg) == cudaSuccess && n > 0)
-      v = 16;
-    cudaGetLastError();  // a refused query leaves clusters of 8
-    known.store(v);
-  }
-  return v;
-}
-
 static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int last_first, int only,
                        int maxcap, double* P, uint8_t* F, int* piv, double rtol, int* rank, int* status,
                        cudaStream_t st) {
@@ -1207,7 +1181,8 @@ static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, in
   // an SM (more, and the shared memory is worth more as L1 cache)
   size_t sm = ((size_t)3 * std::max(maxcap, 1) + 2 + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
   smem_limit((const void*)k_aca, kAcaSmem);
-  const int cs = aca_cluster(kAcaSmem);
+  // CTAs per cluster: 16 where clusters of that size can be scheduled, else 8
+  const int cs = cluster_limit((const void*)k_aca, kAcaThreads, kAcaSmem) >= 16 ? 16 : 8;
   const int per = ((only >= 0 ? 1 : nblocks) * cs + 151) / 152;
   if (per <= 3) sm = std::max(sm, kAcaSmem / per);
   cudaLaunchConfig_t cfg = {};

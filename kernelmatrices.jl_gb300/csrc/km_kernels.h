@@ -12,6 +12,12 @@ namespace km {
 // (the batched and serving forms) cannot shrink it under one another's launches.
 void smem_limit(const void* func, size_t bytes);
 
+// Largest cluster of kernel `func` that can be scheduled on the current device with this block size
+// and dynamic shared memory: 16, 8, 4, 2, or 1 where clusters are refused.  Asked once per kernel and
+// device (so with the most shared memory that the kernel takes); clusters above 8, which need a
+// permission per kernel and device, are allowed on the way.  The first query drops a pending launch
+// error (setting a kernel attribute does), so callers check theirs before it.
+int cluster_limit(const void* func, int threads, size_t smem);
 
 // Operand of the leaf triangular kernels: leaf j's block starts at ptr + start(j) * bmul with
 // leading dimension m_j (ld_is_m) or ld.

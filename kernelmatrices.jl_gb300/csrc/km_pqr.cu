@@ -344,11 +344,9 @@ int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, doubl
   // CTAs per panel: enough for the rows to fit, then as many as keep a CTA per SM and 128 rows or
   // more each (a column's work shrinks with the rows, its barrier does not)
   int cs = 1;
-  while (cs < 16 && mmax > (int64_t)cs * kRowsMax) cs <<= 1;
-  while (cs < 16 && n * cs * 2 <= 152 && mmax > (int64_t)cs * 128) cs <<= 1;
-  static const bool wide = cudaFuncSetAttribute((const void*)k_pqr_factor,
-                                                cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  (void)wide;
+  const int most = cluster_limit((const void*)k_pqr_factor, kThreads, (size_t)kPB * (kRowsMax | 1) * sizeof(double));
+  while (cs < most && mmax > (int64_t)cs * kRowsMax) cs <<= 1;
+  while (cs < most && n * cs * 2 <= 152 && mmax > (int64_t)cs * 128) cs <<= 1;
   int launches = 0;
   const int frows = pqr_rows(n, mmax, kApplyRows);
   auto apply = [&](int j0, int nt, int transT) {

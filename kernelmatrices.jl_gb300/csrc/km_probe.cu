@@ -108,4 +108,33 @@ void smem_limit(const void* func, size_t bytes) {
     cudaGetLastError();  // the launch then reports the size error itself
 }
 
+int cluster_limit(const void* func, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  int& limit = known[{func, dev}];
+  if (limit > 0) return limit;
+  smem_limit(func, smem);
+  const bool wide = cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  for (limit = wide ? 16 : 8; limit > 1; limit >>= 1) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)limit);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)limit;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, func, &cfg) == cudaSuccess && n > 0) break;
+  }
+  cudaGetLastError();  // a refused query leaves smaller clusters
+  return limit;
+}
+
 }  // namespace km

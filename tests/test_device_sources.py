@@ -26,3 +26,11 @@ def test_kernels_that_start_early_do_not_restrict_their_vectors():
              if "wait_for_previous()" in body or "griddepcontrol.wait" in body]
     assert {name for name, _ in early} == {"k_up", "k_down"}
     assert [name for name, args in early if "__restrict__" in args] == []
+
+
+def test_cluster_permission_is_set_per_device():
+    """The permission for clusters above 8 belongs to a kernel on a device: one place asks for it, by device."""
+    users = {f.name for f in CSRC.glob("*.cu*") if "NonPortableClusterSizeAllowed" in f.read_text()}
+    assert users == {"km_probe.cu"}
+    body = (CSRC / "km_probe.cu").read_text().split("int cluster_limit(", 1)[1]
+    assert "known[{func, dev}]" in body
