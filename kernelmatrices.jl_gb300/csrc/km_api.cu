@@ -489,9 +489,6 @@ NodeMatsH node_mats(km_handle* h) {
 // Nodes at least this large (rows of both children) update the coarser panels of the factorisation
 // by FP64 products over all SMs (launch_dgemm): those updates have hundreds of columns.
 constexpr int64_t kGapplyBig = 16384;
-// Panels of more rows than a cluster's shared memory holds are factored by all SMs
-// (launch_panel_qr_gemm), the others by clusters (launch_panel_qr).
-constexpr int64_t kPanelBig = kPanelRowsMax + 1;
 
 // Applies the node factors of items [a, b) of a level (host list hl, device list dl), modes as in
 // k_gapply: 0 W^{-1}, 1 W'^{-1}, 2 W, 3 W', 4 pre-factor product (Q1 = V rows c1, Q2 = U rows c2;
@@ -1450,6 +1447,9 @@ static int general_factorize(km_handle* h) {
   cudaStream_t st = h->stream;
   const int nb = (int)h->blk.size();
   int rc;
+  // panels of more rows than a cluster's shared memory holds are factored by all SMs
+  // (launch_panel_qr_gemm), the others by clusters (launch_panel_qr)
+  const int64_t rows_max = panel_rows_max();
   timer_start(h);
   KM_CUDA(h, cudaMemsetAsync(h->d_info, 0, sizeof(int) * (t.nleaf + nb + 1), st));  // + grid-barrier word
   if (!leaf_chol_f64(h, 0))
@@ -1483,9 +1483,9 @@ static int general_factorize(km_handle* h) {
         int64_t o = 0;
         for (int p = 0; p < q; ++p) o += (int64_t)h->brank[p] * h->brank[p];
         const int rq = h->brank[q];
-        pd.push_back(PanelDesc{h->d_panels + b.offV, b.ncl, b.ncl, rq, h->d_R12 + 2 * o, b.ncl >= kPanelBig ? 1 : 0});
+        pd.push_back(PanelDesc{h->d_panels + b.offV, b.ncl, b.ncl, rq, h->d_R12 + 2 * o, b.ncl > rows_max ? 1 : 0});
         pd.push_back(PanelDesc{h->d_panels + b.offU, b.nro, b.nro, rq, h->d_R12 + 2 * o + (int64_t)rq * rq,
-                               b.nro >= kPanelBig ? 1 : 0});
+                               b.nro > rows_max ? 1 : 0});
         for (int lev = l + 1; lev <= t.L; ++lev) {
           const int64_t kp = k >> (lev - l);
           const int qp = (int)(h->lvoff[lev] + kp);

@@ -15,7 +15,7 @@ void smem_limit(const void* func, size_t bytes);
 // Largest cluster of kernel `func` that can be scheduled on the current device with this block size
 // and dynamic shared memory: 16, 8, 4, 2, or 1 where clusters are refused.  Asked once per kernel and
 // device (so with the most shared memory that the kernel takes); clusters above 8, which need a
-// permission per kernel and device, are allowed on the way.  The first query drops a pending launch
+// permission per kernel and device, are allowed on the way.  KM_CLUSTER_MAX=1, 2, 4, 8 or 16 caps it.  The first query drops a pending launch
 // error (setting a kernel attribute does), so callers check theirs before it.
 int cluster_limit(const void* func, int threads, size_t smem);
 
@@ -253,9 +253,11 @@ int64_t aca_grid_scratch(int cap);
 void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b, int maxcap, double* P,
                     uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st);
 // Householder QR with explicit Q of the panels that are not marked big (km_pqr.cu): n descriptors,
-// largest column count kmax, largest row count mmax <= kPanelRowsMax of those panels; scratch of
+// largest column count kmax, largest row count mmax <= panel_rows_max() of those panels; scratch of
 // panel_qr_scratch(n, kmax, mmax) doubles.  Returns the number of kernels launched.
-constexpr int64_t kPanelRowsMax = 12288;  // 16 CTAs of 768 rows x 32 columns of shared memory
+// panel_rows_max: rows that the largest cluster of the current device holds (768 a CTA: 12288 with 16;
+// asks cluster_limit)
+int64_t panel_rows_max();
 int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, double* scratch, cudaStream_t st);
 int64_t panel_qr_scratch(int n, int kmax, int64_t mmax);
 void launch_panel_rout(const PanelDesc* descs, int n, int kmax, int big, cudaStream_t st);

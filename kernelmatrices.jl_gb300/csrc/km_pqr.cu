@@ -317,6 +317,12 @@ __global__ void __launch_bounds__(kThreads) k_pqr_form(const PanelDesc* __restri
 
 }  // namespace
 
+static int pqr_cluster_limit() {
+  return cluster_limit((const void*)k_pqr_factor, kThreads, (size_t)kPB * (kRowsMax | 1) * sizeof(double));
+}
+
+int64_t panel_rows_max() { return (int64_t)kRowsMax * pqr_cluster_limit(); }
+
 // rows of a CTA when `others` CTAs share a row range of mmax: the most that still give four CTAs an
 // SM, at least 64 (an update CTA repeats the 32 x 32 x 32 product with T)
 static int pqr_rows(int64_t others, int64_t mmax, int most) {
@@ -344,7 +350,7 @@ int launch_panel_qr(const PanelDesc* descs, int n, int kmax, int64_t mmax, doubl
   // CTAs per panel: enough for the rows to fit, then as many as keep a CTA per SM and 128 rows or
   // more each (a column's work shrinks with the rows, its barrier does not)
   int cs = 1;
-  const int most = cluster_limit((const void*)k_pqr_factor, kThreads, (size_t)kPB * (kRowsMax | 1) * sizeof(double));
+  const int most = pqr_cluster_limit();
   while (cs < most && mmax > (int64_t)cs * kRowsMax) cs <<= 1;
   while (cs < most && n * cs * 2 <= 152 && mmax > (int64_t)cs * 128) cs <<= 1;
   int launches = 0;

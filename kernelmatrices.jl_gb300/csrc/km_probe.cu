@@ -1,5 +1,7 @@
 // Device FP64 FMA throughput probe (the roofline denominator of FP64-ALU-bound kernels: the
 // measured peaks file of the GPU pool carries only HBM copy and bf16 tensor rates).
+#include <algorithm>
+#include <cstdlib>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -111,6 +113,11 @@ void smem_limit(const void* func, size_t bytes) {
 int cluster_limit(const void* func, int threads, size_t smem) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, int> known;
+  static const int cap = [] {
+    const char* e = std::getenv("KM_CLUSTER_MAX");
+    const int v = e ? std::atoi(e) : 16;
+    return v >= 16 ? 16 : v >= 8 ? 8 : v >= 4 ? 4 : v >= 2 ? 2 : 1;
+  }();
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(mu);
@@ -118,7 +125,7 @@ int cluster_limit(const void* func, int threads, size_t smem) {
   if (limit > 0) return limit;
   smem_limit(func, smem);
   const bool wide = cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  for (limit = wide ? 16 : 8; limit > 1; limit >>= 1) {
+  for (limit = std::min(cap, wide ? 16 : 8); limit > 1; limit >>= 1) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)limit);
     cfg.blockDim = dim3((unsigned)threads);
