@@ -347,8 +347,9 @@ __global__ void __launch_bounds__(512) k_leaf_nys_apply(const double* __restrict
   }
   // beta = S^{-1} a = Sc^{-T} Sc^{-1} a, one warp per column, with the reciprocals of Sc's diagonal (a
   // division in each of the 2 r steps of the chain took most of its time: 256 leaves of 256, rank 72, one
-  // column, the whole kernel 174 us with them, 149 without)
-  __shared__ double rdiag[kMaxNysRank];
+  // column, the whole kernel 174 us with them, 149 without); they lie where the parts are added later
+  double* red = bs + 8 * r;  // kNaParts x kNaRows x 8
+  double* rdiag = red;
   for (int l = threadIdx.x; l < r; l += blockDim.x) rdiag[l] = 1.0 / Sc[(int64_t)l * r + l];
   __syncthreads();
   if (w < nc) {
@@ -377,7 +378,6 @@ __global__ void __launch_bounds__(512) k_leaf_nys_apply(const double* __restrict
   // entry feeding the nc columns; the parts are added in order through shared memory.
   const double* K = Kl + d_leaf_koff(t, leaf);
   const double* P = Phi + s * r;
-  double* red = bs + 8 * r;  // kNaParts x kNaRows x 8
   const int il = threadIdx.x % kNaRows, part = threadIdx.x / kNaRows;
   const int l0 = (int)((int64_t)m * part / kNaParts), l1 = (int)((int64_t)m * (part + 1) / kNaParts);
   const int q0 = r * part / kNaParts, q1 = r * (part + 1) / kNaParts;
