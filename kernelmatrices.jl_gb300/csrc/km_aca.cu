@@ -937,10 +937,14 @@ __global__ void __launch_bounds__(kGaThreads) k_gproj(const GApplyItem* __restri
   double* xs = Z + CB * r;
   const int nc = min(CB, ncols - col), n = (int)min((int64_t)sp.rows, s - i0);
   for (int e = threadIdx.x; e < CB * r; e += kGaThreads) Z[e] = 0.0;
-  for (int c = 0; c < CB; ++c)
-    for (int i = threadIdx.x; i < n; i += kGaThreads) xs[c * kGaStage + i] = c < nc ? x[c * ld + i] : 0.0;
-  __syncthreads();
-  ga_proj<CB>((first ? N.Q1 : N.Q2) + i0, s, r, n, xs, kGaStage, Z, r, 1.0);
+  for (int j0 = 0; j0 < n; j0 += kGaStage) {
+    const int nj = min(kGaStage, n - j0);
+    __syncthreads();
+    for (int c = 0; c < CB; ++c)
+      for (int i = threadIdx.x; i < nj; i += kGaThreads) xs[c * kGaStage + i] = c < nc ? x[c * ld + j0 + i] : 0.0;
+    __syncthreads();
+    ga_proj<CB>((first ? N.Q1 : N.Q2) + i0 + j0, s, r, nj, xs, kGaStage, Z, r, 1.0);
+  }
   __syncthreads();
   double* out = sp.part + ((((int64_t)2 * blockIdx.x + d) * sp.nchunk + h) * sp.ncol + col) * sp.ldr;
   for (int e = threadIdx.x; e < CB * r; e += kGaThreads) out[(int64_t)(e / r) * sp.ldr + e % r] = Z[e];
@@ -1046,7 +1050,8 @@ int ga_width(int ncols, int r) {
 
 // Shape of an application: how many columns a CTA takes and, when the items alone would not give
 // six CTAs an SM, how the rows are split so that the projections and expansions do (chunks of 64
-// to kGaStage rows, at most 64 of them, so that their sums stay a small part of the middle step).
+// rows or more, at most 64 of them, so that their sums stay a small part of the middle step and,
+// with fewer than 12 CTAs an SM in all, their scratch small whatever the rows and columns).
 struct GShape {
   int cb, cols, rows, nchunk;  // nchunk 0: one launch
 };
@@ -1057,8 +1062,7 @@ GShape ga_shape(int n, int maxr, int maxcols, int64_t maxs) {
   const int64_t ctas = (int64_t)n * g.cols;
   if (ctas >= 6 * 152) return g;
   const int64_t want = std::min<int64_t>((6 * 152 + 2 * ctas - 1) / (2 * ctas), 64);
-  int64_t rows = std::max<int64_t>(64, ((maxs + want - 1) / want + 31) / 32 * 32);
-  g.rows = (int)std::min<int64_t>(rows, kGaStage);
+  g.rows = (int)std::max<int64_t>(64, ((maxs + want - 1) / want + 31) / 32 * 32);
   g.nchunk = (int)((maxs + g.rows - 1) / g.rows);
   return g;
 }
@@ -1067,7 +1071,7 @@ template <int CB>
 void gapply_launch(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, const GShape& g, int mode,
                    double* X, const double* Xin, int64_t ldX, int kX, double* scratch, cudaStream_t st) {
   const size_t sm = ga_smem(CB, maxr);
-  if (g.nchunk == 0) {
+  if (g.nchunk == 0 || !scratch) {
     smem_limit((const void*)k_gapply<CB>, sm);
     k_gapply<CB><<<dim3((unsigned)n, (unsigned)g.cols), kGaThreads, sm, st>>>(items, nodes, mode, X, Xin, ldX, kX);
     return;
@@ -1540,7 +1544,7 @@ int launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int ma
    : g.cb == 4 ? gapply_launch<4>
    : g.cb == 2 ? gapply_launch<2>
                : gapply_launch<1>)(items, n, nodes, maxr, g, mode, X, Xin, ldX, kX, scratch, st);
-  return g.nchunk > 0 ? 3 : 1;
+  return g.nchunk > 0 && scratch ? 3 : 1;
 }
 
 void launch_gsmall(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2,

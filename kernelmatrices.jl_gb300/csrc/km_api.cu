@@ -501,7 +501,7 @@ static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyIte
   // scratch of the whole sweep, so that its levels do not regrow it one after the other
   const std::vector<int64_t>& off = &hl == &h->gsolve_h ? h->lvoff : h->gfoff;
   int maxr = 1, maxcols = 0;  // of this level, over the items that are not big
-  int64_t maxs = 1, need = 0, split = 0, room = 0;
+  int64_t maxs = 1, need = 0, split = 0, room = 0, least = 0;
   for (int l = 1; l <= h->tree.L; ++l) {
     int r1 = 1, c1 = 0;
     int64_t s1 = 1, nd = 0, sp = 0;
@@ -517,7 +517,8 @@ static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyIte
         s1 = std::max(s1, std::max(N.s1, N.s2));
       }
     }
-    room = std::max(room, std::max(nd + sp, gapply_scratch((int)(off[l + 1] - off[l]), r1, c1, s1)));
+    least = std::max(least, nd + sp);  // (for the products; the other items can do without)
+    room = std::max(room, gapply_scratch((int)(off[l + 1] - off[l]), r1, c1, s1));
     if (off[l] == a) {
       maxr = r1;
       maxcols = c1;
@@ -527,11 +528,12 @@ static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyIte
     }
   }
   int rc;
-  if ((rc = grow(h, &h->d_gz, room)) != KM_OK) return rc;
+  const bool spread = grow(h, &h->d_gz, std::max(room, least)) == KM_OK;
+  if (!spread && least > 0 && (rc = grow(h, &h->d_gz, least)) != KM_OK) return rc;
   int nk = 0;
   if (maxcols > 0) {
     KLV(h, KM_PROF_SWEEP, nk = launch_gapply(dl + a, (int)(b - a), h->d_gnodes, maxr, maxcols, maxs, mode, X, Xin, ldX,
-                                             kX, h->d_gz, st));
+                                             kX, spread ? h->d_gz : nullptr, st));
     h->stats.kernel_launches += nk - 1;
   }
   for (int64_t q = a; q < b && need > 0; ++q) {

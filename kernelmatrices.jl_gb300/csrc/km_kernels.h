@@ -282,7 +282,8 @@ int64_t dgemm_scratch(int transA, int64_t M, int64_t N, int64_t K);
 // entry; returns the number of kernels launched
 int launch_gnode(const GNodeDesc* nodes, int n, int maxr, int* info, cudaStream_t st);
 // Applies the factors of n items (nodes of rank at most maxr and at most maxs rows a side) to at
-// most maxcols columns each; scratch of gapply_scratch(...) doubles; returns the kernels launched.
+// most maxcols columns each; scratch of gapply_scratch(...) doubles, or null: one launch without the
+// split over the rows; returns the kernels launched.
 int launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int maxr, int maxcols, int64_t maxs, int mode,
                   double* X, const double* Xin, int64_t ldX, int kX, double* scratch, cudaStream_t st);
 int64_t gapply_scratch(int n, int maxr, int maxcols, int64_t maxs);

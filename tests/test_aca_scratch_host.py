@@ -26,3 +26,15 @@ def test_level_without_items_needs_none(lib, n, cols):
     """The root level has no panel to update; a level may also hold only items that go through the products
     over all SMs, which are not counted here (0 columns)."""
     assert gapply_scratch(lib, n, 1, cols, 1) == 0
+
+
+@pytest.mark.parametrize("n,r,cols,rows", [(1, 300, 1000, 131072), (1, 300, 1, 131072), (2, 300, 200, 65536), (1, 64, 4096, 1 << 20),
+                                           (16, 100, 8, 8192), (1, 24, 5, 700)])
+def test_scratch_does_not_grow_with_the_rows(lib, n, r, cols, rows):
+    """Two sides and the coefficients besides; the split stops at 6 CTAs an SM (152 SMs, 8 columns a CTA at most)
+    and at 64 chunks: 2 r values for each column of a chunk, of which there are fewer than 6 * 152 / 2 more than
+    CTAs of 8 columns, plus the coefficients' own 2 r values a column."""
+    ctas = n * -(-cols // 8)
+    most = 2 * r * 8 * (2 * ctas + 6 * 152 // 2)
+    got = gapply_scratch(lib, n, r, cols, rows)
+    assert 0 <= got <= min(most, 2 * r * 65 * 8 * ctas)

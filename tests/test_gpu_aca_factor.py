@@ -48,3 +48,49 @@ def test_unsorted_points_full_rank(lib):
     want = np.linalg.solve(A, b)
     assert np.linalg.norm(hk.ldiv(b) - want) < 1e-9 * np.linalg.norm(want)
     assert abs(hk.logdet() - np.linalg.slogdet(A)[1]) < 1e-8 * n
+
+
+def test_solve_at_the_memory_budget(lib):
+    """Where the scratch of the split does not fit, the node applications run without it: the same solution to
+    1e-12 (only the order of the sums over the rows differs; condition number below 1e2)."""
+    import ctypes as C
+    import torch
+    from kmhodlr import _lib as L, hodlr as KH
+    from kmhodlr.data import uniform_points
+    n, k = 4100, 512
+    pts, p = uniform_points(n, 3), np.array([1.0, 0.005, 1.0])
+    b = np.asfortranarray(np.random.default_rng(4).standard_normal((n, k)))
+
+    def solve(fraction):
+        h = C.c_void_p()
+        cfg = L.KmConfig(device=0, precision=L.KM_PREC_FP64, hbm_budget_fraction=fraction, refine_max_iter=0, refine_tol=0.0)
+        assert lib.km_create(C.byref(cfg), C.byref(h)) == L.KM_OK
+        assert lib.km_assemble(h, KH._dp(pts), n, L.KM_KERNEL_MATERN32, KH._dp(p), 3, L.KM_METHOD_ACA, 1e-13, 40,
+                               L.KM_LEVEL_FIXED, 2) == L.KM_OK, lib.km_last_error(h)
+        assert lib.km_factorize(h) == L.KM_OK, lib.km_last_error(h)
+        x, st = np.empty_like(b, order="F"), L.KmStats()
+        assert lib.km_solve(h, KH._dp(b), KH._dp(x), k) == L.KM_OK, lib.km_last_error(h)
+        assert lib.km_get_stats(h, C.byref(st)) == L.KM_OK
+        lib.km_destroy(h)
+        return x, st.device_bytes
+
+    want, used = solve(0.8)
+    got, less = solve((used - 4096) / torch.cuda.mem_get_info()[1])
+    assert less < used - 4096
+    assert np.linalg.norm(got - want) < 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n,lv,k", [(40000, 5, 17), (70000, 6, 300)])
+def test_tall_sides(lib, n, lv, k):
+    """Sides of 20000 and 35000 rows: row chunks above the 512 rows that a projection stages at a time."""
+    import kmhodlr as K
+    from kmhodlr.data import uniform_points
+    pts = uniform_points(n, 3)
+    hk = K.KernelHODLR(K.KernelMatrix(pts, pts, np.array([1.0, 0.003, 1.0]), K.Matern32()), 1e-13, 24, K.FixedLevel(lv))
+    x = np.random.default_rng(4).standard_normal((n, k))
+    y = hk @ x
+    K.symmetricfactorize(hk)
+    close = lambda a, b: np.linalg.norm(a - b) < 1e-10 * np.linalg.norm(b)  # noqa: E731
+    assert close(hk @ x, y)
+    assert close(hk.ldiv(y), x)
+    assert close(hk.W.ldiv(hk.W @ x), x)
