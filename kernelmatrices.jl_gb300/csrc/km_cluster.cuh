@@ -6,7 +6,10 @@
 
 namespace km {
 
-constexpr long long kWaitCycles = 1ll << 28;  // clock cycles before a barrier wait gives up (0.13 s)
+// Polls before a wait on a barrier or a shared-memory flag gives up: a few tens of cycles each, so well
+// above any legitimate wait inside one leaf or node, far below a watchdog.  (Not a time: the clock also
+// runs while the process has been switched off the GPU for another one.)
+constexpr int kWaitPolls = 1 << 22;
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -56,12 +59,12 @@ __device__ __forceinline__ bool bar_try(unsigned bar, int cs) {
   return ok != 0;
 }
 
-// Waits for phase 0 of the barrier; false if it gave up (after wait_limit tries, < 0: kWaitCycles)
+// Waits for phase 0 of the barrier; false if it gave up (after wait_limit polls, < 0: kWaitPolls)
 __device__ __forceinline__ bool bar_wait(unsigned bar, int wait_limit, int cs) {
-  const long long t0 = clock64();
+  const int lim = wait_limit < 0 ? kWaitPolls : wait_limit;
   int n = 0;
   while (wait_limit == 0 || !bar_try(bar, cs))
-    if (wait_limit >= 0 ? ++n > wait_limit : clock64() - t0 > kWaitCycles) return false;
+    if (++n > lim) return false;
   return true;
 }
 

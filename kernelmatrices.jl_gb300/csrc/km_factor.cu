@@ -160,11 +160,6 @@ __global__ void __launch_bounds__(NT) k_leaf_chol(const double* __restrict__ K, 
 // v = x/(alpha-beta); a zero column x gives tau = 0 (H = I).  One CTA per leaf; the panel is
 // copied to shared memory when it fits.
 // ---------------------------------------------------------------------------------------------
-// Iteration bound of a spin wait on a shared-memory flag (a few tens of cycles per iteration:
-// well above any legitimate wait inside one leaf or node, far below a watchdog).  The waiter of the
-// critical column does not sleep: it would wake too late for the column-to-column handoff.
-constexpr int kWaitLimit = 1 << 22;
-
 // Householder QR of the leaf panels (m x r, in place: R above, the scaled reflectors below), a CTA per
 // leaf, in dataflow order: of the NW warps warp w owns the columns w, w + NW, ...; reflector j + 1 is formed
 // by the warp that owns its column as soon as it has applied reflector j to it, before its other columns,
@@ -186,7 +181,7 @@ __global__ void __launch_bounds__(32 * leaf_qr_warps<T>()) k_leaf_qr(T* __restri
   T* sm = reinterpret_cast<T*>(smraw);
   __shared__ T red[32], sc[kMaxNysRank], ta[kMaxNysRank];
   __shared__ volatile int flag[kMaxNysRank];
-  const int lim = wait_limit < 0 ? kWaitLimit : wait_limit;
+  const int lim = wait_limit < 0 ? kWaitPolls : wait_limit;
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   T* G = Pan + d_leaf_start(t, leaf) * r;
@@ -497,7 +492,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_node_factor(T* __restrict__ R,
   constexpr int ld = kNodeLd;
   // polls of a flag before a wait gives up; wait_limit 0: every wait gives up at its first poll,
   // as if its flag were never set (the test of the timeout path)
-  const int lim = wait_limit < 0 ? kWaitLimit : wait_limit;
+  const int lim = wait_limit < 0 ? kWaitPolls : wait_limit;
   T* X0 = sm;
   T* X1 = X0 + r * ld;
   T* X2 = X1 + r * ld;

@@ -41,7 +41,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kSpin = 1 << 22;     // polls of a shared-memory flag before a wait gives up
 
 // v into the same location of every CTA (local store if the cluster is one CTA)
 __device__ __forceinline__ void put_all(double* p, double v, int cs) {
@@ -119,7 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_node_factor_f64(double* __restr
   const double* R2 = R + (cbase + 2 * k + 1) * (int64_t)r * r;
   const int nch = (r + 31) >> 5, gw = rank * kWarps + w, ngw = cs * kWarps;
   // a wait_limit of 0 makes every wait give up at its first poll, as if its flag were never set
-  const int lim = wait_limit < 0 ? kSpin : wait_limit;
+  const int lim = wait_limit < 0 ? kWaitPolls : wait_limit;
   for (int c = w; c < r; c += kWarps)
     for (int i = lane; i < r; i += 32) {
       const int e = i + c * r;

@@ -34,3 +34,9 @@ def test_cluster_permission_is_set_per_device():
     assert users == {"km_probe.cu"}
     body = (CSRC / "km_probe.cu").read_text().split("int cluster_limit(", 1)[1]
     assert "known[{func, dev}]" in body
+
+
+def test_waits_count_polls():
+    """A bounded wait counts polls, as km_set_wait_limit documents: the clock also runs while another process has
+    the GPU."""
+    assert [f.name for f in CSRC.glob("*.cu*") if re.search(r"\bclock(64)?\(|globaltimer", f.read_text())] == []
