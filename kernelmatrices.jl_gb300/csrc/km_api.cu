@@ -1894,8 +1894,14 @@ int km_factorize(km_handle* h) {
   h->stats.factorize_ms = timer_stop(h);
   if ((rc = sync(h, "factorize")) != KM_OK) return rc;
   rc = check_info_words(h, h->h_info, t.nleaf, "leaf");
+  const int* info = h->h_info + t.nleaf;
+  if (rc == KM_ERR_TIMEOUT) {
+    // (the node kernels ran all the same: the message says whether they gave up too)
+    if (std::any_of(info, info + t.nnode, [](int v) { return v < 0; }))
+      h->err += "; a bounded wait inside the node factorisation ran out";
+    return rc;
+  }
   if (rc == KM_OK) {
-    const int* info = h->h_info + t.nleaf;
     for (int64_t i = 0; i < t.nnode && rc == KM_OK; ++i) {
       if (info[i] < 0) return fail(h, KM_ERR_TIMEOUT, "a bounded wait inside the node factorisation ran out");
       if (info[i]) rc = fail(h, KM_ERR_NOT_SPD, "PosDefException: a low-rank capacitance block is not positive definite");
