@@ -1319,7 +1319,7 @@ static int aca_assemble(km_handle* h, const double* pts, bool dev, const Tree& t
   h->lvoff[t.L + 1] = (int64_t)h->blk.size();
   const int nb = (int)h->blk.size();
   // panel capacity: the largest column count (256 .. kAcaMaxCap, powers of two) whose panels
-  // fit in 40% of the budget; the ACA kernel keeps two capacity-long vectors in shared memory
+  // fit in 40% of the budget; the ACA kernel keeps three capacity-long vectors in shared memory
   int capmax = 256;
   for (int c = kAcaMaxCap; c > 256; c >>= 1) {
     int64_t tot = 0;

@@ -94,3 +94,21 @@ def test_tall_sides(lib, n, lv, k):
     assert close(hk @ x, y)
     assert close(hk.ldiv(y), x)
     assert close(hk.W.ldiv(hk.W @ x), x)
+
+
+@pytest.mark.parametrize("n,lv", [(24575, 4), (24576, 4), (24577, 4), (24578, 4)])
+def test_panels_at_the_cluster_limit(lib, n, lv):
+    """Top panels of 12287 to 12289 rows: 12288 is what 16 CTAs hold, one more goes to the kernels of all SMs, and
+    at 24577 points the two panels of one level go different ways."""
+    import kmhodlr as K
+    from kmhodlr.data import uniform_points
+    pts = uniform_points(n, 3)
+    hk = K.KernelHODLR(K.KernelMatrix(pts, pts, np.array([1.0, 0.005, 1.0]), K.Matern32()), 1e-13, 33, K.FixedLevel(lv))
+    x = np.random.default_rng(4).standard_normal((n, 2))
+    y = hk @ x
+    K.symmetricfactorize(hk)
+    close = lambda a, b: np.linalg.norm(a - b) < 1e-10 * np.linalg.norm(b)  # noqa: E731
+    assert close(hk @ x, y)
+    assert close(hk.ldiv(y), x)
+    assert close(hk.W.ldiv(hk.W @ x), x)
+    assert close(hk.W.T.ldiv(hk.W.T @ x), x)
