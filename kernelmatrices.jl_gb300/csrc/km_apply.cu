@@ -387,6 +387,16 @@ __global__ void __launch_bounds__(512) k_leaf_nys_apply(const double* __restrict
     if (i < m && nc == 1) {  // one column: two independent chains, no idle column slots
       double a1 = 0.0;
       int l = l0;
+      for (; l + 7 < l1; l += 8) {  // eight entries loaded ahead of their multiply-adds
+        double kv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) kv[u] = K[i + (int64_t)(l + u) * m];
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          acc[0] += kv[u] * xs[l + u];
+          a1 += kv[u + 1] * xs[l + u + 1];
+        }
+      }
       for (; l + 1 < l1; l += 2) {
         acc[0] += K[i + (int64_t)l * m] * xs[l];
         a1 += K[i + (int64_t)(l + 1) * m] * xs[l + 1];
