@@ -67,41 +67,17 @@ __device__ void leaf_tri_body(const T* __restrict__ L, int m, int op, const T* B
       // update of the remaining rows with the solved block: items of (row, 4 columns), so that
       // each loaded L entry feeds 4 multiply-adds and all threads stay busy as the remaining
       // rows shrink
-      if (op == 1) {
-        // rows i < i0 take L[i0 + l, i]: along l in memory, so 32 x 32 tiles go through shared
-        // memory (over D, which this block has finished with); items of (row, 2 columns)
-        for (int r0 = 0; r0 < i0; r0 += 32) {
-          for (int e = tid; e < 32 * 32; e += blockDim.x) {
-            const int l = e & 31, i = e >> 5;
-            if (l < ib) D[l * 33 + i] = L[(int64_t)(r0 + i) * m + i0 + l];
-          }
-          __syncthreads();
-          for (int e = tid; e < 32 * ((nc + 1) >> 1); e += blockDim.x) {
-            const int i = e & 31, cb = 2 * (e >> 5);
-            const T* xc = xs + cb * m + i0;
-            acc_t<T> acc[2] = {};
-            const int c2 = cb + 1 < nc ? m : 0;
-#pragma unroll 4
-            for (int l = 0; l < ib; ++l) {
-              const T a = D[l * 33 + i];
-              acc[0] += a * xc[l];
-              acc[1] += a * xc[c2 + l];
-            }
-            xs[cb * m + r0 + i] -= accv(acc[0]);
-            if (c2) xs[cb * m + m + r0 + i] -= accv(acc[1]);
-          }
-          __syncthreads();
-        }
-        continue;
-      }
-      const int R = m - (i0 + ib);
-      const int r0 = i0 + ib;
+      const int R = (op == 0) ? m - (i0 + ib) : i0;
+      const int r0 = (op == 0) ? i0 + ib : 0;
       const int ng = (nc + 3) >> 2;
       for (int e = tid; e < R * ng; e += blockDim.x) {
         const int g = e / R, i = r0 + (e - g * R), cb = 4 * g;
         const T* xc = xs + cb * m + i0;
         acc_t<T> acc[4] = {};
-        auto ld = [&](int l) { return L[(int64_t)(i0 + l) * m + i]; };  // L[i, i0 + l]
+        auto ld = [&](int l) {
+          return (op == 0) ? L[(int64_t)(i0 + l) * m + i]   // L[i, i0 + l]
+                           : L[(int64_t)i * m + i0 + l];    // L[i0 + l, i]
+        };
         int l = 0;
         for (; l + 3 < ib; l += 4) {  // four entries loaded ahead of their multiply-adds
           const T a0 = ld(l), a1 = ld(l + 1), a2 = ld(l + 2), a3 = ld(l + 3);
