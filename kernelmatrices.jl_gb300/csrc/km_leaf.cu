@@ -338,15 +338,29 @@ __global__ void __launch_bounds__(128) k_leaf_diaginv(double* __restrict__ Lf, D
     if (lane < i) L[(int64_t)i * m + lane] = X[i * 33 + lane];
 }
 
-template <int NC>
-__global__ void __launch_bounds__(256) k_leaf_solve(const double* __restrict__ Lf, DTree t, int op,
+// The row updates of the backward solve read L along its columns, a row a lane.  With large leaves and several
+// CTAs an SM these loads of 32 lines each bound it (128 leaves of 1025, 16 columns: 7.1 ms, the
+// substitution 3.6), so that there a warp turns its entries round in shared memory (2.9 ms).  Up to 768 points
+// or with a CTA an SM the direct loads are as fast or faster (128 of 700, 13 columns: 1.33 against 1.57 ms).
+enum { kForward = 0, kDirect = 1, kTurned = 2 };
+// CTAs an SM holds by their registers: 32 a thread with one or two columns, 48 with more; turned 48 and 64
+__host__ __device__ constexpr int solve_ctas(int nc, int form) {
+  return nc <= 2 ? (form == kTurned ? 5 : 8) : form == kTurned ? 4 : 5;
+}
+__host__ __device__ constexpr int solve_bound(int nc, int form) {  // (the compiler takes 32 by itself)
+  return nc <= 2 && form != kTurned ? 0 : solve_ctas(nc, form);
+}
+
+template <int NC, int FORM>
+__global__ void __launch_bounds__(256, solve_bound(NC, FORM)) k_leaf_solve(const double* __restrict__ Lf, DTree t,
                                                     double* __restrict__ Xg, int64_t ldx, int k) {
+  constexpr int OP = FORM == kForward ? 0 : 1;
   extern __shared__ __align__(16) unsigned char smraw[];
   double* xs = reinterpret_cast<double*>(smraw);  // NC x m
   const int64_t leaf = blockIdx.x;
   const int m = d_leaf_size(t, leaf);
   const double* L = Lf + d_leaf_koff(t, leaf);
-  double* D = xs + NC * m;                        // 32 x 33
+  double* D = xs + NC * m;                        // 32 x 33 (turned: 8 x 32 x 9 while rows are updated)
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int c0 = blockIdx.y * NC, nc = min(NC, k - c0);
   double* X = Xg + d_leaf_start(t, leaf) + (int64_t)c0 * ldx;
@@ -354,7 +368,7 @@ __global__ void __launch_bounds__(256) k_leaf_solve(const double* __restrict__ L
     for (int i = tid; i < m; i += 256) xs[c * m + i] = X[(int64_t)c * ldx + i];
   const int nblk = (m + 31) / 32;
   for (int q = 0; q < nblk; ++q) {
-    const int i0 = 32 * (op == 0 ? q : nblk - 1 - q), ib = min(32, m - i0);
+    const int i0 = 32 * (OP == 0 ? q : nblk - 1 - q), ib = min(32, m - i0);
     __syncthreads();
     // op 0: D[a][l] = X_q[a][l], l <= a; op 1: D[a][l] = X_q[31 - l][31 - a], the transpose with rows
     // and columns reversed, again lower triangular (rows beyond the block are zero)
@@ -364,7 +378,7 @@ __global__ void __launch_bounds__(256) k_leaf_solve(const double* __restrict__ L
         const double e = L[(int64_t)(i0 + i) * m + i0 + lane];
         v = lane == i ? 1.0 / e : e;
       }
-      if (lane <= i) D[op == 0 ? i * 33 + lane : (31 - lane) * 33 + 31 - i] = v;
+      if (lane <= i) D[OP == 0 ? i * 33 + lane : (31 - lane) * 33 + 31 - i] = v;
     }
     __syncthreads();
     for (int c = 2 * w; c < nc; c += 16) {
@@ -378,26 +392,63 @@ __global__ void __launch_bounds__(256) k_leaf_solve(const double* __restrict__ L
           acc = 0.0;
         }
         const int row = one ? lane : 31 - lane, l = one ? u : u - lane - 1;
-        const int i = op == 0 ? l : 31 - l;
+        const int i = OP == 0 ? l : 31 - l;
         const double b = i < ib ? (one ? b0 : b1)[i] : 0.0;
         acc += D[row * 33 + l] * b;
       }
       const double second = acc;
       __syncwarp();
-      const int ra = op == 0 ? lane : 31 - lane, rb = 31 - ra;
+      const int ra = OP == 0 ? lane : 31 - lane, rb = 31 - ra;
       if (ra < ib) b0[ra] = first;
       __syncwarp();
       if (c + 1 < nc && rb < ib) b1[rb] = second;
     }
     __syncthreads();
-    const int R = op == 0 ? m - (i0 + ib) : i0, r0 = op == 0 ? i0 + ib : 0;
+    const int R = OP == 0 ? m - (i0 + ib) : i0, r0 = OP == 0 ? i0 + ib : 0;
     constexpr int CG = NC < 4 ? NC : 4;
     const int ng = (nc + CG - 1) / CG;
+    if constexpr (FORM == kTurned) {
+      // row i takes L[i0 + l, i], which runs along l in memory: a warp reads 8 entries of each of its 32 rows
+      // (R is a multiple of 32), 4 rows a load, and turns them round in its part of shared memory
+      double* ts = D + w * 32 * 9;
+      const int nr = R / 32, lq = lane & 7;
+      for (int e = w; e < nr * ng; e += 8) {
+        const int g = e / nr, ib0 = 32 * (e - g * nr), cb = CG * g;
+        const double* xc = xs + cb * m + i0;
+        const double* a = L + (int64_t)(ib0 + (lane >> 3)) * m + i0 + lq;
+        double acc[CG] = {}, pre[8];
+        auto fetch = [&](int l) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) pre[u] = l + lq < ib ? a[(int64_t)4 * u * m + l] : 0.0;
+        };
+        fetch(0);
+        for (int l = 0; l < ib; l += 8) {
+          __syncwarp();
+#pragma unroll
+          for (int u = 0; u < 8; ++u) ts[(4 * u + (lane >> 3)) * 9 + lq] = pre[u];
+          __syncwarp();
+          if (l + 8 < ib) fetch(l + 8);
+          const int n = min(8, ib - l);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (u < n) {
+              const double v = ts[lane * 9 + u];
+#pragma unroll
+              for (int j = 0; j < CG; ++j)
+                if (cb + j < nc) acc[j] += v * xc[j * m + l + u];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < CG; ++j)
+          if (cb + j < nc) xs[(cb + j) * m + ib0 + lane] -= acc[j];
+      }
+      continue;
+    }
     for (int e = tid; e < R * ng; e += 256) {
       const int g = e / R, i = r0 + (e - g * R), cb = CG * g;
       const double* xc = xs + cb * m + i0;
-      const double* a = op == 0 ? L + (int64_t)i0 * m + i : L + (int64_t)i * m + i0;
-      const int64_t sa = op == 0 ? m : 1;
+      const double* a = OP == 0 ? L + (int64_t)i0 * m + i : L + (int64_t)i * m + i0;
+      const int64_t sa = OP == 0 ? m : 1;
       double acc[CG] = {};
       int l = 0;
       for (; l + 7 < ib; l += 8) {  // eight entries loaded ahead of their multiply-adds
@@ -510,13 +561,28 @@ void launch_leaf_diaginv(double* Lf, const Tree& t, cudaStream_t st) {
   k_leaf_diaginv<<<dim3((unsigned)t.nleaf, (unsigned)((t.max_leaf + 31) / 32)), 128, 0, st>>>(Lf, dtree(t));
 }
 
+template <int NC, int FORM>
+static bool solve_form(const double* Lf, const Tree& t, double* X, int64_t ldx, int k, size_t sm, cudaStream_t st) {
+  smem_limit((const void*)k_leaf_solve<NC, FORM>, sm);
+  k_leaf_solve<NC, FORM><<<dim3((unsigned)t.nleaf, (unsigned)((k + NC - 1) / NC)), 256, sm, st>>>(Lf, dtree(t), X, ldx, k);
+  return true;
+}
+
+static int solve_form_of(const Tree& t, int op, int nc, int k) {
+  return op == 0 ? kForward : t.max_leaf > 768 && t.nleaf * (int64_t)((k + nc - 1) / nc) > 152 ? kTurned : kDirect;
+}
+static size_t solve_smem(const Tree& t, int nc, int form) {
+  return ((size_t)nc * t.max_leaf + (form == kTurned ? 8 * 32 * 9 : 32 * 33)) * sizeof(double);
+}
+
 template <int NC>
 static bool solve_launch(const double* Lf, const Tree& t, int op, double* X, int64_t ldx, int k, cudaStream_t st) {
-  const size_t sm = ((size_t)NC * t.max_leaf + 32 * 33) * sizeof(double);
+  const int form = solve_form_of(t, op, NC, k);
+  const size_t sm = solve_smem(t, NC, form);
   if (sm > 200 * 1024) return false;
-  smem_limit((const void*)k_leaf_solve<NC>, sm);
-  k_leaf_solve<NC><<<dim3((unsigned)t.nleaf, (unsigned)((k + NC - 1) / NC)), 256, sm, st>>>(Lf, dtree(t), op, X, ldx, k);
-  return true;
+  return form == kForward  ? solve_form<NC, kForward>(Lf, t, X, ldx, k, sm, st)
+         : form == kDirect ? solve_form<NC, kDirect>(Lf, t, X, ldx, k, sm, st)
+                           : solve_form<NC, kTurned>(Lf, t, X, ldx, k, sm, st);
 }
 
 bool launch_leaf_solve_f64(const double* Lf, const Tree& t, int op, double* X, int64_t ldx, int k, cudaStream_t st) {
@@ -525,7 +591,13 @@ bool launch_leaf_solve_f64(const double* Lf, const Tree& t, int op, double* X, i
   const int64_t want = 4 * 152;
   if (k > 8 && ctas(16) >= want && solve_launch<16>(Lf, t, op, X, ldx, k, st)) return true;
   if (k > 4 && ctas(8) >= want && solve_launch<8>(Lf, t, op, X, ldx, k, st)) return true;
-  if (k > 2 && ctas(4) >= want && solve_launch<4>(Lf, t, op, X, ldx, k, st)) return true;
+  // few CTAs: two columns each, or four where only those run all at once, by registers and shared memory
+  // (32 leaves of 2800, 33 columns, backward: 12.0 ms in two waves, 10.0 in one)
+  auto at_once = [&](int nc) {
+    const int form = solve_form_of(t, op, nc, k);
+    return ctas(nc) <= 152 * std::min<int64_t>(solve_ctas(nc, form), 227 * 1024 / (solve_smem(t, nc, form) + 1024));
+  };
+  if (k > 2 && (ctas(4) >= want || (!at_once(2) && at_once(4))) && solve_launch<4>(Lf, t, op, X, ldx, k, st)) return true;
   if (k > 1 && solve_launch<2>(Lf, t, op, X, ldx, k, st)) return true;
   return solve_launch<1>(Lf, t, op, X, ldx, k, st);
 }

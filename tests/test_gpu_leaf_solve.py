@@ -35,3 +35,23 @@ def test_solves_and_projections(lib, precision, tol, n, lv, r, k):
     # the estimator depends on the factor's basis in the null directions of the leaf panels
     want = O.stoch_gradient(O.KernelMatrix(pts, pts, p, O.KERNEL_MATERN32), ok, b[:, 0], 3, [z[:, j] for j in range(k)])
     assert np.linalg.norm(g - want) < 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n,lv,k", [(16 * 768 + 15, 4, 20), (16 * 769, 4, 19), (16 * 800 + 3, 4, 40), (16 * 1057, 4, 33),
+                                    (32 * 900 + 1, 5, 9), (8 * 1120, 3, 80)])
+def test_backward_solves_of_large_leaves(lib, n, lv, k):
+    """Leaves above 768 points with more CTAs than SMs turn the factor's entries round in shared memory: last blocks
+    of 1 to 32 rows, chunks of 2 and 4 columns, ragged ones too.  A column alone takes the direct form; both
+    against W' to 1e-12 (unit diagonal plus a nugget of 1, condition number below 1e3)."""
+    import kmhodlr as K
+    from kmhodlr.data import uniform_points
+    pts = uniform_points(n, 41)
+    b = np.random.default_rng(42).standard_normal((n, k))
+    hk = K.KernelHODLR(K.KernelMatrix(pts, pts, np.array([1.0, 0.02, 1.0]), K.Matern32()), 0.0, 16, K.FixedLevel(lv),
+                       nystrom=True)
+    K.symmetricfactorize(hk)
+    x = hk.W.T.ldiv(b)
+    assert np.linalg.norm(hk.W.T @ x - b) < 1e-12 * np.linalg.norm(b)
+    for c in (0, k // 2, k - 1):
+        one = hk.W.T.ldiv(b[:, c])
+        assert np.linalg.norm(one - x[:, c]) < 1e-12 * np.linalg.norm(one)
