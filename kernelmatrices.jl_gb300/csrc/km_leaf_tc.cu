@@ -838,7 +838,10 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
       else if (left > 1) fetch(op == 0 ? q + 1 : q - 1, op == 0 ? q + 1 : q - 1);
       acc_t<ff> a[3] = {};
       // the inverse is a triangle: 32 of its rows need half of the tile
-      const int l0 = v == 0 && op == 1 ? 32 * (w & 1) : 0, l1 = v == 0 && op == 0 ? 32 * (w & 1) + 32 : kLcNB;
+      const int l0 = v == 0 && op == 1 ? 32 * (w & 1) : 0;
+      // (nothing beyond the leaf: columns in pairs, rows by warps)
+      const bool live = kLcNB * b + 32 * (w & 1) < m;
+      const int l1 = live ? min(v == 0 && op == 0 ? 32 * (w & 1) + 32 : kLcNB, (m - kLcNB * q + 1) & ~1) : 0;
       const ff* x = xc + kLcNB * q;
 #pragma unroll 4
       for (int l = l0; l < l1; l += 2) {
@@ -852,8 +855,9 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
       }
       if (v == 0) __syncthreads();
       ff* out = xc + kLcNB * b + i;
+      if (live)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) out[c * mp] = v == 0 ? accv(a[c]) : out[c * mp] - accv(a[c]);
+        for (int c = 0; c < 3; ++c) out[c * mp] = v == 0 ? accv(a[c]) : out[c * mp] - accv(a[c]);
     }
   }
   __syncthreads();
@@ -864,10 +868,16 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
 bool launch_leaf_tri_blk(const ff* Lf, const Tree& t, int op, ff* X, int64_t ldx, int k, cudaStream_t st) {
   if (k <= 0) return true;
   if (t.max_leaf > kLcMaxLeaf || (op != 0 && op != 1)) return false;
-  const int64_t mp = (t.max_leaf + kLcNB - 1) / kLcNB * kLcNB;
+  const int64_t nb = (t.max_leaf + kLcNB - 1) / kLcNB, mp = nb * kLcNB, few = (k + kTfCols - 1) / kTfCols;
+  // Many leaves whose triangle fills little of its tiles, up to 37 points and 65 and 66: the substitution (16
+  // columns, a backward call: 4096 leaves of 16 0.44 ms, by tiles 0.63; 2048 of 65 0.75 against 0.93).  With few
+  // CTAs the tiles are faster (32 of 65, 100 columns: 0.15 against 0.17 ms).
+  if (t.max_leaf * (t.max_leaf + 1) * 100 < 18 * kLcNB * kLcNB * nb * (nb + 1) && t.nleaf * few > 8 * 152)
+    return launch_leaf_tri<ff>(Lf, t, op, X, 1, t.n, 0, X, 1, t.n, 0, k, st);
   // 12 columns a CTA take as long as 2.1 chunks of 4 columns (256 leaves of 256: 81 us against 31, 50, 90,
-  // 124 us for 1, 4, 8, 12 columns; 16 columns 155 against 146, 24 columns 156 against 220)
-  if (2 * ((k + kTwCols - 1) / kTwCols) >= (k + kTfCols - 1) / kTfCols) {
+  // 124 us for 1, 4, 8, 12 columns; 16 columns 155 against 146, 24 columns 156 against 220), unless the SMs
+  // hold all chunks of 4 at once (one leaf of 1024, 33 columns: the call 634 us against 424)
+  if (2 * ((k + kTwCols - 1) / kTwCols) >= few || t.nleaf * few <= 152) {
     const size_t sm = ((size_t)kTfCols * mp + (size_t)4 * kTfCols * kLcNB + (size_t)kLcNB * kTwLd) * sizeof(ff);
     smem_limit((const void*)k_leaf_tri_few, sm);
     k_leaf_tri_few<<<dim3((unsigned)t.nleaf, (unsigned)((k + kTfCols - 1) / kTfCols)), 256, sm, st>>>(Lf, dtree(t), op, X,

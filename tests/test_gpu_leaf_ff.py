@@ -28,3 +28,22 @@ def test_solve(lib, n, lv, r, k):
     assert abs(h[1].logdet() - h[0].logdet()) < 1e-6
     z = h[1].W @ h[1].W.ldiv(b)
     assert np.linalg.norm(z - b) < 1e-9 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n,lv,r,k", [(16 * 512, 9, 8, 20), (37 * 512, 9, 16, 16), (38 * 512, 9, 16, 20), (65 * 256, 8, 24, 33),
+                                      (66 * 256 + 7, 8, 24, 48), (67 * 128, 7, 24, 100), (1024, 0, 2, 33), (1000, 0, 2, 9)])
+def test_small_leaves_and_few_ctas(lib, n, lv, r, k):
+    """Both sides of the rules that send many leaves with ill-filled tiles to the substitution and the chunks of few
+    leaves to the kernel of 4 columns.  Tolerances as above."""
+    import kmhodlr as K
+    from kmhodlr.data import uniform_points
+    pts = uniform_points(n, 41)
+    km = K.KernelMatrix(pts, pts, np.array([1.0, 0.1, 1e-1]), K.Matern32())
+    b = np.random.default_rng(42).standard_normal((n, k))
+    h = [K.KernelHODLR(km, 0.0, r, K.FixedLevel(lv), nystrom=True, precision=p) for p in (K.KM_PREC_FP64, K.KM_PREC_MIXED)]
+    for x in h:
+        K.symmetricfactorize(x)
+    want, got = (x.ldiv(b) for x in h)
+    assert np.linalg.norm(got - want) < 1e-8 * np.linalg.norm(want)
+    z = h[1].W.T @ h[1].W.T.ldiv(b)
+    assert np.linalg.norm(z - b) < 1e-9 * np.linalg.norm(b)
