@@ -19,6 +19,10 @@ void smem_limit(const void* func, size_t bytes);
 // error (setting a kernel attribute does), so callers check theirs before it.
 int cluster_limit(const void* func, int threads, size_t smem);
 
+// Leaf solves by inverses of diagonal blocks: a block whose inverse has an entry above kIllBlock / L[0][0] (the
+// diagonal of K is constant and L[0][0] its square root) is solved by substitution instead.
+constexpr float kIllBlock = 48.f;
+
 // Operand of the leaf triangular kernels: leaf j's block starts at ptr + start(j) * bmul with
 // leading dimension m_j (ld_is_m) or ld.
 struct LeafOperand {

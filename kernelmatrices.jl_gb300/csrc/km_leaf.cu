@@ -311,6 +311,13 @@ __global__ void __launch_bounds__(kExpRows) k_leaf_qexpand(const T* __restrict__
 // lives in the block's upper triangle of Lf, which nothing else uses.
 // Measured: 128 leaves of 312 points, 32 right-hand sides 0.67 -> 0.54 ms; 2 leaves of 500, one right-hand
 // side 270 -> 205 us.
+//
+// A product with X_q loses up to the block's condition number against the substitution (points closer to
+// each other than the nugget hides, next to each other in a leaf), so a block whose X_q has an entry above
+// kIllBlock times 1 / L[0][0] is solved by substitution.
+// Blocks of a nugget of 1e-3 and more stay below 32.  Right-hand sides K x of a smooth x, 160 points with
+// neighbours 1e-3 apart, error of x: nugget 1e-3 (entries to 25) 1.0e-12 both ways; 1e-5 (229) 8e-10 by products,
+// 7e-11 by substitution.
 // ---------------------------------------------------------------------------------------------
 
 // X_q of every diagonal block: grid (nleaf, blocks), 4 warps, lane = column of X; warp i mod 4 keeps
@@ -343,16 +350,30 @@ __global__ void __launch_bounds__(128) k_leaf_diaginv(double* __restrict__ Lf, D
 // substitution 3.6), so that there a warp turns its entries round in shared memory (2.9 ms).  Up to 768 points
 // or with a CTA an SM the direct loads are as fast or faster (128 of 700, 13 columns: 1.33 against 1.57 ms).
 enum { kForward = 0, kDirect = 1, kTurned = 2 };
-// CTAs an SM holds by their registers: 32 a thread with one or two columns, 48 with more; turned 48 and 64
+// CTAs an SM holds by their registers: 40 a thread forward with one or two columns, else 48; turned with more 64
 __host__ __device__ constexpr int solve_ctas(int nc, int form) {
-  return nc <= 2 ? (form == kTurned ? 5 : 8) : form == kTurned ? 4 : 5;
+  return nc <= 2 ? (form == kForward ? 6 : 5) : form == kTurned ? 4 : 5;
 }
-__host__ __device__ constexpr int solve_bound(int nc, int form) {  // (the compiler takes 32 by itself)
-  return nc <= 2 && form != kTurned ? 0 : solve_ctas(nc, form);
+
+// x of the 32-row block at row i0 of nc columns (column c at xs[c m]) by substitution: a warp per column, lane =
+// row; D holds the block of L (row-major, leading dimension 33), the diagonal as reciprocals
+template <int OP>
+__device__ __noinline__ void block_subst(const double* D, double* xs, int m, int i0, int ib, int nc) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int c = w; c < nc; c += 8) {
+    double v = lane < ib ? xs[c * m + i0 + lane] : 0.0;
+    for (int u = 0; u < ib; ++u) {
+      const int l = OP == 0 ? u : ib - 1 - u;
+      if (lane == l) v *= D[l * 33 + l];
+      const double x = __shfl_sync(0xffffffffu, v, l);
+      if (OP == 0 ? (lane > l && lane < ib) : lane < l) v -= (OP == 0 ? D[lane * 33 + l] : D[l * 33 + lane]) * x;
+    }
+    if (lane < ib) xs[c * m + i0 + lane] = v;
+  }
 }
 
 template <int NC, int FORM>
-__global__ void __launch_bounds__(256, solve_bound(NC, FORM)) k_leaf_solve(const double* __restrict__ Lf, DTree t,
+__global__ void __launch_bounds__(256, solve_ctas(NC, FORM)) k_leaf_solve(const double* __restrict__ Lf, DTree t,
                                                     double* __restrict__ Xg, int64_t ldx, int k) {
   constexpr int OP = FORM == kForward ? 0 : 1;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -367,8 +388,10 @@ __global__ void __launch_bounds__(256, solve_bound(NC, FORM)) k_leaf_solve(const
   for (int c = 0; c < nc; ++c)
     for (int i = tid; i < m; i += 256) xs[c * m + i] = X[(int64_t)c * ldx + i];
   const int nblk = (m + 31) / 32;
+  const int ill = __double2hiint((double)(kIllBlock / (float)L[0]));
   for (int q = 0; q < nblk; ++q) {
     const int i0 = 32 * (OP == 0 ? q : nblk - 1 - q), ib = min(32, m - i0);
+    bool above = false;
     __syncthreads();
     // op 0: D[a][l] = X_q[a][l], l <= a; op 1: D[a][l] = X_q[31 - l][31 - a], the transpose with rows
     // and columns reversed, again lower triangular (rows beyond the block are zero)
@@ -377,31 +400,41 @@ __global__ void __launch_bounds__(256, solve_bound(NC, FORM)) k_leaf_solve(const
       if (i < ib && lane <= i) {
         const double e = L[(int64_t)(i0 + i) * m + i0 + lane];
         v = lane == i ? 1.0 / e : e;
+        above |= (__double2hiint(v) & 0x7fffffff) > ill;
       }
       if (lane <= i) D[OP == 0 ? i * 33 + lane : (31 - lane) * 33 + 31 - i] = v;
     }
-    __syncthreads();
-    for (int c = 2 * w; c < nc; c += 16) {
-      double* b0 = xs + c * m + i0;
-      double* b1 = c + 1 < nc ? b0 + m : b0;
-      double first = 0.0, acc = 0.0;
-      for (int u = 0; u <= 32; ++u) {
-        const bool one = u <= lane;
-        if (u == lane + 1) {
-          first = acc;
-          acc = 0.0;
+    if (__syncthreads_or(above)) {
+      for (int l = w; l < ib; l += 8)
+        if (lane >= l && lane < ib) {
+          const double e = L[(int64_t)(i0 + l) * m + i0 + lane];
+          D[lane * 33 + l] = lane == l ? 1.0 / e : e;
         }
-        const int row = one ? lane : 31 - lane, l = one ? u : u - lane - 1;
-        const int i = OP == 0 ? l : 31 - l;
-        const double b = i < ib ? (one ? b0 : b1)[i] : 0.0;
-        acc += D[row * 33 + l] * b;
+      __syncthreads();
+      block_subst<OP>(D, xs, m, i0, ib, nc);
+    } else {
+      for (int c = 2 * w; c < nc; c += 16) {
+        double* b0 = xs + c * m + i0;
+        double* b1 = c + 1 < nc ? b0 + m : b0;
+        double first = 0.0, acc = 0.0;
+        for (int u = 0; u <= 32; ++u) {
+          const bool one = u <= lane;
+          if (u == lane + 1) {
+            first = acc;
+            acc = 0.0;
+          }
+          const int row = one ? lane : 31 - lane, l = one ? u : u - lane - 1;
+          const int i = OP == 0 ? l : 31 - l;
+          const double b = i < ib ? (one ? b0 : b1)[i] : 0.0;
+          acc += D[row * 33 + l] * b;
+        }
+        const double second = acc;
+        __syncwarp();
+        const int ra = OP == 0 ? lane : 31 - lane, rb = 31 - ra;
+        if (ra < ib) b0[ra] = first;
+        __syncwarp();
+        if (c + 1 < nc && rb < ib) b1[rb] = second;
       }
-      const double second = acc;
-      __syncwarp();
-      const int ra = OP == 0 ? lane : 31 - lane, rb = 31 - ra;
-      if (ra < ib) b0[ra] = first;
-      __syncwarp();
-      if (c + 1 < nc && rb < ib) b1[rb] = second;
     }
     __syncthreads();
     const int R = OP == 0 ? m - (i0 + ib) : i0, r0 = OP == 0 ? i0 + ib : 0;

@@ -691,6 +691,60 @@ static int64_t lc_rp_max(const Tree& t, int r) { return lc_rows_padded(t.max_lea
 // ---------------------------------------------------------------------------------------------
 constexpr int kTfCols = 4, kTwLd = kLcNB + 1;
 
+// x of 64-row block q by substitution in place of the product with its inverse (kIllBlock, km_kernels.h): a warp per
+// column (column c at xs[c mp]), rows lane and lane + 32, L's block through T (64 x 65), the diagonal as
+// reciprocals.  Called by all 256 threads; begins and ends with a barrier.
+__device__ __noinline__ void block_subst_ff(const ff* L, ff* T, ff* xs, int m, int mp, int q, int nc, int op) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, fast = tid & 63;
+  const int i0 = kLcNB * q, nb = min(kLcNB, m - i0);
+  __syncthreads();
+  for (int sl = tid >> 6; sl < kLcNB; sl += 4)
+    if (sl <= fast && fast < nb) {
+      const ff v = L[(int64_t)(i0 + sl) * m + i0 + fast];
+      T[sl * kTwLd + fast] = sl == fast ? ff(1.0) / v : v;
+    }
+  __syncthreads();
+  // columns w and w + 8 together: two independent chains (at most 16 columns)
+  if (w < nc) {
+    const bool two = w + 8 < nc;
+    ff* x[2] = {xs + w * mp + i0, xs + (two ? w + 8 : w) * mp + i0};
+    acc_t<ff> v[2][2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) v[c][s] = x[c][lane + 32 * s];
+    for (int u = 0; u < nb; ++u) {
+      const int l = op == 0 ? u : nb - 1 - u;
+      const ff inv = T[l * kTwLd + l];
+      ff xl[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (c == 0 || two) xl[c] = shfl_idx(accv(l < 32 ? v[c][0] : v[c][1]) * inv, l & 31);
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int i = lane + 32 * s;
+        if (i == l) {
+          v[0][s] = xl[0];
+          v[1][s] = xl[1];
+        } else if (op == 0 ? (i > l && i < nb) : i < l) {
+          const ff a = op == 0 ? T[l * kTwLd + i] : T[i * kTwLd + l];
+          v[0][s] -= a * xl[0];
+          if (two) v[1][s] -= a * xl[1];
+        }
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+      if (lane + 32 * s < nb) {
+        x[0][lane + 32 * s] = accv(v[0][s]);
+        if (two) x[1][lane + 32 * s] = accv(v[1][s]);
+      }
+  }
+  __syncthreads();
+}
+
+// CHECK: diagonal blocks with an ill-conditioned inverse are substituted (kIllBlock, km_kernels.h)
+template <bool CHECK>
 __global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ Lf, DTree t, int op, ff* __restrict__ X,
                                                       int64_t ldx, int k) {
   extern __shared__ __align__(16) unsigned char lc_smem_s[];
@@ -716,6 +770,7 @@ __global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ 
 #pragma unroll
     for (int u = 0; u < 16; ++u, p += 4 * m) pre[u] = 4 * u < cols ? *p : ff(0.0);
   };
+  const float ill = kIllBlock / L[0].hi;
   fetch(op == 0 ? 0 : nbk - 1, op == 0 ? 0 : nbk - 1);
   __syncthreads();
   for (int step = 0; step < nbk; ++step) {
@@ -723,6 +778,7 @@ __global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ 
     for (int v = 0; v < left; ++v) {
       const int b = op == 0 ? q + v : q - v;
       ff cur[16];  // columns g + 4 u of row `fast` of the tile
+      bool above = false;
 #pragma unroll
       for (int u = 0; u < 16; ++u) cur[u] = pre[u];
       if (v == 0) {  // a triangle, its diagonal the reciprocal (fast <= column or row g + 4 u)
@@ -732,17 +788,28 @@ __global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ 
           if (fast == g + 4 * u && kLcNB * q + fast < m) d = cur[u];
         d = ff(1.0) / d;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) cur[u] = fast < g + 4 * u ? cur[u] : fast == g + 4 * u ? d : ff(0.0);
+        for (int u = 0; u < 16; ++u) {
+          cur[u] = fast < g + 4 * u ? cur[u] : fast == g + 4 * u ? d : ff(0.0);
+          if (CHECK) above |= !(fabsf(cur[u].hi) <= ill) && kLcNB * q + fast < m;  // (one in rows beyond the leaf)
+        }
       }
+      bool by_rows = false;
       if ((v == 0) == (op == 0)) {
 #pragma unroll
         for (int u = 0; u < 16; ++u) T[fast * kTwLd + g + 4 * u] = cur[u];
-        __syncthreads();
+        if (CHECK) by_rows = __syncthreads_or(above);
+        else __syncthreads();
 #pragma unroll
         for (int u = 0; u < 16; ++u) cur[u] = T[(g + 4 * u) * kTwLd + fast];
+      } else if (CHECK && v == 0) {
+        by_rows = __syncthreads_or(above);
       }
       if (v + 1 < left) fetch(q, op == 0 ? b + 1 : b - 1);
       else if (left > 1) fetch(op == 0 ? q + 1 : q - 1, op == 0 ? q + 1 : q - 1);
+      if (CHECK && by_rows) {
+        block_subst_ff(L, T, xs, m, mp, q, nc, op);
+        continue;
+      }
       for (int c = 0; c < nc; ++c) {
         const ff* x = xs + c * mp + kLcNB * q + g;
         acc_t<ff> a{};
@@ -771,7 +838,8 @@ __global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ 
 // two rows of x five loads from shared memory feed six multiply-adds, so that the FP32 pipe bounds the
 // kernel (12 instructions a multiply-add).  512 leaves of 488, 72 columns: the substitution of
 // k_leaf_tri took 4.4 ms, this 2.8 ms; the FP32 floor is 1.5 ms.  The chunks of a leaf are neighbours in
-// the grid and find its tiles in L2.  grid nleaf ceil(k / 12), block 256.
+// the grid and find its tiles in L2.  A diagonal block with an ill-conditioned inverse is substituted
+// (kIllBlock, km_kernels.h).  grid nleaf ceil(k / 12), block 256.
 constexpr int kTwCols = 12;
 
 __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__ Lf, DTree t, int op, ff* __restrict__ X,
@@ -804,8 +872,11 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
 #pragma unroll
     for (int u = 0; u < 16; ++u, p += 4 * m) pre[u] = 4 * u < cols ? *p : ff(0.0);
   };
+  // true if a thread's part of the inverse has an entry above kIllBlock / L[0][0]
+  const float ill = kIllBlock / L[0].hi;
   auto put = [&](int q, int b) {
     const bool across = (b == q) == (op == 0);
+    bool above = false;
     if (b == q) {
       ff d(1.f, 0.f);
 #pragma unroll
@@ -815,7 +886,9 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const int sl = slow + 4 * u;  // kept: l <= i (op 0) or l >= i (op 1), fast <= sl for both
-        T[across ? fast * kTwLd + sl : sl * kTwLd + fast] = fast < sl ? pre[u] : fast == sl ? d : ff(0.0);
+        const ff v = fast < sl ? pre[u] : fast == sl ? d : ff(0.0);
+        above |= !(fabsf(v.hi) <= ill) && kLcNB * q + fast < m;  // (one in rows beyond the leaf)
+        T[across ? fast * kTwLd + sl : sl * kTwLd + fast] = v;
       }
     } else {
       ff* to = across ? T + fast * kTwLd + slow : T + slow * kTwLd + fast;
@@ -823,6 +896,7 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
 #pragma unroll
       for (int u = 0; u < 16; ++u) to[u * step] = pre[u];
     }
+    return above;
   };
   const int i = 32 * (w & 1) + lane;
   ff* xc = xs + 3 * (w >> 1) * mp;
@@ -832,10 +906,13 @@ __global__ void __launch_bounds__(256, 2) k_leaf_tri_wide(const ff* __restrict__
     for (int v = 0; v < left; ++v) {
       const int b = op == 0 ? q + v : q - v;
       __syncthreads();
-      put(q, b);
-      __syncthreads();
+      const bool by_rows = __syncthreads_or(put(q, b));
       if (v + 1 < left) fetch(q, op == 0 ? b + 1 : b - 1);
       else if (left > 1) fetch(op == 0 ? q + 1 : q - 1, op == 0 ? q + 1 : q - 1);
+      if (by_rows) {  // (a diagonal block)
+        block_subst_ff(L, T, xs, m, mp, q, nc, op);
+        continue;
+      }
       acc_t<ff> a[3] = {};
       // the inverse is a triangle: 32 of its rows need half of the tile
       const int l0 = v == 0 && op == 1 ? 32 * (w & 1) : 0;
@@ -879,9 +956,15 @@ bool launch_leaf_tri_blk(const ff* Lf, const Tree& t, int op, ff* X, int64_t ldx
   // hold all chunks of 4 at once (one leaf of 1024, 33 columns: the call 634 us against 424)
   if (2 * ((k + kTwCols - 1) / kTwCols) >= few || t.nleaf * few <= 152) {
     const size_t sm = ((size_t)kTfCols * mp + (size_t)4 * kTfCols * kLcNB + (size_t)kLcNB * kTwLd) * sizeof(ff);
-    smem_limit((const void*)k_leaf_tri_few, sm);
-    k_leaf_tri_few<<<dim3((unsigned)t.nleaf, (unsigned)((k + kTfCols - 1) / kTfCols)), 256, sm, st>>>(Lf, dtree(t), op, X,
-                                                                                                    ldx, k);
+    const dim3 grid((unsigned)t.nleaf, (unsigned)few);
+    // (from 32 columns on the substitution has been the rule: none of its accuracy is given up)
+    if (k < 32) {
+      smem_limit((const void*)k_leaf_tri_few<false>, sm);
+      k_leaf_tri_few<false><<<grid, 256, sm, st>>>(Lf, dtree(t), op, X, ldx, k);
+    } else {
+      smem_limit((const void*)k_leaf_tri_few<true>, sm);
+      k_leaf_tri_few<true><<<grid, 256, sm, st>>>(Lf, dtree(t), op, X, ldx, k);
+    }
     return true;
   }
   const size_t sm = ((size_t)kTwCols * mp + (size_t)kLcNB * kTwLd) * sizeof(ff);
