@@ -1,6 +1,6 @@
 // ACA assembly and the general (per-block basis) HODLR factorisation used for ACA blocks.
 //
-// ACA: one cluster of CTAs per off-diagonal block runs the partially pivoted adaptive cross approximation of
+// ACA: one cluster of CTAs per off-diagonal block (16, for many small blocks 4 or 2) runs the partially pivoted adaptive cross approximation of
 // the reference (src/factorizations.jl:9-84) step for step: the start-row search, the pivot
 // rule of restrictedmaxabs (src/utils.jl:2-15: first strict maximum of |x| outside the used set,
 // the first unused index when nothing is non-zero), residual updates as a multiply followed by a
@@ -1179,14 +1179,14 @@ bool launch_aca_grid(const double* pts, KParams kp, const AcaBlock* blocks, int 
 }
 
 static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int last_first, int only,
-                       int maxcap, double* P, uint8_t* F, int* piv, double rtol, int* rank, int* status,
+                       int most, int maxcap, double* P, uint8_t* F, int* piv, double rtol, int* rank, int* status,
                        cudaStream_t st) {
   // the fixed arrays, then this CTA's share of an SM for slices when the CTAs fit at most three to
   // an SM (more, and the shared memory is worth more as L1 cache)
   size_t sm = ((size_t)3 * std::max(maxcap, 1) + 2 + 2 * kAcaChunk * kAcaSplit) * sizeof(double);
   smem_limit((const void*)k_aca, kAcaSmem);
   // CTAs per cluster: 16 where clusters of that size can be scheduled, else 8
-  const int cs = cluster_limit((const void*)k_aca, kAcaThreads, kAcaSmem) >= 16 ? 16 : 8;
+  const int cs = std::min(most, cluster_limit((const void*)k_aca, kAcaThreads, kAcaSmem) >= 16 ? 16 : 8);
   const int per = ((only >= 0 ? 1 : nblocks) * cs + 151) / 152;
   if (per <= 3) sm = std::max(sm, kAcaSmem / per);
   cudaLaunchConfig_t cfg = {};
@@ -1205,15 +1205,15 @@ static void aca_launch(const double* pts, KParams kp, const AcaBlock* blocks, in
 
 void launch_aca_one(const double* pts, KParams kp, const AcaBlock* blocks, int b, int maxcap, double* P,
                     uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st) {
-  aca_launch(pts, kp, blocks, 1, 0, b, maxcap, P, F, piv, rtol, rank, status, st);
+  aca_launch(pts, kp, blocks, 1, 0, b, 16, maxcap, P, F, piv, rtol, rank, status, st);
 }
 
 // ---------------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------------
 void launch_aca(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int maxcap, double* P,
-                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first) {
-  aca_launch(pts, kp, blocks, nblocks, last_first, -1, maxcap, P, F, piv, rtol, rank, status, st);
+                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first, int cluster) {
+  aca_launch(pts, kp, blocks, nblocks, last_first, -1, cluster, maxcap, P, F, piv, rtol, rank, status, st);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -486,6 +486,8 @@ NodeMatsH node_mats(km_handle* h) {
 
 // ---- general (ACA) path -------------------------------------------------------------------
 
+// Sides of the ACA blocks that clusters of 2 and of 4 CTAs take where there are 64 of them and more
+constexpr int64_t kAcaSide2 = 40, kAcaSide4 = 130;
 // Nodes at least this large (rows of both children) update the coarser panels of the factorisation
 // by FP64 products over all SMs (launch_dgemm): those updates have hundreds of columns.
 constexpr int64_t kGapplyBig = 16384;
@@ -1367,16 +1369,38 @@ static int aca_assemble(km_handle* h, const double* pts, bool dev, const Tree& t
   KLV(h, KM_PROF_EVAL, launch_eval_leaves(h->d_pts, t, h->kp, -1, h->d_K, st));
   // (now: setting a kernel attribute, as the first ACA launch of a process does, drops a pending error)
   if ((rc = check_launch(h, "leaf evaluation")) != KM_OK) return rc;
-  if (nb > 0)
-    KLV(h, KM_PROF_ACA, launch_aca(h->d_pts, h->kp, h->d_blk, nb, maxcap, h->d_panels, h->d_flags, h->d_piv, tol,
-                                   h->d_brank, h->d_bstatus, st, 1));
+  // The blocks of the finest levels, where they are many, by clusters of 2 or 4 beside the others: 16 CTAs leave
+  // them slices of a few rows, and a warp's FP64 instruction costs the same whatever its active lanes
+  // (65536 points, leaves of 16, rank 20: 60.7 ms with 16 throughout, 37.8 with a CTA a block, now 15.5;
+  // 16384 points, leaves of 128, 32.0 -> 26.6 ms).
+  auto small_to = [&](int64_t side, int from) {  // blocks from `from` on with both sides up to `side`
+    int q = from;
+    while (q < nb && std::max(h->blk[q].nro, h->blk[q].ncl) <= side) ++q;
+    return q - from >= 64 ? q : from;
+  };
+  const int n2 = small_to(kAcaSide2, 0), n4 = small_to(kAcaSide4, n2);
+  auto aca_part = [&](int a, int b, int cluster, cudaStream_t s) {
+    int cap = 0;
+    for (int q = a; q < b; ++q) cap = std::max(cap, h->blk[q].cap);
+    launch_aca(h->d_pts, h->kp, h->d_blk + a, b - a, cap, h->d_panels, h->d_flags, h->d_piv, tol, h->d_brank + a,
+               h->d_bstatus + a, s, 1, cluster);
+  };
+  if (n4 > 0) {
+    side_begin(h);
+    if (n4 > n2) aca_part(n2, n4, 4, h->side);
+    if (n2 > 0) aca_part(0, n2, 2, h->side);
+  }
+  if (nb > n4) KLV(h, KM_PROF_ACA, aca_part(n4, nb, 16, st));
   // large blocks: one cooperative launch each, all SMs on one block
   {
     int gmax = 0;
     for (const auto& b : h->blk)
       if (b.grid) gmax = std::max(gmax, b.cap);
     if (gmax > 0) {
-      if ((rc = grow(h, &h->d_acascr, aca_grid_scratch(gmax)))) return rc;
+      if ((rc = grow(h, &h->d_acascr, aca_grid_scratch(gmax)))) {
+        if (n4 > 0) side_end(h);
+        return rc;
+      }
       for (int q = 0; q < nb; ++q) {
         if (!h->blk[q].grid) continue;
         bool ok = false;
@@ -1389,6 +1413,7 @@ static int aca_assemble(km_handle* h, const double* pts, bool dev, const Tree& t
       }
     }
   }
+  if (n4 > 0) side_end(h);
   if ((rc = check_launch(h, "aca")) != KM_OK) return rc;
   h->stats.assemble_ms = timer_stop(h);
   if ((rc = sync(h, "aca")) != KM_OK) return rc;

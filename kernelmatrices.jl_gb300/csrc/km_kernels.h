@@ -242,9 +242,11 @@ void launch_col_dots(const double* A, int64_t lda, const double* B, int64_t ldb,
 // ACA and the general factorisation
 constexpr int kAcaMaxCap = 4096;       // ACA panel columns per block (3 x 4096 doubles of shared memory)
 constexpr int64_t kAcaGridMin = 8192;  // blocks at least this wide run the grid-wide ACA kernel
-// last_first: start with the last blocks (they are the large ones of a HODLR level order)
+// last_first: start with the last blocks (they are the large ones of a HODLR level order); cluster: CTAs per
+// block at most
 void launch_aca(const double* pts, KParams kp, const AcaBlock* blocks, int nblocks, int maxcap, double* P,
-                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first = 0);
+                uint8_t* F, int* piv, double rtol, int* rank, int* status, cudaStream_t st, int last_first = 0,
+                int cluster = 16);
 // ACA of one large block (blocks[b].grid == 1) by all SMs in one cooperative launch, with
 // bounded grid barriers; scratch of aca_grid_scratch(cap) doubles.  Returns false when the
 // cooperative launch is unavailable (the caller then runs the block in one cluster).
