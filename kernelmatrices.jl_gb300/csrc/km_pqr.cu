@@ -331,9 +331,12 @@ static int pqr_rows(int64_t others, int64_t mmax, int most) {
   return (int)std::min<int64_t>(std::max<int64_t>(rows, 64), most);
 }
 
-// T factors (two kPB x kPB values per block) and the partial products of one block
+// T factors (two kPB x kPB values per block) and the partial products of one block (most chunks: one
+// column tile left)
 int64_t panel_qr_scratch(int n, int kmax, int64_t mmax) {
-  const int64_t nblk = (kmax + kPB - 1) / kPB, nchunk = (mmax + 63) / 64;
+  if (n <= 0 || kmax <= 0) return 0;
+  const int64_t rows = pqr_rows(n, mmax, kVtcRows);
+  const int64_t nblk = (kmax + kPB - 1) / kPB, nchunk = (mmax + rows - 1) / rows;
   return n * nblk * 2 * kPB * kPB + n * nchunk * std::max(kmax, 1) * kPB;
 }
 

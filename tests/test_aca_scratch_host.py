@@ -1,7 +1,9 @@
-"""Scratch of the node applications of an ACA factor (km_aca.cu): host arithmetic, no GPU.
+"""Scratch of the node applications (km_aca.cu) and of the panel QR (km_pqr.cu) of an ACA factor: host arithmetic,
+no GPU.
 
 The calls run in a process of their own: an integer division by zero ends it on x86-64.
 """
+import ctypes
 import subprocess
 import sys
 
@@ -38,3 +40,13 @@ def test_scratch_does_not_grow_with_the_rows(lib, n, r, cols, rows):
     most = 2 * r * 8 * (2 * ctas + 6 * 152 // 2)
     got = gapply_scratch(lib, n, r, cols, rows)
     assert 0 <= got <= min(most, 2 * r * 65 * 8 * ctas)
+
+
+@pytest.mark.parametrize("n,k,rows", [(32, 400, 8192), (1024, 100, 256), (2, 350, 8192), (8, 4000, 12288), (2, 1, 1)])
+def test_panel_scratch_is_what_its_chunks_take(lib, n, k, rows):
+    """Partial products: 32 values a column and row chunk of a panel, with at most 4 CTAs an SM (152 SMs) more than
+    panels, or chunks of 512 rows; two 32 x 32 factors a block."""
+    lib._ZN2km16panel_qr_scratchEiil.restype = ctypes.c_int64
+    got = lib._ZN2km16panel_qr_scratchEiil(ctypes.c_int(n), ctypes.c_int(k), ctypes.c_int64(rows))
+    chunks = max(4 * 152 + n, n * -(-rows // 512))
+    assert 0 < got <= n * -(-k // 32) * 2 * 32 * 32 + chunks * k * 32
