@@ -1080,8 +1080,8 @@ static int sm_count() {
 
 // CTAs per node of the node kernels (form 0: FP64, 1: float pairs): the largest of 8, 4, 2 with
 // nodes x csize <= the SM count and as many such clusters schedulable at once (asked once per form,
-// size and device: clusters do not straddle the groups that SMs come in, so 16 of 8 may not fit
-// 152 SMs), else 1.  max_cs (the handle's setting) and KM_NODE_CLUSTER=1, 2, 4 or 8 cap it
+// device, size and number of CTAs that an SM's shared memory holds: clusters do not straddle the groups
+// that SMs come in, so 16 of 8 may not fit 152 SMs), else 1.  max_cs (the handle's setting) and KM_NODE_CLUSTER=1, 2, 4 or 8 cap it
 // (1 gives the one-CTA form).
 static int node_cluster_size(int form, const void* fn, int64_t nodes, int threads, size_t smem, int max_cs) {
   static const int cap = [] {
@@ -1090,17 +1090,18 @@ static int node_cluster_size(int form, const void* fn, int64_t nodes, int thread
     return v >= 8 ? 8 : v >= 4 ? 4 : v >= 2 ? 2 : 1;
   }();
   constexpr int kDevMax = 64;
-  // per form, device, size 1, 2, 4, 8 and whether a CTA takes more than half an SM's shared memory:
-  // clusters at once, 0 unknown, -1 none (handles on several host threads may ask at once; a
-  // repeated query gives the same answer)
-  static std::atomic<int> room[2][kDevMax][4][2];
+  // per form, device, size 1, 2, 4, 8 and CTAs an SM by shared memory (1, 2, 3, 4 and more): clusters at
+  // once, 0 unknown, -1 none (handles on several host threads may ask at once; a repeated query gives the
+  // same answer)
+  static std::atomic<int> room[2][kDevMax][4][4];
+  const int per_sm = (int)std::min<size_t>(std::max<size_t>(228 * 1024 / (smem + 1024), 1), 4);
   const int nsm = sm_count();
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevMax) return 1;
   const int top = std::min(cap, max_cs);
   for (int cs = top, lg = top >= 8 ? 3 : top == 4 ? 2 : top == 2 ? 1 : 0; cs > 1; cs >>= 1, --lg) {
     if (nodes * cs > nsm) continue;
-    std::atomic<int>& n = room[form][dev][lg][smem > 113 * 1024];
+    std::atomic<int>& n = room[form][dev][lg][per_sm - 1];
     if (n.load() == 0) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)cs);
