@@ -1012,12 +1012,12 @@ __global__ void __launch_bounds__(kGaThreads) k_gexpand(const GApplyItem* __rest
   }
 }
 
-// The r x r part alone for a node whose projections and expansions run as products over all SMs
-// (columns of Z1, Z2, G1, G2: r consecutive values), CB columns per CTA.
+// The r x r part of mode 0 alone for a node whose projections and expansion run as products over all SMs
+// (columns of Z1, Z2, G2: r consecutive values), CB columns per CTA.
 template <int CB>
-__global__ void __launch_bounds__(kGaThreads) k_gsmall(const GNodeDesc* __restrict__ node, int mode,
+__global__ void __launch_bounds__(kGaThreads) k_gsmall(const GNodeDesc* __restrict__ node,
                                                        const double* __restrict__ Z1, const double* __restrict__ Z2,
-                                                       double* __restrict__ G1, double* __restrict__ G2, int ncols) {
+                                                       double* __restrict__ G2, int ncols) {
   extern __shared__ double sm[];
   const GNodeDesc N = *node;
   const int r = N.r, col = blockIdx.x * CB, nc = min(CB, ncols - col);
@@ -1027,15 +1027,12 @@ __global__ void __launch_bounds__(kGaThreads) k_gsmall(const GNodeDesc* __restri
   double* xs = T + CB * r;
   const int64_t off = (int64_t)col * r;
   for (int e = threadIdx.x; e < CB * r; e += kGaThreads) {
-    z1[e] = (e < nc * r && (mode == 0 || mode == 2)) ? Z1[off + e] : 0.0;
+    z1[e] = e < nc * r ? Z1[off + e] : 0.0;
     z2[e] = e < nc * r ? Z2[off + e] : 0.0;
   }
   __syncthreads();
-  ga_middle<CB>(N, mode, z1, z2, T, xs);
-  for (int e = threadIdx.x; e < nc * r; e += kGaThreads) {
-    if (mode == 1 || mode == 3) G1[off + e] = z1[e];
-    G2[off + e] = z2[e];
-  }
+  ga_middle<CB>(N, 0, z1, z2, T, xs);
+  for (int e = threadIdx.x; e < nc * r; e += kGaThreads) G2[off + e] = z2[e];
 }
 
 // shared memory of CB columns at rank r; the widest CB <= want whose vectors fit
@@ -1089,11 +1086,11 @@ void gapply_launch(const GApplyItem* items, int n, const GNodeDesc* nodes, int m
 }
 
 template <int CB>
-void gsmall_launch(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2, int r,
-                   int ncols, cudaStream_t st) {
+void gsmall_launch(const GNodeDesc* node, const double* Z1, const double* Z2, double* G2, int r, int ncols,
+                   cudaStream_t st) {
   const size_t sm = ga_smem(CB, r);
   smem_limit((const void*)k_gsmall<CB>, sm);
-  k_gsmall<CB><<<(unsigned)((ncols + CB - 1) / CB), kGaThreads, sm, st>>>(node, mode, Z1, Z2, G1, G2, ncols);
+  k_gsmall<CB><<<(unsigned)((ncols + CB - 1) / CB), kGaThreads, sm, st>>>(node, Z1, Z2, G2, ncols);
 }
 
 }  // namespace
@@ -1547,12 +1544,12 @@ int launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int ma
   return g.nchunk > 0 && scratch ? 3 : 1;
 }
 
-void launch_gsmall(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2,
-                   int r, int ncols, cudaStream_t st) {
+void launch_gsmall(const GNodeDesc* node, const double* Z1, const double* Z2, double* G2, int r, int ncols,
+                   cudaStream_t st) {
   if (ncols <= 0 || r <= 0) return;
   const int cb = ga_width(ncols, r);
   (cb == 8 ? gsmall_launch<8> : cb == 4 ? gsmall_launch<4> : cb == 2 ? gsmall_launch<2> : gsmall_launch<1>)(
-      node, mode, Z1, Z2, G1, G2, r, ncols, st);
+      node, Z1, Z2, G2, r, ncols, st);
 }
 
 void launch_glogdet(const GNodeDesc* nodes, int nn, double* partial, cudaStream_t st) {

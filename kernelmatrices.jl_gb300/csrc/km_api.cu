@@ -138,7 +138,7 @@ struct km_handle {
   GApplyItem* d_gfact = nullptr;      // factorisation updates, grouped by level
   std::vector<GNodeDesc> gnodes_h;    // host copies: the library-GEMM path of large nodes reads them
   std::vector<GApplyItem> gsolve_h, gfact_h;
-  double* d_gz = nullptr;             // projections and coefficients of one large node (4 x r x ncols),
+  double* d_gz = nullptr;             // projections and coefficients of one large node (3 x r x ncols),
                                       // then the partial products of its split projections
   double* d_pqg = nullptr;            // explicit reflector block and products of the tall-panel QR
   std::vector<int64_t> gfoff;
@@ -511,7 +511,7 @@ static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyIte
       const GNodeDesc& N = h->gnodes_h[hl[q].node];
       const int nc = hl[q].base ? hl[q].ncols : kX;
       if (hl[q].big) {
-        nd = std::max<int64_t>(nd, 4 * (int64_t)N.r * nc);
+        nd = std::max<int64_t>(nd, 3 * (int64_t)N.r * nc);
         sp = std::max(sp, std::max(dgemm_scratch(1, N.r, nc, N.s1), dgemm_scratch(1, N.r, nc, N.s2)));
       } else {
         r1 = std::max(r1, N.r);
@@ -546,13 +546,12 @@ static int run_gapply(km_handle* h, const std::vector<GApplyItem>& hl, GApplyIte
     if (r <= 0 || nc <= 0) continue;
     double* Z1 = h->d_gz;
     double* Z2 = Z1 + (int64_t)r * nc;
-    double* G1 = Z2 + (int64_t)r * nc;
-    double* G2 = G1 + (int64_t)r * nc;
+    double* G2 = Z2 + (int64_t)r * nc;
     double* spl = G2 + (int64_t)r * nc;  // partial products of the split Q' x reductions
     KLV(h, KM_PROF_SWEEP, {
       launch_dgemm(1, r, nc, N.s1, 1.0, N.Q1, N.s1, I.base + I.off1, I.ld, 0.0, Z1, r, spl, split, st);
       launch_dgemm(1, r, nc, N.s2, 1.0, N.Q2, N.s2, I.base + I.off2, I.ld, 0.0, Z2, r, spl, split, st);
-      launch_gsmall(h->d_gnodes + I.node, mode, Z1, Z2, G1, G2, r, nc, st);
+      launch_gsmall(h->d_gnodes + I.node, Z1, Z2, G2, r, nc, st);
       launch_dgemm(0, N.s2, nc, r, -1.0, N.Q2, N.s2, G2, r, 1.0, I.base + I.off2, I.ld, nullptr, 0, st);
     });
   }

@@ -294,10 +294,10 @@ int launch_gapply(const GApplyItem* items, int n, const GNodeDesc* nodes, int ma
                   double* X, const double* Xin, int64_t ldX, int kX, double* scratch, cudaStream_t st);
 int64_t gapply_scratch(int n, int maxr, int maxcols, int64_t maxs);
 void launch_glogdet(const GNodeDesc* nodes, int nn, double* partial, cudaStream_t st);
-// the r x r part of k_gapply for one node and ncols columns: from the projections Z1 = Q1' x1,
-// Z2 = Q2' x2 (r x ncols each; mode 4 is not handled here) to the expansion coefficients G1, G2
-void launch_gsmall(const GNodeDesc* node, int mode, const double* Z1, const double* Z2, double* G1, double* G2,
-                   int r, int ncols, cudaStream_t st);
+// the r x r part of k_gapply's mode 0 for one node and ncols columns: from the projections Z1 = Q1' x1,
+// Z2 = Q2' x2 (r x ncols each) to the expansion coefficients G2
+void launch_gsmall(const GNodeDesc* node, const double* Z1, const double* Z2, double* G2, int r, int ncols,
+                   cudaStream_t st);
 bool launch_leaf_tri_desc(const double* Lf, const Tree& t, int op, const LeafDesc* descs, int n, int maxcols,
                           cudaStream_t st);
 
