@@ -347,7 +347,8 @@ __global__ void __launch_bounds__(512) k_leaf_nys_apply(const double* __restrict
   }
   // beta = S^{-1} a = Sc^{-T} Sc^{-1} a, one warp per column, with the reciprocals of Sc's diagonal (a
   // division in each of the 2 r steps of the chain took most of its time: 256 leaves of 256, rank 72, one
-  // column, the whole kernel 174 us with them, 149 without); they lie where the parts are added later
+  // column, the whole kernel 174 us with them, 149 without, 112 with the loads of one column batched besides); they
+  // lie where the parts are added later
   double* red = bs + 8 * r;  // kNaParts x kNaRows x 8
   double* rdiag = red;
   for (int l = threadIdx.x; l < r; l += blockDim.x) rdiag[l] = 1.0 / Sc[(int64_t)l * r + l];

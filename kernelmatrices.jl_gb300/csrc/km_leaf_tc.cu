@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(256, 3) k_leaf_tri_few(const ff* __restrict__ 
 // while the present one is multiplied.  Thread (row 32 (w & 1) + lane, columns 3 (w >> 1) .. + 2): per
 // two rows of x five loads from shared memory feed six multiply-adds, so that the FP32 pipe bounds the
 // kernel (12 instructions a multiply-add).  512 leaves of 488, 72 columns: the substitution of
-// k_leaf_tri took 4.4 ms, this 2.8 ms; the FP32 floor is 1.5 ms.  The chunks of a leaf are neighbours in
+// k_leaf_tri took 4.4 ms, this 2.6 ms; the FP32 floor is 1.5 ms.  The chunks of a leaf are neighbours in
 // the grid and find its tiles in L2.  A diagonal block with an ill-conditioned inverse is substituted
 // (kIllBlock, km_kernels.h).  grid nleaf ceil(k / 12), block 256.
 constexpr int kTwCols = 12;
